@@ -123,6 +123,16 @@ struct Groups {
   int m_rows, b_rows, k_rows, bm_rows;
 };
 
+// Consecutive row groups of any length (routed tokens sorted by expert; the lengths are known on the host): group g
+// holds rows [row0[g], row0[g + 1]) of A / C and is cut into tiles of its own, m-tiles [mt0[g], mt0[g + 1]) of the
+// launch. Its B is shifted by g * Groups::b_rows as above. A tile's loads may run into the rows of the next group,
+// its stores stop at the group's end. n == 0: off.
+constexpr int RAGGED_MAX = 64;
+struct Ragged {
+  int n;
+  int row0[RAGGED_MAX + 1], mt0[RAGGED_MAX + 1];
+};
+
 ATB_DEVICE uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -193,7 +203,8 @@ ATB_DEVICE void mbar_arrive_remote(uint32_t bar_cluster_addr) {
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epi ep, int M,
-                      int N, int K, Groups grp, Gate gate, Sched sched, int* status) {
+                      int N, int K, Groups grp, Gate gate, Sched sched, const __grid_constant__ Ragged rag,
+                      int* status) {
   constexpr int BNH = Cfg<BN>::BNH, STAGES = Cfg<BN>::STAGES, B_BYTES = Cfg<BN>::B_BYTES,
                 BAR_OFF = Cfg<BN>::BAR_OFF;
   extern __shared__ uint8_t smem_raw[];
@@ -217,7 +228,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   // both CTAs of a pair read the same word, so they take the same decision
   const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
 
-  const int tiles_m = (M + 2 * BM - 1) / (2 * BM);
+  const int tiles_m = rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM);
   const int tile_cols = ep.gated ? BN / 2 : BN;      // output columns per tile
   const int tiles_n = (N + tile_cols - 1) / tile_cols;
   const int num_tiles = skip ? 0 : tiles_m * tiles_n;
@@ -275,7 +286,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     return k0 - g * grp.k_rows < grp.counts[g];
   };
 
-  auto tile_coords = [&](int tile, int& m0, int& n0) {
+  // first row / column of a tile, the end of its rows and the index of its B operand
+  auto tile_coords = [&](int tile, int& m0, int& n0, int& m_end, int& b_idx) {
     const int band_tiles = BAND * tiles_n;
     const int band = tile / band_tiles;
     const int rem = tile - band * band_tiles;
@@ -291,8 +303,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (tm >= tiles_m) tm -= tiles_m;
       }
     }
-    m0 = tm * 2 * BM;
     n0 = tn * tile_cols;
+    if (rag.n > 0) {
+      int g = 0;
+      while (tm >= rag.mt0[g + 1]) ++g;
+      m0 = rag.row0[g] + (tm - rag.mt0[g]) * 2 * BM;
+      m_end = rag.row0[g + 1];
+      b_idx = g;
+    } else {
+      m0 = tm * 2 * BM;
+      m_end = M;
+      b_idx = grp.b_rows > 0 ? m0 / grp.bm_rows : 0;
+    }
   };
 
   // The idx-th tile of this pair, the same number in every role of both CTAs. Static: a fixed stride. Dynamic: the
@@ -344,11 +366,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           free_tile_slot(idx);
         }
         if (tile < 0) break;
-        int m0, n0;
-        tile_coords(tile, m0, n0);
+        int m0, n0, m_end, b_idx;
+        tile_coords(tile, m0, n0, m_end, b_idx);
         if (!tile_active(m0)) continue;
         const int am0 = m0 + (int)rank * BM;   // this CTA's rows of A
-        const int bshift = grp.b_rows > 0 ? (m0 / grp.bm_rows) * grp.b_rows : 0;   // this expert's own B
+        const int bshift = b_idx * grp.b_rows;   // this expert's own B
         // this CTA's rows of B (gated: CTA 0 takes gate rows, CTA 1 the up rows of the same features)
         const int bn0 = ep.gated ? n0 + (int)rank * N : n0 + (int)rank * BNH + (B_MN ? 0 : bshift);
         const int bk0 = B_MN ? bshift : 0;
@@ -394,8 +416,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         free_tile_slot(idx);
         if (tile < 0) break;
         {
-          int m0, n0;
-          tile_coords(tile, m0, n0);
+          int m0, n0, m_end, b_idx;
+          tile_coords(tile, m0, n0, m_end, b_idx);
           if (!tile_active(m0)) continue;
         }
         const int acc = local & 1;
@@ -440,8 +462,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       __syncwarp();
       if (lane == 0) free_tile_slot(idx);
       if (tile < 0) break;
-      int m0, n0;
-      tile_coords(tile, m0, n0);
+      int m0, n0, m_end, b_idx;
+      tile_coords(tile, m0, n0, m_end, b_idx);
       if (!tile_active(m0)) {
         // an empty tile: its output is all zeros (left alone when accumulating)
         const int zrow = m0 + (int)rank * BM + q * 32 + lane;
@@ -474,7 +496,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           tmem_ld_32x32(t_addr + BN / 2 + c * 32, u);
           tmem_ld_wait();
           const int col0 = n0 + c * 32;
-          if (row < M && col0 < N) {
+          if (row < m_end && col0 < N) {
             __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
             __nv_bfloat16* grow = ep.gu_out == nullptr ? nullptr
                 : reinterpret_cast<__nv_bfloat16*>(ep.gu_out) + (long long)row * ep.ldgu + col0;
@@ -511,7 +533,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tmem_ld_32x32(t_addr + c * 32, r);
         tmem_ld_wait();
         const int col0 = n0 + c * 32;
-        if (row < M && col0 < N) {
+        if (row < m_end && col0 < N) {
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ep.alpha;
@@ -649,7 +671,8 @@ int* sched_counters(cudaStream_t stream) {
 
 template <int BN, bool A_MN, bool B_MN>
 int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, long long lda, long long ldb,
-           int max_ctas, const Groups& grp, int b_extent_rows, const Gate& gate, cudaStream_t stream, int* status) {
+           int max_ctas, const Groups& grp, int b_extent_rows, const Gate& gate, const Ragged& rag, cudaStream_t stream,
+           int* status) {
   CUtensorMap tmA, tmB;
   bool ok;
   if (!A_MN)
@@ -673,7 +696,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     attr_set = true;
   }
   const int tile_cols = ep.gated ? BN / 2 : BN;
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
+  const int tiles = (rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
   int clusters = sm_count() / 2;
   if (tiles < clusters) clusters = tiles;
   if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
@@ -683,7 +706,8 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     const char* e = getenv("ATB_GEMM_DYNAMIC");
     g_dynamic = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
-  if (g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && grp.b_rows == 0 && gate.flags == nullptr)
+  if (g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
+      gate.flags == nullptr)
     sched.counters = sched_counters(stream);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters, 1, 1);
@@ -697,9 +721,11 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, ep, M, N, K, grp, gate, sched, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, ep, M, N, K, grp, gate, sched, rag, status);
   return e == cudaSuccess ? 0 : -5;
 }
+
+const Ragged kNoGroups = {};
 
 // extra arguments of the next launch of this host thread (set and cleared by atb_gemm_bf16_2cta_fused)
 struct FusedArgs {
@@ -758,12 +784,12 @@ extern "C" int atb_gemm_bf16_2cta_grouped(const void* A, const void* B, void* C,
 #define ATB_PAIR_DISPATCH(BN_)                                                                                     \
   do {                                                                                                             \
     if (!a_mn_major && !b_mn_major)                                                                                \
-      return launch<BN_, false, false>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, st, status);          \
+      return launch<BN_, false, false>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, kNoGroups, st, status);  \
     if (!a_mn_major && b_mn_major)                                                                                 \
-      return launch<BN_, false, true>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, st, status);           \
+      return launch<BN_, false, true>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, kNoGroups, st, status);  \
     if (a_mn_major && b_mn_major)                                                                                  \
-      return launch<BN_, true, true>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, st, status);            \
-    return launch<BN_, true, false>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, st, status);             \
+      return launch<BN_, true, true>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, kNoGroups, st, status);  \
+    return launch<BN_, true, false>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent, gate, kNoGroups, st, status);  \
   } while (0)
   if (narrow) ATB_PAIR_DISPATCH(128);
   ATB_PAIR_DISPATCH(256);
@@ -777,6 +803,37 @@ extern "C" int atb_gemm_bf16_2cta(const void* A, const void* B, void* C, const v
   return atb_gemm_bf16_2cta_grouped(A, B, C, bias, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, out_fp32,
                                     accumulate, alpha, tile_n, max_ctas, residual, ldr, nullptr, 0, 0, 0, 0, 0, stream,
                                     status);
+}
+
+// C[rows of group g] = A[rows of group g] * B_g^T for `n_groups` (at most 64) consecutive row groups of `sizes` rows
+// (host memory, the sum is M) and as many stacked operands: B is [n_groups * N, K] (K-major) or [n_groups * K, N]
+// (MN-major, K a multiple of 64 so that no k-block reaches into the next operand). A is K-major, C is bf16.
+// One launch in place of one per group: the tiles of all groups share the waves. Experts of a routed layer get unequal
+// numbers of rows, and a launch of its own leaves 74 CTA pairs with a short last wave once per expert. Forward and
+// backward of the expert MLP 8 x 14336 x 4096 on 8192 routed rows: 9.9 ms, against 148 ms when every group whose
+// length is no multiple of 8 took the fp32 fallback and w2 was transposed by a copy first.
+extern "C" int atb_gemm_bf16_2cta_ragged(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                                         long long ldb, long long ldc, int b_mn_major, const int* sizes, int n_groups,
+                                         void* stream, int* status) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((N & 7) || (lda & 7) || (ldb & 7) || (ldc & 7)) return -1;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -1;
+  if (n_groups < 1 || n_groups > RAGGED_MAX || (b_mn_major && (K % BK))) return -1;
+  Ragged rag = {};
+  rag.n = n_groups;
+  for (int g = 0; g < n_groups; ++g) {
+    if (sizes[g] < 0 || sizes[g] > M - rag.row0[g]) return -1;
+    rag.row0[g + 1] = rag.row0[g] + sizes[g];
+    rag.mt0[g + 1] = rag.mt0[g] + (sizes[g] + 2 * BM - 1) / (2 * BM);
+  }
+  if (rag.row0[n_groups] != M) return -1;
+  Epi ep{C, nullptr, ldc, 1.f, 0, 0, nullptr, 0, {nullptr}, 0, 0, nullptr, 0};
+  Groups grp{nullptr, 0, b_mn_major ? K : N, 0, 0};
+  Gate gate{nullptr, 0u, 1, 0};
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (b_mn_major)
+    return launch<256, false, true>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * K, gate, rag, st, status);
+  return launch<256, false, false>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * N, gate, rag, st, status);
 }
 
 // act[M, F] = silu(x Wg^T) * (x Wu^T) for the fused weight W = [Wg; Wu] ([2 F, K], K-major, pitch ldb): the GEMM with
@@ -793,7 +850,7 @@ extern "C" int atb_gemm_bf16_2cta_swiglu(const void* A, const void* B, void* act
   Epi ep{act, nullptr, ld_act, 1.f, 0, 0, nullptr, 0, {nullptr}, 0, 1, gu_out, ldgu};
   Groups grp{nullptr, 0, 0, 0, 0};
   Gate gate{nullptr, 0u, 1, 0};
-  return launch<256, false, false>(A, B, ep, M, F, K, lda, ldb, 0, grp, 2 * F, gate,
+  return launch<256, false, false>(A, B, ep, M, F, K, lda, ldb, 0, grp, 2 * F, gate, kNoGroups,
                                    reinterpret_cast<cudaStream_t>(stream), status);
 }
 

@@ -31,6 +31,26 @@ def _pitch(t: torch.Tensor) -> int:
     return t.stride(0) if t.dim() == 2 else t.shape[-1]
 
 
+def _sizes_ok(a, b, M, N, K, a_mn, b_mn, out, groups, bias, residual) -> bool:
+    """Whether the kernels take these sizes. They store 8 columns at a time and load 16-byte pieces along the dim in
+    which an operand is contiguous; the other dim of an operand may have any length (rows of A in the forward product
+    and in dgrad, the reduction dim in wgrad: the tensor maps read zeros past the end), which is where the token count
+    of a ragged batch goes. Evaluating a 1.3B model of 8 layers on 777 tokens (25 such products) takes 1.8 ms of GPU
+    time with them here, 11.3 ms with them on the fp32 fallback."""
+    if N % 8 == 0 and K % 8 == 0 and M % 8 == 0:
+        return True
+    if N % 8 or (a_mn and M % 8) or (K % 8 and not (a_mn and b_mn)) or groups is not None:
+        return False
+    if residual is not None and (out.dtype != torch.bfloat16 or residual.dtype != torch.bfloat16
+                                 or residual.stride(-1) != 1):
+        return False
+    if bias is not None and not (bias.dtype == torch.bfloat16 and bias.is_contiguous() and bias.is_cuda):
+        return False
+    # inputs that are not laid out for the kernel stay on the fallback, which they always took at these sizes
+    return all(t is None or (t.stride(-1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
+               for t in (a, b, out, residual)) and out.dtype in (torch.bfloat16, torch.float32)
+
+
 def gemm_reference(a, b, a_mn=False, b_mn=False, out=None, out_dtype=None, accumulate=False, alpha=1.0, bias=None):
     """fp32-accumulated PyTorch evaluation of the same contract (the oracle for the kernel)."""
     A = a.t() if a_mn else a
@@ -87,7 +107,8 @@ def gemm(
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype or torch.bfloat16, device=a.device)
         assert not accumulate
-    if not _lib.use_kernels(a, b, out) or a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 or (N % 8) or (K % 8) or (M % 8):
+    if not _lib.use_kernels(a, b, out) or a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16 \
+            or not _sizes_ok(a, b, M, N, K, a_mn, b_mn, out, groups, bias, residual):
         if n_b > 1:                  # reference: one product per stacked operand (inputs are zero beyond the counts)
             R = groups["bm_rows"]
             for e in range(n_b):
@@ -145,6 +166,35 @@ def gemm(
         _lib.stream_ptr(), _lib.ptr(_lib.status_word(a.device)),
     )
     _lib.check(rc, f"atb_gemm_bf16 M={M} N={N} K={K}")
+    return out
+
+
+MAX_RAGGED_GROUPS = 64
+
+
+def ragged_ok(x: torch.Tensor, w: torch.Tensor, b_mn: bool, n_groups: int) -> bool:
+    """Whether ``gemm_ragged`` takes these operands: bf16 on the GPU, laid out for 16-byte loads and stores, and a
+    reduction dim of whole 64-row blocks where the stacked operands follow each other along it."""
+    N, K = (w.shape[2], w.shape[1]) if b_mn else (w.shape[1], w.shape[2])
+    return (_lib.use_kernels(x, w) and _lib.lib().has("atb_gemm_bf16_2cta_ragged") and PAIR_KERNEL_DEFAULT
+            and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and 0 < n_groups <= MAX_RAGGED_GROUPS
+            and w.shape[0] == n_groups and x.dim() == 2 and x.shape[1] == K and N % 8 == 0
+            and K % (64 if b_mn else 8) == 0 and w.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_ragged(x: torch.Tensor, w: torch.Tensor, sizes, b_mn: bool) -> torch.Tensor:
+    """Rows of ``x`` in consecutive groups of ``sizes`` rows (host numbers), group ``g`` times ``w[g]`` (``[K, N]``)
+    when ``b_mn`` else times ``w[g]^T`` (``[N, K]``): one launch for all groups. See :func:`ragged_ok`."""
+    M, K = x.shape
+    N = w.shape[2] if b_mn else w.shape[1]
+    out = torch.empty(M, N, dtype=x.dtype, device=x.device)
+    rc = _lib.lib().atb_gemm_bf16_2cta_ragged(
+        _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
+        ctypes.c_longlong(_pitch(x)), ctypes.c_longlong(w.shape[2]), ctypes.c_longlong(N), ctypes.c_int(int(b_mn)),
+        (ctypes.c_int * len(sizes))(*sizes), ctypes.c_int(len(sizes)), _lib.stream_ptr(),
+        _lib.ptr(_lib.status_word(x.device)))
+    _lib.check(rc, f"atb_gemm_bf16_2cta_ragged M={M} N={N} K={K} groups={len(sizes)}")
     return out
 
 

@@ -16,7 +16,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
-from .gemm import gemm, linear
+from .gemm import gemm, gemm_ragged, linear, ragged_ok
 
 
 def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tensor:
@@ -49,37 +49,49 @@ def unpermute(permuted: torch.Tensor, sorted_idx: torch.Tensor, probs: Optional[
 
 
 class _GroupedLinear(torch.autograd.Function):
-    """y[g] = x[g] @ W[g]^T for consecutive row groups (W stored [G, N, K])."""
+    """y[g] = x[g] @ W[g]^T for consecutive row groups (W stored [G, N, K]), or x[g] @ W[g] (W stored [G, K, N])
+    when ``b_mn``: the GEMM reads either as it lies in memory. Forward and dgrad are one launch over all groups where
+    the kernel takes the operands; wgrad is one product per group (each of its outputs alone fills the GPU)."""
 
     @staticmethod
-    def forward(ctx, x, w, sizes: Tuple[int, ...]):
-        ctx.sizes = sizes
-        ctx.save_for_backward(x, w)
-        out = torch.empty(x.shape[0], w.shape[1], dtype=x.dtype, device=x.device)
+    def _rows(x, w, sizes, b_mn):
+        if ragged_ok(x, w, b_mn, len(sizes)):
+            return gemm_ragged(x, w, sizes, b_mn)
+        out = torch.empty(x.shape[0], w.shape[2] if b_mn else w.shape[1], dtype=x.dtype, device=x.device)
         r = 0
         for g, n in enumerate(sizes):
             if n:
-                gemm(x[r: r + n], w[g], out=out[r: r + n])
+                gemm(x[r: r + n], w[g], b_mn=b_mn, out=out[r: r + n])
             r += n
         return out
+
+    @staticmethod
+    def forward(ctx, x, w, sizes: Tuple[int, ...], b_mn: bool):
+        ctx.sizes, ctx.b_mn = sizes, b_mn
+        ctx.save_for_backward(x, w)
+        return _GroupedLinear._rows(x, w, sizes, b_mn)
 
     @staticmethod
     def backward(ctx, dy):
         x, w = ctx.saved_tensors
         dy = dy.contiguous()
-        dx = torch.empty_like(x)
+        dx = _GroupedLinear._rows(dy, w, ctx.sizes, not ctx.b_mn).to(x.dtype) if ctx.needs_input_grad[0] else None
+        if not ctx.needs_input_grad[1]:
+            return dx, None, None, None
         mg = getattr(w, "main_grad", None)
-        dw = mg if mg is not None else torch.zeros_like(w)
+        dw = mg if mg is not None else torch.empty(w.shape, dtype=w.dtype, device=w.device)
+        a, b = (x, dy) if ctx.b_mn else (dy, x)         # dW[g] = a[g]^T b[g]
         r = 0
         for g, n in enumerate(ctx.sizes):
             if n:
-                gemm(dy[r: r + n], w[g], b_mn=True, out=dx[r: r + n])
-                gemm(dy[r: r + n], x[r: r + n], a_mn=True, b_mn=True, out=dw[g], accumulate=mg is not None)
+                gemm(a[r: r + n], b[r: r + n], a_mn=True, b_mn=True, out=dw[g], accumulate=mg is not None)
+            elif mg is None:
+                dw[g].zero_()
             r += n
         if mg is not None:
             w.grad_added_to_main_grad = True
-            return dx, None, None
-        return dx, dw, None
+            return dx, None, None, None
+        return dx, dw, None, None
 
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, batch_sizes, trans_b: bool = False) -> torch.Tensor:
@@ -87,6 +99,4 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, batch_sizes, trans_b: bool = 
     ``b[g]`` (``[K, N]``) or ``b[g]^T`` when ``trans_b`` (``[N, K]``)."""
     sizes = tuple(int(s) for s in (batch_sizes.tolist() if isinstance(batch_sizes, torch.Tensor) else batch_sizes))
     assert sum(sizes) == a.shape[0], "batch_sizes must cover all rows"
-    if trans_b:
-        return _GroupedLinear.apply(a, b, sizes)
-    return _GroupedLinear.apply(a, b.transpose(1, 2).contiguous(), sizes)
+    return _GroupedLinear.apply(a, b, sizes, not trans_b)

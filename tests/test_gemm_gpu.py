@@ -218,3 +218,45 @@ def test_dynamic_tile_schedule_matches_static():
                 assert torch.equal(o, ref)
     finally:
         L.atb_gemm_set_dynamic(1)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 72), (129, 264, 136), (255, 256, 64), (257, 512, 200), (777, 1032, 520)])
+def test_gemm_odd_token_counts(M, N, K):
+    """Token counts that are no multiple of 8: rows of A in forward and dgrad, the reduction dim in wgrad."""
+    torch.manual_seed(M)
+    x, w, dy = _mk(M, K), _mk(N, K), _mk(M, N)
+    bias, res = _mk(1, N)[0], _mk(M, N)
+    _check(gemm(x, w, bias=bias, residual=res), x.float() @ w.float().t() + bias.float() + res.float(), K)
+    _check(gemm(dy, w, b_mn=True), dy.float() @ w.float(), N)
+    _check(gemm(dy, x, a_mn=True, b_mn=True), dy.float().t() @ x.float(), M)
+    c0 = torch.randn(N, K, device="cuda")
+    out = c0.clone()
+    gemm(dy, x, a_mn=True, b_mn=True, out=out, accumulate=True)
+    _check(out, c0 + dy.float().t() @ x.float(), M)
+
+
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("sizes", [(0, 1, 255, 0), (257, 0, 64, 129, 3), (512, 513), (0, 0, 40)])
+def test_grouped_gemm_ragged_groups(sizes, trans_b):
+    """Groups of any length in one launch, against one fp32 product per group; rows past a group's end belong to the
+    next one and must not be touched by it."""
+    from atorch_b200.ops.moe import grouped_gemm
+
+    torch.manual_seed(sum(sizes))
+    G, K, N = len(sizes), 192, 328
+    x = _mk(sum(sizes), K).requires_grad_(True)
+    w = (torch.randn(G, N, K, device="cuda") if trans_b else torch.randn(G, K, N, device="cuda")).bfloat16()
+    w.requires_grad_(True)
+    dy = _mk(sum(sizes), N)
+    y = grouped_gemm(x, w, sizes, trans_b)
+    y.backward(dy)
+    r = 0
+    for g, n in enumerate(sizes):
+        xs, ds, wg = x.detach()[r: r + n].float(), dy[r: r + n].float(), w.detach()[g].float()
+        wk = wg.t() if trans_b else wg                              # [K, N]
+        if n:
+            _check(y.detach()[r: r + n], xs @ wk, K)
+            _check(x.grad[r: r + n], ds @ wk.t(), N)
+        dw = xs.t() @ ds
+        _check(w.grad[g], dw.t() if trans_b else dw, max(n, 1))
+        r += n
