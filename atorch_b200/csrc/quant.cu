@@ -11,6 +11,7 @@
 // Counterparts in the reference: atorch/ops/csrc/quantization/{quantize,dequantize,swizzled_quantize,
 // quant_reduce}.cu and atorch/ops/csrc/quantization_optimizer/quantization_optimizer.cu.
 #include "common.cuh"
+#include <type_traits>
 
 namespace {
 using namespace atb;
@@ -67,6 +68,111 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ x, 
   }
 }
 
+// The same quantisation with every group held in registers: one read of x. A warp (WARPS = 1) or a block of WARPS warps
+// owns a group of at most WARPS * 32 * V pieces of 8 elements; lane i of them takes pieces i, i + 32 WARPS, ...
+// Bound by memory: 16-byte loads, all V pieces of a thread in flight, 8- or 4-byte stores. 67 M bf16 values in groups
+// of 2048 to int8: 87.5 -> 45.2 us (201 MB, 4.5 TB/s); the kernel above reads x twice, 2 bytes a thread.
+template <typename T>
+struct Piece8 {
+  uint4 r[sizeof(T) / 2];
+  ATB_DEVICE void load(const T* p) {
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(T) / 2); ++i) r[i] = reinterpret_cast<const uint4*>(p)[i];
+  }
+  ATB_DEVICE float at(int i) const { return to_f32<T>(reinterpret_cast<const T*>(r)[i]); }
+};
+
+template <typename T, int WARPS, int V>
+__global__ void __launch_bounds__(128) quantize_regs_kernel(const T* __restrict__ x, int8_t* __restrict__ q,
+                                                            float* __restrict__ params, int groups, int group_size,
+                                                            int bits, int asym, const int* __restrict__ group_map) {
+  __shared__ float red[2][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = WARPS == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
+  if (g >= groups) return;                       // WARPS == 1 only: whole warps leave, nothing below syncs the block
+  const int t = WARPS == 1 ? lane : threadIdx.x;
+  const int n = group_size / 8;
+  const T* xg = x + (long long)g * group_size;
+  Piece8<T> v[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i)
+    if (t + i * 32 * WARPS < n) v[i].load(xg + (t + i * 32 * WARPS) * 8);
+  float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    if (t + i * 32 * WARPS < n) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        lo = fminf(lo, v[i].at(j));
+        hi = fmaxf(hi, v[i].at(j));
+      }
+    }
+  }
+  hi = warp_max(hi);
+  lo = -warp_max(-lo);
+  if (WARPS > 1) {
+    if (lane == 0) { red[0][warp] = hi; red[1][warp] = lo; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < WARPS; ++i) { hi = fmaxf(hi, red[0][i]); lo = fminf(lo, red[1][i]); }
+  }
+  const int qmax = (1 << (bits - 1)) - 1, half = 1 << (bits - 1);
+  float s = asym ? (hi - lo) / (float)((1 << bits) - 1) : fmaxf(fabsf(hi), fabsf(lo)) / (float)qmax;
+  const float off = asym ? lo : 0.f;
+  if (s == 0.f) s = 1.f;
+  const float inv = 1.f / s;
+  const int og = group_map ? group_map[g] : g;
+  if (t == 0) {
+    params[(long long)og * (asym ? 2 : 1)] = s;
+    if (asym) params[(long long)og * 2 + 1] = off;
+  }
+  const float fh = (float)half, fm = (float)qmax, shift = asym ? fh : 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const int k = t + i * 32 * WARPS;
+    if (k >= n) continue;
+    uint32_t c[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      c[j] = (uint32_t)(int)fminf(fmaxf(rintf((v[i].at(j) - off) * inv) - shift, -fh), fm);
+    if (bits == 8) {
+      uint2 o = make_uint2(0u, 0u);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        o.x |= (c[j] & 0xFFu) << (8 * j);
+        o.y |= (c[4 + j] & 0xFFu) << (8 * j);
+      }
+      *reinterpret_cast<uint2*>(q + (long long)og * group_size + (long long)k * 8) = o;
+    } else {
+      uint32_t o = 0u;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o |= (c[j] & 0xFu) << (4 * j);
+      *reinterpret_cast<uint32_t*>(q + (long long)og * (group_size / 2) + (long long)k * 4) = o;
+    }
+  }
+}
+
+// A warp per group up to 2048 elements (8 pieces a lane: 32 registers of 16-bit, 64 of 32-bit values), a block of 4
+// warps up to 8192. Longer groups, groups that are no multiple of 8 and unaligned inputs take quantize_kernel.
+template <typename T>
+bool quantize_regs(const T* x, int8_t* q, float* params, int groups, int group_size, int bits, int asym,
+                   const int* group_map, cudaStream_t st) {
+  if (group_size % 8 || group_size > 8192 || (reinterpret_cast<uintptr_t>(x) & 15) ||
+      (reinterpret_cast<uintptr_t>(q) & 7))
+    return false;
+#define ATB_QUANT(W_, V_)                                                                                     \
+  quantize_regs_kernel<T, W_, V_><<<(W_) == 1 ? (groups + 3) / 4 : groups, 128, 0, st>>>(x, q, params, groups, \
+                                                                                         group_size, bits, asym, group_map)
+  if (group_size <= 256) ATB_QUANT(1, 1);
+  else if (group_size <= 512) ATB_QUANT(1, 2);
+  else if (group_size <= 1024) ATB_QUANT(1, 4);
+  else if (group_size <= 2048) ATB_QUANT(1, 8);
+  else if (group_size <= 4096) ATB_QUANT(4, 4);
+  else ATB_QUANT(4, 8);
+#undef ATB_QUANT
+  return true;
+}
+
 ATB_DEVICE float deq(int v, float s, float off, int asym, int half) { return asym ? (v + half) * s + off : v * s; }
 ATB_DEVICE int sext4(int v) { return (v & 8) ? v - 16 : v; }
 
@@ -86,6 +192,57 @@ __global__ void dequantize_kernel(const int8_t* __restrict__ q, const float* __r
     }
     out[i] = from_f32<T>(deq(v, s, off, asym, half));
   }
+}
+
+// The same for groups of a multiple of 8 elements: a thread turns pieces of 8 codes into 16-byte stores, four pieces in
+// flight, one division by the group length per piece in place of one (64-bit) per element. Bound by memory: 67 M int8
+// codes to bf16 146.5 -> 29.4 us (201 MB, part of the codes still in L2).
+template <typename T>
+__global__ void __launch_bounds__(256) dequantize8_kernel(const int8_t* __restrict__ q, const float* __restrict__ params,
+                                                          T* __restrict__ out, unsigned pieces, unsigned per_group,
+                                                          int bits, int asym) {
+  constexpr int U = 4;
+  const int half = 1 << (bits - 1);
+  const unsigned first = blockIdx.x * (256u * U) + threadIdx.x;
+  uint2 c[U];
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    const unsigned k = first + i * 256u;
+    if (k >= pieces) break;
+    if (bits == 8) c[i] = reinterpret_cast<const uint2*>(q)[k];
+    else c[i].x = reinterpret_cast<const uint32_t*>(q)[k];
+  }
+#pragma unroll
+  for (int i = 0; i < U; ++i) {
+    const unsigned k = first + i * 256u;
+    if (k >= pieces) break;
+    const unsigned g = k / per_group;
+    const float s = params[(size_t)g * (asym ? 2 : 1)], off = asym ? params[(size_t)g * 2 + 1] : 0.f;
+    Piece8<T> o;
+    T* ov = reinterpret_cast<T*>(o.r);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      int v;
+      if (bits == 8) v = (int)(int8_t)((j < 4 ? c[i].x : c[i].y) >> (8 * (j & 3)));
+      else v = sext4((c[i].x >> (4 * j)) & 0xF);
+      ov[j] = from_f32<T>(deq(v, s, off, asym, half));
+    }
+#pragma unroll
+    for (int j = 0; j < (int)(sizeof(T) / 2); ++j)
+      reinterpret_cast<uint4*>(out + (size_t)k * 8)[j] = o.r[j];
+  }
+}
+
+template <typename T>
+bool dequantize8(const int8_t* q, const float* params, T* out, long long total, int group_size, int bits, int asym,
+                 cudaStream_t st) {
+  if (group_size % 8 || total % 8 || total / 8 > 0x7fffffffLL || (reinterpret_cast<uintptr_t>(out) & 15) ||
+      (reinterpret_cast<uintptr_t>(q) & 7))
+    return false;
+  const unsigned pieces = (unsigned)(total / 8);
+  dequantize8_kernel<T><<<(pieces + 1023) / 1024, 256, 0, st>>>(q, params, out, pieces, (unsigned)group_size / 8, bits,
+                                                                asym);
+  return true;
 }
 
 // out group g = requantised sum over `n_in` tensors' group g (all tensors share the group layout);
@@ -231,20 +388,30 @@ extern "C" int atb_quantize(const void* x, void* q, float* params, int groups, i
                             const int* group_map, int dtype, void* stream) {
   if (groups <= 0) return 0;
   if ((bits != 4 && bits != 8) || (bits == 4 && (group_size & 1))) return -1;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == 0) quantize_kernel<__nv_bfloat16><<<groups, 256, 0, st>>>((const __nv_bfloat16*)x, (int8_t*)q, params, group_size, bits, asym, group_map, groups);
-  else if (dtype == 1) quantize_kernel<__half><<<groups, 256, 0, st>>>((const __half*)x, (int8_t*)q, params, group_size, bits, asym, group_map, groups);
-  else quantize_kernel<float><<<groups, 256, 0, st>>>((const float*)x, (int8_t*)q, params, group_size, bits, asym, group_map, groups);
+  auto run = [&](auto* xt) {
+    using T = std::remove_cv_t<std::remove_pointer_t<decltype(xt)>>;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!quantize_regs<T>(xt, (int8_t*)q, params, groups, group_size, bits, asym, group_map, st))
+      quantize_kernel<T><<<groups, 256, 0, st>>>(xt, (int8_t*)q, params, group_size, bits, asym, group_map, groups);
+  };
+  if (dtype == 0) run((const __nv_bfloat16*)x);
+  else if (dtype == 1) run((const __half*)x);
+  else run((const float*)x);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 extern "C" int atb_dequantize(const void* q, const float* params, void* out, long long total, int group_size, int bits,
                               int asym, int dtype, void* stream) {
   if (total <= 0) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int g = cap_grid(total, 256);
-  if (dtype == 0) dequantize_kernel<__nv_bfloat16><<<g, 256, 0, st>>>((const int8_t*)q, params, (__nv_bfloat16*)out, total, group_size, bits, asym);
-  else if (dtype == 1) dequantize_kernel<__half><<<g, 256, 0, st>>>((const int8_t*)q, params, (__half*)out, total, group_size, bits, asym);
-  else dequantize_kernel<float><<<g, 256, 0, st>>>((const int8_t*)q, params, (float*)out, total, group_size, bits, asym);
+  auto run = [&](auto* o) {
+    using T = std::remove_pointer_t<decltype(o)>;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!dequantize8<T>((const int8_t*)q, params, o, total, group_size, bits, asym, st))
+      dequantize_kernel<T><<<cap_grid(total, 256), 256, 0, st>>>((const int8_t*)q, params, o, total, group_size, bits,
+                                                                 asym);
+  };
+  if (dtype == 0) run((__nv_bfloat16*)out);
+  else if (dtype == 1) run((__half*)out);
+  else run((float*)out);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 extern "C" int atb_dequant_reduce(const void* q_in, const float* p_in, void* q_out, float* p_out, int n_in,

@@ -58,3 +58,32 @@ def test_state_packing():
         assert torch.equal(s1, s2) and not torch.equal(s1, s3)
         mean_err = (lowbit.unpack_nonlinear(s1, am, qm, x.numel(), bits, gs) - x).mean().abs()
         assert mean_err < 5e-3            # stochastic rounding is unbiased
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("group", [8, 248, 256, 520, 1024, 2040, 2056, 4096, 8192, 8200, 30])
+def test_quantize_group_lengths(group, dtype):
+    """Every split of a group over lanes and warps, the lengths at its edges, and the general kernel beyond it."""
+    torch.manual_seed(group)
+    groups = 37
+    x = (torch.randn(groups, group, device="cuda") * torch.rand(groups, 1, device="cuda")).to(dtype)
+    x[3] = 0
+    for bits in (8, 4):
+        for sym in (True, False):
+            q, p = quantizer.quantize(x.reshape(-1), groups, bits, sym)
+            qr, pr = quantizer.quantize_reference(x.reshape(-1), groups, bits, sym)
+            assert torch.allclose(p, pr, rtol=1e-6, atol=0)
+            # the kernel multiplies by the rounded reciprocal of the scale, the reference divides: x / s differs by
+            # 2^-23 |x / s| <= 2^-15, so an element may differ only if its exact quotient is that close to a tie. Of a
+            # 16-bit input many lie exactly on one (the scale is absmax / 127 of the same grid), hence no fixed share
+            lo = 0.0 if sym else pr.double()[:, 1:2]
+            v = (x.double() - lo) / pr.double()[:, :1]
+            near = ((v - v.floor() - 0.5).abs() < 2 ** -14).reshape(-1)
+            if bits == 8:
+                assert not bool(((q != qr) & ~near).any()) and (q.int() - qr.int()).abs().max() <= 1
+            else:
+                assert not bool(((q != qr) & ~(near[0::2] | near[1::2])).any())
+            for out in (torch.float32, dtype):
+                d = quantizer.dequantize(q, p, groups, bits, sym, out)
+                dr = quantizer.dequantize_reference(q, p, groups, bits, sym, out)     # one rounding to `out`
+                assert torch.equal(d, dr) or torch.allclose(d.float(), dr.float(), rtol=2 ** -7, atol=1e-6)
