@@ -156,6 +156,41 @@ __global__ void sumsq_kernel(const G* __restrict__ x, long long n, float* __rest
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
+// The same over 16-byte aligned buffers: 16-byte loads, four of them in flight per thread, an accumulator each (shorter
+// fp32 chains than one). Bound by memory: 268 M bf16 values (537 MB) 269 -> 100.3 us; two bytes a thread kept too few
+// bytes in flight.
+template <typename G>
+__global__ void __launch_bounds__(256) sumsq16_kernel(const G* __restrict__ x, long long n, float* __restrict__ partial) {
+  constexpr int U = 4, PER = 16 / sizeof(G);
+  __shared__ float red[33];
+  const uint4* xv = reinterpret_cast<const uint4*>(x);
+  const long long nv = n / PER, stride = (long long)gridDim.x * 256;
+  float s[U] = {0.f, 0.f, 0.f, 0.f};
+  auto add = [&](float& acc, const uint4& u) {
+    const G* e = reinterpret_cast<const G*>(&u);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const float v = to_f32<G>(e[j]);
+      acc += v * v;
+    }
+  };
+  long long i = blockIdx.x * 256LL + threadIdx.x;
+  for (; i + (U - 1) * stride < nv; i += U * stride) {
+    uint4 u[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) u[k] = xv[i + k * stride];
+#pragma unroll
+    for (int k = 0; k < U; ++k) add(s[k], u[k]);
+  }
+  for (; i < nv; i += stride) add(s[0], xv[i]);
+  if (blockIdx.x == 0 && threadIdx.x < n - nv * PER) {   // fewer than PER values are left over
+    const float v = to_f32<G>(x[nv * PER + threadIdx.x]);
+    s[1] += v * v;
+  }
+  const float t = block_sum((s[0] + s[1]) + (s[2] + s[3]), red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = t;
+}
+
 // Nesterov / momentum SGD outer step of local SGD on a flat shard:
 //   g = pseudo-gradient (already reduced); buf = mu*buf + g; p_sync -= lr*(g + mu*buf) (nesterov)
 //   or p_sync -= lr*buf; then param <- p_sync.
@@ -251,8 +286,12 @@ extern "C" int atb_sumsq_parts() { return 148 * 4; }
 extern "C" int atb_sumsq(const void* x, long long n, float* partial, int dtype, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = atb_sumsq_parts();
-  if (dtype == 0) sumsq_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, n, partial);
-  else sumsq_kernel<float><<<grid, 256, 0, st>>>((const float*)x, n, partial);
+  auto run = [&](const auto* xt) {
+    if (reinterpret_cast<uintptr_t>(x) & 15) sumsq_kernel<<<grid, 256, 0, st>>>(xt, n, partial);
+    else sumsq16_kernel<<<grid, 256, 0, st>>>(xt, n, partial);
+  };
+  if (dtype == 0) run((const __nv_bfloat16*)x);
+  else run((const float*)x);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
