@@ -40,6 +40,10 @@ ATB_DEVICE uint64_t globaltimer_ns() {
   return t;
 }
 
+// A value that is the same in every lane, as one the compiler knows to be (it can then use uniform registers and branches).
+template <typename T>
+ATB_DEVICE T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 ATB_DEVICE bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -91,21 +95,46 @@ ATB_DEVICE bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Bounded wait. `abort_flag` is a shared-memory word: once any role of the CTA has
 // timed out, all later waits return false at once so the CTA can drain.
+// The clock is read only after a thousand polls: a read of %globaltimer costs several hundred clocks, which every wait
+// that was not already satisfied used to pay between its first and its second poll.
 ATB_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
-  if (mbar_try_wait(bar, parity)) return true;
-  uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+  while (!mbar_try_wait(bar, parity)) {
     if ((++spins & 0x3ff) == 0) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > ATB_WAIT_LIMIT_NS) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > ATB_WAIT_LIMIT_NS) {
         *abort_flag = 1;
         if (status) atomicCAS(status, 0, (int)ATB_ERR_WAIT_TIMEOUT);
         return false;
       }
     }
   }
+  return true;
+}
+
+// The same by a whole converged warp, with one answer for all lanes: a satisfied wait costs 27 clocks, against 103 in the
+// loop above, which every lane may leave on its own, and 267 when that loop runs in an `if (lane == 0)` branch (2000
+// waits on a completed barrier, clock64). The warps that feed the tensor core wait several times per tile in series with
+// the products, so they use this one, and leave to one elected lane only the instructions that must be issued once.
+ATB_DEVICE bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
+  uint64_t t0 = 0;
+  uint32_t spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 0x3ff) == 0) {
+      const uint64_t now = warp_uniform(globaltimer_ns());
+      if (t0 == 0) t0 = now;
+      const bool late = now - t0 > ATB_WAIT_LIMIT_NS;
+      if (late) {
+        *abort_flag = 1;
+        if (status) atomicCAS(status, 0, (int)ATB_ERR_WAIT_TIMEOUT);
+      }
+      if (__any_sync(0xffffffffu, late || *abort_flag != 0)) return false;
+    }
+  }
+  return true;
 }
 
 // ----------------------------------------------------------------------------------
@@ -307,12 +336,82 @@ ATB_DEVICE uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint
 // place of rebuilding the descriptor, which matters when one thread issues an MMA every 64 clocks.
 ATB_DEVICE uint64_t umma_desc_advance(uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); }
 
+// The issue path of a whole warp: every lane runs the code, lanes with issue != 0 (one, from elect_one()) execute the
+// instruction. The predicate sits on the instruction itself, not on a branch around it, and a descriptor is its low word
+// (start address and LBO; the high word is the same for every tile with 1024-byte row groups). Measured for groups of 8
+// products of 32 clocks, each group behind a satisfied barrier: 268 clocks a group, 336 with `if (issue)` around 64-bit
+// descriptors.
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+ATB_DEVICE uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
+  return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);
+}
+template <int CTA_GROUP = 1>
+ATB_DEVICE void umma_ss_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
+                              uint32_t issue) {
+#define ATB_UMMA_SS(GROUP)                                          \
+  asm volatile(                                                     \
+      "{\n"                                                         \
+      ".reg .pred p, q;\n"                                          \
+      ".reg .b64 a, b;\n"                                           \
+      "mov.b64 a, {%1, %3};\n"                                      \
+      "mov.b64 b, {%2, %3};\n"                                      \
+      "setp.ne.b32 p, %5, 0;\n"                                     \
+      "setp.ne.b32 q, %6, 0;\n"                                     \
+      "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], a, b, %4, p;\n" \
+      "}\n" ::"r"(tmem_d),                                          \
+      "r"(a_lo), "r"(b_lo), "r"(UMMA_DESC_HI), "r"(idesc), "r"(accumulate), "r"(issue) \
+      : "memory")
+  if constexpr (CTA_GROUP == 1) ATB_UMMA_SS("1");
+  else ATB_UMMA_SS("2");
+#undef ATB_UMMA_SS
+}
+ATB_DEVICE void umma_ts_issue(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
+                              uint32_t issue) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 b;\n"
+      "mov.b64 b, {%2, %3};\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "setp.ne.b32 q, %6, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %4, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(UMMA_DESC_HI), "r"(idesc), "r"(accumulate), "r"(issue)
+      : "memory");
+}
+ATB_DEVICE void umma_commit_issue(uint64_t* bar, uint32_t issue) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(smem_u32(bar)), "r"(issue)
+      : "memory");
+}
+
+ATB_DEVICE void umma_commit_cg2_issue(uint32_t bar_cluster_addr, uint32_t issue) {
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "setp.ne.b32 q, %1, 0;\n"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+      "}\n" ::"r"(bar_cluster_addr), "r"(issue)
+      : "memory");
+}
+
 // Instruction descriptor for kind::f16 / kind::f8f6f4 with fp32 accumulation.
 //   fmt: kind::f16: 0 = f16, 1 = bf16;  kind::f8f6f4: 0 = e4m3, 1 = e5m2
 ATB_DEVICE constexpr uint32_t umma_idesc(int m, int n, int a_fmt, int b_fmt, bool a_mn_major, bool b_mn_major) {
   return (1u << 4) | ((uint32_t)a_fmt << 7) | ((uint32_t)b_fmt << 10) | ((a_mn_major ? 1u : 0u) << 15) |
          ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+
+// Registers per thread of this warpgroup (executed by all its warps; N a multiple of 8). The warpgroups' shares must
+// add up to no more than the block was launched with, or the increase waits forever.
+template <int N>
+ATB_DEVICE void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+ATB_DEVICE void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ----------------------------------------------------------------------------------
 // small helpers

@@ -1,19 +1,28 @@
-// Flash attention forward, two query tiles per CTA (head dim 128, bf16) for sm_100a.
+// Flash attention forward, two query tiles per CTA (head dim 128 or 64, bf16) for sm_100a.
 //
 // One CTA owns 256 query rows as two 128-row tiles A and B that share every K/V tile. Warp 0 = TMA
-// producer, warp 1 = MMA issuer / TMEM owner, warps 2..5 = softmax of tile A, warps 6..9 = softmax of
-// tile B; a softmax thread owns one whole row (128 scores), so no row statistics are exchanged.
+// producer, warp 1 = MMA issuer / TMEM owner, warp 2 = key range, warps 4..7 = softmax of tile A, warps 8..11 =
+// softmax of tile B; a softmax thread owns one whole row (128 scores), so no row statistics are exchanged.
 //
 //   TMEM:  S_A | S_B | O_A | O_B   (4 x 128 fp32 columns); P_T (bf16) overwrites the first 64 columns of S_T
 //   per K/V tile j:   S_T = Q_T K_j^T  ->  P_T = 2^(S_T c - m_T c)  ->  O_T += P_T V_j
 //
 // P never leaves tensor memory: the softmax thread stores its packed row with tcgen05.st and the P.V
-// product reads it as the A operand of tcgen05.mma. O accumulates in tensor memory. The reference maximum
+// product reads it as the A operand of tcgen05.mma. O accumulates in tensor memory. What bounds the kernel is the
+// chain S -> maximum -> exponentials -> P -> P.V -> next S of one tile, so it is kept short: the 128 scores of a row
+// are read out of tensor memory once and stay in registers, hidden keys are turned into -inf there (32 keys per bit
+// mask, so that a partly visible tile costs little more than a full one), and P is handed over in two halves of 64
+// keys, so that the first half of P.V runs under the second half of the exponentials. The reference maximum
 // m_T of a row is only raised when the new row maximum exceeds it by more than 2^8 (in the exponent
 // domain); then the row of O_T is rescaled in TMEM by the owning thread, which is safe because the scores
 // S_T(j) it has just waited for were issued after the product P_T(j-1) V and complete after it.
 // While tile A's warps exponentiate, the tensor core works for tile B and vice versa:
 // issue order  PV_A(j), S_A(j+1), PV_B(j), S_B(j+1).
+//
+// 8192 keys, 32 heads of 128: full 825 us (1333 TFLOP/s), causal 489 us (before: 945 and 578-625 us); a step of both
+// tiles takes 3100 clocks, 1900 of them softmax and 1200 tensor work of the same tile. Tried: K/V tiles of 64 keys with
+// two score buffers per tile, which takes the tensor work out of that chain - 887 us, because a 128 x 64 x 16 score
+// product takes 48 clocks for its shared-memory operands where it should take 32; P in one piece - 859 us.
 //
 // Masks: per-row key interval [lo, hi) exactly as in flash_attn.cu; each query tile walks only the K/V
 // tiles up to the last one that any of its rows can see.
@@ -23,10 +32,12 @@
 namespace {
 using namespace atb;
 
-constexpr int BQ = 128, BKV = 128, HD = 128;
+constexpr int BQ = 128, BKV = 128;
 constexpr int PANEL = 128 * 64 * 2;
-constexpr int TILE = 2 * PANEL;
-constexpr int THREADS = 64 + 256;
+constexpr int THREADS = 128 + 256;
+// 168 registers a thread at launch (384 x 168 = 64512); the control warpgroup gives up what the softmax warps need to
+// hold a row of scores: 128 x 80 + 256 x 208 = 63488
+constexpr int REGS_CONTROL = 80, REGS_SOFTMAX = 208;
 constexpr float RESCALE_THRESHOLD = 8.f;   // log2 units
 
 struct Params {
@@ -39,77 +50,78 @@ struct Params {
   int* status;
 };
 
+template <int HD>
 struct L2 {
+  static constexpr int TILE = (HD / 64) * PANEL;
   static constexpr int Q_OFF = 0;                    // tile A, tile B
   static constexpr int K_OFF = Q_OFF + 2 * TILE;     // 2 stages
   static constexpr int V_OFF = K_OFF + 2 * TILE;     // 2 stages
   static constexpr int BAR_OFF = V_OFF + 2 * TILE;   // 192 KB
-  static constexpr int NBARS = 1 + 8 + 2 + 2 + 2;
+  static constexpr int NBARS = 1 + 8 + 2 + 4 + 2;
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
 };
 
-// P = 2^(S c - m c) for one row: the 128 scores are read back from tensor memory in chunks of 32 (the next
-// chunk's load is in flight while this one is exponentiated) and the packed bf16 result overwrites the first
-// 64 columns of S; each chunk is read before the 16 columns it turns into are written, and those lie below
-// the next chunk. Returns the row sum. MASK: per-element key interval test (tiles that are not fully visible).
-template <bool MASK>
-ATB_DEVICE float softmax_exp_row(uint32_t s_addr, float scale_log2, float neg_ms, int kv0, int lo, int hi) {
-  const uint64_t sc2 = f2_pack(scale_log2, scale_log2), nm2 = f2_pack(neg_ms, neg_ms);
-  uint64_t acc0 = 0ull, acc1 = 0ull;   // (0.f, 0.f)
-  uint32_t xa[32], xb[32];
-  tmem_ld_32x32(s_addr, xa);
+// -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi)
+ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi) {
+  const int a = min(max(lo - kv0, 0), 32), e = min(max(hi - kv0, 0), 32);
+  const uint32_t below_e = e == 32 ? 0xffffffffu : (1u << e) - 1u, below_a = a == 32 ? 0xffffffffu : (1u << a) - 1u;
+  const uint32_t vis = below_e & ~below_a;
 #pragma unroll
-  for (int cc = 0; cc < 4; ++cc) {
-    uint32_t (&x)[32] = (cc & 1) ? xb : xa;
-    uint32_t (&xn)[32] = (cc & 1) ? xa : xb;
-    tmem_ld_wait();
-    if (cc + 1 < 4) tmem_ld_32x32(s_addr + (cc + 1) * 32, xn);
-    uint32_t pk[16];
-#pragma unroll
-    for (int c = 0; c < 32; c += 2) {
-      float t0, t1;
-      f2_unpack(f2_fma(f2_pack_bits(x[c], x[c + 1]), sc2, nm2), t0, t1);
-      float p0 = fast_exp2(t0), p1 = fast_exp2(t1);
-      if (MASK) {
-        const int kk = kv0 + cc * 32 + c;
-        if (kk < lo || kk >= hi) p0 = 0.f;
-        if (kk + 1 < lo || kk + 1 >= hi) p1 = 0.f;
-      }
-      const uint64_t pp = f2_pack(p0, p1);
-      if ((c >> 1) & 1) acc1 = f2_add(acc1, pp);
-      else acc0 = f2_add(acc0, pp);
-      pk[c >> 1] = pack_bf16x2(p0, p1);
-    }
-    tmem_st_32x16(s_addr + cc * 16, pk);
-  }
-  float a, b, c, d;
-  f2_unpack(acc0, a, b);
-  f2_unpack(acc1, c, d);
-  return (a + b) + (c + d);
+  for (int c = 0; c < 32; ++c)
+    if (!(vis & (1u << c))) x[c] = 0xff800000u;
 }
 
+ATB_DEVICE float max_of(const uint32_t (&x)[32]) {
+  float m0 = __uint_as_float(x[0]), m1 = __uint_as_float(x[1]);
+#pragma unroll
+  for (int c = 2; c < 32; c += 2) {
+    m0 = fmaxf(m0, __uint_as_float(x[c]));
+    m1 = fmaxf(m1, __uint_as_float(x[c + 1]));
+  }
+  return fmaxf(m0, m1);
+}
+
+// P = 2^(S c - m c) of 64 scores as packed bf16; the sums of the even and the odd keys are added to `sum`
+ATB_DEVICE void exp_half(const uint32_t (&xa)[32], const uint32_t (&xb)[32], uint64_t sc2, uint64_t nm2, uint64_t& sum0,
+                         uint64_t& sum1, uint32_t (&pk)[32]) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 2) {
+    float t0, t1, u0, u1;
+    f2_unpack(f2_fma(f2_pack_bits(xa[c], xa[c + 1]), sc2, nm2), t0, t1);
+    f2_unpack(f2_fma(f2_pack_bits(xb[c], xb[c + 1]), sc2, nm2), u0, u1);
+    const float p0 = fast_exp2(t0), p1 = fast_exp2(t1), r0 = fast_exp2(u0), r1 = fast_exp2(u1);
+    sum0 = f2_add(sum0, f2_pack(p0, p1));
+    sum1 = f2_add(sum1, f2_pack(r0, r1));
+    pk[c >> 1] = pack_bf16x2(p0, p1);
+    pk[16 + (c >> 1)] = pack_bf16x2(r0, r1);
+  }
+}
+
+template <int HD>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, Params p) {
+  using L = L2<HD>;
+  constexpr int TILE = L::TILE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem + L2::Q_OFF;
-  uint8_t* sK = smem + L2::K_OFF;
-  uint8_t* sV = smem + L2::V_OFF;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L2::BAR_OFF);
+  uint8_t* sQ = smem + L::Q_OFF;
+  uint8_t* sK = smem + L::K_OFF;
+  uint8_t* sV = smem + L::V_OFF;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* q_full = bars;
   uint64_t* k_full = bars + 1;      // [2]
   uint64_t* k_empty = bars + 3;     // [2]
   uint64_t* v_full = bars + 5;      // [2]
   uint64_t* v_empty = bars + 7;     // [2]
   uint64_t* s_full = bars + 9;      // [2] per query tile: S_T(j) is in TMEM (and P_T(j-1) V has completed)
-  uint64_t* p_full = bars + 11;     // [2] per query tile: P_T(j) is in TMEM
-  uint64_t* o_full = bars + 13;     // [2] per query tile: the last P.V product has completed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L2::NBARS);
+  uint64_t* p_full = bars + 11;     // [2][2] per query tile and half of the keys: P_T(j) is in TMEM
+  uint64_t* o_full = bars + 15;     // [2] per query tile: the last P.V product has completed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // t0, t1 of tile A, t1 of tile B
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
   const int qb = gridDim.x - 1 - blockIdx.x;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -122,8 +134,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&o_full[i], 1);
     }
+    for (int i = 0; i < 4; ++i) mbar_init(&p_full[i], 4);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -157,96 +170,103 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int t0 = kv_range[0];
-  const int n_a = kv_range[1] - t0, n_b = kv_range[2] - t0;   // K/V tiles of query tile A / B
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int t0 = warp_uniform(kv_range[0]);
+  const int n_a = warp_uniform(kv_range[1]) - t0, n_b = warp_uniform(kv_range[2]) - t0;   // K/V tiles of query tile A / B
   const int n = max(n_a, n_b);
   const long long q_row0 = (long long)b * p.Sq + q0;
   const long long k_row0 = (long long)b * p.Sk;
 
-  if (warp == 0) {
-    if (lane == 0 && n > 0) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-      mbar_expect_tx(q_full, 2 * TILE);
+  if (warp < 4) {
+    reg_dealloc<REGS_CONTROL>();
+    if (warp == 0 && n > 0) {
+      const bool el = elect_one();
+      if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
+      if (el) mbar_expect_tx(q_full, 2 * TILE);
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
-        tma_load_2d(sQ + t * TILE, &tmQ, q_full, h * HD, (int)(q_row0 + t * BQ));
-        tma_load_2d(sQ + t * TILE + PANEL, &tmQ, q_full, h * HD + 64, (int)(q_row0 + t * BQ));
+        if (el) tma_load_2d(sQ + t * TILE, &tmQ, q_full, h * HD, (int)(q_row0 + t * BQ));
+        if (HD == 128 && el) tma_load_2d(sQ + t * TILE + PANEL, &tmQ, q_full, h * HD + 64, (int)(q_row0 + t * BQ));
       }
       for (int j = 0; j < n; ++j) {
         const int s = j & 1;
         const uint32_t ph = (j >> 1) & 1;
         const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
-        if (!mbar_wait(&k_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&k_full[s], TILE);
-        tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HD, krow);
-        tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HD + 64, krow);
-        if (!mbar_wait(&v_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&v_full[s], TILE);
-        tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HD, krow);
-        tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HD + 64, krow);
+        if (!mbar_wait_warp(&k_empty[s], ph ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&k_full[s], TILE);
+        if (el) tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HD, krow);
+        if (HD == 128 && el) tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HD + 64, krow);
+        if (!mbar_wait_warp(&v_empty[s], ph ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&v_full[s], TILE);
+        if (el) tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HD, krow);
+        if (HD == 128 && el) tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HD + 64, krow);
       }
     }
-  } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (warp == 1 && n > 0) {
+      const uint32_t el = elect_one();  // the lane that issues and commits
       constexpr uint32_t idesc_s = umma_idesc(BQ, BKV, 1, 1, false, false);
       constexpr uint32_t idesc_o = umma_idesc(BQ, HD, 1, 1, false, true);
       int k_ready = -1, v_ready = -1;   // newest K / V tile whose arrival has been waited for
       // descriptors of the tiles' first MMA operands; the loops below only advance them
       // (kept in scalars and picked with selects: an array indexed at run time would live in local memory)
-      const uint64_t q_desc0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), k_desc0 = umma_desc_sw128(smem_u32(sK), 16, 1024),
-                     v_desc0 = umma_desc_sw128(smem_u32(sV), PANEL, 1024);
-      // S_T(j) = Q_T K_j^T into the tile's S columns
-      auto issue_s = [&](int t, int j) -> bool {
-        const int s = j & 1;
-        if (k_ready < j) {
-          if (!mbar_wait(&k_full[s], (j >> 1) & 1, abort_flag, p.status)) return false;
-          k_ready = j;
-          tc_fence_after();
-        }
-        const uint64_t qd = umma_desc_advance(q_desc0, t ? TILE : 0), kd = umma_desc_advance(k_desc0, s ? TILE : 0);
+      const uint32_t q_desc0 = umma_desc_lo(smem_u32(sQ), 16), k_desc0 = umma_desc_lo(smem_u32(sK), 16),
+                     v_desc0 = umma_desc_lo(smem_u32(sV), PANEL);
+      auto wait_k = [&](int j) -> bool {
+        if (k_ready >= j) return true;
+        k_ready = j;
+        return mbar_wait_warp(&k_full[j & 1], (j >> 1) & 1, abort_flag, p.status);
+      };
+      auto wait_v = [&](int j) -> bool {
+        if (v_ready >= j) return true;
+        v_ready = j;
+        return mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, abort_flag, p.status);
+      };
+      // S_T(j) = Q_T K_j^T into the tile's S columns (K_j has arrived)
+      auto issue_s = [&](int t, int j) {
+        const uint32_t qd = q_desc0 + ((t ? TILE : 0) >> 4), kd = k_desc0 + (((j & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tmem_base + t * BKV, umma_desc_advance(qd, off), umma_desc_advance(kd, off), idesc_s, k != 0);
+          umma_ss_issue(tmem_base + t * BKV, qd + (off >> 4), kd + (off >> 4), idesc_s, k != 0, el);
         }
-        umma_commit(&s_full[t]);
-        return true;
+        umma_commit_issue(&s_full[t], el);
       };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status);
-      if (ok && n_a > 0) ok = issue_s(0, 0);
-      if (ok && n_b > 0) ok = issue_s(1, 0);
-      if (ok) umma_commit(&k_empty[0]);
+      bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status) && wait_k(0);
+      if (ok && n_a > 0) issue_s(0, 0);
+      if (ok && n_b > 0) issue_s(1, 0);
+      if (ok) umma_commit_issue(&k_empty[0], el);
       // one half-step of the ping-pong for query tile T (compile-time, so that nothing is indexed at run time):
-      // P_T(j) V_j into O_T, then the next scores S_T(j+1)
+      // P_T(j) V_j into O_T, then the next scores S_T(j+1). The waits for V_j and K_{j+1} come before the wait for P,
+      // so that nothing lies between P's arrival and the products that depend on it.
       auto half_step = [&](auto tile, int j) -> bool {
         constexpr int t = decltype(tile)::value;
         const int n_t = t ? n_b : n_a;
         const int s = j & 1;
         if (j < n_t) {
-          if (!mbar_wait(&p_full[t], j & 1, abort_flag, p.status)) return false;
-          if (v_ready < j) {
-            if (!mbar_wait(&v_full[s], (j >> 1) & 1, abort_flag, p.status)) return false;
-            v_ready = j;
-          }
-          tc_fence_after();
-          const uint64_t vd = umma_desc_advance(v_desc0, s ? TILE : 0);
+          if (!wait_v(j) || (j + 1 < n_t && !wait_k(j + 1))) return false;
+          const uint32_t vd = v_desc0 + ((s ? TILE : 0) >> 4);
 #pragma unroll
-          for (int k = 0; k < BKV / 16; ++k)   // A = P_T: 16 bf16 keys per step = 8 TMEM columns
-            umma_f16_ts(tmem_base + 2 * BKV + t * HD, tmem_base + t * BKV + k * 8, umma_desc_advance(vd, k * 2048),
-                        idesc_o, (j | k) != 0);
-          if (j == n_t - 1) umma_commit(&o_full[t]);
+          for (int k = 0; k < BKV / 16; ++k) {   // A = P_T: 16 bf16 keys per step = 8 TMEM columns
+            if (k % (BKV / 32) == 0) {
+              if (!mbar_wait_warp(&p_full[2 * t + k / (BKV / 32)], j & 1, abort_flag, p.status)) return false;
+              tc_fence_after();
+            }
+            umma_ts_issue(tmem_base + 2 * BKV + t * HD, tmem_base + t * BKV + k * 8, vd + k * 128,
+                          idesc_o, (j | k) != 0, el);
+          }
+          if (j == n_t - 1) umma_commit_issue(&o_full[t], el);
         }
-        if (t == 1) umma_commit(&v_empty[s]);
-        if (j + 1 < n_t && !issue_s(t, j + 1)) return false;
-        if (t == 1 && j + 1 < n) umma_commit(&k_empty[(j + 1) & 1]);
+        if (j + 1 < n_t) issue_s(t, j + 1);
+        if (t == 1) umma_commit_issue(&v_empty[s], el);
+        if (t == 1 && j + 1 < n) umma_commit_issue(&k_empty[(j + 1) & 1], el);
         return true;
       };
       for (int j = 0; ok && j < n; ++j)
         ok = half_step(std::integral_constant<int, 0>{}, j) && half_step(std::integral_constant<int, 1>{}, j);
     }
   } else {
-    const int t = (warp - 2) >> 2;            // query tile of this warp
+    reg_alloc<REGS_SOFTMAX>();
+    const int t = (warp - 4) >> 2;            // query tile of this warp
     const int quarter = warp & 3;             // TMEM lane quarter
     const int r = quarter * 32 + lane;        // row inside the tile
     const int i = q0 + t * BQ + r;            // global query row
@@ -264,36 +284,23 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     bool ok = true;
     for (int j = 0; j < n_t; ++j) {
       const int kv0 = (t0 + j) * BKV;
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[t], j & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       // the mask tests are compiled into a separate path taken only by warps with a partly visible row
       const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
-      // ---- pass 1: row maximum
-      float mx;
-      {
-        uint32_t x0[32], x1[32], x2[32], x3[32];
-        tmem_ld_32x32(s_addr, x0);
-        tmem_ld_32x32(s_addr + 32, x1);
-        tmem_ld_32x32(s_addr + 64, x2);
-        tmem_ld_32x32(s_addr + 96, x3);
-        tmem_ld_wait();
-        if (!full) {
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            if (kv0 + c < lo || kv0 + c >= hi) x0[c] = 0xff800000u;
-            if (kv0 + 32 + c < lo || kv0 + 32 + c >= hi) x1[c] = 0xff800000u;
-            if (kv0 + 64 + c < lo || kv0 + 64 + c >= hi) x2[c] = 0xff800000u;
-            if (kv0 + 96 + c < lo || kv0 + 96 + c >= hi) x3[c] = 0xff800000u;
-          }
-        }
-        float m4[4] = {__uint_as_float(x0[0]), __uint_as_float(x1[0]), __uint_as_float(x2[0]), __uint_as_float(x3[0])};
-#pragma unroll
-        for (int c = 1; c < 32; ++c) {
-          m4[0] = fmaxf(m4[0], __uint_as_float(x0[c])); m4[1] = fmaxf(m4[1], __uint_as_float(x1[c]));
-          m4[2] = fmaxf(m4[2], __uint_as_float(x2[c])); m4[3] = fmaxf(m4[3], __uint_as_float(x3[c]));
-        }
-        mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      uint32_t x0[32], x1[32], x2[32], x3[32];
+      tmem_ld_32x32(s_addr, x0);
+      tmem_ld_32x32(s_addr + 32, x1);
+      tmem_ld_32x32(s_addr + 64, x2);
+      tmem_ld_32x32(s_addr + 96, x3);
+      tmem_ld_wait();
+      if (!full) {
+        mask_scores(x0, kv0, lo, hi);
+        mask_scores(x1, kv0 + 32, lo, hi);
+        mask_scores(x2, kv0 + 64, lo, hi);
+        mask_scores(x3, kv0 + 96, lo, hi);
       }
+      const float mx = fmaxf(fmaxf(max_of(x0), max_of(x1)), fmaxf(max_of(x2), max_of(x3)));
       // raise the reference maximum only when it pays: a stale one costs nothing while 2^(gap) fits bf16/fp32
       const bool raise = (mx > m_ref) && (m_ref == -INFINITY || (mx - m_ref) * p.scale_log2 > RESCALE_THRESHOLD);
       if (__any_sync(0xffffffffu, raise)) {
@@ -304,8 +311,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           l_run *= alpha;
         }
         if (j > 0) {   // O_T holds the products up to tile j-1 (complete: S_T(j) was issued after them)
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
+#pragma unroll 1
+          for (int cc = 0; cc < HD / 32; ++cc) {
             uint32_t tr[32];
             tmem_ld_32x32(o_addr + cc * 32, tr);
             tmem_ld_wait();
@@ -315,22 +322,35 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           }
         }
       }
-      // ---- pass 2: P = 2^(S c - m c) as packed bf16 over the first 64 columns of S
+      // ---- P = 2^(S c - m c) as packed bf16 over the first 64 columns of S, in two halves
       const float neg_ms = (m_ref == -INFINITY) ? 0.f : -m_ref * p.scale_log2;
-      l_run += full ? softmax_exp_row<false>(s_addr, p.scale_log2, neg_ms, kv0, lo, hi)
-                    : softmax_exp_row<true>(s_addr, p.scale_log2, neg_ms, kv0, lo, hi);
+      const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nm2 = f2_pack(neg_ms, neg_ms);
+      uint64_t sum0 = 0ull, sum1 = 0ull;   // (0.f, 0.f)
+      uint32_t pk[32];
+      exp_half(x0, x1, sc2, nm2, sum0, sum1, pk);
+      tmem_st_32x32(s_addr, pk);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[t]);
+      if (lane == 0) mbar_arrive(&p_full[2 * t]);
+      exp_half(x2, x3, sc2, nm2, sum0, sum1, pk);
+      tmem_st_32x32(s_addr + 32, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_full[2 * t + 1]);
+      float a, b2, c2, d2;
+      f2_unpack(sum0, a, b2);
+      f2_unpack(sum1, c2, d2);
+      l_run += (a + b2) + (c2 + d2);
     }
-    if (ok && n_t > 0) ok = __all_sync(0xffffffffu, mbar_wait(&o_full[t], 0, abort_flag, p.status));
+    if (ok && n_t > 0) ok = mbar_wait_warp(&o_full[t], 0, abort_flag, p.status);
     if (ok) {
       if (n_t > 0) tc_fence_after();
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       __nv_bfloat16* orow = p.O + (((long long)b * p.Sq + i) * p.Hq + h) * HD;
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
+      for (int cc = 0; cc < HD / 32; ++cc) {
         uint32_t tr[32];
         if (n_t > 0) {
           tmem_ld_32x32(o_addr + cc * 32, tr);
@@ -366,38 +386,43 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (warp == 1) { tc_fence_after(); tmem_dealloc<1>(tmem_base, 512); }
 }
 
-}  // namespace
-
-// Same contract as atb_flash_fwd (flash_attn.cu).
-extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_lo,
-                                const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
-                                long long k_stride, long long v_stride, int causal, float softmax_scale, void* stream,
-                                int* status) {
-  if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  if (Hq % Hkv) return -1;
-  if ((q_stride | k_stride | v_stride) & 7) return -1;
+template <int HD>
+int launch_fwd2(const void* q, const void* k, const void* v, const Params& p, long long q_stride, long long k_stride,
+                long long v_stride, cudaStream_t stream) {
   CUtensorMap tmQ, tmK, tmV;
-  if (!make_tmap_2d(&tmQ, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sq, (uint64_t)Hq * HD, q_stride, BQ,
-                    64, CU_TENSOR_MAP_SWIZZLE_128B))
-    return -2;
-  if (!make_tmap_2d(&tmK, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sk, (uint64_t)Hkv * HD, k_stride,
-                    BKV, 64, CU_TENSOR_MAP_SWIZZLE_128B))
-    return -2;
-  if (!make_tmap_2d(&tmV, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sk, (uint64_t)Hkv * HD, v_stride,
-                    BKV, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+  const auto bf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
+  if (!make_tmap_2d(&tmQ, q, bf16, 2, (uint64_t)p.B * p.Sq, (uint64_t)p.Hq * HD, q_stride, BQ, 64, sw) ||
+      !make_tmap_2d(&tmK, k, bf16, 2, (uint64_t)p.B * p.Sk, (uint64_t)p.Hkv * HD, k_stride, BKV, 64, sw) ||
+      !make_tmap_2d(&tmV, v, bf16, 2, (uint64_t)p.B * p.Sk, (uint64_t)p.Hkv * HD, v_stride, BKV, 64, sw))
     return -2;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_fwd2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L2::TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(flash_fwd2_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, L2<HD>::TOTAL) !=
+        cudaSuccess)
       return -4;
     attr_set = true;
   }
+  dim3 grid((p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B);
+  flash_fwd2_kernel<HD><<<grid, THREADS, L2<HD>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+}  // namespace
+
+// Same contract as atb_flash_fwd (flash_attn.cu), for a positive softmax_scale and head dim 128 or 64.
+extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_lo,
+                                const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
+                                long long k_stride, long long v_stride, int causal, float softmax_scale, void* stream,
+                                int* status, int head_dim) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
+  if (Hq % Hkv || (head_dim != 128 && head_dim != 64) || !(softmax_scale > 0.f)) return -1;
+  if ((q_stride | k_stride | v_stride) & 7) return -1;
   Params p;
   p.O = (__nv_bfloat16*)o; p.lse = lse; p.row_lo = row_lo; p.row_hi = row_hi;
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  dim3 grid((Sq + 2 * BQ - 1) / (2 * BQ), Hq, B);
-  flash_fwd2_kernel<<<grid, THREADS, L2::TOTAL, (cudaStream_t)stream>>>(tmQ, tmK, tmV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return head_dim == 64 ? launch_fwd2<64>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream)
+                        : launch_fwd2<128>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream);
 }

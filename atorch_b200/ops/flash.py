@@ -30,8 +30,9 @@ import os
 import weakref
 
 # forward kernel with two 128-row query tiles per CTA that share every K/V tile (csrc/flash_attn_v2.cu): the
-# default from 256 query rows on (measured 201 us against 256 us for the single-tile kernel at S=4096, H=32,
-# causal); ATB_FLASH_V2=0 keeps the single-tile kernel everywhere
+# default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 167 us against
+# 256 us for the single-tile kernel; at B=16, S=512, H=16, D=64 with padding: 53 us against 80 us); ATB_FLASH_V2=0
+# keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
 # backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch): measured 667 us
 # against 696 us for the single key-block kernel at S=4096, H=32, causal. ATB_FLASH_BWD_SPLIT=0 selects the latter.
@@ -255,16 +256,18 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     out = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
     L = _lib.lib()
-    # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences; the single-tile kernel otherwise
-    if D != 128:
+    # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences; the single-tile kernel otherwise, and for
+    # dropout, a bias, and a scale that is not positive (hidden scores are -inf before they are scaled)
+    if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0:
+        fwd, extra = L.atb_flash_fwd_v2, (ctypes.c_int(D),)
+    elif D != 128:
         fwd, extra = L.atb_flash_fwd_ex, _extra_args(drop, bias, D)      # single-tile kernel, head dim 64
     elif bias is not None:
         fwd, extra = L.atb_flash_fwd_bias, _extra_args(drop, bias)
     elif drop is not None:
         fwd, extra = L.atb_flash_fwd_dropout, _extra_args(drop, None)
     else:
-        fwd = L.atb_flash_fwd_v2 if (FWD_TWO_TILES and Sq >= 256 and L.has("atb_flash_fwd_v2")) else L.atb_flash_fwd
-        extra = ()
+        fwd, extra = L.atb_flash_fwd, ()
     rc = fwd(
         _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(row_lo), _lib.ptr(row_hi),
         ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk), ctypes.c_int(Hq), ctypes.c_int(Hkv),
