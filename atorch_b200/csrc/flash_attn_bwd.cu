@@ -106,7 +106,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* q_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [2]: first, last+1 q block
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   // a wait already ran out somewhere in this stream of work: do not start, so that a failing
   // launch ends after one wait limit instead of one per wave of CTAs
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
@@ -166,40 +166,42 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int qb0 = q_range[0], qb1 = q_range[1];
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int qb0 = warp_uniform(q_range[0]), qb1 = warp_uniform(q_range[1]);
   const int nblk = qb1 - qb0;
   const long long q_row_base = (long long)b * p.Sq;
   const long long k_row = (long long)b * p.Sk + kv0;
 
   if (warp == 0) {
-    if (lane == 0 && nblk > 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmdO);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmdQ);
+    if (nblk > 0) {
+      const bool el = elect_one();
+      if (el) tma_prefetch_desc(&tmQ);
+      if (el) tma_prefetch_desc(&tmdO);
+      if (el) tma_prefetch_desc(&tmK);
+      if (el) tma_prefetch_desc(&tmV);
+      if (el) tma_prefetch_desc(&tmdQ);
       constexpr int TILE_B = (HDIM / 64) * PANEL;   // bytes of a [128 x HDIM] tile
-      mbar_expect_tx(kv_full, 2 * TILE_B);
-      tma_load_2d(sK, &tmK, kv_full, hk * HDIM, (int)k_row);
-      if (HDIM == 128) tma_load_2d(sK + PANEL, &tmK, kv_full, hk * HDIM + 64, (int)k_row);
-      tma_load_2d(sV, &tmV, kv_full, hk * HDIM, (int)k_row);
-      if (HDIM == 128) tma_load_2d(sV + PANEL, &tmV, kv_full, hk * HDIM + 64, (int)k_row);
+      if (el) mbar_expect_tx(kv_full, 2 * TILE_B);
+      if (el) tma_load_2d(sK, &tmK, kv_full, hk * HDIM, (int)k_row);
+      if (HDIM == 128 && el) tma_load_2d(sK + PANEL, &tmK, kv_full, hk * HDIM + 64, (int)k_row);
+      if (el) tma_load_2d(sV, &tmV, kv_full, hk * HDIM, (int)k_row);
+      if (HDIM == 128 && el) tma_load_2d(sV + PANEL, &tmV, kv_full, hk * HDIM + 64, (int)k_row);
       for (int it = 0; it < nblk; ++it) {
         const int qs = it & 1;
         const int qrow = (int)(q_row_base + (long long)(qb0 + it) * BQ);
-        if (!mbar_wait(&q_free[qs], ((it >> 1) & 1) ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&q_full[qs], TILE_B);
-        tma_load_2d(sQ + qs * TILE, &tmQ, &q_full[qs], h * HDIM, qrow);
-        if (HDIM == 128) tma_load_2d(sQ + qs * TILE + PANEL, &tmQ, &q_full[qs], h * HDIM + 64, qrow);
-        if (!mbar_wait(do_free, (it & 1) ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(do_full, TILE_B);
-        tma_load_2d(sdO, &tmdO, do_full, h * HDIM, qrow);
-        if (HDIM == 128) tma_load_2d(sdO + PANEL, &tmdO, do_full, h * HDIM + 64, qrow);
+        if (!mbar_wait_warp(&q_free[qs], ((it >> 1) & 1) ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&q_full[qs], TILE_B);
+        if (el) tma_load_2d(sQ + qs * TILE, &tmQ, &q_full[qs], h * HDIM, qrow);
+        if (HDIM == 128 && el) tma_load_2d(sQ + qs * TILE + PANEL, &tmQ, &q_full[qs], h * HDIM + 64, qrow);
+        if (!mbar_wait_warp(do_free, (it & 1) ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(do_full, TILE_B);
+        if (el) tma_load_2d(sdO, &tmdO, do_full, h * HDIM, qrow);
+        if (HDIM == 128 && el) tma_load_2d(sdO + PANEL, &tmdO, do_full, h * HDIM + 64, qrow);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
+      const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t id_kk = umma_idesc(128, 128, 1, 1, false, false);
       constexpr uint32_t id_mm = umma_idesc(128, HDIM, 1, 1, true, true);     // dV, dK: [keys x d]
       constexpr uint32_t id_km = umma_idesc(128, HDIM, 1, 1, false, true);    // dQ: [queries x d]
@@ -207,61 +209,61 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
       // descriptors of every operand in the form(s) it is read in; the loops below only advance them
       // (scalars and selects: an array indexed at run time would live in local memory)
-      const uint64_t dQk0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), dQm0 = umma_desc_sw128(smem_u32(sQ), PANEL, 1024);
-      const uint64_t dKk = umma_desc_sw128(aK, 16, 1024), dKm = umma_desc_sw128(aK, PANEL, 1024);
-      const uint64_t dVk = umma_desc_sw128(aV, 16, 1024);
-      const uint64_t dOk = umma_desc_sw128(adO, 16, 1024), dOm = umma_desc_sw128(adO, PANEL, 1024);
-      const uint64_t dPm = umma_desc_sw128(aP, PANEL, 1024);
-      const uint64_t dSk = umma_desc_sw128(adS, 16, 1024), dSm = umma_desc_sw128(adS, PANEL, 1024);
+      const uint32_t dQk0 = umma_desc_lo(smem_u32(sQ), 16), dQm0 = umma_desc_lo(smem_u32(sQ), PANEL);
+      const uint32_t dKk = umma_desc_lo(aK, 16), dKm = umma_desc_lo(aK, PANEL);
+      const uint32_t dVk = umma_desc_lo(aV, 16);
+      const uint32_t dOk = umma_desc_lo(adO, 16), dOm = umma_desc_lo(adO, PANEL);
+      const uint32_t dPm = umma_desc_lo(aP, PANEL);
+      const uint32_t dSk = umma_desc_lo(adS, 16), dSm = umma_desc_lo(adS, PANEL);
       auto issue_s = [&](int it) -> bool {   // S(it) = Q(it) K^T over d
-        if (!mbar_wait(&q_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t qd = umma_desc_advance(dQk0, (it & 1) ? TILE : 0);
+        const uint32_t qd = dQk0 + (((it & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < HDIM / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tS, umma_desc_advance(qd, off), umma_desc_advance(dKk, off), id_kk, k != 0);
+          umma_ss_issue(tS, qd + (off >> 4), dKk + (off >> 4), id_kk, k != 0, el);
         }
-        umma_commit(s_full);
+        umma_commit_issue(s_full, el);
         return true;
       };
       auto issue_dp = [&](int it) -> bool {  // dP(it) = dO(it) V^T over d
-        if (!mbar_wait(do_full, it & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(do_full, it & 1, abort_flag, p.status)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < HDIM / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tdP, umma_desc_advance(dOk, off), umma_desc_advance(dVk, off), id_kk, k != 0);
+          umma_ss_issue(tdP, dOk + (off >> 4), dVk + (off >> 4), id_kk, k != 0, el);
         }
-        umma_commit(dp_full);
+        umma_commit_issue(dp_full, el);
         return true;
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status);
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status);
       ok = ok && issue_s(0) && issue_dp(0);
       for (int it = 0; ok && it < nblk; ++it) {
-        if (!mbar_wait(pds_full, it & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(pds_full, it & 1, abort_flag, p.status)) break;
         tc_fence_after();
         if (it + 1 < nblk && !issue_s(it + 1)) break;
-        const uint64_t qm = umma_desc_advance(dQm0, (it & 1) ? TILE : 0);
+        const uint32_t qm = dQm0 + (((it & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k)  // dV += P^T dO over q
-          umma_f16<1>(tdV, umma_desc_advance(dPm, k * 2048), umma_desc_advance(dOm, k * 2048), id_mm, (it | k) != 0);
-        umma_commit(do_free);
+          umma_ss_issue(tdV, dPm + k * 128, dOm + k * 128, id_mm, (it | k) != 0, el);
+        umma_commit_issue(do_free, el);
 #pragma unroll
         for (int k = 0; k < 8; ++k)  // dK += dS^T Q over q
-          umma_f16<1>(tdK, umma_desc_advance(dSm, k * 2048), umma_desc_advance(qm, k * 2048), id_mm, (it | k) != 0);
-        umma_commit(&q_free[it & 1]);
+          umma_ss_issue(tdK, dSm + k * 128, qm + k * 128, id_mm, (it | k) != 0, el);
+        umma_commit_issue(&q_free[it & 1], el);
         if constexpr (WITH_DQ) {
 #pragma unroll
           for (int k = 0; k < 8; ++k) {  // dQ = dS K over keys (into the dP columns)
             const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-            umma_f16<1>(tdP, umma_desc_advance(dSk, off), umma_desc_advance(dKm, k * 2048), id_km, k != 0);
+            umma_ss_issue(tdP, dSk + (off >> 4), dKm + k * 128, id_km, k != 0, el);
           }
         }
-        umma_commit(dq_full);
+        umma_commit_issue(dq_full, el);
         if (it + 1 < nblk) {
           if constexpr (WITH_DQ) {
-            if (!mbar_wait(dp_free, it & 1, abort_flag, p.status)) break;
+            if (!mbar_wait_warp(dp_free, it & 1, abort_flag, p.status)) break;
             tc_fence_after();
           }
           if (!issue_dp(it + 1)) break;
@@ -303,7 +305,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     uint8_t* stage = sP;
     const bool reducer = threadIdx.x == 64;     // first element-wise thread issues the TMA operations
     auto drain_dq = [&](int it) -> bool {
-      if (!__all_sync(0xffffffffu, mbar_wait(dq_full, it & 1, abort_flag, p.status))) return false;
+      if (!mbar_wait_warp(dq_full, it & 1, abort_flag, p.status)) return false;
       if constexpr (!WITH_DQ) return true;   // the products that read P and dS have completed: nothing to move
       tc_fence_after();
       // this thread's HDIM / 2 columns of dQ: boxes (2 half, 2 half + 1) for 128, box `half` for 64
@@ -349,7 +351,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // warp-uniform, so that the per-element interval tests are a separate path that full tiles never enter
       const bool row_full = __all_sync(0xffffffffu, cur.valid && cur.lo <= kv0 && cur.hi >= kv0 + BKV);
       // ---- P(it) = exp2(S c - lse): runs while the tensor core accumulates dV, dK and forms dQ of block it-1
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, it & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       float pv[64];
       {
@@ -396,10 +398,10 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ---- dQ(it-1) out of the dP columns, which frees them for dP(it)
       if (it > 0 && !drain_dq(it - 1)) { ok = false; break; }
       // ---- dS(it) = P (dP - delta) scale; P and dS to shared memory (free: dq_full(it-1) has been waited for)
-      if (!__all_sync(0xffffffffu, mbar_wait(dp_full, it & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(dp_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       // P and dS share their memory with the staged dQ(it-1): wait until the TMA unit has read it
       if (WITH_DQ && it > 0 &&
-          !__all_sync(0xffffffffu, mbar_wait(stage_free, (it - 1) & 1, abort_flag, p.status))) {
+          !mbar_wait_warp(stage_free, (it - 1) & 1, abort_flag, p.status)) {
         ok = false;
         break;
       }

@@ -87,7 +87,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* q_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [2]: first, last+1 q block
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
   const int kb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int hk = h / (p.Hq / p.Hkv);
@@ -143,15 +143,16 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int qb0 = q_range[0], nblk = q_range[1] - q_range[0];
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int qb0 = warp_uniform(q_range[0]), nblk = warp_uniform(q_range[1]) - qb0;
   const long long q_row_base = (long long)b * p.Sq;
   const long long k_row = (long long)b * p.Sk + kv0;
   const uint32_t tSt = tmem_base, tdPt = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 384;
 
   if (warp == 0) {
     if (nblk > 0) {
-      if (lane == 0) {
+      const bool el = elect_one();
+      if (el) {
         tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
         mbar_expect_tx(kv_full, 2 * TILE);
         tma_load_2d(sK, &tmK, kv_full, hk * HD, (int)k_row);
@@ -163,16 +164,12 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const int st = it & 1;
         const uint32_t ph = ((it >> 1) & 1) ^ 1;
         const int qrow = (int)(q_row_base + (long long)(qb0 + it) * BQ);
-        bool ok = true;
-        if (lane == 0) {
-          ok = mbar_wait(&q_free[st], ph, abort_flag, p.status);
-          if (ok) {
-            mbar_expect_tx(&q_full[st], TILE);
-            tma_load_2d(sQ + st * TILE, &tmQ, &q_full[st], h * HD, qrow);
-            tma_load_2d(sQ + st * TILE + PANEL, &tmQ, &q_full[st], h * HD + 64, qrow);
-          }
+        if (!mbar_wait_warp(&q_free[st], ph, abort_flag, p.status)) break;
+        if (el) {
+          mbar_expect_tx(&q_full[st], TILE);
+          tma_load_2d(sQ + st * TILE, &tmQ, &q_full[st], h * HD, qrow);
+          tma_load_2d(sQ + st * TILE + PANEL, &tmQ, &q_full[st], h * HD + 64, qrow);
         }
-        if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
         // row values of this query block (the stage is free: q_free covers its previous user)
         RowVals& rv = rows[st];
 #pragma unroll
@@ -196,70 +193,68 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           rv.neg_lse2[r] = nl; rv.neg_delta[r] = nd; rv.lo[r] = lo; rv.hi[r] = hi;
         }
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&rows_full[st]);
-          ok = mbar_wait(&do_free[st], ph, abort_flag, p.status);
-          if (ok) {
-            mbar_expect_tx(&do_full[st], TILE);
-            tma_load_2d(sdO + st * TILE, &tmdO, &do_full[st], h * HD, qrow);
-            tma_load_2d(sdO + st * TILE + PANEL, &tmdO, &do_full[st], h * HD + 64, qrow);
-          }
+        if (el) mbar_arrive(&rows_full[st]);
+        if (!mbar_wait_warp(&do_free[st], ph, abort_flag, p.status)) break;
+        if (el) {
+          mbar_expect_tx(&do_full[st], TILE);
+          tma_load_2d(sdO + st * TILE, &tmdO, &do_full[st], h * HD, qrow);
+          tma_load_2d(sdO + st * TILE + PANEL, &tmdO, &do_full[st], h * HD + 64, qrow);
         }
-        if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
+      const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t id_kk = umma_idesc(128, 128, 1, 1, false, false);
       constexpr uint32_t id_km = umma_idesc(128, 128, 1, 1, false, true);
-      const uint64_t dKk = umma_desc_sw128(smem_u32(sK), 16, 1024), dVk = umma_desc_sw128(smem_u32(sV), 16, 1024);
-      const uint64_t dQk0 = umma_desc_sw128(smem_u32(sQ), 16, 1024), dQm0 = umma_desc_sw128(smem_u32(sQ), PANEL, 1024);
-      const uint64_t dOk0 = umma_desc_sw128(smem_u32(sdO), 16, 1024), dOm0 = umma_desc_sw128(smem_u32(sdO), PANEL, 1024);
+      const uint32_t dKk = umma_desc_lo(smem_u32(sK), 16), dVk = umma_desc_lo(smem_u32(sV), 16);
+      const uint32_t dQk0 = umma_desc_lo(smem_u32(sQ), 16), dQm0 = umma_desc_lo(smem_u32(sQ), PANEL);
+      const uint32_t dOk0 = umma_desc_lo(smem_u32(sdO), 16), dOm0 = umma_desc_lo(smem_u32(sdO), PANEL);
       auto issue_st = [&](int it) -> bool {   // S^T(it) = K Q(it)^T
-        if (!mbar_wait(&q_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&q_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t qd = umma_desc_advance(dQk0, (it & 1) ? TILE : 0);
+        const uint32_t qd = dQk0 + (((it & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tSt, umma_desc_advance(dKk, off), umma_desc_advance(qd, off), id_kk, k != 0);
+          umma_ss_issue(tSt, dKk + (off >> 4), qd + (off >> 4), id_kk, k != 0, el);
         }
-        umma_commit(st_full);
+        umma_commit_issue(st_full, el);
         return true;
       };
       auto issue_dpt = [&](int it) -> bool {  // dP^T(it) = V dO(it)^T
-        if (!mbar_wait(&do_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&do_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t od = umma_desc_advance(dOk0, (it & 1) ? TILE : 0);
+        const uint32_t od = dOk0 + (((it & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tdPt, umma_desc_advance(dVk, off), umma_desc_advance(od, off), id_kk, k != 0);
+          umma_ss_issue(tdPt, dVk + (off >> 4), od + (off >> 4), id_kk, k != 0, el);
         }
-        umma_commit(dpt_full);
+        umma_commit_issue(dpt_full, el);
         return true;
       };
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.status);
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.status);
       ok = ok && issue_st(0) && issue_dpt(0);
       for (int it = 0; ok && it < nblk; ++it) {
         const int st = it & 1;
-        if (!mbar_wait(p_full, it & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(p_full, it & 1, abort_flag, p.status)) break;
         tc_fence_after();
-        const uint64_t om = umma_desc_advance(dOm0, st ? TILE : 0);
+        const uint32_t om = dOm0 + ((st ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // dV += P^T dO(it): 16 queries per step = 8 TMEM columns of packed bf16
-          umma_f16_ts(tdV, tSt + k * 8, umma_desc_advance(om, k * 2048), id_km, (it | k) != 0);
-        umma_commit(&do_free[st]);
+          umma_ts_issue(tdV, tSt + k * 8, om + k * 128, id_km, (it | k) != 0, el);
+        umma_commit_issue(&do_free[st], el);
         if (it + 1 < nblk && !issue_st(it + 1)) break;
-        if (!mbar_wait(ds_full, it & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(ds_full, it & 1, abort_flag, p.status)) break;
         tc_fence_after();
-        const uint64_t qm = umma_desc_advance(dQm0, st ? TILE : 0);
+        const uint32_t qm = dQm0 + ((st ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // dK += dS^T Q(it)
-          umma_f16_ts(tdK, tdPt + k * 8, umma_desc_advance(qm, k * 2048), id_km, (it | k) != 0);
-        umma_commit(&q_free[st]);
+          umma_ts_issue(tdK, tdPt + k * 8, qm + k * 128, id_km, (it | k) != 0, el);
+        umma_commit_issue(&q_free[st], el);
         if (it + 1 < nblk && !issue_dpt(it + 1)) break;
-        if (it == nblk - 1) umma_commit(acc_full);
+        if (it == nblk - 1) umma_commit_issue(acc_full, el);
       }
     }
   } else {
@@ -275,9 +270,9 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int i0 = (qb0 + it) * BQ;             // first query row of the block
       // every query of the block sees every key of this block: no per-element tests (warp-uniform)
       const bool full = analytic && (!p.causal || i0 + shift + 1 >= kv0 + BKV) && (kv0 + BKV <= p.Sk);
-      if (!__all_sync(0xffffffffu, mbar_wait(&rows_full[it & 1], (it >> 1) & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(&rows_full[it & 1], (it >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
       // ---- P^T(it) = exp2(S^T c - lse[q])
-      if (!__all_sync(0xffffffffu, mbar_wait(st_full, it & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(st_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       float pv[64];
       {
@@ -309,7 +304,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
         for (int c = 0; c < 64; c += 2) pk[c >> 1] = pack_bf16x2(pv[c], pv[c + 1]);
         // the other half's thread of this key row must hold its S^T before these columns are overwritten
-        if (!__all_sync(0xffffffffu, mbar_wait(&pair_a[quarter], it & 1, abort_flag, p.status))) { ok = false; break; }
+        if (!mbar_wait_warp(&pair_a[quarter], it & 1, abort_flag, p.status)) { ok = false; break; }
         tmem_st_32x32(tSt + lane_addr + half * 32, pk);   // queries [64h, 64h+64) as packed bf16: columns [32h, 32h+32)
         tmem_st_wait();
       }
@@ -317,7 +312,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
       // ---- dS^T(it) = P^T (dP^T - delta[q]) scale
-      if (!__all_sync(0xffffffffu, mbar_wait(dpt_full, it & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(dpt_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       {
         uint32_t d0[32], d1[32];
@@ -340,7 +335,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           dk_[c >> 1] = pack_bf16x2(x0, x1);
           dk_[16 + (c >> 1)] = pack_bf16x2(y0, y1);
         }
-        if (!__all_sync(0xffffffffu, mbar_wait(&pair_c[quarter], it & 1, abort_flag, p.status))) { ok = false; break; }
+        if (!mbar_wait_warp(&pair_c[quarter], it & 1, abort_flag, p.status)) { ok = false; break; }
         tmem_st_32x32(tdPt + lane_addr + half * 32, dk_);
         tmem_st_wait();
       }
@@ -351,7 +346,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // dV / dK of this key block: TMEM lane = key row. tcgen05.ld is a warp-wide (.sync.aligned) instruction:
     // every lane executes it, only the global stores are predicated per row.
     ok = __all_sync(0xffffffffu, ok);
-    if (ok && nblk > 0) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.status));
+    if (ok && nblk > 0) ok = mbar_wait_warp(acc_full, 0, abort_flag, p.status);
     if (ok) {
       const bool store = kk < p.Sk;
       __nv_bfloat16* dvrow = p.dv + ((long long)b * p.Sk + kk) * p.dkv_stride + h * HD + half * 64;

@@ -75,7 +75,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [4]: t0, t1, full_lo, full_hi
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
   const int qb = gridDim.x - 1 - blockIdx.x;  // heaviest (last) causal blocks first
   const int h = blockIdx.y, b = blockIdx.z;
@@ -129,82 +129,84 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int t0 = kv_range[0], n = kv_range[1] - kv_range[0];
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int t0 = warp_uniform(kv_range[0]), n = warp_uniform(kv_range[1]) - t0;
   const int full_lo = kv_range[2], full_hi = kv_range[3];
   const long long q_row0 = (long long)b * p.Sq + q0;
   const long long k_row0 = (long long)b * p.Sk;
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 384;   // dP buffer j&1 at tdP + 128*(j&1)
 
   if (warp == 0) {
-    if (lane == 0 && n > 0) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-      mbar_expect_tx(qdo_full, 2 * TILE);
-      tma_load_2d(sQ, &tmQ, qdo_full, h * HD, (int)q_row0);
-      tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, (int)q_row0);
-      tma_load_2d(sdO, &tmdO, qdo_full, h * HD, (int)q_row0);
-      tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, (int)q_row0);
+    if (n > 0) {
+      const bool el = elect_one();
+      if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
+      if (el) mbar_expect_tx(qdo_full, 2 * TILE);
+      if (el) tma_load_2d(sQ, &tmQ, qdo_full, h * HD, (int)q_row0);
+      if (el) tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, (int)q_row0);
+      if (el) tma_load_2d(sdO, &tmdO, qdo_full, h * HD, (int)q_row0);
+      if (el) tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, (int)q_row0);
       for (int j = 0; j < n; ++j) {
         const int ks = j % K_STAGES, vs = j % V_STAGES;
         const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
-        if (!mbar_wait(&k_empty[ks], ((j / K_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&k_full[ks], TILE);
-        tma_load_2d(sK + ks * TILE, &tmK, &k_full[ks], hk * HD, krow);
-        tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
-        if (!mbar_wait(&v_empty[vs], ((j / V_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&v_full[vs], TILE);
-        tma_load_2d(sV + vs * TILE, &tmV, &v_full[vs], hk * HD, krow);
-        tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
+        if (!mbar_wait_warp(&k_empty[ks], ((j / K_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&k_full[ks], TILE);
+        if (el) tma_load_2d(sK + ks * TILE, &tmK, &k_full[ks], hk * HD, krow);
+        if (el) tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
+        if (!mbar_wait_warp(&v_empty[vs], ((j / V_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&v_full[vs], TILE);
+        if (el) tma_load_2d(sV + vs * TILE, &tmV, &v_full[vs], hk * HD, krow);
+        if (el) tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n > 0) {
+    if (n > 0) {
+      const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t id_kk = umma_idesc(128, 128, 1, 1, false, false);
       constexpr uint32_t id_km = umma_idesc(128, 128, 1, 1, false, true);
-      const uint64_t dQk = umma_desc_sw128(smem_u32(sQ), 16, 1024), dOk = umma_desc_sw128(smem_u32(sdO), 16, 1024);
-      const uint64_t dKk0 = umma_desc_sw128(smem_u32(sK), 16, 1024), dKm0 = umma_desc_sw128(smem_u32(sK), PANEL, 1024);
-      const uint64_t dVk0 = umma_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint32_t dQk = umma_desc_lo(smem_u32(sQ), 16), dOk = umma_desc_lo(smem_u32(sdO), 16);
+      const uint32_t dKk0 = umma_desc_lo(smem_u32(sK), 16), dKm0 = umma_desc_lo(smem_u32(sK), PANEL);
+      const uint32_t dVk0 = umma_desc_lo(smem_u32(sV), 16);
       // S(j) = Q K_j^T and dP(j) = dO V_j^T
       auto issue_sdp = [&](int j) -> bool {
         const int ks = j % K_STAGES, vs = j % V_STAGES;
-        if (!mbar_wait(&k_full[ks], (j / K_STAGES) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&k_full[ks], (j / K_STAGES) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t kd = umma_desc_advance(dKk0, ks * TILE);
+        const uint32_t kd = dKk0 + ((ks * TILE) >> 4);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tS, umma_desc_advance(dQk, off), umma_desc_advance(kd, off), id_kk, k != 0);
+          umma_ss_issue(tS, dQk + (off >> 4), kd + (off >> 4), id_kk, k != 0, el);
         }
-        if (!mbar_wait(&v_full[vs], (j / V_STAGES) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&v_full[vs], (j / V_STAGES) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint64_t vd = umma_desc_advance(dVk0, vs * TILE);
+        const uint32_t vd = dVk0 + ((vs * TILE) >> 4);
         const uint32_t dst = tdP + 128 * (j & 1);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(dst, umma_desc_advance(dOk, off), umma_desc_advance(vd, off), id_kk, k != 0);
+          umma_ss_issue(dst, dOk + (off >> 4), vd + (off >> 4), id_kk, k != 0, el);
         }
-        umma_commit(sdp_full);
-        umma_commit(&v_empty[vs]);
+        umma_commit_issue(sdp_full, el);
+        umma_commit_issue(&v_empty[vs], el);
         return true;
       };
-      bool ok = mbar_wait(qdo_full, 0, abort_flag, p.status);
+      bool ok = mbar_wait_warp(qdo_full, 0, abort_flag, p.status);
       ok = ok && issue_sdp(0);
       for (int j = 0; ok && j < n; ++j) {
         if (j + 1 < n) {
-          if (!mbar_wait(s_free, j & 1, abort_flag, p.status)) break;
+          if (!mbar_wait_warp(s_free, j & 1, abort_flag, p.status)) break;
           tc_fence_after();
           if (!issue_sdp(j + 1)) break;
         }
-        if (!mbar_wait(ds_full, j & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(ds_full, j & 1, abort_flag, p.status)) break;
         tc_fence_after();
-        const uint64_t km = umma_desc_advance(dKm0, (j % K_STAGES) * TILE);
+        const uint32_t km = dKm0 + (((j % K_STAGES) * TILE) >> 4);
         const uint32_t a = tdP + 128 * (j & 1);
 #pragma unroll
         for (int k = 0; k < 8; ++k)   // dQ += dS K_j: 16 keys per step = 8 TMEM columns of packed bf16
-          umma_f16_ts(tdQ, a + k * 8, umma_desc_advance(km, k * 2048), id_km, (j | k) != 0);
-        umma_commit(&k_empty[j % K_STAGES]);
-        if (j == n - 1) umma_commit(dq_full);
+          umma_ts_issue(tdQ, a + k * 8, km + k * 128, id_km, (j | k) != 0, el);
+        umma_commit_issue(&k_empty[j % K_STAGES], el);
+        if (j == n - 1) umma_commit_issue(dq_full, el);
       }
     }
   } else {
@@ -236,7 +238,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int j = 0; j < n; ++j) {
       const int kv0 = (t0 + j) * BKV;
       const uint32_t dp_addr = tdP + 128 * (j & 1) + lane_addr;
-      if (!__all_sync(0xffffffffu, mbar_wait(sdp_full, j & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(sdp_full, j & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       uint32_t s0[32], s1[32], d0[32], d1[32];
       tmem_ld_32x32(tS + lane_addr + half * 64, s0);
@@ -252,7 +254,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       // both threads of every row of this lane quarter hold their S and dP before either stores dS (a bounded
       // mbarrier wait, not a named barrier, so that a warp whose partner gave up cannot wait forever)
-      if (!__all_sync(0xffffffffu, mbar_wait(&pair_bar[quarter], j & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(&pair_bar[quarter], j & 1, abort_flag, p.status)) { ok = false; break; }
       // tiles inside the intersection of the rows' intervals run without per-element tests
       const bool tile_full = (kv0 >= full_lo) && (kv0 + BKV <= full_hi);
       const int c0 = kv0 + half * 64;
@@ -289,7 +291,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (lane == 0) mbar_arrive(ds_full);
     }
     ok = __all_sync(0xffffffffu, ok);
-    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(dq_full, 0, abort_flag, p.status));
+    if (ok && n > 0) ok = mbar_wait_warp(dq_full, 0, abort_flag, p.status);
     if (ok) {
       if (n > 0) tc_fence_after();
       __nv_bfloat16* row = p.dq + ((long long)b * p.Sq + i) * p.dq_stride + h * HD + half * 64;
