@@ -169,7 +169,8 @@ struct Sched {
 ATB_DEVICE void st_remote_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
-// Wait on a barrier whose phase is completed by an arrive of another CTA of the cluster that published data with it.
+// Wait (by a whole converged warp, one answer for all lanes) on a barrier whose phase is completed by an arrive of
+// another CTA of the cluster that published data with it.
 ATB_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
   uint64_t t0 = 0;
   uint32_t spins = 0;
@@ -184,15 +185,16 @@ ATB_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* 
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
     if ((++spins & 0x3ff) == 0) {
-      if (t0 == 0) t0 = globaltimer_ns();
-      if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > ATB_WAIT_LIMIT_NS) {
+      const uint64_t now = warp_uniform(globaltimer_ns());
+      if (t0 == 0) t0 = now;
+      const bool late = now - t0 > ATB_WAIT_LIMIT_NS;
+      if (late) {
         *abort_flag = 1;
         if (status) atomicCAS(status, 0, (int)ATB_ERR_WAIT_TIMEOUT);
-        return false;
       }
+      if (__any_sync(0xffffffffu, late || *abort_flag != 0)) return false;
     }
   }
 }
@@ -222,11 +224,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* tq_tile = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [TQ] tile ids (-1: no more tiles)
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const uint32_t rank = warp_uniform(cluster_ctarank());
   const bool leader = rank == 0;
   // both CTAs of a pair read the same word, so they take the same decision
-  const bool skip = status != nullptr && *reinterpret_cast<volatile int*>(status) != 0;
+  const bool skip = warp_uniform((int)(status != nullptr && *reinterpret_cast<volatile int*>(status) != 0)) != 0;
 
   const int tiles_m = rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM);
   const int tile_cols = ep.gated ? BN / 2 : BN;      // output columns per tile
@@ -263,7 +265,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   tc_fence_before();
   cluster_sync_all();  // barriers of both CTAs initialised and visible before any remote arrive
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   // identical decisions in every role: which tiles and which k-blocks carry data
   auto tile_active = [&](int m0) -> bool {
@@ -325,36 +327,45 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int t = cluster_id + idx * num_clusters;
     return t < num_tiles ? t : -1;
   };
-  auto publish_tile = [&](int idx, int t) -> bool {          // leader's producer thread
+  auto publish_tile = [&](int idx, int t) -> bool {          // leader's producer warp
     const int slot = idx % TQ;
-    if (!mbar_wait(&tq_empty[slot], ((idx / TQ) & 1) ^ 1, abort_flag, status)) return false;
-    tq_tile[slot] = t;
-    st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), 1), (uint32_t)t);
-    mbar_arrive(&tq_full[slot]);
-    mbar_arrive_remote(map_to_cta(&tq_full[slot], 1));       // release.cluster: orders the store above
+    if (!mbar_wait_warp(&tq_empty[slot], ((idx / TQ) & 1) ^ 1, abort_flag, status)) return false;
+    if (lane == 0) {
+      tq_tile[slot] = t;
+      st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), 1), (uint32_t)t);
+      mbar_arrive(&tq_full[slot]);
+      mbar_arrive_remote(map_to_cta(&tq_full[slot], 1));     // release.cluster: orders the store above
+    }
     return true;
   };
-  auto read_tile = [&](int idx) -> int {                      // any other role (one thread, or all lanes of a warp)
+  auto read_tile = [&](int idx) -> int {                      // any other role, a whole warp
     if (!dyn) return static_tile(idx);
     const int slot = idx % TQ;
     if (!mbar_wait_cluster(&tq_full[slot], (idx / TQ) & 1, abort_flag, status)) return -1;
-    return tq_tile[slot];
+    return warp_uniform((int)tq_tile[slot]);
   };
-  auto free_tile_slot = [&](int idx) {                        // one thread per consumer, after read_tile
-    if (dyn) mbar_arrive_remote(map_to_cta(&tq_empty[idx % TQ], 0));
+  auto free_tile_slot = [&](int idx) {                        // once per consumer warp, after read_tile by all its lanes
+    __syncwarp();
+    if (dyn && lane == 0) mbar_arrive_remote(map_to_cta(&tq_empty[idx % TQ], 0));
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    {
       uint32_t it = 0;
-      int drawn = (dyn && leader) ? atomicAdd(&sched.counters[0], 1) : 0;
+      // lane 0 draws, all lanes know the number
+      auto draw = [&]() -> int {
+        int d = 0;
+        if (lane == 0) d = atomicAdd(&sched.counters[0], 1);
+        return warp_uniform(d);
+      };
+      int drawn = (dyn && leader) ? draw() : 0;
       for (int idx = 0;; ++idx) {
         int tile;
         if (dyn && leader) {
           tile = drawn < num_tiles ? drawn : -1;
-          if (tile >= 0) drawn = atomicAdd(&sched.counters[0], 1);     // the next one, fetched under this tile's loads
+          if (tile >= 0) drawn = draw();                       // the next one, fetched under this tile's loads
           if (!publish_tile(idx, tile)) goto producer_done;
-          if (tile < 0) {      // every pair draws exactly one number past the end; the last pair to do so resets
+          if (tile < 0 && lane == 0) {   // every pair draws exactly one number past the end; the last to do so resets
             if (atomicAdd(&sched.counters[1], 1) == num_clusters - 1) {
               sched.counters[0] = 0;
               sched.counters[1] = 0;
@@ -375,31 +386,35 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int bn0 = ep.gated ? n0 + (int)rank * N : n0 + (int)rank * BNH + (B_MN ? 0 : bshift);
         const int bk0 = B_MN ? bshift : 0;
         if (gate.flags != nullptr) {
-          const bool here = gate.on_b ? gate_wait(gate, min(bn0, N - 1), min(bn0 + BNH, N), abort_flag, status)
-                                      : gate_wait(gate, am0, min(am0 + BM, M), abort_flag, status);
-          if (!here) goto producer_done;
+          bool here = true;
+          if (lane == 0)
+            here = gate.on_b ? gate_wait(gate, min(bn0, N - 1), min(bn0 + BNH, N), abort_flag, status)
+                             : gate_wait(gate, am0, min(am0 + BM, M), abort_flag, status);
+          if (!__all_sync(0xffffffffu, here)) goto producer_done;
         }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!kb_active(kb)) continue;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, status)) goto producer_done;
-          if (leader) mbar_expect_tx(&full[s], 2 * (A_BYTES + B_BYTES));
-          const uint32_t bar = map_to_cta(&full[s], 0);
-          uint8_t* a_dst = sA + s * A_BYTES;
-          uint8_t* b_dst = sB + s * B_BYTES;
-          if constexpr (!A_MN) {
-            tma_load_2d_pair(a_dst, &tmA, bar, kb * BK, am0);
-          } else {
+          if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, status)) goto producer_done;
+          if (lane == 0) {
+            if (leader) mbar_expect_tx(&full[s], 2 * (A_BYTES + B_BYTES));
+            const uint32_t bar = map_to_cta(&full[s], 0);
+            uint8_t* a_dst = sA + s * A_BYTES;
+            uint8_t* b_dst = sB + s * B_BYTES;
+            if constexpr (!A_MN) {
+              tma_load_2d_pair(a_dst, &tmA, bar, kb * BK, am0);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(a_dst + j * 8192, &tmA, bar, am0 + j * 64, kb * BK);
-          }
-          if constexpr (!B_MN) {
-            tma_load_2d_pair(b_dst, &tmB, bar, kb * BK, bn0);
-          } else {
+              for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(a_dst + j * 8192, &tmA, bar, am0 + j * 64, kb * BK);
+            }
+            if constexpr (!B_MN) {
+              tma_load_2d_pair(b_dst, &tmB, bar, kb * BK, bn0);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BNH / 64; ++j)
-              tma_load_2d_pair(b_dst + j * 8192, &tmB, bar, bn0 + j * 64, bk0 + kb * BK);
+              for (int j = 0; j < BNH / 64; ++j)
+                tma_load_2d_pair(b_dst + j * 8192, &tmB, bar, bn0 + j * 64, bk0 + kb * BK);
+            }
           }
           ++it;
         }
@@ -407,7 +422,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   producer_done:;
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const uint32_t el = elect_one();      // the lane that issues and commits
+      const uint32_t a_desc = umma_desc_lo(smem_u32(sA), A_MN ? 8192 : 16), b_desc = umma_desc_lo(smem_u32(sB), B_MN ? 8192 : 16);
+      const uint32_t empty0 = smem_u32(empty), empty1 = map_to_cta(empty, 1), tfull0 = smem_u32(tfull), tfull1 = map_to_cta(tfull, 1);
       constexpr uint32_t idesc = umma_idesc(2 * BM, BN, 1, 1, A_MN, B_MN);
       uint32_t it = 0;
       int local = 0;
@@ -422,7 +440,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
         const int acc = local & 1;
         const uint32_t acc_ph = (local >> 1) & 1;
-        if (!mbar_wait(&tempty[acc], acc_ph ^ 1, abort_flag, status)) goto mma_done;
+        if (!mbar_wait_warp(&tempty[acc], acc_ph ^ 1, abort_flag, status)) goto mma_done;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         bool first_kb = true;
@@ -430,25 +448,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (!kb_active(kb)) continue;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(&full[s], ph, abort_flag, status)) goto mma_done;
+          if (!mbar_wait_warp(&full[s], ph, abort_flag, status)) goto mma_done;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + s * A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + s * B_BYTES);
+          const uint32_t a_s = a_desc + ((s * A_BYTES) >> 4), b_s = b_desc + ((s * B_BYTES) >> 4);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t adesc = A_MN ? umma_desc_sw128(a_addr + k * 2048, 8192, 1024)
-                                        : umma_desc_sw128(a_addr + k * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_desc_sw128(b_addr + k * 2048, 8192, 1024)
-                                        : umma_desc_sw128(b_addr + k * 32, 16, 1024);
-            umma_f16<2>(d_tmem, adesc, bdesc, idesc, (first_kb && k == 0) ? 0u : 1u);
-          }
+          for (int k = 0; k < BK / 16; ++k)   // 16 elements of the reduction: 16 rows MN-major, 32 bytes of a row K-major
+            umma_ss_issue<2>(d_tmem, a_s + k * (A_MN ? 128 : 2), b_s + k * (B_MN ? 128 : 2), idesc,
+                             (first_kb && k == 0) ? 0u : 1u, el);
           first_kb = false;
-          umma_commit_cg2(smem_u32(&empty[s]));
-          umma_commit_cg2(map_to_cta(&empty[s], 1));
+          umma_commit_cg2_issue(empty0 + s * 8, el);
+          umma_commit_cg2_issue(empty1 + s * 8, el);
           ++it;
         }
-        umma_commit_cg2(smem_u32(&tfull[acc]));
-        umma_commit_cg2(map_to_cta(&tfull[acc], 1));
+        umma_commit_cg2_issue(tfull0 + acc * 8, el);
+        umma_commit_cg2_issue(tfull1 + acc * 8, el);
         ++local;
       }
     }
@@ -458,9 +471,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     int local = 0;
     const uint32_t tempty_leader[2] = {map_to_cta(&tempty[0], 0), map_to_cta(&tempty[1], 0)};
     for (int idx = 0;; ++idx) {
-      const int tile = __shfl_sync(0xffffffffu, read_tile(idx), 0);
-      __syncwarp();
-      if (lane == 0) free_tile_slot(idx);
+      const int tile = read_tile(idx);
+      free_tile_slot(idx);
       if (tile < 0) break;
       int m0, n0, m_end, b_idx;
       tile_coords(tile, m0, n0, m_end, b_idx);
@@ -484,7 +496,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       const int acc = local & 1;
       const uint32_t acc_ph = (local >> 1) & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(&tfull[acc], acc_ph, abort_flag, status))) break;
+      if (!mbar_wait_warp(&tfull[acc], acc_ph, abort_flag, status)) break;
       tc_fence_after();
       const int row = m0 + (int)rank * BM + q * 32 + lane;
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
