@@ -448,6 +448,13 @@ ATB_DEVICE float block_max(float v, float* red) {
   return t;
 }
 
+// 32-byte global store (32-byte aligned): one whole sector per thread.
+ATB_DEVICE void stg_v8(void* p, const uint32_t* r) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+
 // Two fp32 values in one 64-bit register and the packed arithmetic of sm_100 on them: one instruction
 // does two fused multiply-adds (or adds), which halves the issue slots of element-wise fp32 work.
 ATB_DEVICE uint64_t f2_pack(float a, float b) {
