@@ -1,4 +1,5 @@
-// Flash attention backward for sm_100a (head dim 128, bf16), tcgen05 + TMEM + TMA.
+// Flash attention backward in one kernel for sm_100a (head dim 128 or 64, bf16; dropout, additive bias), tcgen05 + TMEM
+// + TMA. Without dropout and bias the two kernels of flash_attn_bwd_dkv.cu and flash_attn_bwd_dq.cu are the default.
 //
 // One CTA per (128 keys, head, batch) walks the query blocks that can see its keys. Per query block:
 //   S  = Q K^T,  dP = dO V^T                      2 x tcgen05.mma -> TMEM   (K-major operands)
@@ -72,10 +73,8 @@ struct RowInfo {
   float lse2, delta;
 };
 
-// WITH_DQ = false: key/value gradients only (the query gradient then comes from flash_attn_bwd_dq.cu): the
-// dQ product, its staging and the reduce-add are compiled out and dP(i+1) follows dK(i) without a hand-shake.
 // HDIM = 128 or 64 (64: one 64-column panel per Q / dO / K / V tile, 64-column dV / dK / dQ accumulators).
-template <bool WITH_DQ, bool DROP = false, bool BIAS = false, int HDIM = 128>
+template <bool DROP, bool BIAS, int HDIM>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                  const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -253,19 +252,15 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int k = 0; k < 8; ++k)  // dK += dS^T Q over q
           umma_ss_issue(tdK, dSm + k * 128, qm + k * 128, id_mm, (it | k) != 0, el);
         umma_commit_issue(&q_free[it & 1], el);
-        if constexpr (WITH_DQ) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {  // dQ = dS K over keys (into the dP columns)
-            const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-            umma_ss_issue(tdP, dSk + (off >> 4), dKm + k * 128, id_km, k != 0, el);
-          }
+        for (int k = 0; k < 8; ++k) {  // dQ = dS K over keys (into the dP columns)
+          const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
+          umma_ss_issue(tdP, dSk + (off >> 4), dKm + k * 128, id_km, k != 0, el);
         }
         umma_commit_issue(dq_full, el);
         if (it + 1 < nblk) {
-          if constexpr (WITH_DQ) {
-            if (!mbar_wait_warp(dp_free, it & 1, abort_flag, p.status)) break;
-            tc_fence_after();
-          }
+          if (!mbar_wait_warp(dp_free, it & 1, abort_flag, p.status)) break;
+          tc_fence_after();
           if (!issue_dp(it + 1)) break;
         }
       }
@@ -306,7 +301,6 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const bool reducer = threadIdx.x == 64;     // first element-wise thread issues the TMA operations
     auto drain_dq = [&](int it) -> bool {
       if (!mbar_wait_warp(dq_full, it & 1, abort_flag, p.status)) return false;
-      if constexpr (!WITH_DQ) return true;   // the products that read P and dS have completed: nothing to move
       tc_fence_after();
       // this thread's HDIM / 2 columns of dQ: boxes (2 half, 2 half + 1) for 128, box `half` for 64
       uint32_t t0[32], t1[32];
@@ -400,8 +394,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // ---- dS(it) = P (dP - delta) scale; P and dS to shared memory (free: dq_full(it-1) has been waited for)
       if (!mbar_wait_warp(dp_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       // P and dS share their memory with the staged dQ(it-1): wait until the TMA unit has read it
-      if (WITH_DQ && it > 0 &&
-          !mbar_wait_warp(stage_free, (it - 1) & 1, abort_flag, p.status)) {
+      if (it > 0 && !mbar_wait_warp(stage_free, (it - 1) & 1, abort_flag, p.status)) {
         ok = false;
         break;
       }
@@ -469,7 +462,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       cur = nxt;
     }
     if (ok && nblk > 0) ok = drain_dq(nblk - 1);
-    if (WITH_DQ && reducer) tma_store_wait<0>();
+    if (reducer) tma_store_wait<0>();
     // dV / dK of this key block: TMEM lane = key row. tcgen05.ld is a warp-wide (.sync.aligned)
     // instruction: every lane executes it, only the global stores are predicated per row.
     const int j = kv0 + r;
@@ -564,41 +557,60 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16*
 extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const float* lse,
                                 const float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
-                                long long do_stride, long long dq_stride, int causal, float softmax_scale,
+                                long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
                                 void* stream, int* status);
 
 extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k, const void* v, const float* lse,
                                  const float* delta, void* dk, void* dv, const int* row_lo, const int* row_hi, int B,
                                  int Sq, int Sk, int Hq, int Hkv, long long q_stride, long long k_stride,
                                  long long v_stride, long long do_stride, long long dkv_stride, int causal,
-                                 float softmax_scale, void* stream, int* status);
+                                 float softmax_scale, int fold, int head_dim, void* stream, int* status);
 
-// Which key-block kernel the two-kernel form uses: 1 = flash_attn_bwd_dkv.cu (transposed products, P and dS kept
-// in tensor memory), 0 = this file's kernel without its dQ part (P and dS through shared memory), -1 (default) =
-// by shape: measured at H=32, D=128 the shared-memory form is ahead up to 4096 keys (667 vs 681 us causal, 1067
-// vs 1281 us full) and the transposed form from 8192 causal keys on (2121 vs 2151 us).
-static int g_dkv_transposed = -1;
-extern "C" void atb_flash_bwd_set_dkv(int transposed) { g_dkv_transposed = transposed; }
+static int delta_launch(const void* dout, const void* out, float* delta, int B, int Sq, int Hq, long long do_stride,
+                        int head_dim, cudaStream_t st) {
+  const long long blocks = ((long long)B * Sq * Hq * 32 + 255) / 256;
+  flash_delta_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, B, Sq,
+                                                       Hq, do_stride, head_dim);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
 
-// Two forms. dq_acc == nullptr (default of the Python wrapper): the key-block kernel writes dK and dV, the
-// query-block kernel of flash_attn_bwd_dq.cu writes dQ; no atomics, results do not depend on scheduling.
-// dq_acc != nullptr: one key-block kernel for all three; dQ goes through TMA reduce-adds into dq_acc
-// (fp32 [B, Sq, Hq, 128], zero on entry) and a conversion pass.
-// dq_acc must be zero on entry; dq/dk/dv are written as token-major rows of pitch dq_stride / dkv_stride
-// elements (so they may be slices of one fused [tokens, (Hq + 2 Hq) * 128] gradient buffer). dk, dv are per
-// query head; the caller sums head groups for grouped-query attention. `delta` is scratch [B, Hq, Sq].
+// The two-kernel form, the default without dropout and bias: dK and dV per key block (flash_attn_bwd_dkv.cu; `fold`:
+// see there), dQ per query block (flash_attn_bwd_dq.cu). No atomics, results do not depend on scheduling. dq/dk/dv are
+// token-major rows of pitch dq_stride / dkv_stride elements (so they may be slices of one fused
+// [tokens, (Hq + 2 Hkv) * head_dim] gradient buffer); `delta` is scratch [B, Hq, Sq].
+extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* k, const void* v, const void* out,
+                                   const float* lse, float* delta, void* dq, void* dk, void* dv, const int* row_lo,
+                                   const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
+                                   long long k_stride, long long v_stride, long long do_stride, long long dq_stride,
+                                   long long dkv_stride, int causal, float softmax_scale, void* stream, int* status,
+                                   int fold, int head_dim) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
+  if ((head_dim != 128 && head_dim != 64) || Hq % Hkv || (do_stride & 7)) return -1;
+  int rc = delta_launch(dout, out, delta, B, Sq, Hq, do_stride, head_dim, (cudaStream_t)stream);
+  if (rc == 0)
+    rc = atb_flash_bwd_dkv(dout, q, k, v, lse, delta, dk, dv, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
+                           v_stride, do_stride, dkv_stride, causal, softmax_scale, fold, head_dim, stream, status);
+  if (rc == 0)
+    rc = atb_flash_bwd_dq(dout, q, k, v, lse, delta, dq, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride, v_stride,
+                          do_stride, dq_stride, causal, softmax_scale, head_dim, stream, status);
+  return rc;
+}
+
+// One key-block kernel for all three gradients: dropout, an additive bias, or on request. dQ goes through TMA
+// reduce-adds into dq_acc (fp32 [B, Sq, Hq, head_dim], zero on entry) and a conversion pass; dk, dv are per query head,
+// the caller sums head groups for grouped-query attention.
 // One-kernel form (dQ through the fp32 buffer) for a given dropout / bias / head-dim combination.
 template <bool DROP, bool BIAS, int HDIM>
 static int bwd_variant(dim3 grid, cudaStream_t st, const CUtensorMap& tmQ, const CUtensorMap& tmdO, const CUtensorMap& tmK,
                        const CUtensorMap& tmV, const CUtensorMap& tmdQ, const BwdParams& p) {
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_bwd_kernel<true, DROP, BIAS, HDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(flash_bwd_kernel<DROP, BIAS, HDIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              SmemB::TOTAL) != cudaSuccess)
       return -4;
     attr_set = true;
   }
-  flash_bwd_kernel<true, DROP, BIAS, HDIM><<<grid, THREADS, SmemB::TOTAL, st>>>(tmQ, tmdO, tmK, tmV, tmdQ, p);
+  flash_bwd_kernel<DROP, BIAS, HDIM><<<grid, THREADS, SmemB::TOTAL, st>>>(tmQ, tmdO, tmK, tmV, tmdQ, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
@@ -610,10 +622,8 @@ static int flash_bwd_launch(const void* dout, const void* q, const void* k, cons
                             int* status, DropParams drop, BiasParams bias = BiasParams{nullptr, 0, 0, 0},
                             int head_dim = 128) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  // dropout, the additive bias and head dim 64 are implemented in the one-kernel form only
-  if (head_dim != 128 && head_dim != 64) return -1;
+  if ((head_dim != 128 && head_dim != 64) || dq_acc == nullptr) return -1;
   const int HDv = head_dim;
-  if ((drop.thr16 != 0 || bias.ptr != nullptr || HDv != 128) && dq_acc == nullptr) return -1;
   if (bias.ptr != nullptr &&
       ((Sk & 7) || ((bias.sb | bias.sh | bias.sq) & 7) || (reinterpret_cast<uintptr_t>(bias.ptr) & 15) ||
        !(softmax_scale > 0.f)))
@@ -635,26 +645,11 @@ static int flash_bwd_launch(const void* dout, const void* q, const void* k, cons
                     64, CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
   // fp32 accumulation buffer as [B*Sq, Hq*HD]; the kernel adds [128 x 32] boxes to it
-  if (dq_acc == nullptr) {
-    tmdQ = tmQ;   // unused by the kernel variant without dQ
-  } else if (!make_tmap_2d(&tmdQ, dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)B * Sq, (uint64_t)Hq * HDv,
-                           (uint64_t)Hq * HDv, BQ, 32, CU_TENSOR_MAP_SWIZZLE_128B)) {
+  if (!make_tmap_2d(&tmdQ, dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)B * Sq, (uint64_t)Hq * HDv,
+                    (uint64_t)Hq * HDv, BQ, 32, CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
-  }
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemB::TOTAL) !=
-        cudaSuccess)
-      return -4;
-    attr_set = true;
-  }
-  {
-    const long long warps = (long long)B * Sq * Hq;
-    const int threads = 256;
-    const long long blocks = (warps * 32 + threads - 1) / threads;
-    flash_delta_kernel<<<(unsigned)blocks, threads, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out,
-                                                             delta, B, Sq, Hq, do_stride, HDv);
-  }
+  const int rd = delta_launch(dout, out, delta, B, Sq, Hq, do_stride, HDv, st);
+  if (rd != 0) return rd;
   BwdParams p;
   p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.dkv_stride = dkv_stride;
@@ -666,18 +661,6 @@ static int flash_bwd_launch(const void* dout, const void* q, const void* k, cons
   p.bias = bias;
   p.inv_scale = 1.f / softmax_scale;
   dim3 grid((Sk + BKV - 1) / BKV, Hq, B);
-  if (dq_acc == nullptr) {
-    if (g_dkv_transposed > 0 || (g_dkv_transposed < 0 && causal && Sk >= 8192)) {
-      const int rc = atb_flash_bwd_dkv(dout, q, k, v, lse, delta, dk, dv, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride,
-                                       k_stride, v_stride, do_stride, dkv_stride, causal, softmax_scale, stream, status);
-      if (rc != 0) return rc;
-    } else {
-      flash_bwd_kernel<false><<<grid, THREADS, SmemB::TOTAL, st>>>(tmQ, tmdO, tmK, tmV, tmdQ, p);
-      if (cudaGetLastError() != cudaSuccess) return -5;
-    }
-    return atb_flash_bwd_dq(dout, q, k, v, lse, delta, dq, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
-                            v_stride, do_stride, dq_stride, causal, softmax_scale, stream, status);
-  }
   {
     const bool dr = drop.thr16 != 0, bi = bias.ptr != nullptr;
     int rc;
@@ -738,7 +721,6 @@ extern "C" int atb_flash_bwd_bias(const void* dout, const void* q, const void* k
 }
 
 // The general entry point: head dim 128 or 64, optional dropout (thr16 != 0) and additive bias (bias != null).
-// Anything but the plain head-dim-128 case needs dq_acc (one-kernel form).
 extern "C" int atb_flash_bwd_ex(const void* dout, const void* q, const void* k, const void* v, const void* out,
                                 const float* lse, float* delta, float* dq_acc, void* dq, void* dk, void* dv,
                                 const int* row_lo, const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv,

@@ -1,8 +1,8 @@
-// Flash attention backward, query-gradient kernel for sm_100a (head dim 128, bf16), tcgen05 + TMEM + TMA.
+// Flash attention backward, query-gradient kernel for sm_100a (head dim 128 or 64, bf16), tcgen05 + TMEM + TMA.
 //
 // One CTA per (128 query rows, head, batch) walks the key blocks its rows can see and keeps dQ in tensor
 // memory from the first block to the last, so the query gradient needs no atomic adds, no fp32 scratch buffer
-// and no conversion pass (the key/value gradients come from the key-block kernel of flash_attn_bwd.cu):
+// and no conversion pass (the key/value gradients come from flash_attn_bwd_dkv.cu):
 //   S  = Q K_j^T,  dP = dO V_j^T              2 x tcgen05.mma  smem x smem -> TMEM
 //   P  = exp2(S c - lse),  dS = P (dP - delta) s   registers; dS written as bf16 over the dP columns
 //   dQ += dS K_j                                tcgen05.mma  TMEM x smem (MN-major K) -> TMEM
@@ -20,9 +20,8 @@
 namespace {
 using namespace atb;
 
-constexpr int BQ = 128, BKV = 128, HD = 128;
+constexpr int BQ = 128, BKV = 128;
 constexpr int PANEL = 128 * 64 * 2;
-constexpr int TILE = 2 * PANEL;
 constexpr int K_STAGES = 3, V_STAGES = 2;
 constexpr int N_EW = 256;
 constexpr int THREADS = 64 + N_EW;
@@ -39,7 +38,9 @@ struct DqParams {
   int* status;
 };
 
+template <int HD>
 struct SmemQ {
+  static constexpr int TILE = (HD / 64) * PANEL;
   static constexpr int Q_OFF = 0;
   static constexpr int DO_OFF = Q_OFF + TILE;
   static constexpr int K_OFF = DO_OFF + TILE;
@@ -48,12 +49,14 @@ struct SmemQ {
   static constexpr int NBARS = 1 + 2 * K_STAGES + 2 * V_STAGES + 4 + 4;
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
 };
-static_assert(SmemQ::TOTAL <= 232448, "shared memory of the dQ kernel exceeds 227 KB");
+static_assert(SmemQ<128>::TOTAL <= 232448, "shared memory of the dQ kernel exceeds 227 KB");
 
+template <int HD>
 __global__ void __launch_bounds__(THREADS, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, DqParams p) {
-  using L = SmemQ;
+  using L = SmemQ<HD>;
+  constexpr int TILE = L::TILE;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::Q_OFF;
@@ -142,27 +145,27 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
       if (el) mbar_expect_tx(qdo_full, 2 * TILE);
       if (el) tma_load_2d(sQ, &tmQ, qdo_full, h * HD, (int)q_row0);
-      if (el) tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, (int)q_row0);
+      if (HD == 128 && el) tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, (int)q_row0);
       if (el) tma_load_2d(sdO, &tmdO, qdo_full, h * HD, (int)q_row0);
-      if (el) tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, (int)q_row0);
+      if (HD == 128 && el) tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, (int)q_row0);
       for (int j = 0; j < n; ++j) {
         const int ks = j % K_STAGES, vs = j % V_STAGES;
         const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
         if (!mbar_wait_warp(&k_empty[ks], ((j / K_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
         if (el) mbar_expect_tx(&k_full[ks], TILE);
         if (el) tma_load_2d(sK + ks * TILE, &tmK, &k_full[ks], hk * HD, krow);
-        if (el) tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
+        if (HD == 128 && el) tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
         if (!mbar_wait_warp(&v_empty[vs], ((j / V_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
         if (el) mbar_expect_tx(&v_full[vs], TILE);
         if (el) tma_load_2d(sV + vs * TILE, &tmV, &v_full[vs], hk * HD, krow);
-        if (el) tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
+        if (HD == 128 && el) tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
       }
     }
   } else if (warp == 1) {
     if (n > 0) {
       const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t id_kk = umma_idesc(128, 128, 1, 1, false, false);
-      constexpr uint32_t id_km = umma_idesc(128, 128, 1, 1, false, true);
+      constexpr uint32_t id_km = umma_idesc(128, HD, 1, 1, false, true);
       const uint32_t dQk = umma_desc_lo(smem_u32(sQ), 16), dOk = umma_desc_lo(smem_u32(sdO), 16);
       const uint32_t dKk0 = umma_desc_lo(smem_u32(sK), 16), dKm0 = umma_desc_lo(smem_u32(sK), PANEL);
       const uint32_t dVk0 = umma_desc_lo(smem_u32(sV), 16);
@@ -173,7 +176,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after();
         const uint32_t kd = dKk0 + ((ks * TILE) >> 4);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
           umma_ss_issue(tS, dQk + (off >> 4), kd + (off >> 4), id_kk, k != 0, el);
         }
@@ -182,7 +185,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint32_t vd = dVk0 + ((vs * TILE) >> 4);
         const uint32_t dst = tdP + 128 * (j & 1);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
+        for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
           umma_ss_issue(dst, dOk + (off >> 4), vd + (off >> 4), id_kk, k != 0, el);
         }
@@ -294,12 +297,12 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (ok && n > 0) ok = mbar_wait_warp(dq_full, 0, abort_flag, p.status);
     if (ok) {
       if (n > 0) tc_fence_after();
-      __nv_bfloat16* row = p.dq + ((long long)b * p.Sq + i) * p.dq_stride + h * HD + half * 64;
+      __nv_bfloat16* row = p.dq + ((long long)b * p.Sq + i) * p.dq_stride + h * HD + half * (HD / 2);
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
+      for (int cc = 0; cc < HD / 64; ++cc) {
         uint32_t t[32];
         if (n > 0) {
-          tmem_ld_32x32(tdQ + lane_addr + half * 64 + cc * 32, t);
+          tmem_ld_32x32(tdQ + lane_addr + half * (HD / 2) + cc * 32, t);
           tmem_ld_wait();
         } else {
 #pragma unroll
@@ -332,45 +335,48 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
 }
 
-}  // namespace
-
-// dq rows of pitch dq_stride elements (head h at columns [h*128, h*128+128)); lse, delta: [B, Hq, Sq] fp32
-// (delta = rowsum(dO * O), written by the pre-pass of atb_flash_bwd).
-extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const float* lse,
-                                const float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
-                                int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
-                                long long do_stride, long long dq_stride, int causal, float softmax_scale,
-                                void* stream, int* status) {
-  if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  if (Hq % Hkv) return -1;
-  if ((q_stride | k_stride | v_stride | do_stride | dq_stride) & 7) return -1;
+template <int HD>
+int launch_dq(const void* dout, const void* q, const void* k, const void* v, const DqParams& p, long long q_stride,
+              long long k_stride, long long v_stride, long long do_stride, cudaStream_t stream) {
   CUtensorMap tmQ, tmdO, tmK, tmV;
-  if (!make_tmap_2d(&tmQ, q, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sq, (uint64_t)Hq * HD, q_stride, BQ, 64,
-                    CU_TENSOR_MAP_SWIZZLE_128B))
-    return -2;
-  if (!make_tmap_2d(&tmdO, dout, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sq, (uint64_t)Hq * HD, do_stride,
-                    BQ, 64, CU_TENSOR_MAP_SWIZZLE_128B))
-    return -2;
-  if (!make_tmap_2d(&tmK, k, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sk, (uint64_t)Hkv * HD, k_stride, BKV,
-                    64, CU_TENSOR_MAP_SWIZZLE_128B))
-    return -2;
-  if (!make_tmap_2d(&tmV, v, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * Sk, (uint64_t)Hkv * HD, v_stride, BKV,
-                    64, CU_TENSOR_MAP_SWIZZLE_128B))
+  const auto bf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
+  if (!make_tmap_2d(&tmQ, q, bf16, 2, (uint64_t)p.B * p.Sq, (uint64_t)p.Hq * HD, q_stride, BQ, 64, sw) ||
+      !make_tmap_2d(&tmdO, dout, bf16, 2, (uint64_t)p.B * p.Sq, (uint64_t)p.Hq * HD, do_stride, BQ, 64, sw) ||
+      !make_tmap_2d(&tmK, k, bf16, 2, (uint64_t)p.B * p.Sk, (uint64_t)p.Hkv * HD, k_stride, BKV, 64, sw) ||
+      !make_tmap_2d(&tmV, v, bf16, 2, (uint64_t)p.B * p.Sk, (uint64_t)p.Hkv * HD, v_stride, BKV, 64, sw))
     return -2;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemQ::TOTAL) !=
+    if (cudaFuncSetAttribute(flash_bwd_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemQ<HD>::TOTAL) !=
         cudaSuccess)
       return -4;
     attr_set = true;
   }
+  dim3 grid((p.Sq + BQ - 1) / BQ, p.Hq, p.B);
+  flash_bwd_dq_kernel<HD><<<grid, THREADS, SmemQ<HD>::TOTAL, stream>>>(tmQ, tmdO, tmK, tmV, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+}  // namespace
+
+// dq rows of pitch dq_stride elements (head h at columns [h*head_dim, (h+1)*head_dim)); lse, delta: [B, Hq, Sq] fp32
+// (delta = rowsum(dO * O), written by the pre-pass of atb_flash_bwd_split).
+extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const float* lse,
+                                const float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
+                                int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
+                                long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
+                                void* stream, int* status) {
+  if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
+  if (Hq % Hkv || (head_dim != 128 && head_dim != 64)) return -1;
+  if ((q_stride | k_stride | v_stride | do_stride | dq_stride) & 7) return -1;
   DqParams p;
   p.lse = lse; p.delta = delta; p.dq = (__nv_bfloat16*)dq; p.dq_stride = dq_stride;
   p.row_lo = row_lo; p.row_hi = row_hi;
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale = softmax_scale; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  dim3 grid((Sq + BQ - 1) / BQ, Hq, B);
-  flash_bwd_dq_kernel<<<grid, THREADS, SmemQ::TOTAL, (cudaStream_t)stream>>>(tmQ, tmdO, tmK, tmV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return head_dim == 64
+             ? launch_dq<64>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream)
+             : launch_dq<128>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream);
 }

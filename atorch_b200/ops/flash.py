@@ -34,10 +34,13 @@ import weakref
 # 256 us for the single-tile kernel; at B=16, S=512, H=16, D=64 with padding: 53 us against 80 us); ATB_FLASH_V2=0
 # keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
-# backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch): measured 667 us
-# against 696 us for the single key-block kernel at S=4096, H=32, causal. ATB_FLASH_BWD_SPLIT=0 selects the latter.
+# backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch) where there is neither
+# dropout nor a bias. ATB_FLASH_BWD_SPLIT=0 selects the one key-block kernel with TMA reduce-adds of dQ everywhere.
 BWD_SPLIT = os.environ.get("ATB_FLASH_BWD_SPLIT", "1") == "1"
-_DKV_SET = False   # ATB_FLASH_BWD_DKV=0 / 1 forces the shared-memory / transposed key-block kernel (default: by shape)
+# dK/dV kernel: one CTA per key block and key/value head sums the query heads of its group in tensor memory, if that
+# still gives every SM a CTA; else one CTA per query head, and the groups are summed by a pass over their bf16 results
+# (packed documents, S=4096, 32 heads on 8: 140 us folded, 179 us and 135 us of passes otherwise)
+FOLD_MIN_CTAS = 148
 
 
 def kernels_built() -> bool:
@@ -285,15 +288,9 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
     like a fused q|k|v projection output, so the gradient of that projection needs no concatenation."""
     B, Sq, Hq, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
-    global _DKV_SET
-    if not _DKV_SET:
-        _DKV_SET = True
-        if os.environ.get("ATB_FLASH_BWD_DKV", "") in ("0", "1"):
-            _lib.lib().atb_flash_bwd_set_dkv(ctypes.c_int(int(os.environ["ATB_FLASH_BWD_DKV"])))
-    # two kernels (dK/dV per key block, dQ per query block: no atomics, no fp32 scratch) unless
-    # ATB_FLASH_BWD_SPLIT=0 asks for the single key-block kernel with TMA reduce-adds of dQ
-    dq_acc = None if (BWD_SPLIT and drop is None and bias is None and D == 128) else \
-        torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=q.device)
+    split = BWD_SPLIT and drop is None and bias is None
+    dq_acc = None if split else torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=q.device)
+    fold = Hq // Hkv if split and B * Hkv * ((Sk + 127) // 128) >= FOLD_MIN_CTAS else 1
     delta = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
     if fused_out and Hkv == Hq and Sq == Sk:
         fused = torch.empty(B, Sq, 3 * Hq, D, dtype=q.dtype, device=q.device)
@@ -301,28 +298,33 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
     else:
         fused = None
         dq = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
-        dk = torch.empty(B, Sk, Hq, D, dtype=q.dtype, device=q.device)
-        dv = torch.empty(B, Sk, Hq, D, dtype=q.dtype, device=q.device)
+        dk = torch.empty(B, Sk, Hq // fold, D, dtype=q.dtype, device=q.device)
+        dv = torch.empty(B, Sk, Hq // fold, D, dtype=q.dtype, device=q.device)
     dout = dout if (dout.stride(-1) == 1 and dout.stride(2) == D and dout.stride(0) == dout.stride(1) * Sq) \
         else dout.contiguous()
-    if D != 128:
-        bwd, extra = _lib.lib().atb_flash_bwd_ex, _extra_args(drop, bias, D)
-    elif bias is not None:
-        bwd, extra = _lib.lib().atb_flash_bwd_bias, _extra_args(drop, bias)
-    elif drop is not None:
-        bwd, extra = _lib.lib().atb_flash_bwd_dropout, _extra_args(drop, None)
+    L = _lib.lib()
+    if split:
+        bwd, acc, extra = L.atb_flash_bwd_split, (), (ctypes.c_int(fold), ctypes.c_int(D))
     else:
-        bwd, extra = _lib.lib().atb_flash_bwd, ()
+        acc = (_lib.ptr(dq_acc),)
+        if D != 128:
+            bwd, extra = L.atb_flash_bwd_ex, _extra_args(drop, bias, D)
+        elif bias is not None:
+            bwd, extra = L.atb_flash_bwd_bias, _extra_args(drop, bias)
+        elif drop is not None:
+            bwd, extra = L.atb_flash_bwd_dropout, _extra_args(drop, None)
+        else:
+            bwd, extra = L.atb_flash_bwd, ()
     rc = bwd(
-        _lib.ptr(dout), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(delta),
-        _lib.ptr(dq_acc), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(row_lo), _lib.ptr(row_hi),
+        _lib.ptr(dout), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(delta), *acc,
+        _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(row_lo), _lib.ptr(row_hi),
         ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk), ctypes.c_int(Hq), ctypes.c_int(Hkv),
         ctypes.c_longlong(_token_stride(q)), ctypes.c_longlong(_token_stride(k)), ctypes.c_longlong(_token_stride(v)),
         ctypes.c_longlong(_token_stride(dout)), ctypes.c_longlong(_token_stride(dq)),
         ctypes.c_longlong(_token_stride(dk)), ctypes.c_int(int(causal)), ctypes.c_float(softmax_scale),
         _lib.stream_ptr(), _lib.ptr(_lib.status_word(q.device)), *extra)
     _lib.check(rc, "atb_flash_bwd")
-    if Hkv != Hq:
+    if Hkv != Hq and fold == 1:
         g = Hq // Hkv
         dk = dk.view(B, Sk, Hkv, g, D).float().sum(3).to(q.dtype)
         dv = dv.view(B, Sk, Hkv, g, D).float().sum(3).to(q.dtype)

@@ -381,3 +381,27 @@ def test_flash_head_dim_64_masks_and_dropout():
     for name, a, b_ in zip("qkv", qs, rs):
         err = (a.grad.float() - b_.grad).abs().max().item()
         assert err / (b_.grad.abs().max().item() + 1e-6) < 3e-2, (name, err)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("fold", [True, False])
+@pytest.mark.parametrize("mask", ["causal", "packed", "padding", "glm"])
+def test_backward_grouped_queries_folded_into_the_key_block_kernel(mask, fold, D, monkeypatch):
+    """dK / dV summed over a group of query heads in one CTA and by the pass over per-head results: the same gradients
+    as the fp32 reference, with lengths that leave a ragged block and key blocks that no row of a sample sees."""
+    monkeypatch.setattr(flash, "FOLD_MIN_CTAS", 1 if fold else 1 << 30)
+    torch.manual_seed(len(mask) + D)
+    B, S, Hq, Hkv = (1 if mask == "packed" else 2), 421, 6, 2
+    q, k, v, dout = (torch.randn(B, S, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    kw = {"causal": {"causal": True},
+          "packed": {"causal": True, "cu_seqlens": torch.tensor([0, 3, 130, 300, 421], device="cuda", dtype=torch.int32)},
+          "padding": {"key_padding_mask": torch.arange(S, device="cuda")[None] < torch.tensor([[90], [421]], device="cuda")},
+          "glm": {"glm_mask": torch.tensor([0, 333], device="cuda")}}[mask]
+    ins = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    got = torch.autograd.grad(flash.flash_attention(*ins, **kw), ins, dout)
+    ref_in = [t.float().requires_grad_(True) for t in (q, k, v)]
+    ref = torch.autograd.grad(attention_reference(*ref_in, **kw), ref_in, dout.float())
+    torch.cuda.synchronize()
+    _lib.check_status(torch.device("cuda", 0))
+    for g, r in zip(got, ref):
+        assert g.shape == r.shape and (g.float() - r).norm() <= 1e-2 * r.norm()   # bf16 P, dS and results: 2^-9 each
