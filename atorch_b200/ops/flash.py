@@ -82,6 +82,45 @@ def row_intervals(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_ma
     analytic causal / full form inside the kernel is enough."""
     if glm_mask is None and pack_glm_mask is None and key_padding_mask is None and cu_seqlens is None:
         return None, None
+    out = _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens)
+    return out if out is not None else row_intervals_reference(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask,
+                                                               key_padding_mask, cu_seqlens)
+
+
+def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens):
+    """The lowering in one launch (csrc/masks.cu), or ``None`` for arguments it does not read as they are. With a key
+    padding mask one host synchronisation: an interval can only describe valid keys that lie next to each other."""
+    device = torch.device(device)
+    if device.type != "cuda" or B < 1 or B > 65535 or Sq < 1 or Sk < 1 or _lib.lib() is None:
+        return None
+    ints = (torch.int32, torch.int64)
+    glm, pack, kp, cu = (None if t is None else t.to(device) for t in (glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens))
+    if not ((glm is None or (glm.dtype in ints and glm.numel() == B))
+            and (pack is None or (pack.dtype in ints and pack.dim() == 3 and pack.shape[0] == B and pack.shape[1] >= 2
+                                  and pack.shape[2] > 0))
+            and (kp is None or (kp.dtype in (torch.bool, torch.uint8) and kp.shape == (B, Sk)))
+            and (cu is None or (cu.dtype in ints and cu.dim() == 1 and cu.numel() >= 2))):
+        return None
+    glm, kp, cu = (None if t is None else t.contiguous() for t in (glm, kp, cu))
+    pack = None if pack is None else pack[:, :2].contiguous()
+    is64 = lambda t: ctypes.c_int(int(t is not None and t.dtype == torch.int64))
+    buf = torch.empty(2 * B * Sq + B, dtype=torch.int32, device=device)
+    lo, hi, holes = buf[: B * Sq].view(B, Sq), buf[B * Sq: 2 * B * Sq].view(B, Sq), buf[2 * B * Sq:]
+    with torch.cuda.device(device):
+        rc = _lib.lib().atb_row_intervals(
+            _lib.ptr(lo), _lib.ptr(hi), _lib.ptr(holes), ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk),
+            ctypes.c_int(int(causal or glm is not None or pack is not None)), _lib.ptr(glm), is64(glm), _lib.ptr(pack),
+            is64(pack), ctypes.c_int(0 if pack is None else pack.shape[2]), _lib.ptr(kp), _lib.ptr(cu), is64(cu),
+            ctypes.c_int(0 if cu is None else cu.numel()), _lib.stream_ptr())
+    _lib.check(rc, "atb_row_intervals")
+    if kp is not None and any(holes.tolist()):
+        raise NonContiguousKeyMask()
+    return lo, hi
+
+
+def row_intervals_reference(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask=None, pack_glm_mask=None,
+                            key_padding_mask=None, cu_seqlens=None):
+    """The same in tensor operations: any device, any argument dtype (and the oracle of the kernel's test)."""
     i = torch.arange(Sq, device=device, dtype=torch.int64)
     shift = Sk - Sq
     causal_like = causal or glm_mask is not None or pack_glm_mask is not None

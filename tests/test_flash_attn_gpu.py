@@ -405,3 +405,35 @@ def test_backward_grouped_queries_folded_into_the_key_block_kernel(mask, fold, D
     _lib.check_status(torch.device("cuda", 0))
     for g, r in zip(got, ref):
         assert g.shape == r.shape and (g.float() - r).norm() <= 1e-2 * r.norm()   # bf16 P, dS and results: 2^-9 each
+
+
+@pytest.mark.parametrize("idx", [torch.int32, torch.int64])
+@pytest.mark.parametrize("B,Sq,Sk", [(1, 1, 1), (3, 255, 255), (2, 257, 513), (2, 300, 128)])
+def test_row_intervals_kernel_matches_the_tensor_operations(B, Sq, Sk, idx):
+    """Every mask argument alone and together, index dtypes, cross lengths, empty samples and masks with holes."""
+    g = torch.Generator().manual_seed(B * 1000 + Sq + Sk)
+    rnd = lambda lo, hi, *shape: torch.randint(lo, hi, shape, generator=g)
+    glm = rnd(0, Sk + 3, B).to(idx).cuda()
+    pack = torch.stack([rnd(-1, Sq, B, 3), rnd(-1, Sk + 1, B, 3)], 1).to(idx).cuda()
+    cu = torch.cat([torch.zeros(1, dtype=torch.int64), rnd(0, Sk + 1, 3).sort().values, torch.tensor([Sk])]).to(idx).cuda()
+    n = rnd(0, Sk + 1, B)
+    n[0] = 0
+    pos = torch.arange(Sk)[None]
+    right, left = (pos < n[:, None]).cuda(), (pos >= n[:, None]).cuda()
+    holes = (torch.rand(B, Sk, generator=g) < 0.5).cuda()
+    for causal in (False, True):
+        for kw in ({"glm_mask": glm}, {"pack_glm_mask": pack}, {"cu_seqlens": cu}, {"key_padding_mask": right},
+                   {"key_padding_mask": left.to(torch.uint8) * 3}, {"key_padding_mask": holes},
+                   {"glm_mask": glm.cpu(), "pack_glm_mask": pack, "cu_seqlens": cu, "key_padding_mask": right}):
+            def lower(fn):
+                try:
+                    return fn(B, Sq, Sk, torch.device("cuda"), causal, **kw)
+                except flash.NonContiguousKeyMask:
+                    return None
+            got, ref = lower(flash.row_intervals), lower(flash.row_intervals_reference)
+            assert (got is None) == (ref is None)
+            if ref is not None:
+                assert all(a.dtype == b.dtype and torch.equal(a, b) for a, b in zip(got, ref))
+    before = _lib.launch_count
+    flash.row_intervals(B, Sq, Sk, torch.device("cuda"), True, glm_mask=glm)
+    assert _lib.launch_count == before + 1
