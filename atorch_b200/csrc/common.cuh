@@ -486,6 +486,13 @@ ATB_DEVICE uint64_t f2_mul(uint64_t a, uint64_t b) {
   return d;
 }
 
+// bit c set: key k0 + c lies in [lo, hi)
+ATB_DEVICE uint32_t visible_keys(int k0, int lo, int hi) {
+  const int a = min(max(lo - k0, 0), 32), e = min(max(hi - k0, 0), 32);
+  const uint32_t below_e = e == 32 ? 0xffffffffu : (1u << e) - 1u, below_a = a == 32 ? 0xffffffffu : (1u << a) - 1u;
+  return below_e & ~below_a;
+}
+
 // Attention dropout: a counter-based keep decision per (batch*head, query row, key column), the same in the
 // forward and the backward kernels and reproducible on the host (ops/flash.py: dropout_keep_mask). One hash
 // serves two neighbouring columns: the low 16 bits decide the even column, the high 16 bits the odd one;

@@ -554,8 +554,8 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16*
 
 }  // namespace
 
-extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const float* lse,
-                                const float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
+extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const void* out,
+                                const float* lse, float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
                                 long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
                                 void* stream, int* status);
@@ -566,16 +566,8 @@ extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k,
                                  long long v_stride, long long do_stride, long long dkv_stride, int causal,
                                  float softmax_scale, int fold, int head_dim, void* stream, int* status);
 
-static int delta_launch(const void* dout, const void* out, float* delta, int B, int Sq, int Hq, long long do_stride,
-                        int head_dim, cudaStream_t st) {
-  const long long blocks = ((long long)B * Sq * Hq * 32 + 255) / 256;
-  flash_delta_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, B, Sq,
-                                                       Hq, do_stride, head_dim);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
-
 // The two-kernel form, the default without dropout and bias: dK and dV per key block (flash_attn_bwd_dkv.cu; `fold`:
-// see there), dQ per query block (flash_attn_bwd_dq.cu). No atomics, results do not depend on scheduling. dq/dk/dv are
+// see there), dQ per query block (flash_attn_bwd_dq.cu, which runs first and writes delta). No atomics, results do not depend on scheduling. dq/dk/dv are
 // token-major rows of pitch dq_stride / dkv_stride elements (so they may be slices of one fused
 // [tokens, (Hq + 2 Hkv) * head_dim] gradient buffer); `delta` is scratch [B, Hq, Sq].
 extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* k, const void* v, const void* out,
@@ -586,13 +578,11 @@ extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* 
                                    int fold, int head_dim) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if ((head_dim != 128 && head_dim != 64) || Hq % Hkv || (do_stride & 7)) return -1;
-  int rc = delta_launch(dout, out, delta, B, Sq, Hq, do_stride, head_dim, (cudaStream_t)stream);
+  int rc = atb_flash_bwd_dq(dout, q, k, v, out, lse, delta, dq, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
+                            v_stride, do_stride, dq_stride, causal, softmax_scale, head_dim, stream, status);
   if (rc == 0)
     rc = atb_flash_bwd_dkv(dout, q, k, v, lse, delta, dk, dv, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
                            v_stride, do_stride, dkv_stride, causal, softmax_scale, fold, head_dim, stream, status);
-  if (rc == 0)
-    rc = atb_flash_bwd_dq(dout, q, k, v, lse, delta, dq, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride, v_stride,
-                          do_stride, dq_stride, causal, softmax_scale, head_dim, stream, status);
   return rc;
 }
 
@@ -648,8 +638,11 @@ static int flash_bwd_launch(const void* dout, const void* q, const void* k, cons
   if (!make_tmap_2d(&tmdQ, dq_acc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)B * Sq, (uint64_t)Hq * HDv,
                     (uint64_t)Hq * HDv, BQ, 32, CU_TENSOR_MAP_SWIZZLE_128B))
     return -2;
-  const int rd = delta_launch(dout, out, delta, B, Sq, Hq, do_stride, HDv, st);
-  if (rd != 0) return rd;
+  {
+    const long long blocks = ((long long)B * Sq * Hq * 32 + 255) / 256;
+    flash_delta_kernel<<<(unsigned)blocks, 256, 0, st>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, delta, B,
+                                                         Sq, Hq, do_stride, HDv);
+  }
   BwdParams p;
   p.lse = lse; p.delta = delta; p.dq_acc = dq_acc; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
   p.dkv_stride = dkv_stride;

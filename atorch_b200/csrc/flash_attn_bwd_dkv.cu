@@ -13,7 +13,7 @@
 //   S(i+1) is issued as soon as the warps hold S(i) in registers and runs under the exponentials of block i,
 //   dV(i) starts when P(i) is stored and runs under dS(i),
 //   dK(i), dP(i+1) run under the exponentials of block i+1.
-// S=4096, 32 heads of 128, causal: 353 -> 285 us, S=8192: 1188 -> 938 us; before, S(i+1) was issued after P and dS were
+// S=8192, 32 heads of 128, causal: 1188 -> 865 us (2800 clocks a block, 1024 of them exponentials); before, S(i+1) was issued after P and dS were
 // both stored, or (for long causal inputs) P^T and dS^T went through tensor memory instead, whose element-wise warps need
 // the row statistics per column.
 // For grouped queries the gradients of the group are summed in the accumulator in fp32; with one CTA per query head the
@@ -66,13 +66,6 @@ struct RowInfo {       // one query row as the element-wise thread sees it; -inf
   float lse, delta;
   int lo, hi;          // key interval
 };
-
-// bit c set: key k0 + c lies in [lo, hi)
-ATB_DEVICE uint32_t visible_keys(int k0, int lo, int hi) {
-  const int a = min(max(lo - k0, 0), 32), e = min(max(hi - k0, 0), 32);
-  const uint32_t below_e = e == 32 ? 0xffffffffu : (1u << e) - 1u, below_a = a == 32 ? 0xffffffffu : (1u << a) - 1u;
-  return below_e & ~below_a;
-}
 
 template <int HD>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -133,36 +126,36 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tmem_alloc<1>(tmem_slot, 512);
     tmem_relinquish<1>();
   }
-  if (warp == 2) {   // query rows whose interval meets this key block
-    int rmin = INT_MAX, rmax = -1;
-    if (p.row_lo == nullptr && p.row_hi == nullptr) {
-      if (lane == 0) {
-        rmin = p.causal ? max(0, kv0 - shift) : 0;
-        rmax = p.Sq - 1;
-        if (rmin > rmax) { rmin = INT_MAX; rmax = -1; }
-      }
-    } else {
-      for (int i = lane; i < p.Sq; i += 32) {
-        const int lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-        const int hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-        if (max(lo, kv0) < min(min(hi, p.Sk), kv0 + BKV)) { rmin = min(rmin, i); rmax = max(rmax, i); }
-      }
+  // query rows whose interval meets this key block. With intervals in memory all warps look for them, several rows of a
+  // thread in flight: one warp went through 4096 rows one load after another in 40 us.
+  if (p.row_lo == nullptr && p.row_hi == nullptr) {
+    if (threadIdx.x == 0) {
+      const int rmin = p.causal ? max(0, kv0 - shift) : 0;
+      q_range[0] = rmin < p.Sq ? rmin / BQ : 0;
+      q_range[1] = rmin < p.Sq ? (p.Sq - 1) / BQ + 1 : 0;
+    }
+  } else {
+    if (threadIdx.x == 0) { q_range[0] = INT_MAX; q_range[1] = 0; }
+    __syncthreads();
+    int bmin = INT_MAX, bmax = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < p.Sq; i += THREADS) {
+      const int lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
+      const int hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+      if (max(lo, kv0) < min(min(hi, p.Sk), kv0 + BKV)) { bmin = min(bmin, i / BQ); bmax = max(bmax, i / BQ + 1); }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      rmin = min(rmin, __shfl_xor_sync(0xffffffffu, rmin, o));
-      rmax = max(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+      bmin = min(bmin, __shfl_xor_sync(0xffffffffu, bmin, o));
+      bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
     }
-    if (lane == 0) {
-      q_range[0] = rmax >= 0 ? rmin / BQ : 0;
-      q_range[1] = rmax >= 0 ? rmax / BQ + 1 : 0;
-    }
+    if (lane == 0 && bmax > 0) { atomicMin(&q_range[0], bmin); atomicMax(&q_range[1], bmax); }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int qb0 = warp_uniform(q_range[0]), nq = warp_uniform(q_range[1]) - qb0;
+  const int nq = max(warp_uniform(q_range[1]) - warp_uniform(q_range[0]), 0), qb0 = nq > 0 ? warp_uniform(q_range[0]) : 0;
   const int n = nq * p.fold;                     // block i: query block qb0 + i % nq of head h0 + i / nq
   const long long q_row_base = (long long)b * p.Sq;
   const long long k_row = (long long)b * p.Sk + kv0;
@@ -271,7 +264,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint8_t* dsrow = sdS + half * PANEL + r * 128;
     bool ok = true;
 
-    // Loads only, nothing that depends on their results: the values of block i + 1 arrive under the work of block i.
+    // values of a row: loads only, used one block later
     auto row_info = [&](int h, int qb) -> RowInfo {
       RowInfo ri{-INFINITY, 0.f, 0, p.Sk};
       const int i = (qb0 + qb) * BQ + r;
@@ -286,14 +279,17 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       return ri;
     };
     int h = h0, qb = 0;
-    RowInfo cur = row_info(h, qb);
+    RowInfo raw = row_info(h, qb);
     for (int it = 0; it < n; ++it) {
+      const bool valid = raw.lse != -INFINITY;
+      const float lse2 = valid ? raw.lse * 1.4426950408889634f : 0.f, delta = valid ? raw.delta : 0.f;
+      const int lo = max(raw.lo, 0), hi = valid ? min(raw.hi, p.Sk) : 0;
+      // this block's values are out of `raw` before the loads of the next block's are issued: with both in flight the wait
+      // for the old ones also waited for the new ones, 500 to 700 clocks per block
+      asm volatile("" ::"f"(lse2), "f"(delta), "r"(lo), "r"(hi) : "memory");
       if (++qb == nq) { qb = 0; ++h; }
-      const RowInfo nxt = row_info(h, qb);
+      raw = row_info(h, qb);
       // ---- P(it) = exp2(S c - lse)
-      const bool valid = cur.lse != -INFINITY;
-      const float lse2 = valid ? cur.lse * 1.4426950408889634f : 0.f;
-      const int lo = max(cur.lo, 0), hi = valid ? min(cur.hi, p.Sk) : 0;
       // warp-uniform, so that the interval tests are a separate path that full tiles never enter
       const bool row_full = __all_sync(0xffffffffu, lo <= kv0 && hi >= kv0 + BKV);
       if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.status)) { ok = false; break; }
@@ -346,7 +342,6 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tmem_ld_32x32(tdP + lane_addr + half * 64, d0);
         tmem_ld_32x32(tdP + lane_addr + half * 64 + 32, d1);
         tmem_ld_wait();
-        const float delta = valid ? cur.delta : 0.f;
         const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
@@ -368,7 +363,6 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
-      cur = nxt;
     }
     if (ok && n > 0)
       ok = mbar_wait_warp(p_free, (n - 1) & 1, abort_flag, p.status) &&

@@ -27,8 +27,11 @@ constexpr int N_EW = 256;
 constexpr int THREADS = 64 + N_EW;
 
 struct DqParams {
-  const float* lse;    // [B, Hq, Sq]
-  const float* delta;  // [B, Hq, Sq]
+  const float* lse;            // [B, Hq, Sq]
+  float* delta;                // [B, Hq, Sq], written: rowsum(dO * O)
+  const __nv_bfloat16* dO;     // token-major rows of pitch do_stride, 16-byte aligned like the tensor maps
+  const __nv_bfloat16* O;      // [B, Sq, Hq, HD]
+  long long do_stride;
   __nv_bfloat16* dq;   // token-major, head h at columns [h*HD, h*HD+HD) of a row of pitch dq_stride
   long long dq_stride;
   const int* row_lo;
@@ -46,8 +49,9 @@ struct SmemQ {
   static constexpr int K_OFF = DO_OFF + TILE;
   static constexpr int V_OFF = K_OFF + K_STAGES * TILE;
   static constexpr int BAR_OFF = V_OFF + V_STAGES * TILE;  // 224 KB
-  static constexpr int NBARS = 1 + 2 * K_STAGES + 2 * V_STAGES + 4 + 4;
-  static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
+  static constexpr int NBARS = 1 + 2 * K_STAGES + 2 * V_STAGES + 4 + 4 + 1;
+  static constexpr int DOT_OFF = BAR_OFF + NBARS * 8 + 64;      // float [BQ]: dO . O of the rows
+  static constexpr int TOTAL = DOT_OFF + BQ * 4 + 1024;
 };
 static_assert(SmemQ<128>::TOTAL <= 232448, "shared memory of the dQ kernel exceeds 227 KB");
 
@@ -74,6 +78,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* ds_full = s_free + 1;              // dS(j) is in TMEM
   uint64_t* dq_full = ds_full + 1;             // the last dQ product has completed
   uint64_t* pair_bar = dq_full + 1;            // [4] the two warps of a lane quarter both hold S(j), dP(j)
+  uint64_t* dot_bar = pair_bar + 4;            // every element-wise warp has written its rows' dO . O
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [4]: t0, t1, full_lo, full_hi
@@ -95,6 +100,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(ds_full, N_EW / 32);
     mbar_init(dq_full, 1);
     for (int i = 0; i < 4; ++i) mbar_init(&pair_bar[i], 2);
+    mbar_init(dot_bar, N_EW / 32);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -104,13 +110,17 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   if (warp == 2) {   // key range of this query block: union and intersection of the rows' intervals
     int umin = INT_MAX, umax = 0, ilo = 0, ihi = INT_MAX;
-    for (int r = lane; r < BQ; r += 32) {
-      const int i = q0 + r;
-      if (i >= p.Sq) continue;
-      int lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-      int hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-      lo = max(lo, 0);
-      hi = min(hi, p.Sk);
+    int rlo[BQ / 32], rhi[BQ / 32];      // all loads first, then their use
+#pragma unroll
+    for (int e = 0; e < BQ / 32; ++e) {
+      const int i = min(q0 + lane + 32 * e, p.Sq - 1);
+      rlo[e] = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
+      rhi[e] = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+    }
+#pragma unroll
+    for (int e = 0; e < BQ / 32; ++e) {
+      if (q0 + lane + 32 * e >= p.Sq) continue;
+      const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk);
       if (hi <= lo) { ilo = INT_MAX; ihi = 0; continue; }
       umin = min(umin, lo); umax = max(umax, hi);
       ilo = max(ilo, lo); ihi = min(ihi, hi);
@@ -218,17 +228,50 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int r = quarter * 32 + lane;
     const int i = q0 + r;   // global query row
     const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16);
+    // delta = dO . O of the block's rows, 16 rows per warp and HD / 8 lanes per row, while the first tiles arrive and are
+    // multiplied: a separate pass over both tensors took 26 us at S=4096, 32 heads of 128
+    bool ok = true;
+    float delta;
+    {
+      constexpr int LANES = HD / 8, AT_ONCE = 32 / LANES, STEPS = 16 / AT_ONCE;
+      float* dots = reinterpret_cast<float*>(smem + L::DOT_OFF);
+      const int first = (warp - 2) * 16 + lane / LANES, sub = lane % LANES;
+      uint4 x[STEPS], y[STEPS];
+#pragma unroll
+      for (int e = 0; e < STEPS; ++e) {
+        const long long tok = (long long)b * p.Sq + min(q0 + first + e * AT_ONCE, p.Sq - 1);
+        x[e] = *reinterpret_cast<const uint4*>(p.dO + tok * p.do_stride + h * HD + sub * 8);
+        y[e] = *reinterpret_cast<const uint4*>(p.O + (tok * p.Hq + h) * HD + sub * 8);
+      }
+#pragma unroll
+      for (int e = 0; e < STEPS; ++e) {
+        const uint32_t xs[4] = {x[e].x, x[e].y, x[e].z, x[e].w}, ys[4] = {y[e].x, y[e].y, y[e].z, y[e].w};
+        float acc = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const float2 u = unpack_bf16x2(xs[w]), v = unpack_bf16x2(ys[w]);
+          acc += u.x * v.x + u.y * v.y;
+        }
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (sub == 0) dots[first + e * AT_ONCE] = acc;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(dot_bar);
+      ok = mbar_wait_warp(dot_bar, 0, abort_flag, p.status);
+      delta = dots[r];
+      if (ok && half == 0 && i < p.Sq) p.delta[((long long)b * p.Hq + h) * p.Sq + i] = delta;
+    }
     bool valid = i < p.Sq;
     int lo = 0, hi = 0;
-    float lse2 = 0.f, delta = 0.f;
+    float lse2 = 0.f;
     if (valid) {
-      const long long ridx = ((long long)b * p.Hq + h) * p.Sq + i;
-      const float l = p.lse[ridx];
+      const float l = p.lse[((long long)b * p.Hq + h) * p.Sq + i];
       if (l == -INFINITY) {
         valid = false;
+        delta = 0.f;
       } else {
         lse2 = l * 1.4426950408889634f;
-        delta = p.delta[ridx];
         lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
         hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
         lo = max(lo, 0);
@@ -237,8 +280,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
     const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
-    bool ok = true;
-    for (int j = 0; j < n; ++j) {
+    for (int j = 0; ok && j < n; ++j) {
       const int kv0 = (t0 + j) * BKV;
       const uint32_t dp_addr = tdP + 128 * (j & 1) + lane_addr;
       if (!mbar_wait_warp(sdp_full, j & 1, abort_flag, p.status)) { ok = false; break; }
@@ -271,10 +313,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         pb[c] = fast_exp2(b0); pb[c + 1] = fast_exp2(b1);
       }
       if (!tile_full) {   // a separate pass, so that fully visible tiles execute no interval tests at all
+        const uint32_t m0 = valid ? visible_keys(c0, lo, hi) : 0u, m1 = valid ? visible_keys(c0 + 32, lo, hi) : 0u;
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
-          if (!valid || c0 + c < lo || c0 + c >= hi) pa[c] = 0.f;
-          if (!valid || c0 + 32 + c < lo || c0 + 32 + c >= hi) pb[c] = 0.f;
+          if (!(m0 & (1u << c))) pa[c] = 0.f;
+          if (!(m1 & (1u << c))) pb[c] = 0.f;
         }
       }
       uint32_t ds[32];
@@ -360,17 +403,19 @@ int launch_dq(const void* dout, const void* q, const void* k, const void* v, con
 
 }  // namespace
 
-// dq rows of pitch dq_stride elements (head h at columns [h*head_dim, (h+1)*head_dim)); lse, delta: [B, Hq, Sq] fp32
-// (delta = rowsum(dO * O), written by the pre-pass of atb_flash_bwd_split).
-extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const float* lse,
-                                const float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
+// dq rows of pitch dq_stride elements (head h at columns [h*head_dim, (h+1)*head_dim)); lse: [B, Hq, Sq] fp32;
+// delta: [B, Hq, Sq] fp32, written (rowsum(dO * O), which the key/value-gradient kernel reads); out: [B, Sq, Hq, head_dim].
+extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, const void* v, const void* out,
+                                const float* lse, float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
                                 long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
                                 void* stream, int* status) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || (head_dim != 128 && head_dim != 64)) return -1;
   if ((q_stride | k_stride | v_stride | do_stride | dq_stride) & 7) return -1;
+  if ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
   DqParams p;
+  p.dO = (const __nv_bfloat16*)dout; p.O = (const __nv_bfloat16*)out; p.do_stride = do_stride;
   p.lse = lse; p.delta = delta; p.dq = (__nv_bfloat16*)dq; p.dq_stride = dq_stride;
   p.row_lo = row_lo; p.row_hi = row_hi;
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;

@@ -63,9 +63,7 @@ struct L2 {
 
 // -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi)
 ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi) {
-  const int a = min(max(lo - kv0, 0), 32), e = min(max(hi - kv0, 0), 32);
-  const uint32_t below_e = e == 32 ? 0xffffffffu : (1u << e) - 1u, below_a = a == 32 ? 0xffffffffu : (1u << a) - 1u;
-  const uint32_t vis = below_e & ~below_a;
+  const uint32_t vis = visible_keys(kv0, lo, hi);
 #pragma unroll
   for (int c = 0; c < 32; ++c)
     if (!(vis & (1u << c))) x[c] = 0xff800000u;
@@ -141,30 +139,31 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     mbar_fence_init();
   }
   if (warp == 1) { tmem_alloc<1>(tmem_slot, 512); tmem_relinquish<1>(); }
-  if (warp == 2) {   // union of the key intervals of the rows of each tile
-    int umin[2] = {INT_MAX, INT_MAX}, umax[2] = {0, 0};
+  if (warp == 2) {   // union of the key intervals of the rows of each tile (all loads first, then their use)
+    int rlo[2 * BQ / 32], rhi[2 * BQ / 32];
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      for (int r = lane; r < BQ; r += 32) {
-        const int i = q0 + t * BQ + r;
-        if (i >= p.Sq) continue;
-        int lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-        int hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-        lo = max(lo, 0); hi = min(hi, p.Sk);
-        if (hi > lo) { umin[t] = min(umin[t], lo); umax[t] = max(umax[t], hi); }
-      }
+    for (int e = 0; e < 2 * BQ / 32; ++e) {
+      const int i = min(q0 + lane + 32 * e, p.Sq - 1);
+      rlo[e] = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
+      rhi[e] = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+    }
+    int umin = INT_MAX, umax[2] = {0, 0};
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        umin[t] = min(umin[t], __shfl_xor_sync(0xffffffffu, umin[t], o));
-        umax[t] = max(umax[t], __shfl_xor_sync(0xffffffffu, umax[t], o));
-      }
+    for (int e = 0; e < 2 * BQ / 32; ++e) {
+      const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk), t = e / (BQ / 32);
+      if (q0 + lane + 32 * e < p.Sq && hi > lo) { umin = min(umin, lo); umax[t] = max(umax[t], hi); }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      umin = min(umin, __shfl_xor_sync(0xffffffffu, umin, o));
+      umax[0] = max(umax[0], __shfl_xor_sync(0xffffffffu, umax[0], o));
+      umax[1] = max(umax[1], __shfl_xor_sync(0xffffffffu, umax[1], o));
     }
     if (lane == 0) {
-      const int lo = min(umin[0], umin[1]);
-      const int first = lo == INT_MAX ? 0 : lo / BKV;
+      const int first = umin == INT_MAX ? 0 : umin / BKV;
       kv_range[0] = first;
-      kv_range[1] = umax[0] > umin[0] ? (umax[0] + BKV - 1) / BKV : first;
-      kv_range[2] = umax[1] > umin[1] ? (umax[1] + BKV - 1) / BKV : first;
+      kv_range[1] = umax[0] > 0 ? (umax[0] + BKV - 1) / BKV : first;
+      kv_range[2] = umax[1] > 0 ? (umax[1] + BKV - 1) / BKV : first;
     }
   }
   tc_fence_before();
