@@ -40,11 +40,9 @@ def rope_reference(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, nheads
 def _rope_launch(dst2, src2, cos, sin, positions, nheads, head_dim, backward):
     """dst2 = rope(src2) (rows = tokens); the columns after the rotated heads are copied through."""
     T, W = dst2.shape
-    rc = _lib.lib().atb_rope(_lib.ptr(dst2), _lib.ptr(src2), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions),
-                             ctypes.c_longlong(T), ctypes.c_int(cos.shape[0]), ctypes.c_int(nheads),
-                             ctypes.c_int(head_dim), ctypes.c_longlong(dst2.stride(0)),
-                             ctypes.c_longlong(src2.stride(0)), ctypes.c_int(W - nheads * head_dim),
-                             ctypes.c_int(int(backward)), _lib.stream_ptr())
+    rc = _lib.lib().atb_rope(dst2.data_ptr(), src2.data_ptr(), cos.data_ptr(), sin.data_ptr(), _lib.addr(positions), T,
+                             cos.shape[0], nheads, head_dim, dst2.stride(0), src2.stride(0), W - nheads * head_dim,
+                             int(backward), _lib.stream())
     _lib.check(rc, "atb_rope")
 
 
@@ -130,8 +128,7 @@ class _SwiGLU(torch.autograd.Function):
         gu2 = gu.reshape(-1, shp[-1])
         gu2 = gu2 if gu2.stride(-1) == 1 else gu2.contiguous()
         out = torch.empty(gu2.shape[0], F, dtype=gu.dtype, device=gu.device)
-        rc = _lib.lib().atb_swiglu_fwd(_lib.ptr(gu2), _lib.ptr(out), ctypes.c_longlong(gu2.shape[0]), ctypes.c_int(F),
-                                       ctypes.c_longlong(gu2.stride(0)), ctypes.c_longlong(F), _lib.stream_ptr())
+        rc = _lib.lib().atb_swiglu_fwd(gu2.data_ptr(), out.data_ptr(), gu2.shape[0], F, gu2.stride(0), F, _lib.stream())
         _lib.check(rc, "atb_swiglu_fwd")
         ctx.save_for_backward(gu2)
         ctx.shp = shp
@@ -150,9 +147,8 @@ def swiglu_backward(gu2: torch.Tensor, d2: torch.Tensor) -> torch.Tensor:
     dgu = torch.empty(gu2.shape[0], 2 * F, dtype=gu2.dtype, device=gu2.device)
     # dgu is written with the pitch of gu2; a contiguous gu2 is the common case
     src = gu2 if gu2.is_contiguous() else gu2.contiguous()
-    rc = _lib.lib().atb_swiglu_bwd(_lib.ptr(src), _lib.ptr(d2), _lib.ptr(dgu), ctypes.c_longlong(src.shape[0]),
-                                   ctypes.c_int(F), ctypes.c_longlong(2 * F), ctypes.c_longlong(F),
-                                   _lib.stream_ptr())
+    rc = _lib.lib().atb_swiglu_bwd(src.data_ptr(), d2.data_ptr(), dgu.data_ptr(), src.shape[0], F, 2 * F, F,
+                                   _lib.stream())
     _lib.check(rc, "atb_swiglu_bwd")
     return dgu
 

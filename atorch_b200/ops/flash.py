@@ -71,9 +71,13 @@ def supported(q, k, v, dropout_p=0.0, additive_mask=None, additive_bias=None, ke
     B, Sq, Hq, D = q.shape
     ok = q.dtype == torch.bfloat16 and Hq % k.shape[2] == 0 and \
         (D == 128 or (D == 64 and _lib.lib().has("atb_flash_fwd_ex")))
-    ok = ok and all(t.stride(-1) == 1 and t.stride(2) == D and t.stride(1) % 8 == 0 for t in (q, k, v))
-    ok = ok and all(t.stride(0) == t.stride(1) * t.shape[1] for t in (q, k, v))
-    return ok
+    if not ok:
+        return False
+    for t in (q, k, v):
+        s0, s1, s2, s3 = t.stride()
+        if s3 != 1 or s2 != D or s1 % 8 or s0 != s1 * t.shape[1]:
+            return False
+    return True
 
 
 def row_intervals(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask=None, pack_glm_mask=None,
@@ -103,15 +107,15 @@ def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, ke
         return None
     glm, kp, cu = (None if t is None else t.contiguous() for t in (glm, kp, cu))
     pack = None if pack is None else pack[:, :2].contiguous()
-    is64 = lambda t: ctypes.c_int(int(t is not None and t.dtype == torch.int64))
+    is64 = lambda t: int(t is not None and t.dtype == torch.int64)
     buf = torch.empty(2 * B * Sq + B, dtype=torch.int32, device=device)
     lo, hi, holes = buf[: B * Sq].view(B, Sq), buf[B * Sq: 2 * B * Sq].view(B, Sq), buf[2 * B * Sq:]
     with torch.cuda.device(device):
+        p = _lib.addr
         rc = _lib.lib().atb_row_intervals(
-            _lib.ptr(lo), _lib.ptr(hi), _lib.ptr(holes), ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk),
-            ctypes.c_int(int(causal or glm is not None or pack is not None)), _lib.ptr(glm), is64(glm), _lib.ptr(pack),
-            is64(pack), ctypes.c_int(0 if pack is None else pack.shape[2]), _lib.ptr(kp), _lib.ptr(cu), is64(cu),
-            ctypes.c_int(0 if cu is None else cu.numel()), _lib.stream_ptr())
+            p(lo), p(hi), p(holes), B, Sq, Sk, int(causal or glm is not None or pack is not None), p(glm), is64(glm),
+            p(pack), is64(pack), 0 if pack is None else pack.shape[2], p(kp), p(cu), is64(cu),
+            0 if cu is None else cu.numel(), _lib.stream())
     _lib.check(rc, "atb_row_intervals")
     if kp is not None and any(holes.tolist()):
         raise NonContiguousKeyMask()
@@ -290,6 +294,11 @@ def _extra_args(drop, bias, head_dim=None):
     return extra
 
 
+def _as_ctypes(name, args):
+    """``args`` under the declared types of launcher ``name``, for a launcher that begins with the same arguments."""
+    return tuple(_lib._CTYPE[c](x) for c, x in zip(_lib.SIGNATURES[name], args))
+
+
 def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None):
     """Launch the forward kernel. Returns (out [B,Sq,Hq,D] bf16, lse [B,Hq,Sq] fp32). ``drop``: see
     ``dropout_config``; dropout runs in the single-tile kernel."""
@@ -300,22 +309,18 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     L = _lib.lib()
     # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences; the single-tile kernel otherwise, and for
     # dropout, a bias, and a scale that is not positive (hidden scores are -inf before they are scaled)
+    p = _lib.addr
+    args = (p(q), p(k), p(v), p(out), p(lse), p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q),
+            _token_stride(k), _token_stride(v), int(causal), softmax_scale, _lib.stream(), _lib.status_addr(q))
     if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0:
-        fwd, extra = L.atb_flash_fwd_v2, (ctypes.c_int(D),)
-    elif D != 128:
-        fwd, extra = L.atb_flash_fwd_ex, _extra_args(drop, bias, D)      # single-tile kernel, head dim 64
-    elif bias is not None:
-        fwd, extra = L.atb_flash_fwd_bias, _extra_args(drop, bias)
-    elif drop is not None:
-        fwd, extra = L.atb_flash_fwd_dropout, _extra_args(drop, None)
+        rc = L.atb_flash_fwd_v2(*args, D)
+    elif D == 128 and bias is None and drop is None:
+        rc = L.atb_flash_fwd(*args)
     else:
-        fwd, extra = L.atb_flash_fwd, ()
-    rc = fwd(
-        _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(row_lo), _lib.ptr(row_hi),
-        ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk), ctypes.c_int(Hq), ctypes.c_int(Hkv),
-        ctypes.c_longlong(_token_stride(q)), ctypes.c_longlong(_token_stride(k)), ctypes.c_longlong(_token_stride(v)),
-        ctypes.c_int(int(causal)), ctypes.c_float(softmax_scale), _lib.stream_ptr(),
-        _lib.ptr(_lib.status_word(q.device)), *extra)
+        fwd, extra = (L.atb_flash_fwd_ex, _extra_args(drop, bias, D)) if D != 128 else \
+            (L.atb_flash_fwd_bias, _extra_args(drop, bias)) if bias is not None else \
+            (L.atb_flash_fwd_dropout, _extra_args(drop, None))        # single-tile kernel
+        rc = fwd(*_as_ctypes("atb_flash_fwd", args), *extra)
     _lib.check(rc, "atb_flash_fwd")
     return out, lse
 
@@ -341,11 +346,14 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
         dv = torch.empty(B, Sk, Hq // fold, D, dtype=q.dtype, device=q.device)
     dout = dout if (dout.stride(-1) == 1 and dout.stride(2) == D and dout.stride(0) == dout.stride(1) * Sq) \
         else dout.contiguous()
-    L = _lib.lib()
+    L, p = _lib.lib(), _lib.addr
+    dims = (p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q), _token_stride(k), _token_stride(v),
+            _token_stride(dout), _token_stride(dq), _token_stride(dk), int(causal), softmax_scale, _lib.stream(),
+            _lib.status_addr(q))
+    ins = (p(dout), p(q), p(k), p(v), p(out), p(lse), p(delta))
     if split:
-        bwd, acc, extra = L.atb_flash_bwd_split, (), (ctypes.c_int(fold), ctypes.c_int(D))
+        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D)
     else:
-        acc = (_lib.ptr(dq_acc),)
         if D != 128:
             bwd, extra = L.atb_flash_bwd_ex, _extra_args(drop, bias, D)
         elif bias is not None:
@@ -354,14 +362,8 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
             bwd, extra = L.atb_flash_bwd_dropout, _extra_args(drop, None)
         else:
             bwd, extra = L.atb_flash_bwd, ()
-    rc = bwd(
-        _lib.ptr(dout), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(lse), _lib.ptr(delta), *acc,
-        _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(row_lo), _lib.ptr(row_hi),
-        ctypes.c_int(B), ctypes.c_int(Sq), ctypes.c_int(Sk), ctypes.c_int(Hq), ctypes.c_int(Hkv),
-        ctypes.c_longlong(_token_stride(q)), ctypes.c_longlong(_token_stride(k)), ctypes.c_longlong(_token_stride(v)),
-        ctypes.c_longlong(_token_stride(dout)), ctypes.c_longlong(_token_stride(dq)),
-        ctypes.c_longlong(_token_stride(dk)), ctypes.c_int(int(causal)), ctypes.c_float(softmax_scale),
-        _lib.stream_ptr(), _lib.ptr(_lib.status_word(q.device)), *extra)
+        args = _as_ctypes("atb_flash_bwd_split", (*ins, p(dq), p(dk), p(dv), *dims))
+        rc = bwd(*args[: len(ins)], _lib.ptr(dq_acc), *args[len(ins):], *extra)
     _lib.check(rc, "atb_flash_bwd")
     if Hkv != Hq and fold == 1:
         g = Hq // Hkv

@@ -47,8 +47,10 @@ def _sizes_ok(a, b, M, N, K, a_mn, b_mn, out, groups, bias, residual) -> bool:
     if bias is not None and not (bias.dtype == torch.bfloat16 and bias.is_contiguous() and bias.is_cuda):
         return False
     # inputs that are not laid out for the kernel stay on the fallback, which they always took at these sizes
-    return all(t is None or (t.stride(-1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
-               for t in (a, b, out, residual)) and out.dtype in (torch.bfloat16, torch.float32)
+    for t in (a, b, out, residual):
+        if t is not None and (t.stride(-1) != 1 or t.stride(0) % 8 or t.data_ptr() % 16):
+            return False
+    return out.dtype in (torch.bfloat16, torch.float32)
 
 
 def gemm_reference(a, b, a_mn=False, b_mn=False, out=None, out_dtype=None, accumulate=False, alpha=1.0, bias=None):
@@ -127,45 +129,26 @@ def gemm(
     assert out.stride(-1) == 1 and out.dtype in (torch.bfloat16, torch.float32)
     L = _lib.lib()
     use_pair = kernel == "2cta" or (kernel == "auto" and PAIR_KERNEL_DEFAULT and M >= 256 and N >= 256)
+    pa, pb, po, fp32 = _pitch(a), _pitch(b), _pitch(out), int(out.dtype == torch.float32)
+    pr = _pitch(residual) if residual is not None else 0
+    head = (a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.addr(bias), M, N, K, pa, pb, po, int(a_mn), int(b_mn), fp32,
+            int(accumulate), alpha, tile_n, max_ctas, _lib.addr(residual), pr)
+    tail = (_lib.stream(), _lib.status_addr(a))
     if groups is not None:
         counts = groups.get("counts")
         assert counts is None or (counts.dtype == torch.int32 and counts.is_cuda)
-        rc = L.atb_gemm_bf16_2cta_grouped(
-            _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias),
-            ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-            ctypes.c_longlong(_pitch(a)), ctypes.c_longlong(_pitch(b)), ctypes.c_longlong(_pitch(out)),
-            ctypes.c_int(int(a_mn)), ctypes.c_int(int(b_mn)),
-            ctypes.c_int(int(out.dtype == torch.float32)), ctypes.c_int(int(accumulate)),
-            ctypes.c_float(alpha), ctypes.c_int(tile_n), ctypes.c_int(max_ctas), _lib.ptr(residual),
-            ctypes.c_longlong(_pitch(residual) if residual is not None else 0), _lib.ptr(counts),
-            ctypes.c_int(int(groups.get("m_rows", 0))), ctypes.c_int(int(groups.get("k_rows", 0))),
-            ctypes.c_int((K if b_mn else N) if n_b > 1 else 0), ctypes.c_int(int(groups.get("bm_rows", 0))),
-            ctypes.c_int(n_b), _lib.stream_ptr(), _lib.ptr(_lib.status_word(a.device)))
-        _lib.check(rc, f"atb_gemm_bf16_2cta_grouped M={M} N={N} K={K}")
-        return out
-    if use_pair:
-        rc = L.atb_gemm_bf16_2cta(
-            _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias),
-            ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-            ctypes.c_longlong(_pitch(a)), ctypes.c_longlong(_pitch(b)), ctypes.c_longlong(_pitch(out)),
-            ctypes.c_int(int(a_mn)), ctypes.c_int(int(b_mn)),
-            ctypes.c_int(int(out.dtype == torch.float32)), ctypes.c_int(int(accumulate)),
-            ctypes.c_float(alpha), ctypes.c_int(tile_n), ctypes.c_int(max_ctas), _lib.ptr(residual),
-            ctypes.c_longlong(_pitch(residual) if residual is not None else 0), _lib.stream_ptr(),
-            _lib.ptr(_lib.status_word(a.device)))
-        _lib.check(rc, f"atb_gemm_bf16_2cta M={M} N={N} K={K}")
-        return out
-    rc = L.atb_gemm_bf16(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), _lib.ptr(bias),
-        ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-        ctypes.c_longlong(_pitch(a)), ctypes.c_longlong(_pitch(b)), ctypes.c_longlong(_pitch(out)),
-        ctypes.c_int(int(a_mn)), ctypes.c_int(int(b_mn)),
-        ctypes.c_int(int(out.dtype == torch.float32)), ctypes.c_int(int(accumulate)),
-        ctypes.c_float(alpha), ctypes.c_int(tile_n), ctypes.c_int(max_ctas), _lib.ptr(residual),
-        ctypes.c_longlong(_pitch(residual) if residual is not None else 0),
-        _lib.stream_ptr(), _lib.ptr(_lib.status_word(a.device)),
-    )
-    _lib.check(rc, f"atb_gemm_bf16 M={M} N={N} K={K}")
+        rc = L.atb_gemm_bf16_2cta_grouped(*head, _lib.addr(counts), int(groups.get("m_rows", 0)),
+                                          int(groups.get("k_rows", 0)), (K if b_mn else N) if n_b > 1 else 0,
+                                          int(groups.get("bm_rows", 0)), n_b, *tail)
+        name = "atb_gemm_bf16_2cta_grouped"
+    elif use_pair:
+        rc = L.atb_gemm_bf16_2cta(*head, *tail)
+        name = "atb_gemm_bf16_2cta"
+    else:
+        rc = L.atb_gemm_bf16(*head, *tail)
+        name = "atb_gemm_bf16"
+    if rc != 0:
+        _lib.check(rc, f"{name} M={M} N={N} K={K}")
     return out
 
 
@@ -190,10 +173,8 @@ def gemm_ragged(x: torch.Tensor, w: torch.Tensor, sizes, b_mn: bool) -> torch.Te
     N = w.shape[2] if b_mn else w.shape[1]
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
     rc = _lib.lib().atb_gemm_bf16_2cta_ragged(
-        _lib.ptr(x), _lib.ptr(w), _lib.ptr(out), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-        ctypes.c_longlong(_pitch(x)), ctypes.c_longlong(w.shape[2]), ctypes.c_longlong(N), ctypes.c_int(int(b_mn)),
-        (ctypes.c_int * len(sizes))(*sizes), ctypes.c_int(len(sizes)), _lib.stream_ptr(),
-        _lib.ptr(_lib.status_word(x.device)))
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _pitch(x), w.shape[2], N, int(b_mn),
+        (ctypes.c_int * len(sizes))(*sizes), len(sizes), _lib.stream(), _lib.status_addr(x))
     _lib.check(rc, f"atb_gemm_bf16_2cta_ragged M={M} N={N} K={K} groups={len(sizes)}")
     return out
 
@@ -223,9 +204,8 @@ def gemm_swiglu(x2: torch.Tensor, weight: torch.Tensor, keep_gate_up: bool):
     act = torch.empty(T, F, dtype=x2.dtype, device=x2.device)
     gu = torch.empty(T, 2 * F, dtype=x2.dtype, device=x2.device) if keep_gate_up else None
     rc = _lib.lib().atb_gemm_bf16_2cta_swiglu(
-        _lib.ptr(x2), _lib.ptr(weight), _lib.ptr(act), _lib.ptr(gu), ctypes.c_int(T), ctypes.c_int(F), ctypes.c_int(K),
-        ctypes.c_longlong(_pitch(x2)), ctypes.c_longlong(_pitch(weight)), ctypes.c_longlong(F),
-        ctypes.c_longlong(2 * F), _lib.stream_ptr(), _lib.ptr(_lib.status_word(x2.device)))
+        x2.data_ptr(), weight.data_ptr(), act.data_ptr(), _lib.addr(gu), T, F, K, _pitch(x2), _pitch(weight), F, 2 * F,
+        _lib.stream(), _lib.status_addr(x2))
     _lib.check(rc, f"atb_gemm_bf16_2cta_swiglu T={T} F={F} K={K}")
     return act, gu
 

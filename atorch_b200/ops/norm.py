@@ -34,9 +34,9 @@ def _fwd(x2, res2, w, b, eps, ln):
     s = torch.empty_like(x2) if res2 is not None else None
     rstd = torch.empty(M, dtype=torch.float32, device=x2.device)
     mean = torch.empty(M, dtype=torch.float32, device=x2.device) if ln else None
-    rc = _lib.lib().atb_norm_fwd(_lib.ptr(x2), _lib.ptr(res2), _lib.ptr(w), _lib.ptr(b), _lib.ptr(y), _lib.ptr(s),
-                                 _lib.ptr(mean), _lib.ptr(rstd), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_float(eps),
-                                 ctypes.c_int(int(ln)), ctypes.c_int(_lib.DT[x2.dtype]), _lib.stream_ptr())
+    p = _lib.addr
+    rc = _lib.lib().atb_norm_fwd(p(x2), p(res2), p(w), p(b), p(y), p(s), p(mean), p(rstd), M, N, eps, int(ln),
+                                 _lib.DT[x2.dtype], _lib.stream())
     _lib.check(rc, "atb_norm_fwd")
     return y, s, mean, rstd
 
@@ -48,17 +48,17 @@ def _bwd(dy2, x2, w, mean, rstd, dres2, ln, need_db):
     pdw = torch.empty(parts, N, dtype=torch.float32, device=x2.device)
     pdb = torch.empty(parts, N, dtype=torch.float32, device=x2.device) if (ln and need_db) else None
     dx = torch.empty_like(x2)
-    rc = L.atb_norm_bwd(_lib.ptr(dy2), _lib.ptr(x2), _lib.ptr(w), _lib.ptr(mean), _lib.ptr(rstd), _lib.ptr(dres2),
-                        _lib.ptr(dx), _lib.ptr(pdw), _lib.ptr(pdb), ctypes.c_int(parts), ctypes.c_int(M),
-                        ctypes.c_int(N), ctypes.c_int(int(ln)), ctypes.c_int(_lib.DT[x2.dtype]), _lib.stream_ptr())
+    p = _lib.addr
+    rc = L.atb_norm_bwd(p(dy2), p(x2), p(w), p(mean), p(rstd), p(dres2), p(dx), p(pdw), p(pdb), parts, M, N, int(ln),
+                        _lib.DT[x2.dtype], _lib.stream())
     _lib.check(rc, "atb_norm_bwd")
     return dx, pdw, pdb, parts
 
 
 def _colsum(partial, parts, out, accumulate):
     N = partial.shape[1]
-    rc = _lib.lib().atb_colsum(_lib.ptr(partial), _lib.ptr(out), ctypes.c_int(parts), ctypes.c_int(N),
-                               ctypes.c_int(_lib.DT[out.dtype]), ctypes.c_int(int(accumulate)), _lib.stream_ptr())
+    rc = _lib.lib().atb_colsum(partial.data_ptr(), out.data_ptr(), parts, N, _lib.DT[out.dtype], int(accumulate),
+                               _lib.stream())
     _lib.check(rc, "atb_colsum")
 
 

@@ -438,3 +438,18 @@ def test_dataclass_helpers_dump_diff_map_and_keep_unknown_arguments(monkeypatch)
     assert dyn.to_dict() == {"lr": 0.5, "name": "x", "warmup": 3, "sched": {"k": [1, 2]}}
     with pytest.raises(AttributeError):
         dyn.missing
+
+
+def test_launcher_signatures_match_the_sources():
+    """The argument types that ctypes converts by are those of the C prototypes."""
+    import re
+    from pathlib import Path
+
+    from atorch_b200 import _lib
+
+    src = "\n".join(p.read_text() for p in sorted((Path(_lib.__file__).parent / "csrc").glob("*.cu")))
+    kinds = {"int": "i", "long long": "l", "float": "f"}
+    for name, sig in _lib.SIGNATURES.items():
+        (args,) = re.findall(r'extern "C" int ' + name + r"\(([^)]*)\)\s*\{", src)
+        got = ["p" if "*" in a else kinds[" ".join(a.split()).rsplit(" ", 1)[0]] for a in args.split(",")]
+        assert "".join(got) == sig, name
