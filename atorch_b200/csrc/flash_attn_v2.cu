@@ -48,6 +48,7 @@ struct Params {
   int B, Sq, Sk, Hq, Hkv, causal;
   float scale_log2;
   int* status;
+  KeyBits keys;
 };
 
 template <int HD>
@@ -61,9 +62,9 @@ struct L2 {
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
 };
 
-// -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi)
-ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi) {
-  const uint32_t vis = visible_keys(kv0, lo, hi);
+// -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi) and is a valid key
+ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi, uint32_t valid_keys) {
+  const uint32_t vis = visible_keys(kv0, lo, hi) & valid_keys;
 #pragma unroll
   for (int c = 0; c < 32; ++c)
     if (!(vis & (1u << c))) x[c] = 0xff800000u;
@@ -277,6 +278,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
       lo = max(lo, 0); hi = min(hi, p.Sk);
     }
+    const uint32_t* bits = p.keys.bits != nullptr && *p.keys.any != 0 ? p.keys.bits + (long long)b * ((p.Sk + 31) / 32) : nullptr;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t s_addr = lane_addr + t * BKV, o_addr = lane_addr + 2 * BKV + t * HD;
     float m_ref = -INFINITY, l_run = 0.f;
@@ -286,7 +288,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       // the mask tests are compiled into a separate path taken only by warps with a partly visible row
-      const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
+      const bool full = __all_sync(0xffffffffu, row_valid && bits == nullptr && lo <= kv0 && hi >= kv0 + BKV);
       uint32_t x0[32], x1[32], x2[32], x3[32];
       tmem_ld_32x32(s_addr, x0);
       tmem_ld_32x32(s_addr + 32, x1);
@@ -294,10 +296,15 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tmem_ld_32x32(s_addr + 96, x3);
       tmem_ld_wait();
       if (!full) {
-        mask_scores(x0, kv0, lo, hi);
-        mask_scores(x1, kv0 + 32, lo, hi);
-        mask_scores(x2, kv0 + 64, lo, hi);
-        mask_scores(x3, kv0 + 96, lo, hi);
+        uint32_t ok_keys[4] = {~0u, ~0u, ~0u, ~0u};
+        if (bits != nullptr) {
+#pragma unroll
+          for (int w = 0; w < 4; ++w) ok_keys[w] = kv0 + 32 * w < p.Sk ? bits[kv0 / 32 + w] : 0u;
+        }
+        mask_scores(x0, kv0, lo, hi, ok_keys[0]);
+        mask_scores(x1, kv0 + 32, lo, hi, ok_keys[1]);
+        mask_scores(x2, kv0 + 64, lo, hi, ok_keys[2]);
+        mask_scores(x3, kv0 + 96, lo, hi, ok_keys[3]);
       }
       const float mx = fmaxf(fmaxf(max_of(x0), max_of(x1)), fmaxf(max_of(x2), max_of(x3)));
       // raise the reference maximum only when it pays: a stale one costs nothing while 2^(gap) fits bf16/fp32
@@ -409,11 +416,12 @@ int launch_fwd2(const void* q, const void* k, const void* v, const Params& p, lo
 
 }  // namespace
 
-// Same contract as atb_flash_fwd (flash_attn.cu), for a positive softmax_scale and head dim 128 or 64.
+// Same contract as atb_flash_fwd (flash_attn.cu), for a positive softmax_scale and head dim 128 or 64; key_bits,
+// any_holes: see KeyBits (may be null).
 extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_lo,
                                 const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
                                 long long k_stride, long long v_stride, int causal, float softmax_scale, void* stream,
-                                int* status, int head_dim) {
+                                int* status, int head_dim, const unsigned* key_bits, const int* any_holes) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || (head_dim != 128 && head_dim != 64) || !(softmax_scale > 0.f)) return -1;
   if ((q_stride | k_stride | v_stride) & 7) return -1;
@@ -422,6 +430,7 @@ extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, voi
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
+  p.keys = KeyBits{key_bits, any_holes};
   return head_dim == 64 ? launch_fwd2<64>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream)
                         : launch_fwd2<128>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream);
 }

@@ -122,6 +122,27 @@ def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, ke
     return lo, hi
 
 
+def _padded_intervals(q, k, causal, scale, key_padding_mask, others, drop):
+    """``(row_lo, row_hi, keys)`` for a key padding mask of self-attention, with or without holes, without a host
+    synchronisation; ``keys`` (valid keys as bits, flag) goes to the kernels with the intervals. ``None`` where another
+    kernel than the two-query-tile forward and the two-kernel backward would run: those read intervals only."""
+    B, S = q.shape[:2]
+    if key_padding_mask is None or drop or any(o is not None for o in others) or k.shape[1] != S or S < 256 \
+            or not (FWD_TWO_TILES and BWD_SPLIT) or not scale > 0 or B > 65535 \
+            or key_padding_mask.dtype not in (torch.bool, torch.uint8) or key_padding_mask.shape != (B, S):
+        return None
+    kp = key_padding_mask.to(q.device).contiguous()
+    words = (S + 31) // 32
+    buf = torch.empty(2 * B * S + B * words + 3 * B + 1, dtype=torch.int32, device=q.device)
+    lo, hi, bits, info, flag = buf.split([B * S, B * S, B * words, 3 * B, 1])
+    p = _lib.addr
+    with torch.cuda.device(q.device):
+        rc = _lib.lib().atb_padded_intervals(p(kp), p(lo), p(hi), p(bits), p(info), p(flag), B, S, int(bool(causal)),
+                                             _lib.stream())
+    _lib.check(rc, "atb_padded_intervals")
+    return lo.view(B, S), hi.view(B, S), (bits, flag)
+
+
 def row_intervals_reference(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask=None, pack_glm_mask=None,
                             key_padding_mask=None, cu_seqlens=None):
     """The same in tensor operations: any device, any argument dtype (and the oracle of the kernel's test)."""
@@ -299,7 +320,7 @@ def _as_ctypes(name, args):
     return tuple(_lib._CTYPE[c](x) for c, x in zip(_lib.SIGNATURES[name], args))
 
 
-def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None):
+def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None, keys=None):
     """Launch the forward kernel. Returns (out [B,Sq,Hq,D] bf16, lse [B,Hq,Sq] fp32). ``drop``: see
     ``dropout_config``; dropout runs in the single-tile kernel."""
     B, Sq, Hq, D = q.shape
@@ -313,7 +334,7 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     args = (p(q), p(k), p(v), p(out), p(lse), p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q),
             _token_stride(k), _token_stride(v), int(causal), softmax_scale, _lib.stream(), _lib.status_addr(q))
     if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0:
-        rc = L.atb_flash_fwd_v2(*args, D)
+        rc = L.atb_flash_fwd_v2(*args, D, *(map(p, keys) if keys is not None else (0, 0)))
     elif D == 128 and bias is None and drop is None:
         rc = L.atb_flash_fwd(*args)
     else:
@@ -326,7 +347,7 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
 
 
 def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi, fused_out: bool = False,
-                  drop=None, bias=None):
+                  drop=None, bias=None, keys=None):
     """Launch the backward kernels. Returns (dq, dk, dv) shaped like q, k, v. With ``fused_out`` (and
     equal query / key-value head counts) the three are slices of ONE ``[B, S, 3*H, D]`` buffer laid out
     like a fused q|k|v projection output, so the gradient of that projection needs no concatenation."""
@@ -352,7 +373,7 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
             _lib.status_addr(q))
     ins = (p(dout), p(q), p(k), p(v), p(out), p(lse), p(delta))
     if split:
-        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D)
+        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D, *(map(p, keys) if keys is not None else (0, 0)))
     else:
         if D != 128:
             bwd, extra = L.atb_flash_bwd_ex, _extra_args(drop, bias, D)
@@ -376,18 +397,19 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
 
 class _FlashAttn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, causal, scale, row_lo, row_hi, drop=None, bias=None):
-        out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, drop, bias)
-        ctx.save_for_backward(q, k, v, out, lse, row_lo, row_hi)
+    def forward(ctx, q, k, v, causal, scale, row_lo, row_hi, drop=None, bias=None, keys=None):
+        out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, drop, bias, keys)
+        ctx.save_for_backward(q, k, v, out, lse, row_lo, row_hi, *(keys if keys is not None else (None, None)))
         ctx.cfg = (causal, scale, drop, bias)       # bias: (bf16 tensor, strides), not differentiated
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, lse, row_lo, row_hi = ctx.saved_tensors
+        q, k, v, out, lse, row_lo, row_hi, *keys = ctx.saved_tensors
         causal, scale, drop, bias = ctx.cfg
-        dq, dk, dv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, drop=drop, bias=bias)
-        return dq, dk, dv, None, None, None, None, None, None
+        dq, dk, dv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, drop=drop, bias=bias,
+                                   keys=keys if keys[0] is not None else None)
+        return dq, dk, dv, None, None, None, None, None, None, None
 
 
 def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pack_glm_mask=None,
@@ -401,6 +423,10 @@ def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pa
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     if Sq == 1:
         causal = False   # single-query decode sees every key
+    padded = _padded_intervals(q, k, causal, scale, key_padding_mask,
+                               (glm_mask, pack_glm_mask, cu_seqlens, additive_mask, additive_bias), dropout_p > 0.0)
+    if padded is not None:
+        return _FlashAttn.apply(q, k, v, bool(causal), float(scale), padded[0], padded[1], None, None, padded[2])
     try:
         lo, hi = row_intervals(B, Sq, Sk, q.device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens)
     except NonContiguousKeyMask:
@@ -446,23 +472,24 @@ class _FlashAttnQKV(torch.autograd.Function):
     backward emits one fused gradient tensor in the same layout: no slice-backward zero fills or adds."""
 
     @staticmethod
-    def forward(ctx, qkv, H, causal, scale, row_lo, row_hi, cached):
+    def forward(ctx, qkv, H, causal, scale, row_lo, row_hi, cached, keys=None):
         q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
         if cached is not None:
             out, lse = cached          # output and log-sum-exp kept from the first pass of a checkpointed block
         else:
-            out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi)
-        ctx.save_for_backward(qkv, out, lse, row_lo, row_hi)
+            out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, keys=keys)
+        ctx.save_for_backward(qkv, out, lse, row_lo, row_hi, *(keys if keys is not None else (None, None)))
         ctx.cfg = (H, causal, scale)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        qkv, out, lse, row_lo, row_hi = ctx.saved_tensors
+        qkv, out, lse, row_lo, row_hi, *keys = ctx.saved_tensors
         H, causal, scale = ctx.cfg
         q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
-        dqkv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, fused_out=True)
-        return dqkv, None, None, None, None, None, None
+        dqkv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, fused_out=True,
+                             keys=keys if keys[0] is not None else None)
+        return dqkv, None, None, None, None, None, None, None
 
 
 def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, softmax_scale=None,
@@ -480,10 +507,17 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
 
     B, S, _, D = qkv.shape
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
+    keys = None
+    padded = _padded_intervals(qkv, qkv, causal, scale, mask_kwargs.get("key_padding_mask"),
+                               [v for n, v in mask_kwargs.items() if n not in ("key_padding_mask", "dropout_p", "dropout_seed")],
+                               mask_kwargs.get("dropout_p", 0.0) > 0.0)
     try:
-        lo, hi = row_intervals(B, S, S, qkv.device, causal, mask_kwargs.get("glm_mask"),
-                               mask_kwargs.get("pack_glm_mask"), mask_kwargs.get("key_padding_mask"),
-                               mask_kwargs.get("cu_seqlens"))
+        if padded is not None:
+            lo, hi, keys = padded
+        else:
+            lo, hi = row_intervals(B, S, S, qkv.device, causal, mask_kwargs.get("glm_mask"),
+                                   mask_kwargs.get("pack_glm_mask"), mask_kwargs.get("key_padding_mask"),
+                                   mask_kwargs.get("cu_seqlens"))
     except NonContiguousKeyMask:
         H = num_heads
         return flash_attention(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], causal=causal,
@@ -495,7 +529,7 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
         if not is_recompute and not torch.is_grad_enabled():
             H = num_heads
             out, lse = flash_fwd_raw(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], bool(causal), float(scale),
-                                     lo, hi)
+                                     lo, hi, keys=keys)
             recompute_cache[token] = (out, lse)
             while len(recompute_cache) > RECOMPUTE_CACHE_LIMIT:
                 recompute_cache.popitem(last=False)
@@ -504,7 +538,7 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
             cached = recompute_cache.pop(token, None)
             if cached is not None and cached[0].shape != (B, S, num_heads, D):
                 cached = None
-    return _FlashAttnQKV.apply(qkv, num_heads, bool(causal), float(scale), lo, hi, cached)
+    return _FlashAttnQKV.apply(qkv, num_heads, bool(causal), float(scale), lo, hi, cached, keys)
 
 
 RECOMPUTE_CACHE_LIMIT = 16   # first passes in flight per layer (pipeline micro-batches) before eviction

@@ -437,3 +437,38 @@ def test_row_intervals_kernel_matches_the_tensor_operations(B, Sq, Sk, idx):
     before = _lib.launch_count
     flash.row_intervals(B, Sq, Sk, torch.device("cuda"), True, glm_mask=glm)
     assert _lib.launch_count == before + 1
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("S", [256, 300, 517])
+def test_key_padding_without_a_host_look(S, causal, D, monkeypatch):
+    """Right, left, empty and holed samples in one batch and without holes, in the kernels that test key bits and on
+    the host-decided path (unpadding): the same outputs and gradients, padded rows of a holed batch zero."""
+    g = torch.Generator().manual_seed(S + D)
+    B, Hq, Hkv = 4, 4, 2
+    pos = torch.arange(S)[None]
+    whole = torch.cat([pos < S - 40, pos >= 33, pos < 0, pos < S]).cuda()
+    holed = whole.clone()
+    holed[3] = (torch.rand(S, generator=g) < 0.6).cuda()
+    q, k, v, dout = (torch.randn(B, S, h, D, generator=g).bfloat16().cuda() for h in (Hq, Hkv, Hkv, Hq))
+    for kp in (whole, holed):
+        got, ref = [], []
+        for res, off in ((got, False), (ref, True)):
+            with monkeypatch.context() as m:
+                if off:
+                    m.setattr(flash, "_padded_intervals", lambda *a: None)
+                ins = [t.clone().requires_grad_(True) for t in (q, k, v)]
+                out = flash.flash_attention(*ins, causal=causal, key_padding_mask=kp)
+                res += [out.detach(), *torch.autograd.grad(out, ins, dout)]
+        torch.cuda.synchronize()
+        _lib.check_status(torch.device("cuda", 0))
+        for a, b in zip(got, ref):
+            # both paths round P, dS and the results to bf16 (2^-9 each) but cut the keys into other blocks
+            assert torch.isfinite(a).all() and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+        if kp is holed:
+            assert not got[0][~holed].any()
+        qkv = torch.cat([q[:, :, :2], k, v], 2)
+        fused = flash.flash_attention_qkv(qkv, 2, causal=causal, key_padding_mask=kp)
+        sep = flash.flash_attention(q[:, :, :2], k, v, causal=causal, key_padding_mask=kp)
+        assert torch.equal(fused, sep)
