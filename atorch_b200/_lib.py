@@ -42,6 +42,9 @@ SIGNATURES = {
     "atb_flash_fwd_v2": "pppppppiiiiilllifppipp",
     "atb_flash_fwd": "pppppppiiiiilllifpp",
     "atb_flash_bwd_split": "ppppppppppppiiiiillllllifppiipp",
+    "atb_invert_perm": "ppip",
+    "atb_moe_gather_sum": "pppipiiip",
+    "atb_moe_scatter_mul": "ppppippiiip",
     "atb_padded_intervals": "ppppppiiip",
     "atb_row_intervals": "pppiiiipipiippiip",
 }

@@ -16,6 +16,7 @@ from typing import List, Optional, Sequence, Tuple
 
 import torch
 
+from .. import _lib
 from .gemm import gemm, gemm_ragged, linear, ragged_ok
 
 
@@ -24,12 +25,76 @@ def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tenso
     return torch.bincount(expert_idx.reshape(-1), minlength=num_experts)
 
 
+def _rows_ok(rows: torch.Tensor, order: torch.Tensor) -> bool:
+    """Whether the row kernels (csrc/moe_local.cu) take these rows: bf16 on the GPU in 16-byte pieces, int64 order."""
+    return (_lib.use_kernels(rows, order) and rows.dtype == torch.bfloat16 and rows.dim() == 2 and rows.shape[1] % 8 == 0
+            and rows.shape[1] > 0 and order.dtype == torch.int64 and order.dim() == 1 and order.is_contiguous()
+            and 0 < order.numel() < 1 << 31)
+
+
+def _slots(order: torch.Tensor) -> torch.Tensor:
+    """Row of the sorted buffer of every (token, choice)."""
+    slot = torch.empty(order.numel(), dtype=torch.int32, device=order.device)
+    _lib.check(_lib.lib().atb_invert_perm(order.data_ptr(), slot.data_ptr(), order.numel(), _lib.stream()), "atb_invert_perm")
+    return slot
+
+
+def _gather_sum(rows, slot, w, T, k):
+    out = torch.empty(T, rows.shape[1], dtype=rows.dtype, device=rows.device)
+    rc = _lib.lib().atb_moe_gather_sum(rows.data_ptr(), slot.data_ptr(), _lib.addr(w), 0 if w is None else _lib.DT[w.dtype],
+                                       out.data_ptr(), T, k, rows.shape[1], _lib.stream())
+    _lib.check(rc, "atb_moe_gather_sum")
+    return out
+
+
+def _packed(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _Permute(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, tokens, order, k):
+        ctx.save_for_backward(order)
+        ctx.k, ctx.T = k, tokens.shape[0]
+        return tokens.index_select(0, order // k)
+
+    @staticmethod
+    def backward(ctx, dy):
+        (order,) = ctx.saved_tensors
+        return _gather_sum(_packed(dy), _slots(order), None, ctx.T, ctx.k), None, None
+
+
+class _Unpermute(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, rows, order, probs, k):
+        rows, slot = _packed(rows), _slots(order)
+        w = None if probs is None else probs.contiguous()
+        ctx.save_for_backward(rows, slot, w)
+        ctx.k, ctx.p_shape = k, None if probs is None else probs.shape
+        return _gather_sum(rows, slot, w, order.numel() // k, k)
+
+    @staticmethod
+    def backward(ctx, dout):
+        rows, slot, w = ctx.saved_tensors
+        dout, T, H = _packed(dout), slot.numel() // ctx.k, rows.shape[1]
+        drows = torch.empty_like(rows) if ctx.needs_input_grad[0] else None
+        dw = torch.empty_like(w) if w is not None and ctx.needs_input_grad[2] else None
+        rc = _lib.lib().atb_moe_scatter_mul(dout.data_ptr(), rows.data_ptr(), slot.data_ptr(), _lib.addr(w),
+                                            2 if w is None else _lib.DT[w.dtype], _lib.addr(drows), _lib.addr(dw), T, ctx.k,
+                                            H, _lib.stream())
+        _lib.check(rc, "atb_moe_scatter_mul")
+        return drows, None, None if dw is None else dw.view(ctx.p_shape), None
+
+
 def permute(tokens: torch.Tensor, expert_idx: torch.Tensor, num_out_tokens: Optional[int] = None
             ) -> Tuple[torch.Tensor, torch.Tensor]:
     """tokens ``[T, H]``, expert_idx ``[T, k]`` (or ``[T]``) -> (permuted ``[T*k, H]``, sorted_indices)."""
     k = expert_idx.shape[1] if expert_idx.dim() > 1 else 1
     flat = expert_idx.reshape(-1)
     sorted_idx = torch.argsort(flat, stable=True)
+    if num_out_tokens is None and _rows_ok(tokens, sorted_idx) and sorted_idx.numel() == tokens.shape[0] * k:
+        return _Permute.apply(tokens, sorted_idx, k), sorted_idx
     if num_out_tokens is not None:
         sorted_idx = sorted_idx[:num_out_tokens]
     return tokens.index_select(0, sorted_idx // k), sorted_idx
@@ -40,6 +105,14 @@ def unpermute(permuted: torch.Tensor, sorted_idx: torch.Tensor, probs: Optional[
     """Inverse of :func:`permute`: ``[T*k, H] -> [T, H]`` with optional prob-weighted sum over k."""
     n_slots = (num_tokens * topk) if num_tokens is not None else (probs.numel() if probs is not None
                                                                    else sorted_idx.numel())
+    if topk >= 1 and _rows_ok(permuted, sorted_idx) and n_slots == sorted_idx.numel() == permuted.shape[0] \
+            and n_slots % topk == 0 and (probs is None or (probs.numel() == n_slots and probs.is_cuda
+                                                           and probs.dtype in (torch.bfloat16, torch.float32))):
+        return _Unpermute.apply(permuted, sorted_idx, probs, topk)
+    return unpermute_reference(permuted, sorted_idx, probs, topk, n_slots)
+
+
+def unpermute_reference(permuted, sorted_idx, probs, topk, n_slots):
     out = torch.zeros(n_slots, permuted.shape[-1], dtype=permuted.dtype, device=permuted.device)
     out = out.index_copy(0, sorted_idx, permuted)
     out = out.view(-1, topk, permuted.shape[-1])

@@ -260,3 +260,28 @@ def test_grouped_gemm_ragged_groups(sizes, trans_b):
         dw = xs.t() @ ds
         _check(w.grad[g], dw.t() if trans_b else dw, max(n, 1))
         r += n
+
+
+@pytest.mark.parametrize("T,H,E,k", [(1, 8, 4, 1), (37, 264, 4, 2), (513, 4096, 8, 2), (64, 2048, 8, 3)])
+@pytest.mark.parametrize("probs", [torch.bfloat16, torch.float32, None])
+def test_permute_unpermute_row_kernels(T, H, E, k, probs):
+    """Row movement of a routed layer and its gradients against the tensor operations in fp32 (one bf16 rounding each)."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(T)
+    x, dout = _mk(T, H).requires_grad_(True), _mk(T, H)
+    idx = torch.rand(T, E, device="cuda").topk(k, dim=-1).indices
+    p = None if probs is None else torch.rand(T, k, device="cuda").to(probs).requires_grad_(True)
+    rows, order = M.permute(x, idx)
+    assert torch.equal(rows, x.detach()[order // k])
+    scaled = rows * 2.0
+    out = M.unpermute(scaled, order, p, k, T)
+    got = torch.autograd.grad(out, [x, scaled] + ([p] if p is not None else []), dout)
+    xf = x.detach().float().requires_grad_(True)
+    pf = None if p is None else p.detach().float().requires_grad_(True)
+    sf = xf[order // k] * 2.0
+    of = M.unpermute_reference(sf, order, pf, k, T * k)
+    ref = torch.autograd.grad(of, [xf, sf] + ([pf] if p is not None else []), dout.float())
+    for a, b in zip([out.detach(), *got], [of.detach(), *ref]):
+        # dx passes three bf16 roundings (drows, its double, the sum), everything else one
+        assert a.shape == b.shape and (a.float() - b).norm() <= 2 ** -7 * b.norm() + 1e-6
