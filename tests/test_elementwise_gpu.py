@@ -228,3 +228,40 @@ def test_sum_squares_lengths_and_alignment(n, dtype):
     for x in (buf[:n], buf[1:]):
         ref = x.double().square().sum()
         assert abs(ops.sum_squares(x).double() - ref) <= 1e-5 * ref
+
+
+@pytest.mark.parametrize("M,N,dtype", [(1, 2048, torch.bfloat16), (297, 8, torch.float16), (1187, 2048, torch.bfloat16),
+                                       (1187, 2056, torch.bfloat16), (600, 4104, torch.float16),
+                                       (300, 8192, torch.bfloat16), (1187, 2048, torch.float32),
+                                       (599, 4096, torch.float32), (300, 8192, torch.float32)])
+@pytest.mark.parametrize("layernorm", [False, True])
+def test_norm_backward_row_pairs(M, N, dtype, layernorm):
+    """Backward kernels at the edges of their row pairs (odd chunks, empty chunks, one row) and of each row length, with
+    the residual gradient, against 64 bits. Inputs are exact in both, so what is left in dx is its own rounding (eps / 2) and the
+    fp32 sums (a few N-term sums, taken as 16 times the fp32 eps); dw is rounded once more on its way to the parameter."""
+    from atorch_b200 import _lib
+
+    torch.manual_seed(M + N)
+    x, dy, dres = (torch.randn(M, N, device="cuda").to(dtype) for _ in range(3))
+    w = (1 + 0.1 * torch.randn(N, device="cuda")).to(dtype)
+    xd, wd, dyd = x.double(), w.double(), dy.double()
+    mean = xd.mean(-1) if layernorm else torch.zeros(M, device="cuda", dtype=torch.float64)
+    rstd = ((xd - mean[:, None]).pow(2).mean(-1) + 1e-5).rsqrt()
+    mean, rstd = mean.float(), rstd.float()
+    xh = (xd - mean.double()[:, None]) * rstd.double()[:, None]
+    g = dyd * wd
+    ref = (g - xh * (g * xh).mean(-1, keepdim=True) - (g.mean(-1, keepdim=True) if layernorm else 0)) * rstd.double()[:, None]
+    ref = ref + dres.double()
+    parts = _lib.lib().atb_norm_bwd_parts(M)
+    dx, pw, pb = torch.full_like(x, float("nan")), torch.full((parts, N), float("nan"), device="cuda"), None
+    pb = torch.full_like(pw, float("nan")) if layernorm else None
+    rc = _lib.lib().atb_norm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+                                 dres.data_ptr(), dx.data_ptr(), pw.data_ptr(), _lib.addr(pb), parts, M, N, int(layernorm),
+                                 _lib.DT[dtype], _lib.stream())
+    assert rc == 0
+    eps32 = torch.finfo(torch.float32).eps
+    assert (dx.double() - ref).norm() <= (torch.finfo(dtype).eps / 2 + 16 * eps32) * ref.norm()
+    dw = (dyd * xh).sum(0)
+    assert (pw.double().sum(0) - dw).norm() <= 16 * eps32 * max(1.0, M ** 0.5) * dw.norm()
+    if layernorm:
+        assert (pb.double().sum(0) - dyd.sum(0)).norm() <= 16 * eps32 * max(1.0, M ** 0.5) * dyd.sum(0).norm()
