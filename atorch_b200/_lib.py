@@ -32,6 +32,7 @@ SIGNATURES = {
     "atb_gemm_bf16_2cta_grouped": "ppppiiillliiiifiiplpiiiiipp",
     "atb_gemm_bf16": "ppppiiillliiiifiiplpp",
     "atb_gemm_bf16_2cta_swiglu": "ppppiiillllpp",
+    "atb_gemm_bf16_2cta_rope": "pppiiilllpppiiipp",
     "atb_gemm_bf16_2cta_ragged": "pppiiilllipipp",
     "atb_norm_fwd": "ppppppppiifiip",
     "atb_norm_bwd": "pppppppppiiiiip",

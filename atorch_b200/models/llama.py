@@ -8,8 +8,7 @@ from the Hugging Face parameter names (``q_proj``, ``k_proj``, ``v_proj``, ``gat
 
 Per-layer dataflow (all bf16, fp32 accumulation inside the kernels):
     x   = rms_norm(h)                      csrc/norm.cu
-    qkv = x @ Wqkv^T                       csrc/gemm_bf16.cu
-    qkv = rope(qkv) on the q and k heads   csrc/elementwise.cu
+    qkv = rope(x @ Wqkv^T), q and k heads   csrc/gemm_bf16_2cta.cu (epilogue)
     a   = attention(q, k, v, causal)       csrc/flash_attn.cu
     h   = h + a @ Wo^T                     GEMM epilogue accumulates into the residual stream
     x   = rms_norm(h)
@@ -146,9 +145,12 @@ class LlamaDecoderLayer(nn.Module):
         # are added inside the norm's backward kernel
         pre = type(self.input_layernorm) is RMSNorm and type(self.post_attention_layernorm) is RMSNorm
         x, h = self.input_layernorm(h, carry=True) if pre else (self.input_layernorm(h), h)
-        qkv = self._proj(self.qkv_proj, x)
-        S = qkv.shape[1]      # the projection may have gathered a sequence-sharded input (sequence parallelism)
-        qkv = ops.rope(qkv, cos, sin, self.n_q + self.n_kv, d, positions, inplace=True)   # qkv is read by nothing else
+        if type(self.qkv_proj) is nn.Linear and self.qkv_proj.bias is None:
+            qkv = ops.linear_rope(x, self.qkv_proj.weight, cos, sin, self.n_q + self.n_kv, d, positions)
+        else:
+            qkv = self._proj(self.qkv_proj, x)
+            S = qkv.shape[1]  # the projection may have gathered a sequence-sharded input (sequence parallelism)
+            qkv = ops.rope(qkv, cos, sin, self.n_q + self.n_kv, d, positions, inplace=True)  # read by nothing else
         qkv = qkv.view(B, S, self.n_q + 2 * self.n_kv, d)
         q = qkv[:, :, : self.n_q]
         k = qkv[:, :, self.n_q: self.n_q + self.n_kv]

@@ -249,6 +249,61 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return _LinearSwiGLU.apply(x, weight)
 
 
+class _LinearRope(torch.autograd.Function):
+    """``rope(x @ W^T)`` with the rotation in the GEMM epilogue; its backward rotates the incoming gradient back (in place
+    where it is a contiguous temporary, as ``rope(..., inplace=True)`` does) in front of the projection's products."""
+
+    @staticmethod
+    def forward(ctx, x, weight, cos, sin, positions, nheads, head_dim):
+        shp = x.shape
+        x2 = x.reshape(-1, shp[-1])
+        x2 = x2 if x2.stride(-1) == 1 else x2.contiguous()
+        T, K = x2.shape
+        N = weight.shape[0]
+        out = torch.empty(T, N, dtype=x2.dtype, device=x2.device)
+        rc = _lib.lib().atb_gemm_bf16_2cta_rope(
+            x2.data_ptr(), weight.data_ptr(), out.data_ptr(), T, N, K, _pitch(x2), _pitch(weight), N, cos.data_ptr(),
+            sin.data_ptr(), _lib.addr(positions), cos.shape[0], nheads, head_dim, _lib.stream(), _lib.status_addr(x2))
+        _lib.check(rc, f"atb_gemm_bf16_2cta_rope T={T} N={N} K={K}")
+        ctx.save_for_backward(x2, weight, cos, sin, positions)
+        ctx.x_shape, ctx.weight_ref, ctx.heads = shp, weight, (nheads, head_dim)
+        return out.view(*shp[:-1], N)
+
+    @staticmethod
+    def backward(ctx, dy):
+        from .elementwise import _rope_launch
+
+        x2, weight, cos, sin, positions = ctx.saved_tensors
+        dy = dy if dy.is_contiguous() else dy.contiguous()
+        dy2 = dy.view(-1, dy.shape[-1])
+        _rope_launch(dy2, dy2, cos, sin, positions, *ctx.heads, True)
+        dx, dw = _linear_grads(ctx, dy2, x2, weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return dx, dw, None, None, None, None, None
+
+
+def linear_rope(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, nheads: int, head_dim: int,
+                positions: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=True)`` in one kernel where the pair kernel
+    runs (from 256 tokens on) and whole 128-column halves of its tiles are rotated or not."""
+    from .elementwise import rope
+
+    T = x.numel() // max(x.shape[-1], 1)
+    if not (x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _lib.use_kernels(x, weight, cos, sin, positions)
+            and PAIR_KERNEL_DEFAULT and T >= 256 and head_dim in (64, 128) and weight.dim() == 2
+            and weight.shape[1] == x.shape[-1] and weight.shape[0] % 128 == 0
+            and (nheads * head_dim) % 128 == 0 and 0 < nheads * head_dim <= weight.shape[0] and x.shape[-1] % 8 == 0
+            and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0 and weight.data_ptr() % 16 == 0
+            and x.data_ptr() % 16 == 0 and (x.dim() < 2 or x.is_contiguous()) and cos.dtype == torch.float32
+            and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+            and cos.shape == sin.shape and cos.dim() == 2 and cos.shape[1] == head_dim // 2
+            and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0
+            and (positions is None or (positions.numel() == T and positions.is_contiguous()))):
+        return rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=True)
+    if positions is not None and positions.dtype != torch.int32:
+        positions = positions.to(torch.int32)
+    return _LinearRope.apply(x, weight, cos, sin, positions, nheads, head_dim)
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, residual):

@@ -285,3 +285,30 @@ def test_permute_unpermute_row_kernels(T, H, E, k, probs):
     for a, b in zip([out.detach(), *got], [of.detach(), *ref]):
         # dx passes three bf16 roundings (drows, its double, the sum), everything else one
         assert a.shape == b.shape and (a.float() - b).norm() <= 2 ** -7 * b.norm() + 1e-6
+
+
+@pytest.mark.parametrize("T,K,heads,kv,D", [(256, 128, 2, 1, 128), (777, 264, 4, 2, 128), (300, 512, 4, 2, 64),
+                                            (1000, 256, 3, 3, 128)])
+@pytest.mark.parametrize("with_pos", [False, True])
+def test_linear_rope_epilogue(T, K, heads, kv, D, with_pos):
+    """Projection and rotation in one kernel against the two in fp32; the rounding of the projection is saved, so one
+    bf16 rounding (2^-9) of the values and of the gradients remains. Heads past the rotated ones stay as they are."""
+    from atorch_b200.ops import linear_rope, rope_reference, rope_tables
+
+    torch.manual_seed(T)
+    N = (heads + 2 * kv) * D
+    x, w, dy = _mk(T, K).view(1, T, K).requires_grad_(True), (_mk(N, K) * 0.1).requires_grad_(True), _mk(T, N).view(1, T, N)
+    pos = torch.randint(0, 2 * T, (1, T), device="cuda") if with_pos else None
+    cos, sin = rope_tables(2 * T if with_pos else T, D, device="cuda")
+    before = _lib.launch_count
+    out = linear_rope(x, w, cos, sin, heads + kv, D, pos)
+    rotated = (heads + kv) * D % 128 == 0 and N % 128 == 0
+    assert _lib.launch_count - before == (1 if rotated else 2)
+    got = torch.autograd.grad(out, [x, w], dy.clone())
+    xf, wf = x.detach().float().requires_grad_(True), w.detach().float().requires_grad_(True)
+    ref = rope_reference(xf @ wf.t(), cos, sin, heads + kv, D, pos)
+    rg = torch.autograd.grad(ref, [xf, wf], dy.float())
+    torch.cuda.synchronize()
+    _lib.check_status(out.device)
+    for a, b in zip([out.detach(), *got], [ref.detach(), *rg]):
+        assert (a.float() - b).norm() <= 2 ** -7 * b.norm()
