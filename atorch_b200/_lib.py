@@ -33,7 +33,7 @@ SIGNATURES = {
     "atb_gemm_bf16": "ppppiiillliiiifiiplpp",
     "atb_gemm_bf16_2cta_swiglu": "ppppiiillllpp",
     "atb_gemm_bf16_2cta_rope": "pppiiilllpppiiipp",
-    "atb_gemm_bf16_2cta_ragged": "pppiiilllipipp",
+    "atb_gemm_bf16_2cta_ragged": "pppiiilllipiippp",
     "atb_norm_fwd": "ppppppppiifiip",
     "atb_norm_bwd": "pppppppppiiiiip",
     "atb_colsum": "ppiiiip",

@@ -423,7 +423,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int am0 = m0 + (int)rank * BM;   // this CTA's rows of A
         const int bshift = b_idx * grp.b_rows;   // this expert's own B
         // this CTA's rows of B (gated: CTA 0 takes gate rows, CTA 1 the up rows of the same features)
-        const int bn0 = ep.gated ? n0 + (int)rank * N : n0 + (int)rank * BNH + (B_MN ? 0 : bshift);
+        const int bn0 = n0 + (int)rank * (ep.gated ? N : BNH) + (B_MN ? 0 : bshift);
         const int bk0 = B_MN ? bshift : 0;
         if (gate.flags != nullptr) {
           bool here = true;
@@ -778,7 +778,8 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     ok = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, b_extent_rows > 0 ? b_extent_rows : N, K, ldb,
                       Cfg<BN>::BNH, BK, CU_TENSOR_MAP_SWIZZLE_128B);
   else
-    ok = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, b_extent_rows > 0 ? b_extent_rows : K, N, ldb, BK,
+    ok = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, b_extent_rows > 0 ? b_extent_rows : K,
+                      ep.gated ? 2 * N : N, ldb, BK,
                       64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (!ok) return -3;
   Epi epw = ep;
@@ -910,12 +911,19 @@ extern "C" int atb_gemm_bf16_2cta(const void* A, const void* B, void* C, const v
 // numbers of rows, and a launch of its own leaves 74 CTA pairs with a short last wave once per expert. Forward and
 // backward of the expert MLP 8 x 14336 x 4096 on 8192 routed rows: 9.9 ms, against 148 ms when every group whose
 // length is no multiple of 8 took the fp32 fallback and w2 was transposed by a copy first.
+// gated: every operand holds gate | up features (2 N of them), C [M, N] is silu(gate) * up and gu_out, if given,
+// [M, 2 N] the two as they are, as in atb_gemm_bf16_2cta_swiglu below. Against this
+// launch and the SwiGLU kernel after it, cold L2: 8192 rows, 8 x 14336 x 4096 1687 -> 1541 us, 4000 rows, 4 x 9024 x 4096
+// 490 -> 450, 1000 rows, 4 x 8192 x 2048 103 -> 97.
 extern "C" int atb_gemm_bf16_2cta_ragged(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                                          long long ldb, long long ldc, int b_mn_major, const int* sizes, int n_groups,
-                                         void* stream, int* status) {
+                                         int gated, void* gu_out, void* stream, int* status) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((N & 7) || (lda & 7) || (ldb & 7) || (ldc & 7)) return -1;
-  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -1;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C) |
+       reinterpret_cast<uintptr_t>(gu_out)) & 15)
+    return -1;
+  const int b_cols = gated ? 2 * N : N;
   if (n_groups < 1 || n_groups > RAGGED_MAX || (b_mn_major && (K % BK))) return -1;
   Ragged rag = {};
   rag.n = n_groups;
@@ -925,13 +933,13 @@ extern "C" int atb_gemm_bf16_2cta_ragged(const void* A, const void* B, void* C, 
     rag.mt0[g + 1] = rag.mt0[g] + (sizes[g] + 2 * BM - 1) / (2 * BM);
   }
   if (rag.row0[n_groups] != M) return -1;
-  Epi ep{C, nullptr, ldc, 1.f, 0, 0, nullptr, 0, {nullptr}, 0, 0, nullptr, 0};
-  Groups grp{nullptr, 0, b_mn_major ? K : N, 0, 0};
+  Epi ep{C, nullptr, ldc, 1.f, 0, 0, nullptr, 0, {nullptr}, 0, gated != 0, gated ? gu_out : nullptr, b_cols};
+  Groups grp{nullptr, 0, b_mn_major ? K : b_cols, 0, 0};
   Gate gate{nullptr, 0u, 1, 0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (b_mn_major)
     return launch<256, false, true>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * K, gate, rag, st, status);
-  return launch<256, false, false>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * N, gate, rag, st, status);
+  return launch<256, false, false>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * b_cols, gate, rag, st, status);
 }
 
 // out[M, N] = rope(x W^T): the projection onto fused q | k | v heads with the first rope_heads heads of head_dim (128 or

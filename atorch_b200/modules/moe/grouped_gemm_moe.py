@@ -130,6 +130,8 @@ class Grouped_GEMM_MoE(nn.Module):
             return self.compute_expert_slots(x, tokens_per_expert)
         sizes = tokens_per_expert.tolist()
         w1, w2 = self._scaled(self.w1), self._scaled(self.w2)
+        if self.use_swiglu and self.v1 is None and not self.use_bias and not self.fp8:
+            return self._gmm(moe_ops.grouped_gemm_swiglu(x, w1, sizes, trans_b=self.transpose_w1), w2, sizes, False)
         h = self._gmm(x, w1, sizes, self.transpose_w1)
         if self.use_bias:
             eidx = torch.repeat_interleave(torch.arange(len(sizes), device=x.device), tokens_per_expert)

@@ -166,17 +166,22 @@ def ragged_ok(x: torch.Tensor, w: torch.Tensor, b_mn: bool, n_groups: int) -> bo
             and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
-def gemm_ragged(x: torch.Tensor, w: torch.Tensor, sizes, b_mn: bool) -> torch.Tensor:
+def gemm_ragged(x: torch.Tensor, w: torch.Tensor, sizes, b_mn: bool, gated: bool = False, keep_gate_up: bool = False):
     """Rows of ``x`` in consecutive groups of ``sizes`` rows (host numbers), group ``g`` times ``w[g]`` (``[K, N]``)
-    when ``b_mn`` else times ``w[g]^T`` (``[N, K]``): one launch for all groups. See :func:`ragged_ok`."""
+    when ``b_mn`` else times ``w[g]^T`` (``[N, K]``): one launch for all groups. See :func:`ragged_ok`.
+
+    ``gated``: the weights hold gate | up features; returns ``(silu(gate) * up, gate | up)``, the second only with
+    ``keep_gate_up`` (else None)."""
     M, K = x.shape
     N = w.shape[2] if b_mn else w.shape[1]
+    N = N // 2 if gated else N
     out = torch.empty(M, N, dtype=x.dtype, device=x.device)
+    gu = torch.empty(M, 2 * N, dtype=x.dtype, device=x.device) if gated and keep_gate_up else None
     rc = _lib.lib().atb_gemm_bf16_2cta_ragged(
         x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _pitch(x), w.shape[2], N, int(b_mn),
-        (ctypes.c_int * len(sizes))(*sizes), len(sizes), _lib.stream(), _lib.status_addr(x))
+        (ctypes.c_int * len(sizes))(*sizes), len(sizes), int(gated), _lib.addr(gu), _lib.stream(), _lib.status_addr(x))
     _lib.check(rc, f"atb_gemm_bf16_2cta_ragged M={M} N={N} K={K} groups={len(sizes)}")
-    return out
+    return (out, gu) if gated else out
 
 
 def _linear_grads(ctx, dy2, x2, weight, need_dx, need_dw):

@@ -17,6 +17,7 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 
 from .. import _lib
+from .elementwise import swiglu, swiglu_backward
 from .gemm import gemm, gemm_ragged, linear, ragged_ok
 
 
@@ -145,17 +146,15 @@ class _GroupedLinear(torch.autograd.Function):
         return _GroupedLinear._rows(x, w, sizes, b_mn)
 
     @staticmethod
-    def backward(ctx, dy):
-        x, w = ctx.saved_tensors
-        dy = dy.contiguous()
-        dx = _GroupedLinear._rows(dy, w, ctx.sizes, not ctx.b_mn).to(x.dtype) if ctx.needs_input_grad[0] else None
-        if not ctx.needs_input_grad[1]:
-            return dx, None, None, None
+    def _grads(x, w, dy, sizes, b_mn, need_dx, need_dw):
+        dx = _GroupedLinear._rows(dy, w, sizes, not b_mn).to(x.dtype) if need_dx else None
+        if not need_dw:
+            return dx, None
         mg = getattr(w, "main_grad", None)
         dw = mg if mg is not None else torch.empty(w.shape, dtype=w.dtype, device=w.device)
-        a, b = (x, dy) if ctx.b_mn else (dy, x)         # dW[g] = a[g]^T b[g]
+        a, b = (x, dy) if b_mn else (dy, x)             # dW[g] = a[g]^T b[g]
         r = 0
-        for g, n in enumerate(ctx.sizes):
+        for g, n in enumerate(sizes):
             if n:
                 gemm(a[r: r + n], b[r: r + n], a_mn=True, b_mn=True, out=dw[g], accumulate=mg is not None)
             elif mg is None:
@@ -163,8 +162,33 @@ class _GroupedLinear(torch.autograd.Function):
             r += n
         if mg is not None:
             w.grad_added_to_main_grad = True
-            return dx, None, None, None
-        return dx, dw, None, None
+            return dx, None
+        return dx, dw
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w = ctx.saved_tensors
+        return (*_GroupedLinear._grads(x, w, dy.contiguous(), ctx.sizes, ctx.b_mn, *ctx.needs_input_grad[:2]), None, None)
+
+
+class _GroupedSwiGLU(torch.autograd.Function):
+    """``swiglu`` of :class:`_GroupedLinear` with the activation in the epilogue of its one launch. The gate | up rows
+    are written only when there is a gradient to come."""
+
+    @staticmethod
+    def forward(ctx, x, w, sizes: Tuple[int, ...], b_mn: bool):
+        need = ctx.needs_input_grad[0] or ctx.needs_input_grad[1]
+        act, gu = gemm_ragged(x, w, sizes, b_mn, gated=True, keep_gate_up=need)
+        if need:
+            ctx.save_for_backward(x, w, gu)
+        ctx.sizes, ctx.b_mn = sizes, b_mn
+        return act
+
+    @staticmethod
+    def backward(ctx, dact):
+        x, w, gu = ctx.saved_tensors
+        return (*_GroupedLinear._grads(x, w, swiglu_backward(gu, dact), ctx.sizes, ctx.b_mn, *ctx.needs_input_grad[:2]),
+                None, None)
 
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, batch_sizes, trans_b: bool = False) -> torch.Tensor:
@@ -173,3 +197,16 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, batch_sizes, trans_b: bool = 
     sizes = tuple(int(s) for s in (batch_sizes.tolist() if isinstance(batch_sizes, torch.Tensor) else batch_sizes))
     assert sum(sizes) == a.shape[0], "batch_sizes must cover all rows"
     return _GroupedLinear.apply(a, b, sizes, not trans_b)
+
+
+def grouped_gemm_swiglu(a: torch.Tensor, b: torch.Tensor, batch_sizes, trans_b: bool = False) -> torch.Tensor:
+    """``swiglu(grouped_gemm(a, b, batch_sizes, trans_b))`` for weights of gate | up features, in one kernel where the
+    ragged launch takes the operands and the features come in 16-byte pieces (which the separate kernel needs too)."""
+    N = b.shape[-2] if trans_b else b.shape[-1]
+    if a.dim() == 2 and b.dim() == 3 and N % 16 == 0 and ragged_ok(a, b, not trans_b, b.shape[0]):
+        sizes = tuple(int(s) for s in (batch_sizes.tolist() if isinstance(batch_sizes, torch.Tensor) else batch_sizes))
+        assert sum(sizes) == a.shape[0], "batch_sizes must cover all rows"
+        if len(sizes) == b.shape[0]:
+            return _GroupedSwiGLU.apply(a, b, sizes, not trans_b)
+        batch_sizes = sizes
+    return swiglu(grouped_gemm(a, b, batch_sizes, trans_b))

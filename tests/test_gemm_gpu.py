@@ -312,3 +312,34 @@ def test_linear_rope_epilogue(T, K, heads, kv, D, with_pos):
     _lib.check_status(out.device)
     for a, b in zip([out.detach(), *got], [ref.detach(), *rg]):
         assert (a.float() - b).norm() <= 2 ** -7 * b.norm()
+
+
+@pytest.mark.parametrize("sizes", [(256, 0, 1, 300), (77,), (0, 5, 511, 512, 513, 1)])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("N", [16, 272])
+def test_grouped_gemm_swiglu_epilogue(sizes, trans_b, N):
+    """The activation in the epilogue of the ragged launch: it rounds gate and up and uses the formula of the separate
+    kernel, so results and gradients are the same bits; feature counts that are no multiple of the 128-column tile put
+    columns of the other half, or of the next group, into the last tile."""
+    from atorch_b200.ops import swiglu
+    from atorch_b200.ops.moe import grouped_gemm, grouped_gemm_swiglu
+
+    torch.manual_seed(sum(sizes))
+    G, K = len(sizes), 192
+    x = _mk(sum(sizes), K)
+    w = (torch.randn(G, 2 * N, K, device="cuda") if trans_b else torch.randn(G, K, 2 * N, device="cuda")).bfloat16()
+    dy = _mk(sum(sizes), N)
+    res = []
+    for f in (grouped_gemm_swiglu, lambda *a: swiglu(grouped_gemm(*a))):
+        xs, ws = x.clone().requires_grad_(True), w.clone().requires_grad_(True)
+        before = _lib.launch_count
+        y = f(xs, ws, sizes, trans_b)
+        assert _lib.launch_count - before == (1 if f is grouped_gemm_swiglu else 2)
+        y.backward(dy)
+        with torch.no_grad():
+            assert torch.equal(f(xs, ws, sizes, trans_b), y)
+        res.append((y.detach(), xs.grad, ws.grad))
+    torch.cuda.synchronize()
+    _lib.check_status(x.device)
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
