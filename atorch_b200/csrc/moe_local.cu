@@ -2,6 +2,7 @@
 // of the expert-sorted buffer that holds choice j of token t (-1: none).
 //   gather_sum    out[t] = sum_j w[t, j] src[slot_of[t, j]]     unpermute forward (w = routing probabilities) and
 //                                                               permute backward (no w)
+//   gather_rows   out[i] = src[order[i] / k]                    permute forward
 //   scatter_mul   dsrc[slot_of[t, j]] = w[t, j] dout[t],  dw[t, j] = <dout[t], src[slot_of[t, j]]>   unpermute backward
 // Bound by memory, one pass each with 16-byte pieces and fp32 sums. As tensor operations (zeros, index_copy, product,
 // sum; index_add with atomics backward) this was 13 passes over [T k, H]: for 4096 tokens, top 2, H = 4096 0.75 ms of an
@@ -84,6 +85,84 @@ __global__ void __launch_bounds__(256) scatter_mul_kernel(const __nv_bfloat16* _
   }
 }
 
+// Stable counting sort of n routed expert ids by one block: counts[e], order (the sorted positions) and slot, its inverse.
+// Every warp owns a run of the ids and walks it twice, 32 ids a step: lanes with the same id find each other by
+// match_any, so a step adds each id once (first walk, the warp's histogram) or hands out consecutive places (second walk).
+// Between the walks the histograms become starting places, expert by expert and warp by warp within an expert. Bound by
+// latency: the ids of 8 steps are loaded together. Ids outside [0, E) are counted nowhere and go to the end.
+// 8192 ids of 8 experts: 10 us, in place of a histogram (with a host synchronisation of its own), a radix sort of 64-bit
+// keys and two inversions, 32 launches and 100 us of device time. Forward and backward of 8 experts of 4096 x 1024 on
+// 131 tokens 1200 -> 760 us, of 4 x 8192 x 2048 on 1000 tokens 1000 -> 700. The block takes 84 us for
+// 32768 ids of 256 experts (34 us for 8 experts), by then no less device time than the sort's launches: the limit.
+constexpr int ROUTE_MAX_E = 256, ROUTE_MAX_N = 32768, ROUTE_STEPS = 8;
+__global__ void __launch_bounds__(1024) route_kernel(const long long* __restrict__ idx, int n, int E,
+                                                     long long* __restrict__ counts, long long* __restrict__ order,
+                                                     int* __restrict__ slot) {
+  __shared__ int place[32][ROUTE_MAX_E + 1];
+  __shared__ int scan[2][ROUTE_MAX_E + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int run = ((n + 31) / 32 + 31) / 32 * 32;      // ids per warp, whole steps
+  const int lo = min(n, warp * run), hi = min(n, lo + run);
+  for (int i = threadIdx.x; i < 32 * (ROUTE_MAX_E + 1); i += 1024) (&place[0][0])[i] = 0;
+  __syncthreads();
+  auto walk = [&](auto&& step) {
+    for (int base = lo; base < hi; base += 32 * ROUTE_STEPS) {
+      int e[ROUTE_STEPS];
+#pragma unroll
+      for (int s = 0; s < ROUTE_STEPS; ++s) {
+        const int i = base + s * 32 + lane;
+        const long long v = i < hi ? idx[i] : 0;
+        e[s] = i >= hi ? -1 : v < 0 || v >= E ? E : (int)v;
+      }
+#pragma unroll
+      for (int s = 0; s < ROUTE_STEPS; ++s) {
+        const unsigned same = __match_any_sync(0xffffffffu, e[s]);
+        step(base + s * 32 + lane, e[s], same);
+        __syncwarp();
+        if (e[s] >= 0 && lane == __ffs(same) - 1) place[warp][e[s]] += __popc(same);
+        __syncwarp();
+      }
+    }
+  };
+  walk([](int, int, unsigned) {});
+  __syncthreads();
+  const int b = threadIdx.x;
+  int total = 0;
+  if (b <= E) {
+    for (int w = 0; w < 32; ++w) {
+      const int c = place[w][b];
+      place[w][b] = total;
+      total += c;
+    }
+    scan[0][b] = total;
+    if (b < E) counts[b] = total;
+  }
+  __syncthreads();
+  int cur = 0;
+  for (int d = 1; d <= E; d <<= 1, cur ^= 1) {         // inclusive scan over the experts
+    if (b <= E) scan[cur ^ 1][b] = scan[cur][b] + (b >= d ? scan[cur][b - d] : 0);
+    __syncthreads();
+  }
+  if (b <= E) {
+    const int first = scan[cur][b] - total;
+    for (int w = 0; w < 32; ++w) place[w][b] += first;
+  }
+  __syncthreads();
+  walk([&](int i, int e, unsigned same) {
+    if (e >= 0) {
+      const int p = place[warp][e] + __popc(same & ((1u << lane) - 1));
+      order[p] = i;
+      slot[i] = p;
+    }
+  });
+}
+
+__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ src, const long long* __restrict__ order,
+                                                          uint4* __restrict__ out, int k, int pieces) {
+  const long long s = order[blockIdx.x] / k;
+  for (int c = threadIdx.x; c < pieces; c += 256) out[(long long)blockIdx.x * pieces + c] = src[s * pieces + c];
+}
+
 bool aligned16(const void* a, const void* b, const void* c) {
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
@@ -95,6 +174,22 @@ extern "C" int atb_invert_perm(const long long* order, int* slot_of, int n, void
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemsetAsync(slot_of, 0xff, (size_t)n * 4, st) != cudaSuccess) return -5;
   invert_perm_kernel<<<(n + 255) / 256, 256, 0, st>>>(order, slot_of, n);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// counts [E], order [n] int64, slot [n] int32 from idx [n]; n at most 32768, E at most 256.
+extern "C" int atb_moe_sort_ids(const long long* idx, int n, int E, long long* counts, long long* order, int* slot,
+                             void* stream) {
+  if (n < 0 || n > ROUTE_MAX_N || E < 1 || E > ROUTE_MAX_E) return -1;
+  route_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>(idx, n, E, counts, order, slot);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+// out[i] = src[order[i] / k] for n rows of H bf16; order names rows of src (0 <= order[i] / k < rows).
+extern "C" int atb_moe_gather_rows(const void* src, const long long* order, void* out, int n, int k, int H, void* stream) {
+  if (n <= 0 || H <= 0) return 0;
+  if ((H & 7) || k < 1 || !aligned16(src, out, nullptr)) return -1;
+  gather_rows_kernel<<<n, 256, 0, (cudaStream_t)stream>>>((const uint4*)src, order, (uint4*)out, k, H / 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 

@@ -129,6 +129,7 @@ class Grouped_GEMM_MoE(nn.Module):
         if self.peer_exchange:
             return self.compute_expert_slots(x, tokens_per_expert)
         sizes = tokens_per_expert.tolist()
+        assert sum(sizes) == x.shape[0], "every row must belong to an expert (an expert id is out of range)"
         w1, w2 = self._scaled(self.w1), self._scaled(self.w2)
         if self.use_swiglu and self.v1 is None and not self.use_bias and not self.fp8:
             return self._gmm(moe_ops.grouped_gemm_swiglu(x, w1, sizes, trans_b=self.transpose_w1), w2, sizes, False)

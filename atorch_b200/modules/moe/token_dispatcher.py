@@ -31,8 +31,8 @@ class MoEAllToAllTokenDispatcher:
         self.probs = probs
         x = hidden_states.reshape(-1, hidden_states.shape[-1])
         self.num_tokens = x.shape[0]
-        counts = moe_ops.tokens_per_expert(indices, self.num_experts)             # [E] global ids
-        permuted, self.sorted_idx = moe_ops.permute(x, indices)
+        # counts: [E] global ids
+        counts, permuted, self.sorted_idx, self.slots = moe_ops.route(x, indices, self.num_experts)
         se_out = None
         if self.ep_size == 1:
             if se_fn1 is not None:
@@ -71,7 +71,7 @@ class MoEAllToAllTokenDispatcher:
         if se_fn2 is not None:
             se_out = se_fn2(*se_fn2_additional_input) if isinstance(se_fn2_additional_input, (tuple, list)) \
                 else se_fn2(se_fn2_additional_input)
-        out = moe_ops.unpermute(expert_output, self.sorted_idx, self.probs, self.topk, self.num_tokens)
+        out = moe_ops.unpermute(expert_output, self.sorted_idx, self.probs, self.topk, self.num_tokens, self.slots)
         return out.view(self.hidden_shape), se_out
 
 

@@ -343,3 +343,45 @@ def test_grouped_gemm_swiglu_epilogue(sizes, trans_b, N):
     _lib.check_status(x.device)
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 1), (32, 2), (1025, 1), (2051, 4), (8192, 4), (8193, 4)])
+@pytest.mark.parametrize("E,ids", [(1, "one"), (8, "any"), (8, "last"), (256, "any"), (7, "bad")])
+def test_route_sorts_stably(n, k, E, ids):
+    """Counts, order, its inverse and the gathered rows are the ones of the stable sort, from one id to the largest
+    number that the kernel takes and one above (the general path); ids out of range go to the end, uncounted."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(n)
+    x, dy = _mk(n, 24).requires_grad_(True), _mk(n * k, 24)
+    idx = torch.full((n, k), E - 1) if ids in ("one", "last") else torch.randint(0, E, (n, k))
+    own = n * k <= M.ROUTE_MAX_IDS
+    if ids == "bad":
+        if not own:
+            pytest.skip("the general path refuses these")
+        idx[::3] = E + 5
+        idx[1::5] = -2
+    counts, rows, order, slots = M.route(x, idx.cuda(), E)
+    key = idx.flatten().clone()
+    key[(key < 0) | (key >= E)] = E
+    ref = torch.argsort(key, stable=True).cuda()
+    assert torch.equal(order, ref) and torch.equal(counts.cpu(), torch.bincount(key, minlength=E + 1)[:E])
+    assert (slots is not None) == own and torch.equal(rows, x.detach()[ref // k])
+    if own:
+        assert torch.equal(slots[order].cpu(), torch.arange(n * k, dtype=torch.int32))
+    rows.backward(dy)
+    back = torch.zeros(n, 24, device="cuda").index_add(0, ref // k, dy.float())
+    assert (x.grad.float() - back).norm() <= 2 ** -8 * back.norm()
+
+
+def test_expert_ids_out_of_range_are_refused():
+    from atorch_b200.modules.moe import Grouped_GEMM_MoE
+
+    with torch.device("cuda"):
+        m = Grouped_GEMM_MoE(64, 64, 0.0, 4, 1, use_swiglu=True).bfloat16()
+    x, p = _mk(8, 64), torch.ones(8, 1, device="cuda").bfloat16()
+    for bad in (-1, 4):
+        idx = torch.zeros(8, 1, dtype=torch.int64, device="cuda")
+        idx[3] = bad
+        with pytest.raises((AssertionError, RuntimeError, IndexError)):
+            m(x, p, idx)
