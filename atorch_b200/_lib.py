@@ -47,7 +47,7 @@ SIGNATURES = {
     "atb_flash_bwd_split": "ppppppppppppiiiiillllllifppiipp",
     "atb_invert_perm": "ppip",
     "atb_moe_gather_sum": "pppipiiip",
-    "atb_moe_scatter_mul": "ppppippiiip",
+    "atb_moe_ungather": "ppppippiiip",
     "atb_padded_intervals": "ppppppiiip",
     "atb_row_intervals": "pppiiiipipiippiip",
 }

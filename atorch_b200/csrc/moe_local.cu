@@ -3,7 +3,7 @@
 //   gather_sum    out[t] = sum_j w[t, j] src[slot_of[t, j]]     unpermute forward (w = routing probabilities) and
 //                                                               permute backward (no w)
 //   gather_rows   out[i] = src[order[i] / k]                    permute forward
-//   scatter_mul   dsrc[slot_of[t, j]] = w[t, j] dout[t],  dw[t, j] = <dout[t], src[slot_of[t, j]]>   unpermute backward
+//   ungather      dsrc[i] = w[s] dout[s / k], dw[s] = <dout[s / k], src[i]> with s = order[i]        unpermute backward
 // Bound by memory, one pass each with 16-byte pieces and fp32 sums. As tensor operations (zeros, index_copy, product,
 // sum; index_add with atomics backward) this was 13 passes over [T k, H]: for 4096 tokens, top 2, H = 4096 0.75 ms of an
 // 8.5 ms forward and backward, 0.1 ms here.
@@ -49,22 +49,23 @@ __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* __
   }
 }
 
-__global__ void __launch_bounds__(256) scatter_mul_kernel(const __nv_bfloat16* __restrict__ dout,
-                                                          const __nv_bfloat16* __restrict__ src,
-                                                          const int* __restrict__ slot_of, const void* __restrict__ w,
-                                                          int w_dtype, __nv_bfloat16* __restrict__ dsrc,
-                                                          void* __restrict__ dw, int k, int H) {
+__global__ void __launch_bounds__(256) ungather_kernel(const __nv_bfloat16* __restrict__ dout,
+                                                       const __nv_bfloat16* __restrict__ src,
+                                                       const long long* __restrict__ order, const void* __restrict__ w,
+                                                       int w_dtype, __nv_bfloat16* __restrict__ dsrc,
+                                                       void* __restrict__ dw, int k, int H) {
   __shared__ float red[33];
-  const long long t = blockIdx.x / k;
-  const int s = slot_of[blockIdx.x];
+  const long long s = order[blockIdx.x];
+  if (s < 0 || s >= (long long)gridDim.x) return;
+  const long long t = s / k, row = (long long)blockIdx.x * H;
   float dot = 0.f;
-  if (s >= 0) {
-    const float f = w ? weight_at(w, w_dtype, blockIdx.x) : 1.f;
+  {
+    const float f = w ? weight_at(w, w_dtype, s) : 1.f;
     for (int c = threadIdx.x; c < H / 8; c += 256) {
       const uint4 d = *reinterpret_cast<const uint4*>(dout + t * H + c * 8);
       const uint32_t x[4] = {d.x, d.y, d.z, d.w};
       uint4 u = make_uint4(0u, 0u, 0u, 0u);
-      if (dw != nullptr) u = *reinterpret_cast<const uint4*>(src + (long long)s * H + c * 8);
+      if (dw != nullptr) u = *reinterpret_cast<const uint4*>(src + row + c * 8);
       const uint32_t y[4] = {u.x, u.y, u.z, u.w};
       uint32_t o[4];
 #pragma unroll
@@ -73,14 +74,14 @@ __global__ void __launch_bounds__(256) scatter_mul_kernel(const __nv_bfloat16* _
         dot += a.x * b.x + a.y * b.y;
         o[e] = pack_bf16x2(f * a.x, f * a.y);
       }
-      if (dsrc != nullptr) *reinterpret_cast<uint4*>(dsrc + (long long)s * H + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (dsrc != nullptr) *reinterpret_cast<uint4*>(dsrc + row + c * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
   if (dw != nullptr) {
     dot = block_sum(dot, red);
     if (threadIdx.x == 0) {
-      if (w_dtype == 0) reinterpret_cast<__nv_bfloat16*>(dw)[blockIdx.x] = __float2bfloat16_rn(dot);
-      else reinterpret_cast<float*>(dw)[blockIdx.x] = dot;
+      if (w_dtype == 0) reinterpret_cast<__nv_bfloat16*>(dw)[s] = __float2bfloat16_rn(dot);
+      else reinterpret_cast<float*>(dw)[s] = dot;
     }
   }
 }
@@ -203,12 +204,13 @@ extern "C" int atb_moe_gather_sum(const void* src, const int* slot_of, const voi
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
-// dsrc (rows that no choice names are left alone) or dw may be null; dw has the type of w (bf16 or fp32).
-extern "C" int atb_moe_scatter_mul(const void* dout, const void* src, const int* slot_of, const void* w, int w_dtype,
-                                   void* dsrc, void* dw, int T, int k, int H, void* stream) {
-  if (T <= 0 || H <= 0) return 0;
-  if ((H & 7) || k < 1 || (long long)T * k > 0x7fffffffLL || !aligned16(dout, src, dsrc)) return -1;
-  scatter_mul_kernel<<<(unsigned)T * (unsigned)k, 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)dout, (const __nv_bfloat16*)src, slot_of, w, w_dtype, (__nv_bfloat16*)dsrc, dw, k, H);
+// n sorted rows; dsrc or dw may be null, dw has the type of w (bf16 or fp32). Rows whose entry of `order` is outside [0, n)
+// are left alone.
+extern "C" int atb_moe_ungather(const void* dout, const void* src, const long long* order, const void* w, int w_dtype,
+                                void* dsrc, void* dw, int n, int k, int H, void* stream) {
+  if (n <= 0 || H <= 0) return 0;
+  if ((H & 7) || k < 1 || !aligned16(dout, src, dsrc)) return -1;
+  ungather_kernel<<<n, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)src, order, w,
+                                                       w_dtype, (__nv_bfloat16*)dsrc, dw, k, H);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

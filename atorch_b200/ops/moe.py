@@ -26,11 +26,20 @@ def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tenso
     return torch.bincount(expert_idx.reshape(-1), minlength=num_experts)
 
 
+def _watched(*ts: Optional[torch.Tensor]) -> bool:
+    """Whether something other than reverse-mode autograd looks at these operations (a functorch transform, forward-mode
+    differentiation, a tracer, a tensor subclass): the row kernels would hide them from it, tensor operations do not."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
+            or torch.compiler.is_compiling() or any(type(t) not in (torch.Tensor, torch.nn.Parameter)
+                                                    or torch.autograd.forward_ad.unpack_dual(t).tangent is not None
+                                                    for t in ts if t is not None))
+
+
 def _rows_ok(rows: torch.Tensor, order: torch.Tensor) -> bool:
     """Whether the row kernels (csrc/moe_local.cu) take these rows: bf16 on the GPU in 16-byte pieces, int64 order."""
     return (_lib.use_kernels(rows, order) and rows.dtype == torch.bfloat16 and rows.dim() == 2 and rows.shape[1] % 8 == 0
             and rows.shape[1] > 0 and order.dtype == torch.int64 and order.dim() == 1 and order.is_contiguous()
-            and 0 < order.numel() < 1 << 31)
+            and 0 < order.numel() < 1 << 31 and not _watched(rows, order))
 
 
 def _slots(order: torch.Tensor) -> torch.Tensor:
@@ -70,29 +79,39 @@ class _Permute(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         order, slot = ctx.saved_tensors
+        if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
+            zeros = torch.zeros(ctx.T, dy.shape[1], dtype=dy.dtype, device=dy.device)
+            return zeros.index_add(0, order // ctx.k, dy), None, None, None
         return _gather_sum(_packed(dy), _slots(order) if slot is None else slot, None, ctx.T, ctx.k), None, None, None
 
 
 class _Unpermute(torch.autograd.Function):
     @staticmethod
     def forward(ctx, rows, order, probs, k, slot):
-        rows, slot = _packed(rows), _slots(order) if slot is None else slot
-        w = None if probs is None else probs.contiguous()
-        ctx.save_for_backward(rows, slot, w)
-        ctx.k, ctx.p_shape = k, None if probs is None else probs.shape
-        return _gather_sum(rows, slot, w, order.numel() // k, k)
+        ctx.save_for_backward(rows, order, probs)
+        ctx.k, ctx.sorted = k, slot is not None
+        slot = _slots(order) if slot is None else slot
+        return _gather_sum(_packed(rows), slot, None if probs is None else probs.contiguous(), order.numel() // k, k)
 
     @staticmethod
     def backward(ctx, dout):
-        rows, slot, w = ctx.saved_tensors
-        dout, T, H = _packed(dout), slot.numel() // ctx.k, rows.shape[1]
+        rows, order, probs = ctx.saved_tensors
+        if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
+            d, dw = dout.index_select(0, order // ctx.k), None
+            if probs is not None:
+                dots = (rows * d).sum(-1).to(probs.dtype)
+                dw = torch.zeros_like(dots).index_copy(0, order, dots).view(probs.shape)
+                d = d * probs.reshape(-1, 1).index_select(0, order).to(d.dtype)
+            return d, None, dw, None, None
+        rows, w, dout = _packed(rows), None if probs is None else probs.contiguous(), _packed(dout)
         drows = torch.empty_like(rows) if ctx.needs_input_grad[0] else None
-        dw = torch.empty_like(w) if w is not None and ctx.needs_input_grad[2] else None
-        rc = _lib.lib().atb_moe_scatter_mul(dout.data_ptr(), rows.data_ptr(), slot.data_ptr(), _lib.addr(w),
-                                            2 if w is None else _lib.DT[w.dtype], _lib.addr(drows), _lib.addr(dw), T, ctx.k,
-                                            H, _lib.stream())
-        _lib.check(rc, "atb_moe_scatter_mul")
-        return drows, None, None if dw is None else dw.view(ctx.p_shape), None, None
+        # an order of the caller's own may leave a choice out
+        dw = (torch.empty_like if ctx.sorted else torch.zeros_like)(w) if w is not None and ctx.needs_input_grad[2] else None
+        rc = _lib.lib().atb_moe_ungather(dout.data_ptr(), rows.data_ptr(), order.data_ptr(), _lib.addr(w),
+                                         2 if w is None else _lib.DT[w.dtype], _lib.addr(drows), _lib.addr(dw), order.numel(),
+                                         ctx.k, rows.shape[1], _lib.stream())
+        _lib.check(rc, "atb_moe_ungather")
+        return drows, None, None if dw is None else dw.view(probs.shape), None, None
 
 
 def permute(tokens: torch.Tensor, expert_idx: torch.Tensor, num_out_tokens: Optional[int] = None
@@ -140,7 +159,8 @@ def unpermute(permuted: torch.Tensor, sorted_idx: torch.Tensor, probs: Optional[
                                                                    else sorted_idx.numel())
     if topk >= 1 and _rows_ok(permuted, sorted_idx) and n_slots == sorted_idx.numel() == permuted.shape[0] \
             and n_slots % topk == 0 and (probs is None or (probs.numel() == n_slots and probs.is_cuda
-                                                           and probs.dtype in (torch.bfloat16, torch.float32))):
+                                                           and probs.dtype in (torch.bfloat16, torch.float32)
+                                                           and not _watched(probs))):
         return _Unpermute.apply(permuted, sorted_idx, probs, topk, slots)
     return unpermute_reference(permuted, sorted_idx, probs, topk, n_slots)
 

@@ -385,3 +385,37 @@ def test_expert_ids_out_of_range_are_refused():
         idx[3] = bad
         with pytest.raises((AssertionError, RuntimeError, IndexError)):
             m(x, p, idx)
+
+
+def test_routed_rows_under_transforms_and_second_derivatives():
+    """What the row kernels hide from forward mode, vmap and a second derivative takes tensor operations: the same calls
+    give what the plain composition gives (two bf16 roundings on either side)."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    T, H, E, k = 37, 64, 4, 2
+    x, p = _mk(T, H), torch.rand(T, k, device="cuda").bfloat16()
+    idx = torch.randint(0, E, (T, k), device="cuda")
+
+    def own(x, p):
+        counts, rows, order, slots = M.route(x, idx, E)
+        return M.unpermute(rows * rows, order, p, k, T, slots)
+
+    def plain(x, p):
+        return (x.unsqueeze(1) * x.unsqueeze(1) * p.unsqueeze(-1)).sum(1)
+
+    def close(a, b):
+        return (a.float() - b.float()).norm() <= 2 ** -6 * b.float().norm()
+
+    res = []
+    for f, dt in ((own, torch.bfloat16), (plain, torch.float32)):
+        xs, ps = x.to(dt).requires_grad_(True), p.to(dt).requires_grad_(True)
+        gx, gp = torch.autograd.grad(f(xs, ps).float().sum(), [xs, ps], create_graph=True)
+        res.append(torch.autograd.grad(gx.float().square().sum() + gp.float().square().sum(), [xs, ps]))
+    assert all(close(a, b) for a, b in zip(*res))
+    tx, tp = torch.randn_like(x), torch.randn_like(p)
+    a = torch.func.jvp(own, (x, p), (tx, tp))
+    b = torch.func.jvp(plain, (x.float(), p.float()), (tx.float(), tp.float()))
+    assert close(a[0], b[0]) and close(a[1], b[1])
+    xs = torch.stack([x, tx])
+    assert close(torch.func.vmap(own, (0, None))(xs, p), torch.func.vmap(plain, (0, None))(xs.float(), p.float()))
