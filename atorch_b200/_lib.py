@@ -35,6 +35,7 @@ SIGNATURES = {
     "atb_gemm_bf16_2cta_rope": "pppiiilllpppiiipp",
     "atb_moe_sort_ids": "piipppp",
     "atb_moe_gather_rows": "pppiiip",
+    "atb_gemm_bf16_2cta_kgroups": "pppiiillpiiipp",
     "atb_gemm_bf16_2cta_ragged": "pppiiilllipiippp",
     "atb_norm_fwd": "ppppppppiifiip",
     "atb_norm_bwd": "pppppppppiiiiip",

@@ -164,6 +164,23 @@ struct Ragged {
   int row0[RAGGED_MAX + 1], mt0[RAGGED_MAX + 1];
 };
 
+// Weight gradients of the same groups, C_g = A_g^T B_g (both operands MN-major, the reduction runs over the group's rows):
+// one tensor map per group and operand, so that a group's last k-block ends with its rows (the rest reads as zero). The
+// outputs are stacked, [n * M, N]; a group without rows writes zeros (nothing when accumulating).
+// One launch for up to 16 groups. Against one per group (each with its own prologue, last wave and exposed last epilogue):
+// gradients of 8 experts x 14336 x 4096 over 8192 rows 2518 -> 2468 us; forward and backward of an expert MLP
+// 8 x 4096 x 1024 on 131 tokens 782 -> 515 us, 8 x 3520 x 1024 on 2049 tokens 797 -> 550, 4 x 8192 x 2048 on 1000 tokens
+// 707 -> 657, 4 x 9024 x 4096 on 2000 tokens 2765 -> 2712.
+constexpr int KGROUP_MAX = 16;
+template <bool KG>
+struct KGroups {};
+template <>
+struct KGroups<true> {
+  CUtensorMap a[KGROUP_MAX], b[KGROUP_MAX];
+  int rows[KGROUP_MAX];
+  int n;
+};
+
 ATB_DEVICE uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -242,11 +259,12 @@ ATB_DEVICE void mbar_arrive_remote(uint32_t bar_cluster_addr) {
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool KG>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epi ep, int M,
                       int N, int K, Groups grp, Gate gate, Sched sched, const __grid_constant__ Ragged rag,
-                      int* status) {
+                      const __grid_constant__ KGroups<KG> kg, int* status) {
+  static_assert(!KG || (A_MN && B_MN), "groups along the reduction are rows of MN-major operands");
   constexpr int BNH = Cfg<BN>::BNH, STAGES = Cfg<BN>::STAGES, B_BYTES = Cfg<BN>::B_BYTES,
                 BAR_OFF = Cfg<BN>::BAR_OFF;
   extern __shared__ uint8_t smem_raw[];
@@ -273,8 +291,13 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int tiles_m = rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM);
   const int tile_cols = ep.gated ? BN / 2 : BN;      // output columns per tile
   const int tiles_n = (N + tile_cols - 1) / tile_cols;
-  const int num_tiles = skip ? 0 : tiles_m * tiles_n;
-  const int num_kb = (K + BK - 1) / BK;
+  int groups = 1;
+  if constexpr (KG) groups = kg.n;
+  const int num_tiles = skip ? 0 : tiles_m * tiles_n * groups;
+  auto tile_kbs = [&](int b_idx) -> int {            // k-blocks of a tile
+    if constexpr (KG) return (kg.rows[b_idx] + BK - 1) / BK;
+    else return (K + BK - 1) / BK;
+  };
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
   constexpr int BAND = 8;
 
@@ -294,7 +317,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 0 && lane == 0) {
+  if (!KG && warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
   }
@@ -308,7 +331,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   // identical decisions in every role: which tiles and which k-blocks carry data
-  auto tile_active = [&](int m0) -> bool {
+  auto tile_active = [&](int m0, int b_idx) -> bool {
+    if constexpr (KG) return kg.rows[b_idx] > 0;
     if (grp.counts == nullptr) return true;
     if (grp.m_rows > 0) {
       const int g = m0 / grp.m_rows;
@@ -330,6 +354,11 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   // first row / column of a tile, the end of its rows and the index of its B operand
   auto tile_coords = [&](int tile, int& m0, int& n0, int& m_end, int& b_idx) {
+    int kg_idx = 0;
+    if constexpr (KG) {
+      kg_idx = tile / (tiles_m * tiles_n);
+      tile -= kg_idx * tiles_m * tiles_n;
+    }
     const int band_tiles = BAND * tiles_n;
     const int band = tile / band_tiles;
     const int rem = tile - band * band_tiles;
@@ -355,7 +384,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     } else {
       m0 = tm * 2 * BM;
       m_end = M;
-      b_idx = grp.b_rows > 0 ? m0 / grp.bm_rows : 0;
+      b_idx = KG ? kg_idx : grp.b_rows > 0 ? m0 / grp.bm_rows : 0;
     }
   };
 
@@ -419,7 +448,13 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (tile < 0) break;
         int m0, n0, m_end, b_idx;
         tile_coords(tile, m0, n0, m_end, b_idx);
-        if (!tile_active(m0)) continue;
+        if (!tile_active(m0, b_idx)) continue;
+        const int num_kb = tile_kbs(b_idx);
+        const CUtensorMap *mapA = &tmA, *mapB = &tmB;
+        if constexpr (KG) {
+          mapA = &kg.a[b_idx];
+          mapB = &kg.b[b_idx];
+        }
         const int am0 = m0 + (int)rank * BM;   // this CTA's rows of A
         const int bshift = b_idx * grp.b_rows;   // this expert's own B
         // this CTA's rows of B (gated: CTA 0 takes gate rows, CTA 1 the up rows of the same features)
@@ -443,17 +478,17 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             uint8_t* a_dst = sA + s * A_BYTES;
             uint8_t* b_dst = sB + s * B_BYTES;
             if constexpr (!A_MN) {
-              tma_load_2d_pair(a_dst, &tmA, bar, kb * BK, am0);
+              tma_load_2d_pair(a_dst, mapA, bar, kb * BK, am0);
             } else {
 #pragma unroll
-              for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(a_dst + j * 8192, &tmA, bar, am0 + j * 64, kb * BK);
+              for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(a_dst + j * 8192, mapA, bar, am0 + j * 64, kb * BK);
             }
             if constexpr (!B_MN) {
-              tma_load_2d_pair(b_dst, &tmB, bar, kb * BK, bn0);
+              tma_load_2d_pair(b_dst, mapB, bar, kb * BK, bn0);
             } else {
 #pragma unroll
               for (int j = 0; j < BNH / 64; ++j)
-                tma_load_2d_pair(b_dst + j * 8192, &tmB, bar, bn0 + j * 64, bk0 + kb * BK);
+                tma_load_2d_pair(b_dst + j * 8192, mapB, bar, bn0 + j * 64, bk0 + kb * BK);
             }
           }
           ++it;
@@ -473,10 +508,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int tile = read_tile(idx);
         free_tile_slot(idx);
         if (tile < 0) break;
+        int num_kb;
         {
           int m0, n0, m_end, b_idx;
           tile_coords(tile, m0, n0, m_end, b_idx);
-          if (!tile_active(m0)) continue;
+          if (!tile_active(m0, b_idx)) continue;
+          num_kb = tile_kbs(b_idx);
         }
         const int acc = local & 1;
         const uint32_t acc_ph = (local >> 1) & 1;
@@ -518,18 +555,19 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (tile < 0) break;
       int m0, n0, m_end, b_idx;
       tile_coords(tile, m0, n0, m_end, b_idx);
-      if (!tile_active(m0)) {
+      const long long c_row0 = KG ? (long long)b_idx * M : 0;      // this group's rows of C
+      if (!tile_active(m0, b_idx)) {
         // an empty tile: its output is all zeros (left alone when accumulating)
         const int zrow = m0 + (int)rank * BM + q * 32 + lane;
         if (!ep.accumulate && ep.rs_rows <= 0 && zrow < M) {
           for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 8) {
             if (n0 + c >= N) break;
             if (ep.out_fp32) {
-              float* z = reinterpret_cast<float*>(ep.C) + (long long)zrow * ep.ldc + n0 + c;
+              float* z = reinterpret_cast<float*>(ep.C) + (c_row0 + zrow) * ep.ldc + n0 + c;
               *reinterpret_cast<float4*>(z) = make_float4(0.f, 0.f, 0.f, 0.f);
               *reinterpret_cast<float4*>(z + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
             } else {
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)zrow * ep.ldc + n0 + c) =
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + zrow) * ep.ldc + n0 + c) =
                   make_uint4(0u, 0u, 0u, 0u);
             }
           }
@@ -654,7 +692,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                              : "memory");
             }
           } else if (ep.out_fp32) {
-            float* crow = reinterpret_cast<float*>(ep.C) + (long long)row * ep.ldc + col0;
+            float* crow = reinterpret_cast<float*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               if (col0 + i < N) {
@@ -671,7 +709,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                 if (col0 + i < N) stg_v8(crow + i, reinterpret_cast<const uint32_t*>(v + i));
             }
           } else {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
+            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
             if (ep.accumulate || ep.residual != nullptr) {
 #pragma unroll
               for (int i = 0; i < 32; i += 8) {
@@ -762,19 +800,21 @@ int* sched_counters(cudaStream_t stream) {
   return reinterpret_cast<int*>(p);
 }
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool KG = false>
 int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, long long lda, long long ldb,
            int max_ctas, const Groups& grp, int b_extent_rows, const Gate& gate, const Ragged& rag, cudaStream_t stream,
-           int* status) {
-  CUtensorMap tmA, tmB;
-  bool ok;
-  if (!A_MN)
+           int* status, const KGroups<KG>& kg = KGroups<KG>()) {
+  CUtensorMap tmA = {}, tmB = {};
+  bool ok = true;
+  if (KG) {              // a map per group, made by the caller
+  } else if (!A_MN)
     ok = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, K, lda, BM, BK, CU_TENSOR_MAP_SWIZZLE_128B);
   else
     ok = make_tmap_2d(&tmA, A, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, lda, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B);
   if (!ok) return -2;
   // with per-group B the tensor map spans all groups' weights (b_extent_rows rows)
-  if (!B_MN)
+  if (KG) {
+  } else if (!B_MN)
     ok = make_tmap_2d(&tmB, B, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, b_extent_rows > 0 ? b_extent_rows : N, K, ldb,
                       Cfg<BN>::BNH, BK, CU_TENSOR_MAP_SWIZZLE_128B);
   else
@@ -787,7 +827,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   epw.wide = ep.C != nullptr && ep.rs_rows <= 0 && N % 16 == 0 && (reinterpret_cast<uintptr_t>(ep.C) & 31) == 0 &&
              (ep.ldc * out_bytes) % 32 == 0 &&
              (ep.gu_out == nullptr || ((reinterpret_cast<uintptr_t>(ep.gu_out) & 31) == 0 && (ep.ldgu * 2) % 32 == 0));
-  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN>;
+  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, KG>;
   constexpr int SMEM_TOTAL = Cfg<BN>::SMEM_TOTAL;
   static bool attr_set = false;
   if (!attr_set) {
@@ -795,7 +835,8 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     attr_set = true;
   }
   const int tile_cols = ep.gated ? BN / 2 : BN;
-  const int tiles = (rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
+  int tiles = (rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
+  if constexpr (KG) tiles *= kg.n;
   int clusters = sm_count() / 2;
   if (tiles < clusters) clusters = tiles;
   if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
@@ -820,7 +861,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, epw, M, N, K, grp, gate, sched, rag, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, epw, M, N, K, grp, gate, sched, rag, kg, status);
   return e == cudaSuccess ? 0 : -5;
 }
 
@@ -940,6 +981,46 @@ extern "C" int atb_gemm_bf16_2cta_ragged(const void* A, const void* B, void* C, 
   if (b_mn_major)
     return launch<256, false, true>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * K, gate, rag, st, status);
   return launch<256, false, false>(A, B, ep, M, N, K, lda, ldb, 0, grp, n_groups * b_cols, gate, rag, st, status);
+}
+
+// C[g] (+)= A_g^T B_g for `n_groups` consecutive row groups of `sizes` rows (host memory, T in all): A [T, M] and B [T, N]
+// hold the groups' rows, C [n_groups, M, N] is bf16 or fp32 (see KGroups).
+extern "C" int atb_gemm_bf16_2cta_kgroups(const void* A, const void* B, void* C, int M, int N, int T, long long lda,
+                                          long long ldb, const int* sizes, int n_groups, int out_fp32, int accumulate,
+                                          void* stream, int* status) {
+  if (M <= 0 || N <= 0 || n_groups <= 0) return 0;
+  if ((M & 7) || (N & 7) || (lda & 7) || (ldb & 7) || T < 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15) return -1;
+  const Groups grp{nullptr, 0, 0, 0, 0};
+  const Gate gate{nullptr, 0u, 1, 0};
+  long long row = 0;
+  for (int g = 0; g < n_groups; ++g) {
+    if (sizes[g] < 0 || sizes[g] > T - row) return -1;
+    row += sizes[g];
+  }
+  if (row != T) return -1;
+  row = 0;
+  for (int g0 = 0; g0 < n_groups; g0 += KGROUP_MAX) {
+    KGroups<true> kg = {};
+    kg.n = n_groups - g0 < KGROUP_MAX ? n_groups - g0 : KGROUP_MAX;
+    for (int i = 0; i < kg.n; ++i) {
+      kg.rows[i] = sizes[g0 + i];
+      if (kg.rows[i] == 0) continue;
+      if (!make_tmap_2d(&kg.a[i], reinterpret_cast<const __nv_bfloat16*>(A) + row * lda, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                        kg.rows[i], M, lda, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+        return -2;
+      if (!make_tmap_2d(&kg.b[i], reinterpret_cast<const __nv_bfloat16*>(B) + row * ldb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                        kg.rows[i], N, ldb, BK, 64, CU_TENSOR_MAP_SWIZZLE_128B))
+        return -3;
+      row += kg.rows[i];
+    }
+    char* c = reinterpret_cast<char*>(C) + (long long)g0 * M * N * (out_fp32 ? 4 : 2);
+    Epi ep{c, nullptr, N, 1.f, out_fp32, accumulate, nullptr, 0, {nullptr}, 0, 0, nullptr, 0};
+    const int rc = launch<256, true, true, true>(A, B, ep, M, N, T, lda, ldb, 0, grp, 0, gate, kNoGroups,
+                                                 reinterpret_cast<cudaStream_t>(stream), status, kg);
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 // out[M, N] = rope(x W^T): the projection onto fused q | k | v heads with the first rope_heads heads of head_dim (128 or

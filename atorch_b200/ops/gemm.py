@@ -184,6 +184,27 @@ def gemm_ragged(x: torch.Tensor, w: torch.Tensor, sizes, b_mn: bool, gated: bool
     return (out, gu) if gated else out
 
 
+def k_groups_ok(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether ``gemm_k_groups`` takes these operands: bf16 rows on the GPU in 16-byte pieces, stacked outputs."""
+    return (_lib.use_kernels(a, b, out) and PAIR_KERNEL_DEFAULT and a.dim() == b.dim() == 2 and out.dim() == 3
+            and a.dtype == b.dtype == torch.bfloat16 and out.dtype in (torch.bfloat16, torch.float32)
+            and a.shape[0] == b.shape[0] > 0 and a.shape[1] % 8 == 0 and b.shape[1] % 8 == 0
+            and tuple(out.shape[1:]) == (a.shape[1], b.shape[1]) and out.is_contiguous()
+            and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 for t in (a, b))
+            and all(t.data_ptr() % 16 == 0 for t in (a, b, out)))
+
+
+def gemm_k_groups(a: torch.Tensor, b: torch.Tensor, sizes, out: torch.Tensor, accumulate: bool) -> torch.Tensor:
+    """``out[g] (+)= a_g^T b_g`` over consecutive groups of ``sizes`` rows (host numbers): one launch for up to 16 groups.
+    See :func:`k_groups_ok`."""
+    rc = _lib.lib().atb_gemm_bf16_2cta_kgroups(
+        a.data_ptr(), b.data_ptr(), out.data_ptr(), a.shape[1], b.shape[1], a.shape[0], a.stride(0), b.stride(0),
+        (ctypes.c_int * len(sizes))(*sizes), len(sizes), int(out.dtype == torch.float32), int(accumulate), _lib.stream(),
+        _lib.status_addr(a))
+    _lib.check(rc, f"atb_gemm_bf16_2cta_kgroups T={a.shape[0]} M={a.shape[1]} N={b.shape[1]} groups={len(sizes)}")
+    return out
+
+
 def _linear_grads(ctx, dy2, x2, weight, need_dx, need_dw):
     """dx and dW of ``y = x W^T`` from ``dy``; dW goes straight into ``weight.main_grad`` when there is one."""
     dx = dw = None

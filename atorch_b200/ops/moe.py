@@ -18,7 +18,7 @@ import torch
 
 from .. import _lib
 from .elementwise import swiglu, swiglu_backward
-from .gemm import gemm, gemm_ragged, linear, ragged_ok
+from .gemm import gemm, gemm_k_groups, gemm_ragged, k_groups_ok, linear, ragged_ok
 
 
 def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tensor:
@@ -176,8 +176,8 @@ def unpermute_reference(permuted, sorted_idx, probs, topk, n_slots):
 
 class _GroupedLinear(torch.autograd.Function):
     """y[g] = x[g] @ W[g]^T for consecutive row groups (W stored [G, N, K]), or x[g] @ W[g] (W stored [G, K, N])
-    when ``b_mn``: the GEMM reads either as it lies in memory. Forward and dgrad are one launch over all groups where
-    the kernel takes the operands; wgrad is one product per group (each of its outputs alone fills the GPU)."""
+    when ``b_mn``: the GEMM reads either as it lies in memory. Forward, dgrad and wgrad are one launch each over all
+    groups (wgrad: up to 16) where the kernel takes the operands."""
 
     @staticmethod
     def _rows(x, w, sizes, b_mn):
@@ -205,6 +205,9 @@ class _GroupedLinear(torch.autograd.Function):
         mg = getattr(w, "main_grad", None)
         dw = mg if mg is not None else torch.empty(w.shape, dtype=w.dtype, device=w.device)
         a, b = (x, dy) if b_mn else (dy, x)             # dW[g] = a[g]^T b[g]
+        if len(sizes) == dw.shape[0] and k_groups_ok(a, b, dw):
+            gemm_k_groups(a, b, sizes, dw, mg is not None)
+            sizes = ()
         r = 0
         for g, n in enumerate(sizes):
             if n:

@@ -419,3 +419,36 @@ def test_routed_rows_under_transforms_and_second_derivatives():
     assert close(a[0], b[0]) and close(a[1], b[1])
     xs = torch.stack([x, tx])
     assert close(torch.func.vmap(own, (0, None))(xs, p), torch.func.vmap(plain, (0, None))(xs.float(), p.float()))
+
+
+@pytest.mark.parametrize("sizes", [(1,), (64, 0, 63, 65, 129), (7,) * 17, (0, 300) + (5,) * 15])
+@pytest.mark.parametrize("M,N", [(8, 264), (264, 8), (512, 256)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.float32, True), (torch.float32, False)])
+def test_gemm_k_groups(sizes, M, N, dtype, accumulate):
+    """Weight gradients of row groups in one launch against one fp32 product each: last k-blocks of 1 to 64 rows, empty
+    groups, more groups than a launch takes. Rows of the neighbours hold an infinity, which must not reach a group."""
+    from atorch_b200.ops.gemm import gemm_k_groups, k_groups_ok
+
+    torch.manual_seed(sum(sizes) + M)
+    T, G = sum(sizes), len(sizes)
+    a, b = _mk(T, M), _mk(T, N)
+    a[0] = float("inf")
+    b[0] = 1.0
+    out = torch.randn(G, M, N, device="cuda").to(dtype) if accumulate else torch.full((G, M, N), float("nan"), device="cuda",
+                                                                                      dtype=dtype)
+    before = out.clone()
+    assert k_groups_ok(a, b, out)
+    gemm_k_groups(a, b, sizes, out, accumulate)
+    torch.cuda.synchronize()
+    _lib.check_status(out.device)
+    r, first = 0, True
+    for g, n in enumerate(sizes):
+        ref = a[r: r + n].float().t() @ b[r: r + n].float() + (before[g].float() if accumulate else 0)
+        if n and first:
+            assert torch.isinf(out[g]).all()
+            first = False
+        else:
+            # fp32 sums in another order, and one rounding of the output type
+            tol = torch.finfo(dtype).eps + 2 * max(n, 1) ** 0.5 * 2 ** -23
+            assert (out[g].float() - ref).norm() <= tol * max(ref.norm().item(), 1e-30)
+        r += n
