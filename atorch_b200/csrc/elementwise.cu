@@ -128,6 +128,32 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 }
 
 // out[t, :] = inp[t, :] + bias[expert[t], :]   (MoE per-expert bias)
+// out[r] = sum over the g consecutive heads of row r, in fp32 and in order, for two tensors (blockIdx.y): the gradients of
+// a key/value head from those of its query heads. Bound by memory: one pass, each thread sums 8 columns of one row. As
+// tensor operations (to fp32, sum, back) 31 us for 2 x 4096 rows of 4 heads x 4 x 128, 5.7 us here.
+__global__ void __launch_bounds__(256) head_sum_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
+                                                       uint4* __restrict__ oa, uint4* __restrict__ ob, long long rows, int g,
+                                                       int pieces) {
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (i >= rows * pieces) return;
+  const long long r = i / pieces;
+  const uint4* src = (blockIdx.y ? b : a) + r * g * pieces + (i - r * pieces);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int h = 0; h < g; ++h) {
+    const uint4 u = src[(long long)h * pieces];
+    const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 v = unpack_bf16x2(x[e]);
+      acc[2 * e] += v.x;
+      acc[2 * e + 1] += v.y;
+    }
+  }
+  (blockIdx.y ? ob : oa)[i] = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
+                                         pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+}
+
 __global__ void bias_gather_add_kernel(const __nv_bfloat16* __restrict__ inp, const __nv_bfloat16* __restrict__ bias,
                                        const int* __restrict__ expert, __nv_bfloat16* __restrict__ out, long long T,
                                        int H) {
@@ -203,6 +229,16 @@ extern "C" int atb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long 
   if ((F & 7) || (gu_stride & 7) || (dout_stride & 7)) return -1;
   swiglu_bwd_kernel<<<grid_for(T * (F >> 3), 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, T, F, gu_stride, dout_stride);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+// a, b: [rows, g, D] bf16, contiguous; oa, ob: [rows, D]. D a multiple of 8.
+extern "C" int atb_head_sum(const void* a, const void* b, void* oa, void* ob, long long rows, int g, int D, void* stream) {
+  if (rows <= 0) return 0;
+  if (g < 1 || D < 8 || (D & 7)) return -1;
+  const long long blocks = (rows * (D >> 3) + 255) / 256;
+  if (blocks > 0x7fffffffLL) return -1;
+  head_sum_kernel<<<dim3((unsigned)blocks, 2), 256, 0, (cudaStream_t)stream>>>(
+      (const uint4*)a, (const uint4*)b, (uint4*)oa, (uint4*)ob, rows, g, D >> 3);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 extern "C" int atb_bias_gather_add(const void* inp, const void* bias, const int* expert, void* out, long long T, int H,

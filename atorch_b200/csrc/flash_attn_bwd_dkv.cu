@@ -41,7 +41,7 @@ struct DkvParams {
   const int* row_lo;
   const int* row_hi;
   int B, Sq, Sk, Hq, Hkv, causal;
-  int fold;            // query heads per CTA: Hq / Hkv (gradients of a key/value head) or 1 (of a query head)
+  int fold;            // query heads per CTA, a divisor of Hq / Hkv: Hq / Hkv (gradients of a key/value head) down to 1
   float scale, scale_log2;
   int* status;
   KeyBits keys;
@@ -450,8 +450,8 @@ int launch_dkv(const void* dout, const void* q, const void* k, const void* v, co
 
 }  // namespace
 
-// dk, dv: token-major rows of pitch dkv_stride elements, per key/value head when fold == Hq / Hkv, per query head when
-// fold == 1 (the caller then sums head groups); lse, delta: [B, Hq, Sq] fp32.
+// dk, dv: token-major rows of pitch dkv_stride elements, one head per `fold` query heads (fold == Hq / Hkv: the
+// gradients of a key/value head; below, the caller sums what is left of a group); lse, delta: [B, Hq, Sq] fp32.
 extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k, const void* v, const float* lse,
                                  const float* delta, void* dk, void* dv, const int* row_lo, const int* row_hi, int B,
                                  int Sq, int Sk, int Hq, int Hkv, long long q_stride, long long k_stride,
@@ -459,7 +459,7 @@ extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k,
                                  float softmax_scale, int fold, int head_dim, void* stream, int* status,
                                  const unsigned* key_bits, const int* any_holes) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  if (Hq % Hkv || (fold != 1 && fold != Hq / Hkv) || (head_dim != 128 && head_dim != 64)) return -1;
+  if (Hq % Hkv || fold < 1 || (Hq / Hkv) % fold || (head_dim != 128 && head_dim != 64)) return -1;
   if ((q_stride | k_stride | v_stride | do_stride | dkv_stride) & 7) return -1;
   DkvParams p;
   p.lse = lse; p.delta = delta; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv; p.dkv_stride = dkv_stride;

@@ -37,9 +37,11 @@ FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
 # backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch) where there is neither
 # dropout nor a bias. ATB_FLASH_BWD_SPLIT=0 selects the one key-block kernel with TMA reduce-adds of dQ everywhere.
 BWD_SPLIT = os.environ.get("ATB_FLASH_BWD_SPLIT", "1") == "1"
-# dK/dV kernel: one CTA per key block and key/value head sums the query heads of its group in tensor memory, if that
-# still gives every SM a CTA; else one CTA per query head, and the groups are summed by a pass over their bf16 results
-# (packed documents, S=4096, 32 heads on 8: 140 us folded, 179 us and 135 us of passes otherwise)
+# dK/dV kernel: a CTA sums the query heads of its group in tensor memory, as many of them (a divisor of the group) as still
+# leave this many CTAs; what is left of a group is summed by a pass over the bf16 results. A CTA per SM will do while a
+# head is short (10 x 512, 16 heads on 4, backward in all: 95 us with 160 CTAs, 114 with 320, 132 with 640), from 16 query
+# blocks on half as many again (2560, 32 on 8: 232 us with 160, 210 with 320, 226 with 640; 3584: 345 with 224, 349 with 448,
+# 374 with 896). Long heads that all see every key fold whole groups or none (4000, 32 on 4: 785 us unfolded, 802 by 4).
 FOLD_MIN_CTAS = 148
 
 
@@ -346,6 +348,13 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     return out, lse
 
 
+def _fold(group: int, ctas: int, q_blocks: int, causal: bool) -> int:
+    """Query heads per CTA of the dK/dV kernel (see FOLD_MIN_CTAS); ``ctas``: its CTAs with whole groups."""
+    need = FOLD_MIN_CTAS if q_blocks < 16 else FOLD_MIN_CTAS * 3 // 2
+    return next((f for f in range(group, 1, -1) if group % f == 0 and ctas * (group // f) >= need
+                 and (f == group or causal or q_blocks < 16)), 1)
+
+
 def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi, fused_out: bool = False,
                   drop=None, bias=None, keys=None):
     """Launch the backward kernels. Returns (dq, dk, dv) shaped like q, k, v. With ``fused_out`` (and
@@ -355,7 +364,7 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
     Sk, Hkv = k.shape[1], k.shape[2]
     split = BWD_SPLIT and drop is None and bias is None
     dq_acc = None if split else torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=q.device)
-    fold = Hq // Hkv if split and B * Hkv * ((Sk + 127) // 128) >= FOLD_MIN_CTAS else 1
+    fold = _fold(Hq // Hkv, B * Hkv * ((Sk + 127) // 128), (Sq + 127) // 128, bool(causal)) if split else 1
     delta = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
     if fused_out and Hkv == Hq and Sq == Sk:
         fused = torch.empty(B, Sq, 3 * Hq, D, dtype=q.dtype, device=q.device)
@@ -386,10 +395,10 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
         args = _as_ctypes("atb_flash_bwd_split", (*ins, p(dq), p(dk), p(dv), *dims))
         rc = bwd(*args[: len(ins)], _lib.ptr(dq_acc), *args[len(ins):], *extra)
     _lib.check(rc, "atb_flash_bwd")
-    if Hkv != Hq and fold == 1:
-        g = Hq // Hkv
-        dk = dk.view(B, Sk, Hkv, g, D).float().sum(3).to(q.dtype)
-        dv = dv.view(B, Sk, Hkv, g, D).float().sum(3).to(q.dtype)
+    if Hkv * fold != Hq:
+        parts, (dk, dv) = (dk, dv), (torch.empty(B, Sk, Hkv, D, dtype=q.dtype, device=q.device) for _ in range(2))
+        rc = L.atb_head_sum(*map(p, parts), p(dk), p(dv), B * Sk * Hkv, Hq // Hkv // fold, D, _lib.stream())
+        _lib.check(rc, "atb_head_sum")
     if fused is not None:
         return fused
     return dq, dk, dv
