@@ -448,6 +448,50 @@ ATB_DEVICE float block_max(float v, float* red) {
   return t;
 }
 
+// Order of attention blocks. Under a causal mask the work of a block of rows grows (of a block of keys: shrinks) with its
+// place in the sequence, and one CTA fills an SM: head after head, each from its heaviest block down, the last heads' heavy
+// blocks started when the other SMs were about to run dry. Here the heaviest blocks of all heads of all samples come first
+// and the lightest last (grid: head, place, run), in runs of as many heads as keep what their CTAs stream, two tensors of
+// `rows` rows, in half of the L2. Without a causal mask the blocks weigh the same, and neighbours that stream the same
+// rows are worth more (4096 x 32 heads: 241 us forward, 254 in the other order): grid (place, head, sample) as it was.
+// Causal, before -> after: forward 8192 x 32 heads of 128 497 -> 455 us, 4096 x 32 157 -> 131, 2 x 2048 x 16 60 -> 44; dQ
+// 4096 x 32 204 -> 193; dK/dV 257 -> 245, 2 x 2048 x 16 93 -> 84.
+struct BlockOrder {
+  int heads, all;      // heads of a sample, of the batch; all == 0: the order without a causal mask
+};
+inline void make_block_order(BlockOrder* o, dim3* grid, int blocks, int heads, int batch, bool causal, long long rows,
+                             int head_dim) {
+  const long long all = (long long)heads * batch, fit = (64LL << 20) / (rows * head_dim * 4);
+  const long long run = fit < 1 ? 1 : fit < all ? fit : all, runs = (all + run - 1) / run;
+  if (causal && blocks <= 65535 && runs <= 65535 && all <= 0x7fffffffLL) {
+    *o = BlockOrder{heads, (int)all};
+    *grid = dim3((unsigned)run, blocks, (unsigned)runs);
+  } else {
+    *o = BlockOrder{heads, 0};
+    *grid = dim3(blocks, heads, batch);
+  }
+}
+// place: 0 = the heaviest block of its head. False: no block (the last run is shorter).
+ATB_DEVICE bool block_of(const BlockOrder& o, int& place, int& blocks, int& head, int& sample) {
+  if (o.all == 0) {
+    place = blockIdx.x;
+    blocks = gridDim.x;
+    head = blockIdx.y;
+    sample = blockIdx.z;
+    return true;
+  }
+  place = blockIdx.y;
+  blocks = gridDim.y;
+  head = blockIdx.z * gridDim.x + blockIdx.x;
+  sample = 0;
+  if (head >= o.all) return false;
+  if (o.all != o.heads) {
+    sample = head / o.heads;
+    head -= sample * o.heads;
+  }
+  return true;
+}
+
 // 32-byte global store (32-byte aligned): one whole sector per thread.
 ATB_DEVICE void stg_v8(void* p, const uint32_t* r) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),

@@ -45,6 +45,7 @@ struct DkvParams {
   float scale, scale_log2;
   int* status;
   KeyBits keys;
+  BlockOrder order;
 };
 
 template <int HD>
@@ -101,8 +102,9 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
-  const int kb = blockIdx.x, b = blockIdx.z;
-  const int h0 = blockIdx.y * p.fold;            // first query head of this CTA
+  int kb, blocks, ho, b;                         // key block (the first is the heaviest), head of the results, sample
+  if (!block_of(p.order, kb, blocks, ho, b)) return;
+  const int h0 = ho * p.fold;                    // first query head of this CTA
   const int hk = h0 / (p.Hq / p.Hkv);
   const int kv0 = kb * BKV;
   const int shift = p.Sk - p.Sq;
@@ -378,7 +380,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // dV / dK of this key block: TMEM lane = key row. tcgen05.ld is a warp-wide (.sync.aligned)
     // instruction: every lane executes it, only the global stores are predicated per row.
     if (ok) {
-      const int j = kv0 + r, ho = blockIdx.y;
+      const int j = kv0 + r;
       const bool store = j < p.Sk;
       const long long at = ((long long)b * p.Sk + j) * p.dkv_stride + ho * HD + half * (HD / 2);
       if (n > 0) tc_fence_after();
@@ -426,7 +428,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 template <int HD>
-int launch_dkv(const void* dout, const void* q, const void* k, const void* v, const DkvParams& p, long long q_stride,
+int launch_dkv(const void* dout, const void* q, const void* k, const void* v, DkvParams p, long long q_stride,
                long long k_stride, long long v_stride, long long do_stride, cudaStream_t stream) {
   CUtensorMap tmQ, tmdO, tmK, tmV;
   const auto bf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -443,7 +445,8 @@ int launch_dkv(const void* dout, const void* q, const void* k, const void* v, co
       return -4;
     attr_set = true;
   }
-  dim3 grid((p.Sk + BKV - 1) / BKV, p.Hq / p.fold, p.B);
+  dim3 grid;
+  make_block_order(&p.order, &grid, (p.Sk + BKV - 1) / BKV, p.Hq / p.fold, p.B, p.causal != 0, p.Sq, HD);
   flash_bwd_dkv_kernel<HD><<<grid, THREADS, SmemK<HD>::TOTAL, stream>>>(tmQ, tmdO, tmK, tmV, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -40,6 +40,7 @@ struct DqParams {
   float scale, scale_log2;
   int* status;
   KeyBits keys;
+  BlockOrder order;
 };
 
 template <int HD>
@@ -86,8 +87,9 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
-  const int qb = gridDim.x - 1 - blockIdx.x;  // heaviest (last) causal blocks first
-  const int h = blockIdx.y, b = blockIdx.z;
+  int place, blocks, h, b;
+  if (!block_of(p.order, place, blocks, h, b)) return;
+  const int qb = blocks - 1 - place;   // heaviest (last) causal blocks first
   const int hk = h / (p.Hq / p.Hkv);
   const int q0 = qb * BQ;
   const int shift = p.Sk - p.Sq;
@@ -385,7 +387,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 }
 
 template <int HD>
-int launch_dq(const void* dout, const void* q, const void* k, const void* v, const DqParams& p, long long q_stride,
+int launch_dq(const void* dout, const void* q, const void* k, const void* v, DqParams p, long long q_stride,
               long long k_stride, long long v_stride, long long do_stride, cudaStream_t stream) {
   CUtensorMap tmQ, tmdO, tmK, tmV;
   const auto bf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -402,7 +404,8 @@ int launch_dq(const void* dout, const void* q, const void* k, const void* v, con
       return -4;
     attr_set = true;
   }
-  dim3 grid((p.Sq + BQ - 1) / BQ, p.Hq, p.B);
+  dim3 grid;
+  make_block_order(&p.order, &grid, (p.Sq + BQ - 1) / BQ, p.Hq, p.B, p.causal != 0, p.Sk, HD);
   flash_bwd_dq_kernel<HD><<<grid, THREADS, SmemQ<HD>::TOTAL, stream>>>(tmQ, tmdO, tmK, tmV, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

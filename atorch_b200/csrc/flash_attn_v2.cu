@@ -49,6 +49,7 @@ struct Params {
   float scale_log2;
   int* status;
   KeyBits keys;
+  BlockOrder order;
 };
 
 template <int HD>
@@ -122,8 +123,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
-  const int qb = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
+  int place, blocks, h, b;
+  if (!block_of(p.order, place, blocks, h, b)) return;
+  const int qb = blocks - 1 - place;   // heaviest (last) causal blocks first
   const int hk = h / (p.Hq / p.Hkv);
   const int q0 = qb * 2 * BQ;
   const int shift = p.Sk - p.Sq;
@@ -393,7 +395,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }
 
 template <int HD>
-int launch_fwd2(const void* q, const void* k, const void* v, const Params& p, long long q_stride, long long k_stride,
+int launch_fwd2(const void* q, const void* k, const void* v, Params p, long long q_stride, long long k_stride,
                 long long v_stride, cudaStream_t stream) {
   CUtensorMap tmQ, tmK, tmV;
   const auto bf16 = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -409,7 +411,8 @@ int launch_fwd2(const void* q, const void* k, const void* v, const Params& p, lo
       return -4;
     attr_set = true;
   }
-  dim3 grid((p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B);
+  dim3 grid;
+  make_block_order(&p.order, &grid, (p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B, p.causal != 0, p.Sk, HD);
   flash_fwd2_kernel<HD><<<grid, THREADS, L2<HD>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -472,3 +472,30 @@ def test_key_padding_without_a_host_look(S, causal, D, monkeypatch):
         fused = flash.flash_attention_qkv(qkv, 2, causal=causal, key_padding_mask=kp)
         sep = flash.flash_attention(q[:, :, :2], k, v, causal=causal, key_padding_mask=kp)
         assert torch.equal(fused, sep)
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,fold_at", [(3, 300, 5, 5, 64, None), (1, 4500, 9, 9, 128, None), (2, 260, 8, 2, 128, 24),
+                                                  (2, 260, 12, 2, 64, 24)])
+def test_causal_block_order_and_partly_folded_groups(B, S, Hq, Hkv, D, fold_at, monkeypatch):
+    """Heaviest blocks first over all heads and samples (4500 x 9 heads of 128: runs of 7 heads, the last one short), and
+    groups of 4 and 6 query heads folded by 2 and 3 with the rest summed after: every block is computed once, by the same
+    operations as in the order without a causal mask, which row intervals that spell the same mask select."""
+    if fold_at is not None:
+        monkeypatch.setattr(flash, "FOLD_MIN_CTAS", fold_at)
+        assert 1 < flash._fold(Hq // Hkv, B * Hkv * 3, 3, True) < Hq // Hkv
+    torch.manual_seed(S + D)
+    q, k, v, dout = (torch.randn(B, S, h, D, device="cuda", dtype=torch.bfloat16) for h in (Hq, Hkv, Hkv, Hq))
+    hi = torch.arange(1, S + 1, device="cuda", dtype=torch.int32).expand(B, S).contiguous()
+    res = []
+    for causal, row_hi in ((True, None), (False, hi)):
+        out, lse = flash.flash_fwd_raw(q, k, v, causal, D ** -0.5, None, row_hi)
+        res.append((out, lse, *flash.flash_bwd_raw(dout, q, k, v, out, lse, causal, D ** -0.5, None, row_hi)))
+    torch.cuda.synchronize()
+    _lib.check_status(torch.device("cuda", 0))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+    if S < 1000:
+        ins = [t.float().requires_grad_(True) for t in (q, k, v)]
+        ref = torch.autograd.grad(attention_reference(*ins, causal=True), ins, dout.float())
+        for g, r in zip(res[0][2:], ref):
+            assert (g.float() - r).norm() <= 1e-2 * r.norm()   # bf16 P, dS and results: 2^-9 each
