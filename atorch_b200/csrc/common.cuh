@@ -452,17 +452,20 @@ ATB_DEVICE float block_max(float v, float* red) {
 // place in the sequence, and one CTA fills an SM: head after head, each from its heaviest block down, the last heads' heavy
 // blocks started when the other SMs were about to run dry. Here the heaviest blocks of all heads of all samples come first
 // and the lightest last (grid: head, place, run), in runs of as many heads as keep what their CTAs stream, two tensors of
-// `rows` rows, in half of the L2. Without a causal mask the blocks weigh the same, and neighbours that stream the same
+// `rows` rows, in half of the L2, a quarter for heads of 4 MB and more, whose many blocks leave a short tail in any run, but
+// of 4 heads at least (dK/dV, 16384 x 16 heads of 128: 1619 us in runs of 4, 1706 of 8, 1782 of 16, 1659 of 1; 4096 x 32: 253
+// in one run, 266 in runs of 16, 269 of 8, 295 of 1). Without a causal mask the blocks weigh the same, and neighbours that stream the same
 // rows are worth more (4096 x 32 heads: 241 us forward, 254 in the other order): grid (place, head, sample) as it was.
-// Causal, before -> after: forward 8192 x 32 heads of 128 497 -> 455 us, 4096 x 32 157 -> 131, 2 x 2048 x 16 60 -> 44; dQ
-// 4096 x 32 204 -> 193; dK/dV 257 -> 245, 2 x 2048 x 16 93 -> 84.
+// Causal, before -> after: forward 16384 x 16 1049 -> 878 us, 8192 x 32 heads of 128 503 -> 448, 4096 x 32 157 -> 131,
+// 2 x 2048 x 16 60 -> 44; dQ 8192 x 32 672 -> 655, 4096 x 32 204 -> 193; dK/dV 257 -> 245, 2 x 2048 x 16 93 -> 84.
 struct BlockOrder {
   int heads, all;      // heads of a sample, of the batch; all == 0: the order without a causal mask
 };
 inline void make_block_order(BlockOrder* o, dim3* grid, int blocks, int heads, int batch, bool causal, long long rows,
                              int head_dim) {
-  const long long all = (long long)heads * batch, fit = (64LL << 20) / (rows * head_dim * 4);
-  const long long run = fit < 1 ? 1 : fit < all ? fit : all, runs = (all + run - 1) / run;
+  const long long all = (long long)heads * batch, head = rows * head_dim * 4;
+  const long long fit = (head < (4LL << 20) ? 64LL << 20 : 32LL << 20) / head, least = fit < 4 ? 4 : fit;
+  const long long run = least < all ? least : all, runs = (all + run - 1) / run;
   if (causal && blocks <= 65535 && runs <= 65535 && all <= 0x7fffffffLL) {
     *o = BlockOrder{heads, (int)all};
     *grid = dim3((unsigned)run, blocks, (unsigned)runs);
