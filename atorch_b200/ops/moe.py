@@ -206,15 +206,15 @@ class _GroupedLinear(torch.autograd.Function):
         dw = mg if mg is not None else torch.empty(w.shape, dtype=w.dtype, device=w.device)
         a, b = (x, dy) if b_mn else (dy, x)             # dW[g] = a[g]^T b[g]
         if len(sizes) == dw.shape[0] and k_groups_ok(a, b, dw):
-            gemm_k_groups(a, b, sizes, dw, mg is not None)
-            sizes = ()
-        r = 0
-        for g, n in enumerate(sizes):
-            if n:
-                gemm(a[r: r + n], b[r: r + n], a_mn=True, b_mn=True, out=dw[g], accumulate=mg is not None)
-            elif mg is None:
-                dw[g].zero_()
-            r += n
+            gemm_k_groups(a, b, sizes, dw, mg is not None)      # writes every group
+        else:
+            if mg is None:
+                dw.zero_()                              # groups without rows, and weights that have no group
+            r = 0
+            for g, n in enumerate(sizes):
+                if n:
+                    gemm(a[r: r + n], b[r: r + n], a_mn=True, b_mn=True, out=dw[g], accumulate=mg is not None)
+                r += n
         if mg is not None:
             w.grad_added_to_main_grad = True
             return dx, None

@@ -1,5 +1,6 @@
 """MoE on CPU: permutation round trip, routers, Grouped_GEMM_MoE against a dense per-token evaluation,
 expert parallel (gloo, world 2) against the single-process result for both dispatchers."""
+import pytest
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
@@ -173,3 +174,25 @@ def test_norms_over_parameters_partitioned_on_different_groups_gloo():
     from tests.dist_utils import run_distributed
 
     run_distributed(_group_aware_norms, world=2)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("sizes", [(4, 6), (4, 0, 6), (4, 6, 0, 0, 0)])
+def test_grouped_gemm_with_other_numbers_of_groups_than_weights(sizes, swiglu, trans_b, device, monkeypatch):
+    """Weights without a group get zero gradients (not what the allocator returns, NaN here), extra groups without rows
+    are left out."""
+    real = torch.empty
+    torch.manual_seed(0)
+    x = torch.randn(10, 64).bfloat16().to(device).requires_grad_(True)
+    w = torch.randn(*((4, 32, 64) if trans_b else (4, 64, 32))).bfloat16().to(device).requires_grad_(True)
+    monkeypatch.setattr(torch, "empty", lambda *a, **kw: t.fill_(float("nan"))
+                        if (t := real(*a, **kw)).is_floating_point() else t)
+    y = (moe_ops.grouped_gemm_swiglu if swiglu else moe_ops.grouped_gemm)(x, w, list(sizes), trans_b)
+    y.float().square().sum().backward()
+    used = [g for g, n in enumerate(sizes) if n]
+    for g in range(4):
+        assert torch.isfinite(w.grad[g]).all()
+        assert bool(w.grad[g].any()) == (g in used)
+    assert torch.isfinite(x.grad).all()
