@@ -44,13 +44,12 @@ SIGNATURES = {
     "atb_rope": "pppppliiilliip",
     "atb_swiglu_fwd": "pplillp",
     "atb_swiglu_bwd": "ppplillp",
-    "atb_flash_fwd_v2": "pppppppiiiiilllifppipp",
+    "atb_flash_fwd_v2": "pppppppiiiiilllifppip",
     "atb_flash_fwd": "pppppppiiiiilllifpp",
-    "atb_flash_bwd_split": "ppppppppppppiiiiillllllifppiipp",
+    "atb_flash_bwd_split": "ppppppppppppiiiiillllllifppii",
     "atb_invert_perm": "ppip",
     "atb_moe_gather_sum": "pppipiiip",
     "atb_moe_ungather": "ppppippiiip",
-    "atb_padded_intervals": "ppppppiiip",
     "atb_row_intervals": "pppiiiipipiippiip",
 }
 _CTYPE = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}

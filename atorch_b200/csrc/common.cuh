@@ -540,13 +540,6 @@ ATB_DEVICE uint32_t visible_keys(int k0, int lo, int hi) {
   return below_e & ~below_a;
 }
 
-// Valid keys of the samples as bits [B, ceil(Sk / 32)]; they matter only where *any != 0 (some sample's valid keys are not
-// contiguous, so that no interval describes them). bits == nullptr: none.
-struct KeyBits {
-  const uint32_t* bits;
-  const int* any;
-};
-
 // Attention dropout: a counter-based keep decision per (batch*head, query row, key column), the same in the
 // forward and the backward kernels and reproducible on the host (ops/flash.py: dropout_keep_mask). One hash
 // serves two neighbouring columns: the low 16 bits decide the even column, the high 16 bits the odd one;

@@ -44,7 +44,6 @@ struct DkvParams {
   int fold;            // query heads per CTA, a divisor of Hq / Hkv: Hq / Hkv (gradients of a key/value head) down to 1
   float scale, scale_log2;
   int* status;
-  KeyBits keys;
   BlockOrder order;
 };
 
@@ -263,13 +262,6 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int r = quarter * 32 + lane;
     const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16);
     const int c0 = kv0 + half * 64;              // first key of this thread
-    uint32_t ok0 = ~0u, ok1 = ~0u;               // valid keys among its 64, where no interval describes them
-    const bool holes = p.keys.bits != nullptr && *p.keys.any != 0;
-    if (holes) {
-      const uint32_t* bits = p.keys.bits + (long long)b * ((p.Sk + 31) / 32);
-      ok0 = c0 < p.Sk ? bits[c0 / 32] : 0u;
-      ok1 = c0 + 32 < p.Sk ? bits[c0 / 32 + 1] : 0u;
-    }
     uint8_t* prow = sP + half * PANEL + r * 128;
     uint8_t* dsrow = sdS + half * PANEL + r * 128;
     bool ok = true;
@@ -301,7 +293,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       raw = row_info(h, qb);
       // ---- P(it) = exp2(S c - lse)
       // warp-uniform, so that the interval tests are a separate path that full tiles never enter
-      const bool row_full = __all_sync(0xffffffffu, !holes && lo <= kv0 && hi >= kv0 + BKV);
+      const bool row_full = __all_sync(0xffffffffu, lo <= kv0 && hi >= kv0 + BKV);
       if (!mbar_wait_warp(s_full, it & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       float pv[64];
@@ -323,7 +315,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           pv[32 + c] = fast_exp2(b0); pv[33 + c] = fast_exp2(b1);
         }
         if (!row_full) {
-          const uint32_t m0 = visible_keys(c0, lo, hi) & ok0, m1 = visible_keys(c0 + 32, lo, hi) & ok1;
+          const uint32_t m0 = visible_keys(c0, lo, hi), m1 = visible_keys(c0 + 32, lo, hi);
 #pragma unroll
           for (int c = 0; c < 32; ++c) {
             if (!(m0 & (1u << c))) pv[c] = 0.f;
@@ -459,8 +451,7 @@ extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k,
                                  const float* delta, void* dk, void* dv, const int* row_lo, const int* row_hi, int B,
                                  int Sq, int Sk, int Hq, int Hkv, long long q_stride, long long k_stride,
                                  long long v_stride, long long do_stride, long long dkv_stride, int causal,
-                                 float softmax_scale, int fold, int head_dim, void* stream, int* status,
-                                 const unsigned* key_bits, const int* any_holes) {
+                                 float softmax_scale, int fold, int head_dim, void* stream, int* status) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || fold < 1 || (Hq / Hkv) % fold || (head_dim != 128 && head_dim != 64)) return -1;
   if ((q_stride | k_stride | v_stride | do_stride | dkv_stride) & 7) return -1;
@@ -471,7 +462,6 @@ extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k,
   p.fold = fold;
   p.scale = softmax_scale; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  p.keys = KeyBits{key_bits, any_holes};
   return head_dim == 64
              ? launch_dkv<64>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream)
              : launch_dkv<128>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream);

@@ -39,7 +39,6 @@ struct DqParams {
   int B, Sq, Sk, Hq, Hkv, causal;
   float scale, scale_log2;
   int* status;
-  KeyBits keys;
   BlockOrder order;
 };
 
@@ -281,7 +280,6 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         hi = min(hi, p.Sk);
       }
     }
-    const uint32_t* bits = p.keys.bits != nullptr && *p.keys.any != 0 ? p.keys.bits + (long long)b * ((p.Sk + 31) / 32) : nullptr;
     const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
     const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
     for (int j = 0; ok && j < n; ++j) {
@@ -305,7 +303,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // mbarrier wait, not a named barrier, so that a warp whose partner gave up cannot wait forever)
       if (!mbar_wait_warp(&pair_bar[quarter], j & 1, abort_flag, p.status)) { ok = false; break; }
       // tiles inside the intersection of the rows' intervals run without per-element tests
-      const bool tile_full = bits == nullptr && (kv0 >= full_lo) && (kv0 + BKV <= full_hi);
+      const bool tile_full = (kv0 >= full_lo) && (kv0 + BKV <= full_hi);
       const int c0 = kv0 + half * 64;
       float pa[32], pb[32];   // P for keys c0 .. c0+31 and c0+32 .. c0+63
 #pragma unroll
@@ -317,11 +315,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         pb[c] = fast_exp2(b0); pb[c + 1] = fast_exp2(b1);
       }
       if (!tile_full) {   // a separate pass, so that fully visible tiles execute no interval tests at all
-        uint32_t m0 = valid ? visible_keys(c0, lo, hi) : 0u, m1 = valid ? visible_keys(c0 + 32, lo, hi) : 0u;
-        if (bits != nullptr) {
-          m0 &= c0 < p.Sk ? bits[c0 / 32] : 0u;
-          m1 &= c0 + 32 < p.Sk ? bits[c0 / 32 + 1] : 0u;
-        }
+        const uint32_t m0 = valid ? visible_keys(c0, lo, hi) : 0u, m1 = valid ? visible_keys(c0 + 32, lo, hi) : 0u;
 #pragma unroll
         for (int c = 0; c < 32; ++c) {
           if (!(m0 & (1u << c))) pa[c] = 0.f;
@@ -418,7 +412,7 @@ extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, 
                                 const float* lse, float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
                                 long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
-                                void* stream, int* status, const unsigned* key_bits, const int* any_holes) {
+                                void* stream, int* status) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || (head_dim != 128 && head_dim != 64)) return -1;
   if ((q_stride | k_stride | v_stride | do_stride | dq_stride) & 7) return -1;
@@ -430,7 +424,6 @@ extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, 
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale = softmax_scale; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  p.keys = KeyBits{key_bits, any_holes};
   return head_dim == 64
              ? launch_dq<64>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream)
              : launch_dq<128>(dout, q, k, v, p, q_stride, k_stride, v_stride, do_stride, (cudaStream_t)stream);

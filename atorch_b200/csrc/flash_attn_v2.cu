@@ -48,7 +48,7 @@ struct Params {
   int B, Sq, Sk, Hq, Hkv, causal;
   float scale_log2;
   int* status;
-  KeyBits keys;
+  const int* holes;    // [B] or null: if any is set, the launch does nothing
   BlockOrder order;
 };
 
@@ -63,9 +63,9 @@ struct L2 {
   static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
 };
 
-// -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi) and is a valid key
-ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi, uint32_t valid_keys) {
-  const uint32_t vis = visible_keys(kv0, lo, hi) & valid_keys;
+// -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi)
+ATB_DEVICE void mask_scores(uint32_t (&x)[32], int kv0, int lo, int hi) {
+  const uint32_t vis = visible_keys(kv0, lo, hi);
 #pragma unroll
   for (int c = 0; c < 32; ++c)
     if (!(vis & (1u << c))) x[c] = 0xff800000u;
@@ -123,6 +123,11 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+  if (p.holes != nullptr) {
+    int any = 0;
+    for (int i = threadIdx.x; i < p.B; i += THREADS) any |= p.holes[i];
+    if (__syncthreads_or(any)) return;
+  }
   int place, blocks, h, b;
   if (!block_of(p.order, place, blocks, h, b)) return;
   const int qb = blocks - 1 - place;   // heaviest (last) causal blocks first
@@ -280,7 +285,6 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
       lo = max(lo, 0); hi = min(hi, p.Sk);
     }
-    const uint32_t* bits = p.keys.bits != nullptr && *p.keys.any != 0 ? p.keys.bits + (long long)b * ((p.Sk + 31) / 32) : nullptr;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t s_addr = lane_addr + t * BKV, o_addr = lane_addr + 2 * BKV + t * HD;
     float m_ref = -INFINITY, l_run = 0.f;
@@ -290,7 +294,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       // the mask tests are compiled into a separate path taken only by warps with a partly visible row
-      const bool full = __all_sync(0xffffffffu, row_valid && bits == nullptr && lo <= kv0 && hi >= kv0 + BKV);
+      const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
       uint32_t x0[32], x1[32], x2[32], x3[32];
       tmem_ld_32x32(s_addr, x0);
       tmem_ld_32x32(s_addr + 32, x1);
@@ -298,15 +302,10 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tmem_ld_32x32(s_addr + 96, x3);
       tmem_ld_wait();
       if (!full) {
-        uint32_t ok_keys[4] = {~0u, ~0u, ~0u, ~0u};
-        if (bits != nullptr) {
-#pragma unroll
-          for (int w = 0; w < 4; ++w) ok_keys[w] = kv0 + 32 * w < p.Sk ? bits[kv0 / 32 + w] : 0u;
-        }
-        mask_scores(x0, kv0, lo, hi, ok_keys[0]);
-        mask_scores(x1, kv0 + 32, lo, hi, ok_keys[1]);
-        mask_scores(x2, kv0 + 64, lo, hi, ok_keys[2]);
-        mask_scores(x3, kv0 + 96, lo, hi, ok_keys[3]);
+        mask_scores(x0, kv0, lo, hi);
+        mask_scores(x1, kv0 + 32, lo, hi);
+        mask_scores(x2, kv0 + 64, lo, hi);
+        mask_scores(x3, kv0 + 96, lo, hi);
       }
       const float mx = fmaxf(fmaxf(max_of(x0), max_of(x1)), fmaxf(max_of(x2), max_of(x3)));
       // raise the reference maximum only when it pays: a stale one costs nothing while 2^(gap) fits bf16/fp32
@@ -419,12 +418,13 @@ int launch_fwd2(const void* q, const void* k, const void* v, Params p, long long
 
 }  // namespace
 
-// Same contract as atb_flash_fwd (flash_attn.cu), for a positive softmax_scale and head dim 128 or 64; key_bits,
-// any_holes: see KeyBits (may be null).
+// Same contract as atb_flash_fwd (flash_attn.cu), for a positive softmax_scale and head dim 128 or 64. With
+// `holes` (int32 [B], may be null) the launch writes nothing if any of them is set: the caller, who is about to learn the
+// same, takes another path then.
 extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, void* o, float* lse, const int* row_lo,
                                 const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
                                 long long k_stride, long long v_stride, int causal, float softmax_scale, void* stream,
-                                int* status, int head_dim, const unsigned* key_bits, const int* any_holes) {
+                                int* status, int head_dim, const int* holes) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || (head_dim != 128 && head_dim != 64) || !(softmax_scale > 0.f)) return -1;
   if ((q_stride | k_stride | v_stride) & 7) return -1;
@@ -433,7 +433,7 @@ extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, voi
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
-  p.keys = KeyBits{key_bits, any_holes};
+  p.holes = holes;
   return head_dim == 64 ? launch_fwd2<64>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream)
                         : launch_fwd2<128>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream);
 }

@@ -1,9 +1,6 @@
 // Per-row key intervals [lo, hi) of the flash-attention kernels from the mask arguments of the attention operator, in
 // one launch: causal, GLM break points, packed GLM pairs, key padding (left or right; `holes[b]` reports a sample whose
-// valid keys are not contiguous), packed sequences. With `holes_on_device` the host need not look at `holes`: the valid
-// keys are also written as bits, and if any sample of the batch has holes the rows of padded tokens see nothing (what
-// dropping the padded tokens and putting the results back gives) and *any is set, at which the attention kernels test
-// the bits as well. The host would have to wait for everything queued before the mask. In separate tensor operations the lowering took 13 to 27 launches,
+// valid keys are not contiguous), packed sequences. In separate tensor operations the lowering took 13 to 27 launches,
 // 0.2 to 0.3 ms of host time in front of attention kernels of 0.1 ms.
 #include "common.cuh"
 
@@ -16,51 +13,6 @@ struct MaskArgs {
   int glm64, pack64, cu64;
   int pairs, n_cu;                   // packed GLM pairs per sample; entries of cu (sequences + 1)
 };
-
-struct KeyInfo {                     // of one sample
-  int cnt, first, last;              // valid keys
-};
-
-// bits[b][w]: keys [32 w, 32 w + 32) of sample b; info[b]. One block per sample.
-__global__ void __launch_bounds__(256) key_bits_kernel(const unsigned char* __restrict__ keys, uint32_t* __restrict__ bits,
-                                                       KeyInfo* __restrict__ info, int Sk, int words) {
-  __shared__ int s_cnt, s_first, s_last;
-  const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) { s_cnt = 0; s_first = INT_MAX; s_last = -1; }
-  __syncthreads();
-  for (int w = warp; w < words; w += 8) {
-    const int j = w * 32 + lane;
-    const uint32_t m = __ballot_sync(0xffffffffu, j < Sk && keys[(long long)b * Sk + j] != 0);
-    if (lane == 0) {
-      bits[(long long)b * words + w] = m;
-      if (m != 0u) {
-        atomicAdd(&s_cnt, __popc(m));
-        atomicMin(&s_first, w * 32 + __ffs(m) - 1);
-        atomicMax(&s_last, w * 32 + 31 - __clz(m));
-      }
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) info[b] = KeyInfo{s_cnt, s_first, s_last};
-}
-
-// The rows' intervals from what key_bits_kernel found (self-attention, key padding and causal only).
-__global__ void __launch_bounds__(256) padded_intervals_kernel(int* __restrict__ row_lo, int* __restrict__ row_hi,
-                                                               int* __restrict__ any, const uint32_t* __restrict__ bits,
-                                                               const KeyInfo* __restrict__ info, int B, int S, int words,
-                                                               int causal) {
-  const int b = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
-  int mine = 0;
-  for (int k = threadIdx.x; k < B; k += 256) mine |= info[k].cnt > 0 && info[k].last - info[k].first + 1 != info[k].cnt;
-  const int holes = __syncthreads_or(mine);
-  if (threadIdx.x == 0 && blockIdx.x == 0 && b == 0) *any = holes;
-  if (i >= S) return;
-  const KeyInfo k = info[b];
-  int lo = k.cnt > 0 ? k.first : 0, hi = min(causal ? i + 1 : S, k.cnt > 0 ? k.last + 1 : 0);
-  if (holes && !((bits[(long long)b * words + i / 32] >> (i & 31)) & 1u)) lo = hi = 0;
-  row_lo[(long long)b * S + i] = lo;
-  row_hi[(long long)b * S + i] = hi;
-}
 
 ATB_DEVICE long long ld_index(const void* p, int is64, long long i) {
   return is64 ? reinterpret_cast<const long long*>(p)[i] : reinterpret_cast<const int*>(p)[i];
@@ -120,20 +72,6 @@ __global__ void __launch_bounds__(256) row_intervals_kernel(int* __restrict__ ro
   row_hi[(long long)b * Sq + i] = (int)hi;
 }
 }  // namespace
-
-// Key padding (optionally causal) of self-attention without a look from the host: row_lo, row_hi int32 [B, S], bits
-// [B, ceil(S / 32)], info int32 [B, 3] (scratch), any int32 [1]; all are written.
-extern "C" int atb_padded_intervals(const unsigned char* keys, int* row_lo, int* row_hi, unsigned* bits, int* info,
-                                    int* any, int B, int S, int causal, void* stream) {
-  if (B <= 0 || S <= 0) return 0;
-  if (B > 65535) return -1;
-  const int words = (S + 31) / 32;
-  cudaStream_t st = (cudaStream_t)stream;
-  key_bits_kernel<<<B, 256, 0, st>>>(keys, bits, reinterpret_cast<KeyInfo*>(info), S, words);
-  padded_intervals_kernel<<<dim3((S + 255) / 256, B), 256, 0, st>>>(row_lo, row_hi, any, bits,
-                                                                    reinterpret_cast<KeyInfo*>(info), B, S, words, causal);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
 
 // row_lo, row_hi: int32 [B, Sq]; holes: int32 [B], written when keys != null. glm [B], pack [B, 2, pairs], cu [n_cu] are
 // int32 (x64 == 0) or int64; any may be null. causal_like: causal, or any GLM form.

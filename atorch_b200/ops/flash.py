@@ -93,9 +93,10 @@ def row_intervals(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_ma
                                                                key_padding_mask, cu_seqlens)
 
 
-def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens):
-    """The lowering in one launch (csrc/masks.cu), or ``None`` for arguments it does not read as they are. With a key
-    padding mask one host synchronisation: an interval can only describe valid keys that lie next to each other."""
+def _launch_row_intervals(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens):
+    """The lowering in one launch (csrc/masks.cu): ``(row_lo, row_hi, holes)``, or ``None`` for arguments it does not read
+    as they are. ``holes`` (int32 per sample, None without a key padding mask) is for the host to look at: an interval can
+    only describe valid keys that lie next to each other."""
     device = torch.device(device)
     if device.type != "cuda" or B < 1 or B > 65535 or Sq < 1 or Sk < 1 or _lib.lib() is None:
         return None
@@ -119,30 +120,54 @@ def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, ke
             p(pack), is64(pack), 0 if pack is None else pack.shape[2], p(kp), p(cu), is64(cu),
             0 if cu is None else cu.numel(), _lib.stream())
     _lib.check(rc, "atb_row_intervals")
-    if kp is not None and any(holes.tolist()):
+    return lo, hi, holes if kp is not None else None
+
+
+def _row_intervals_kernel(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens):
+    """``(row_lo, row_hi)`` of the launch; with a key padding mask one host synchronisation."""
+    out = _launch_row_intervals(B, Sq, Sk, device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens)
+    if out is None:
+        return None
+    if out[2] is not None and any(out[2].tolist()):
         raise NonContiguousKeyMask()
-    return lo, hi
+    return out[:2]
+
+
+class _HolesOnTheWay:
+    """The holes that the mask kernel found, on their way to the host: ``device`` for the attention kernel, which does
+    nothing if there are any, :meth:`check` for the host, which waits for the mask kernel only."""
+
+    def __init__(self, holes: torch.Tensor):
+        self.device = holes
+        self.host = holes.to("cpu", non_blocking=True)
+        self.event = torch.cuda.Event()
+        self.event.record(torch.cuda.current_stream(holes.device))
+
+    def check(self) -> None:
+        self.event.synchronize()
+        if any(self.host.tolist()):
+            raise NonContiguousKeyMask()
+
+
+# From two waves of forward CTAs on, the forward kernel goes ahead of the host's look at the holes of a key padding mask.
+# Forward and backward, right padding, against a look that waits first: 16 x 512, 16 heads of 64 (512 CTAs) 273 -> 236 us,
+# 8 x 1024 335 -> 305, 2 x 4096, 32 heads of 128 1820 -> 1750; below two waves the event and the separate copy cost more
+# than the wait (4 x 512, 128 CTAs: 191 -> 203).
+AHEAD_MIN_CTAS = 296
 
 
 def _padded_intervals(q, k, causal, scale, key_padding_mask, others, drop):
-    """``(row_lo, row_hi, keys)`` for a key padding mask of self-attention, with or without holes, without a host
-    synchronisation; ``keys`` (valid keys as bits, flag) goes to the kernels with the intervals. ``None`` where another
-    kernel than the two-query-tile forward and the two-kernel backward would run: those read intervals only."""
-    B, S = q.shape[:2]
+    """``(row_lo, row_hi, look)`` for a key padding mask of self-attention in front of the two-query-tile forward. The host
+    has to know whether the mask has holes (those are unpadded), but the forward kernel need not wait for it: it is
+    launched first and leaves at once if there are any, and ``look.check()`` comes after it, so that the GPU has work while
+    the host waits and starts up again. ``None`` where another forward kernel would run, the mask comes with others or the
+    forward is too short."""
+    B, S, H = q.shape[:3]
     if key_padding_mask is None or drop or any(o is not None for o in others) or k.shape[1] != S or S < 256 \
-            or not (FWD_TWO_TILES and BWD_SPLIT) or not scale > 0 or B > 65535 \
-            or key_padding_mask.dtype not in (torch.bool, torch.uint8) or key_padding_mask.shape != (B, S):
+            or not FWD_TWO_TILES or not scale > 0 or B * H * ((S + 255) // 256) < AHEAD_MIN_CTAS:
         return None
-    kp = key_padding_mask.to(q.device).contiguous()
-    words = (S + 31) // 32
-    buf = torch.empty(2 * B * S + B * words + 3 * B + 1, dtype=torch.int32, device=q.device)
-    lo, hi, bits, info, flag = buf.split([B * S, B * S, B * words, 3 * B, 1])
-    p = _lib.addr
-    with torch.cuda.device(q.device):
-        rc = _lib.lib().atb_padded_intervals(p(kp), p(lo), p(hi), p(bits), p(info), p(flag), B, S, int(bool(causal)),
-                                             _lib.stream())
-    _lib.check(rc, "atb_padded_intervals")
-    return lo.view(B, S), hi.view(B, S), (bits, flag)
+    out = _launch_row_intervals(B, S, S, q.device, causal, None, None, key_padding_mask, None)
+    return None if out is None else (out[0], out[1], _HolesOnTheWay(out[2]))
 
 
 def row_intervals_reference(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask=None, pack_glm_mask=None,
@@ -322,9 +347,9 @@ def _as_ctypes(name, args):
     return tuple(_lib._CTYPE[c](x) for c, x in zip(_lib.SIGNATURES[name], args))
 
 
-def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None, keys=None):
+def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None, holes=None):
     """Launch the forward kernel. Returns (out [B,Sq,Hq,D] bf16, lse [B,Hq,Sq] fp32). ``drop``: see
-    ``dropout_config``; dropout runs in the single-tile kernel."""
+    ``dropout_config``; dropout runs in the single-tile kernel. ``holes``: see ``_padded_intervals`` (two-tile kernel)."""
     B, Sq, Hq, D = q.shape
     Sk, Hkv = k.shape[1], k.shape[2]
     out = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
@@ -336,7 +361,7 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     args = (p(q), p(k), p(v), p(out), p(lse), p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q),
             _token_stride(k), _token_stride(v), int(causal), softmax_scale, _lib.stream(), _lib.status_addr(q))
     if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0:
-        rc = L.atb_flash_fwd_v2(*args, D, *(map(p, keys) if keys is not None else (0, 0)))
+        rc = L.atb_flash_fwd_v2(*args, D, p(holes))
     elif D == 128 and bias is None and drop is None:
         rc = L.atb_flash_fwd(*args)
     else:
@@ -356,7 +381,7 @@ def _fold(group: int, ctas: int, q_blocks: int, causal: bool) -> int:
 
 
 def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi, fused_out: bool = False,
-                  drop=None, bias=None, keys=None):
+                  drop=None, bias=None):
     """Launch the backward kernels. Returns (dq, dk, dv) shaped like q, k, v. With ``fused_out`` (and
     equal query / key-value head counts) the three are slices of ONE ``[B, S, 3*H, D]`` buffer laid out
     like a fused q|k|v projection output, so the gradient of that projection needs no concatenation."""
@@ -382,7 +407,7 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
             _lib.status_addr(q))
     ins = (p(dout), p(q), p(k), p(v), p(out), p(lse), p(delta))
     if split:
-        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D, *(map(p, keys) if keys is not None else (0, 0)))
+        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D)
     else:
         if D != 128:
             bwd, extra = L.atb_flash_bwd_ex, _extra_args(drop, bias, D)
@@ -406,18 +431,19 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
 
 class _FlashAttn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, causal, scale, row_lo, row_hi, drop=None, bias=None, keys=None):
-        out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, drop, bias, keys)
-        ctx.save_for_backward(q, k, v, out, lse, row_lo, row_hi, *(keys if keys is not None else (None, None)))
+    def forward(ctx, q, k, v, causal, scale, row_lo, row_hi, drop=None, bias=None, look=None):
+        out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, drop, bias, None if look is None else look.device)
+        if look is not None:
+            look.check()
+        ctx.save_for_backward(q, k, v, out, lse, row_lo, row_hi)
         ctx.cfg = (causal, scale, drop, bias)       # bias: (bf16 tensor, strides), not differentiated
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q, k, v, out, lse, row_lo, row_hi, *keys = ctx.saved_tensors
+        q, k, v, out, lse, row_lo, row_hi = ctx.saved_tensors
         causal, scale, drop, bias = ctx.cfg
-        dq, dk, dv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, drop=drop, bias=bias,
-                                   keys=keys if keys[0] is not None else None)
+        dq, dk, dv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, drop=drop, bias=bias)
         return dq, dk, dv, None, None, None, None, None, None, None
 
 
@@ -434,9 +460,9 @@ def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pa
         causal = False   # single-query decode sees every key
     padded = _padded_intervals(q, k, causal, scale, key_padding_mask,
                                (glm_mask, pack_glm_mask, cu_seqlens, additive_mask, additive_bias), dropout_p > 0.0)
-    if padded is not None:
-        return _FlashAttn.apply(q, k, v, bool(causal), float(scale), padded[0], padded[1], None, None, padded[2])
     try:
+        if padded is not None:
+            return _FlashAttn.apply(q, k, v, bool(causal), float(scale), padded[0], padded[1], None, None, padded[2])
         lo, hi = row_intervals(B, Sq, Sk, q.device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens)
     except NonContiguousKeyMask:
         if additive_mask is not None or additive_bias is not None:
@@ -481,23 +507,24 @@ class _FlashAttnQKV(torch.autograd.Function):
     backward emits one fused gradient tensor in the same layout: no slice-backward zero fills or adds."""
 
     @staticmethod
-    def forward(ctx, qkv, H, causal, scale, row_lo, row_hi, cached, keys=None):
+    def forward(ctx, qkv, H, causal, scale, row_lo, row_hi, cached, look=None):
         q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
         if cached is not None:
             out, lse = cached          # output and log-sum-exp kept from the first pass of a checkpointed block
         else:
-            out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, keys=keys)
-        ctx.save_for_backward(qkv, out, lse, row_lo, row_hi, *(keys if keys is not None else (None, None)))
+            out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, holes=None if look is None else look.device)
+        if look is not None:
+            look.check()
+        ctx.save_for_backward(qkv, out, lse, row_lo, row_hi)
         ctx.cfg = (H, causal, scale)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        qkv, out, lse, row_lo, row_hi, *keys = ctx.saved_tensors
+        qkv, out, lse, row_lo, row_hi = ctx.saved_tensors
         H, causal, scale = ctx.cfg
         q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
-        dqkv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, fused_out=True,
-                             keys=keys if keys[0] is not None else None)
+        dqkv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, fused_out=True)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -516,38 +543,40 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
 
     B, S, _, D = qkv.shape
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
-    keys = None
-    padded = _padded_intervals(qkv, qkv, causal, scale, mask_kwargs.get("key_padding_mask"),
+    look = None
+    padded = _padded_intervals(qkv[:, :, :num_heads], qkv, causal, scale, mask_kwargs.get("key_padding_mask"),
                                [v for n, v in mask_kwargs.items() if n not in ("key_padding_mask", "dropout_p", "dropout_seed")],
                                mask_kwargs.get("dropout_p", 0.0) > 0.0)
     try:
         if padded is not None:
-            lo, hi, keys = padded
+            lo, hi, look = padded
         else:
             lo, hi = row_intervals(B, S, S, qkv.device, causal, mask_kwargs.get("glm_mask"),
                                    mask_kwargs.get("pack_glm_mask"), mask_kwargs.get("key_padding_mask"),
                                    mask_kwargs.get("cu_seqlens"))
+        cached = None
+        cur = current_pass() if recompute_cache is not None else None
+        if cur is not None:
+            token, is_recompute = cur
+            if not is_recompute and not torch.is_grad_enabled():
+                H = num_heads
+                out, lse = flash_fwd_raw(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], bool(causal),
+                                         float(scale), lo, hi, holes=None if look is None else look.device)
+                if look is not None:
+                    look.check()
+                recompute_cache[token] = (out, lse)
+                while len(recompute_cache) > RECOMPUTE_CACHE_LIMIT:
+                    recompute_cache.popitem(last=False)
+                return out
+            if is_recompute:
+                cached = recompute_cache.pop(token, None)
+                if cached is not None and cached[0].shape != (B, S, num_heads, D):
+                    cached = None
+        return _FlashAttnQKV.apply(qkv, num_heads, bool(causal), float(scale), lo, hi, cached, look)
     except NonContiguousKeyMask:
         H = num_heads
         return flash_attention(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], causal=causal,
                                softmax_scale=softmax_scale, **mask_kwargs)
-    cached = None
-    cur = current_pass() if recompute_cache is not None else None
-    if cur is not None:
-        token, is_recompute = cur
-        if not is_recompute and not torch.is_grad_enabled():
-            H = num_heads
-            out, lse = flash_fwd_raw(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], bool(causal), float(scale),
-                                     lo, hi, keys=keys)
-            recompute_cache[token] = (out, lse)
-            while len(recompute_cache) > RECOMPUTE_CACHE_LIMIT:
-                recompute_cache.popitem(last=False)
-            return out
-        if is_recompute:
-            cached = recompute_cache.pop(token, None)
-            if cached is not None and cached[0].shape != (B, S, num_heads, D):
-                cached = None
-    return _FlashAttnQKV.apply(qkv, num_heads, bool(causal), float(scale), lo, hi, cached, keys)
 
 
 RECOMPUTE_CACHE_LIMIT = 16   # first passes in flight per layer (pipeline micro-batches) before eviction

@@ -1,4 +1,5 @@
 """sm_100a flash attention against the dense fp32 reference, for every mask form."""
+import collections
 import math
 
 import pytest
@@ -442,9 +443,10 @@ def test_row_intervals_kernel_matches_the_tensor_operations(B, Sq, Sk, idx):
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("S", [256, 300, 517])
-def test_key_padding_without_a_host_look(S, causal, D, monkeypatch):
-    """Right, left, empty and holed samples in one batch and without holes, in the kernels that test key bits and on
-    the host-decided path (unpadding): the same outputs and gradients, padded rows of a holed batch zero."""
+def test_key_padding_with_the_forward_ahead_of_the_host_look(S, causal, D, monkeypatch):
+    """Right, left, empty and holed samples in one batch and without holes, with the forward kernel launched before the
+    host knows of the holes and after it: the same outputs and gradients, padded rows of a holed batch zero."""
+    monkeypatch.setattr(flash, "AHEAD_MIN_CTAS", 0)
     g = torch.Generator().manual_seed(S + D)
     B, Hq, Hkv = 4, 4, 2
     pos = torch.arange(S)[None]
@@ -464,8 +466,8 @@ def test_key_padding_without_a_host_look(S, causal, D, monkeypatch):
         torch.cuda.synchronize()
         _lib.check_status(torch.device("cuda", 0))
         for a, b in zip(got, ref):
-            # both paths round P, dS and the results to bf16 (2^-9 each) but cut the keys into other blocks
-            assert torch.isfinite(a).all() and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+            # the same kernels on the same operands
+            assert torch.isfinite(a).all() and torch.equal(a, b)
         if kp is holed:
             assert not got[0][~holed].any()
         qkv = torch.cat([q[:, :, :2], k, v], 2)
@@ -499,3 +501,53 @@ def test_causal_block_order_and_partly_folded_groups(B, S, Hq, Hkv, D, fold_at, 
         ref = torch.autograd.grad(attention_reference(*ins, causal=True), ins, dout.float())
         for g, r in zip(res[0][2:], ref):
             assert (g.float() - r).norm() <= 1e-2 * r.norm()   # bf16 P, dS and results: 2^-9 each
+
+
+@pytest.mark.parametrize("S,D", [(256, 128), (384, 64)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("where", ["q", "k", "v", "dout"])
+@pytest.mark.parametrize("ahead", [0, 1 << 30])
+def test_padded_tokens_of_a_mask_with_holes_are_not_read(where, causal, S, D, ahead, monkeypatch):
+    """A padded token is dropped before the kernels: what stands there (NaN, infinities) reaches no valid token, neither
+    its output nor its gradients, which are those of the same call with other values there."""
+    monkeypatch.setattr(flash, "AHEAD_MIN_CTAS", ahead)
+    g = torch.Generator().manual_seed(S)
+    kp = (torch.rand(2, S, generator=g) < 0.6).cuda()
+    t = {n: torch.randn(2, S, h, D, generator=g).bfloat16().cuda() for n, h in (("q", 4), ("k", 2), ("v", 2), ("dout", 4))}
+    res = []
+    for bad in (0.0, float("nan"), float("inf")):
+        u = dict(t)
+        u[where] = t[where].masked_fill(~kp[:, :, None, None], bad)
+        ins = [u[n].clone().requires_grad_(True) for n in "qkv"]
+        out = flash.flash_attention(*ins, causal=causal, key_padding_mask=kp)
+        res.append([out.detach(), *torch.autograd.grad(out, ins, u["dout"])])
+    torch.cuda.synchronize()
+    _lib.check_status(torch.device("cuda", 0))
+    for other in res[1:]:
+        for a, b in zip(res[0], other):
+            assert torch.isfinite(b).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ahead", [0, 1 << 30])
+def test_fused_projection_attention_with_a_holed_mask_and_kept_outputs(ahead, monkeypatch):
+    """The recomputing path of the fused q|k|v attention: a mask with holes leaves nothing in the cache and both passes
+    take the unpadding path; a mask without holes keeps the first pass."""
+    from atorch_b200.utils.checkpoint import checkpoint_function
+
+    monkeypatch.setattr(flash, "AHEAD_MIN_CTAS", ahead)
+    torch.manual_seed(0)
+    S, H = 300, 4
+    holed = (torch.rand(2, S, device="cuda") < 0.6)
+    right = torch.arange(S, device="cuda")[None] < torch.tensor([[200], [S]], device="cuda")
+    qkv, dout = (torch.randn(2, S, n, 128, device="cuda", dtype=torch.bfloat16) for n in (3 * H, H))
+    for kp in (holed, right):
+        res = []
+        for cache in (collections.OrderedDict(), None):
+            x = qkv.clone().requires_grad_(True)
+            f = lambda t: flash.flash_attention_qkv(t, H, causal=True, recompute_cache=cache, key_padding_mask=kp)
+            out = f(x) if cache is None else checkpoint_function(f, x)
+            assert cache is None or len(cache) == int(kp is right)
+            res.append([out.detach(), *torch.autograd.grad(out, x, dout)])
+            assert not cache
+        for a, b in zip(*res):
+            assert torch.equal(a, b)
