@@ -31,7 +31,7 @@ import weakref
 
 # forward kernel with two 128-row query tiles per CTA that share every K/V tile (csrc/flash_attn_v2.cu): the
 # default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 136 us against
-# 272 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 51 us against 82 us); ATB_FLASH_V2=0
+# 272 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 55 us against 82 us); ATB_FLASH_V2=0
 # keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
 # backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch) where there is neither

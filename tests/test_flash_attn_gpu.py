@@ -551,3 +551,25 @@ def test_fused_projection_attention_with_a_holed_mask_and_kept_outputs(ahead, mo
             assert not cache
         for a, b in zip(*res):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("B,S,H", [(4, 512, 16), (2, 1021, 8), (1, 2048, 8)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_head_dim_64_forward_is_as_exact_as_the_single_tile_kernel(B, S, H, causal, monkeypatch):
+    """Both kernels take P relative to a row's exact running maximum over blocks of 128 keys, so that the same P are
+    rounded to bf16, which is all but the whole error: what is left is the order of fp32 sums (2^-24 against 2^-9)."""
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(B, S, H, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    qd, kd, vd = (t.double().transpose(1, 2) for t in (q, k, v))
+    s = qd @ kd.transpose(-1, -2) / 8
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+    ref = (torch.softmax(s, -1) @ vd).transpose(1, 2)
+    err = {}
+    for two in (True, False):
+        monkeypatch.setattr(flash, "FWD_TWO_TILES", two)
+        out, _ = flash.flash_fwd_raw(q, k, v, causal, 0.125, None, None)
+        err[two] = ((out.double() - ref).norm() / ref.norm()).item()
+    torch.cuda.synchronize()
+    _lib.check_status(torch.device("cuda", 0))
+    assert err[True] <= 1.002 * err[False]
