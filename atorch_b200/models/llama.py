@@ -146,7 +146,8 @@ class LlamaDecoderLayer(nn.Module):
         pre = type(self.input_layernorm) is RMSNorm and type(self.post_attention_layernorm) is RMSNorm
         x, h = self.input_layernorm(h, carry=True) if pre else (self.input_layernorm(h), h)
         if type(self.qkv_proj) is nn.Linear and self.qkv_proj.bias is None:
-            qkv = ops.linear_rope(x, self.qkv_proj.weight, cos, sin, self.n_q + self.n_kv, d, positions)
+            qkv = ops.linear_rope(x, self.qkv_proj.weight, cos, sin, self.n_q + self.n_kv, d, positions,
+                                  inplace_grad=True)      # a temporary of the attention backward
         else:
             qkv = self._proj(self.qkv_proj, x)
             S = qkv.shape[1]  # the projection may have gathered a sequence-sharded input (sequence parallelism)

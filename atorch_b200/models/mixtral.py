@@ -83,7 +83,8 @@ class MixtralDecoderLayer(nn.Module):
         B, S, _ = h.shape
         d = self.config.head_dim
         x = self.input_layernorm(h)
-        qkv = ops.linear_rope(x, self.qkv_proj.weight, cos, sin, self.n_q + self.n_kv, d, positions)
+        qkv = ops.linear_rope(x, self.qkv_proj.weight, cos, sin, self.n_q + self.n_kv, d, positions,
+                              inplace_grad=True)      # a temporary of the attention backward
         qkv = qkv.view(B, S, self.n_q + 2 * self.n_kv, d)
         a = ops.attention(qkv[:, :, : self.n_q], qkv[:, :, self.n_q: self.n_q + self.n_kv],
                           qkv[:, :, self.n_q + self.n_kv:], **(attn_kwargs or {"causal": True}))

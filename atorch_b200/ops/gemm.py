@@ -276,11 +276,11 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 
 class _LinearRope(torch.autograd.Function):
-    """``rope(x @ W^T)`` with the rotation in the GEMM epilogue; its backward rotates the incoming gradient back (in place
-    where it is a contiguous temporary, as ``rope(..., inplace=True)`` does) in front of the projection's products."""
+    """``rope(x @ W^T)`` with the rotation in the GEMM epilogue; its backward rotates the incoming gradient back in front of
+    the projection's products."""
 
     @staticmethod
-    def forward(ctx, x, weight, cos, sin, positions, nheads, head_dim):
+    def forward(ctx, x, weight, cos, sin, positions, nheads, head_dim, inplace_grad):
         shp = x.shape
         x2 = x.reshape(-1, shp[-1])
         x2 = x2 if x2.stride(-1) == 1 else x2.contiguous()
@@ -292,7 +292,7 @@ class _LinearRope(torch.autograd.Function):
             sin.data_ptr(), _lib.addr(positions), cos.shape[0], nheads, head_dim, _lib.stream(), _lib.status_addr(x2))
         _lib.check(rc, f"atb_gemm_bf16_2cta_rope T={T} N={N} K={K}")
         ctx.save_for_backward(x2, weight, cos, sin, positions)
-        ctx.x_shape, ctx.weight_ref, ctx.heads = shp, weight, (nheads, head_dim)
+        ctx.x_shape, ctx.weight_ref, ctx.heads, ctx.inplace_grad = shp, weight, (nheads, head_dim), inplace_grad
         return out.view(*shp[:-1], N)
 
     @staticmethod
@@ -300,17 +300,21 @@ class _LinearRope(torch.autograd.Function):
         from .elementwise import _rope_launch
 
         x2, weight, cos, sin, positions = ctx.saved_tensors
-        dy = dy if dy.is_contiguous() else dy.contiguous()
-        dy2 = dy.view(-1, dy.shape[-1])
-        _rope_launch(dy2, dy2, cos, sin, positions, *ctx.heads, True)
-        dx, dw = _linear_grads(ctx, dy2, x2, weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return dx, dw, None, None, None, None, None
+        own = ctx.inplace_grad or not dy.is_contiguous()        # a gradient, or a copy of it, to write into
+        src = dy.contiguous().view(-1, dy.shape[-1])
+        dst = src if own else torch.empty_like(src)
+        _rope_launch(dst, src, cos, sin, positions, *ctx.heads, True)
+        dx, dw = _linear_grads(ctx, dst, x2, weight, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return dx, dw, None, None, None, None, None, None
 
 
 def linear_rope(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, nheads: int, head_dim: int,
-                positions: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=True)`` in one kernel where the pair kernel
-    runs (from 256 tokens on) and whole 128-column halves of its tiles are rotated or not."""
+                positions: Optional[torch.Tensor] = None, inplace_grad: bool = False) -> torch.Tensor:
+    """``rope(linear(x, weight), cos, sin, nheads, head_dim, positions)`` in one kernel where the pair kernel runs (from 256
+    tokens on) and whole 128-column halves of its tiles are rotated or not.
+
+    ``inplace_grad``: the backward pass overwrites the incoming gradient instead of writing a new tensor; only where that
+    gradient is a temporary, as it is when the result goes straight into attention."""
     from .elementwise import rope
 
     T = x.numel() // max(x.shape[-1], 1)
@@ -324,10 +328,10 @@ def linear_rope(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: t
             and cos.shape == sin.shape and cos.dim() == 2 and cos.shape[1] == head_dim // 2
             and cos.data_ptr() % 16 == 0 and sin.data_ptr() % 16 == 0
             and (positions is None or (positions.numel() == T and positions.is_contiguous()))):
-        return rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=True)
+        return rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=inplace_grad)
     if positions is not None and positions.dtype != torch.int32:
         positions = positions.to(torch.int32)
-    return _LinearRope.apply(x, weight, cos, sin, positions, nheads, head_dim)
+    return _LinearRope.apply(x, weight, cos, sin, positions, nheads, head_dim, inplace_grad)
 
 
 class _Linear(torch.autograd.Function):

@@ -314,6 +314,25 @@ def test_linear_rope_epilogue(T, K, heads, kv, D, with_pos):
         assert (a.float() - b).norm() <= 2 ** -7 * b.norm()
 
 
+@pytest.mark.parametrize("T", [64, 256])
+def test_linear_rope_leaves_the_incoming_gradient_alone(T):
+    """The caller's gradient is read, not rotated in its place, in the fused kernel and in the two: two passes with the same
+    tensor give the same bits. A layer may say that it is a temporary; the gradients are the same."""
+    from atorch_b200.ops import linear_rope, rope_tables
+
+    torch.manual_seed(T)
+    x, w = _mk(T, 128).view(1, T, 128).requires_grad_(True), _mk(384, 128).requires_grad_(True)
+    dy = _mk(T, 384).view(1, T, 384)
+    kept = dy.clone()
+    cos, sin = rope_tables(T, 128, device="cuda")
+    out = linear_rope(x, w, cos, sin, 2, 128)
+    res = [torch.autograd.grad(out, [x, w], dy, retain_graph=True) for _ in range(2)]
+    assert torch.equal(dy, kept)
+    res.append(torch.autograd.grad(linear_rope(x, w, cos, sin, 2, 128, inplace_grad=True), [x, w], dy))
+    for other in res[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(res[0], other))
+
+
 @pytest.mark.parametrize("sizes", [(256, 0, 1, 300), (77,), (0, 5, 511, 512, 513, 1)])
 @pytest.mark.parametrize("trans_b", [False, True])
 @pytest.mark.parametrize("N", [16, 272])
