@@ -142,8 +142,9 @@ def route(tokens: torch.Tensor, expert_idx: torch.Tensor, num_experts: int):
     if not (_rows_ok(tokens, flat) and flat.numel() == tokens.shape[0] * k and flat.numel() <= ROUTE_MAX_IDS
             and 0 < num_experts <= ROUTE_MAX_EXPERTS):
         return (tokens_per_expert(expert_idx, num_experts), *permute(tokens, expert_idx), None)
-    both = torch.empty(num_experts + flat.numel(), dtype=torch.int64, device=flat.device)
-    counts, order = both[:num_experts], both[num_experts:]
+    # the caller's own: changing the counts in place must not touch `order`, which unpermute() keeps for its backward pass
+    counts = torch.empty(num_experts, dtype=torch.int64, device=flat.device)
+    order = torch.empty(flat.numel(), dtype=torch.int64, device=flat.device)
     slot = torch.empty(flat.numel(), dtype=torch.int32, device=flat.device)
     rc = _lib.lib().atb_moe_sort_ids(flat.data_ptr(), flat.numel(), num_experts, counts.data_ptr(), order.data_ptr(),
                                   slot.data_ptr(), _lib.stream())

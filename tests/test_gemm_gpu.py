@@ -393,6 +393,25 @@ def test_route_sorts_stably(n, k, E, ids):
     assert (x.grad.float() - back).norm() <= 2 ** -8 * back.norm()
 
 
+def test_routing_counts_may_be_changed_in_place():
+    """A clamp of the counts (a capacity, a statistic) before the backward pass changes nothing else."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    T, k, E = 40, 2, 4
+    idx = torch.rand(T, E, device="cuda").topk(k, dim=-1).indices
+    res = []
+    for change in (False, True):
+        torch.manual_seed(1)
+        x, p = _mk(T, 64).requires_grad_(True), torch.rand(T, k, device="cuda").bfloat16().requires_grad_(True)
+        counts, rows, order, slots = M.route(x, idx, E)
+        out = M.unpermute(rows, order, p, k, T, slots)
+        if change:
+            counts.clamp_(max=3)
+        res.append(torch.autograd.grad(out, [x, p], torch.ones_like(out)))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
 def test_expert_ids_out_of_range_are_refused():
     from atorch_b200.modules.moe import Grouped_GEMM_MoE
 
