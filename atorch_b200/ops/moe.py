@@ -63,12 +63,15 @@ def _packed(t: torch.Tensor) -> torch.Tensor:
 
 
 class _Permute(torch.autograd.Function):
+    """Keeps the inverse of ``order`` for its backward pass, not ``order``, which is the caller's."""
+
     @staticmethod
     def forward(ctx, tokens, order, k, slot):
-        ctx.save_for_backward(order, slot)
         ctx.k, ctx.T = k, tokens.shape[0]
         if slot is None:
+            ctx.save_for_backward(_slots(order) if ctx.needs_input_grad[0] else None)
             return tokens.index_select(0, order // k)
+        ctx.save_for_backward(slot)
         src = _packed(tokens)                   # ids sorted by route(): their places are rows for certain
         out = torch.empty(order.numel(), src.shape[1], dtype=src.dtype, device=src.device)
         rc = _lib.lib().atb_moe_gather_rows(src.data_ptr(), order.data_ptr(), out.data_ptr(), order.numel(), k, src.shape[1],
@@ -78,11 +81,10 @@ class _Permute(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        order, slot = ctx.saved_tensors
+        (slot,) = ctx.saved_tensors
         if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
-            zeros = torch.zeros(ctx.T, dy.shape[1], dtype=dy.dtype, device=dy.device)
-            return zeros.index_add(0, order // ctx.k, dy), None, None, None
-        return _gather_sum(_packed(dy), _slots(order) if slot is None else slot, None, ctx.T, ctx.k), None, None, None
+            return dy.index_select(0, slot).view(ctx.T, ctx.k, -1).sum(1), None, None, None
+        return _gather_sum(_packed(dy), slot, None, ctx.T, ctx.k), None, None, None
 
 
 class _Unpermute(torch.autograd.Function):

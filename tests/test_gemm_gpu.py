@@ -412,6 +412,24 @@ def test_routing_counts_may_be_changed_in_place():
     assert all(torch.equal(a, b) for a, b in zip(*res))
 
 
+def test_order_of_permute_may_be_changed_in_place():
+    """What permute() and route() return is the caller's: the gradient of the rows does not come from it."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    T, k, E = 40, 2, 4
+    x, dy = _mk(T, 64).requires_grad_(True), _mk(T * k, 64)
+    idx = torch.rand(T, E, device="cuda").topk(k, dim=-1).indices
+    res = []
+    for f in (lambda: M.permute(x, idx), lambda: M.route(x, idx, E)[1:3]):
+        for change in (False, True):
+            rows, order = f()
+            if change:
+                order.zero_()
+            res.append(torch.autograd.grad(rows, x, dy)[0])
+    assert all(torch.equal(res[0], r) for r in res[1:])
+
+
 def test_expert_ids_out_of_range_are_refused():
     from atorch_b200.modules.moe import Grouped_GEMM_MoE
 
