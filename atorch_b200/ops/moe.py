@@ -90,7 +90,8 @@ class _Permute(torch.autograd.Function):
 class _Unpermute(torch.autograd.Function):
     @staticmethod
     def forward(ctx, rows, order, probs, k, slot):
-        ctx.save_for_backward(rows, order, probs)
+        # the rows are read again only for the gradient of the probabilities
+        ctx.save_for_backward(rows if ctx.needs_input_grad[2] else None, order, probs)
         ctx.k, ctx.sorted = k, slot is not None
         slot = _slots(order) if slot is None else slot
         return _gather_sum(_packed(rows), slot, None if probs is None else probs.contiguous(), order.numel() // k, k)
@@ -98,20 +99,24 @@ class _Unpermute(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         rows, order, probs = ctx.saved_tensors
+        need_dw = ctx.needs_input_grad[2]
         if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
             d, dw = dout.index_select(0, order // ctx.k), None
-            if probs is not None:
+            if need_dw:
                 dots = (rows * d).sum(-1).to(probs.dtype)
                 dw = torch.zeros_like(dots).index_copy(0, order, dots).view(probs.shape)
+            if probs is not None:
                 d = d * probs.reshape(-1, 1).index_select(0, order).to(d.dtype)
             return d, None, dw, None, None
-        rows, w, dout = _packed(rows), None if probs is None else probs.contiguous(), _packed(dout)
-        drows = torch.empty_like(rows) if ctx.needs_input_grad[0] else None
+        w, dout = None if probs is None else probs.contiguous(), _packed(dout)
+        rows = _packed(rows) if need_dw else None
+        n, H = order.numel(), dout.shape[1]
+        drows = torch.empty(n, H, dtype=dout.dtype, device=dout.device) if ctx.needs_input_grad[0] else None
         # an order of the caller's own may leave a choice out
-        dw = (torch.empty_like if ctx.sorted else torch.zeros_like)(w) if w is not None and ctx.needs_input_grad[2] else None
-        rc = _lib.lib().atb_moe_ungather(dout.data_ptr(), rows.data_ptr(), order.data_ptr(), _lib.addr(w),
-                                         2 if w is None else _lib.DT[w.dtype], _lib.addr(drows), _lib.addr(dw), order.numel(),
-                                         ctx.k, rows.shape[1], _lib.stream())
+        dw = (torch.empty_like if ctx.sorted else torch.zeros_like)(w) if need_dw else None
+        rc = _lib.lib().atb_moe_ungather(dout.data_ptr(), _lib.addr(rows), order.data_ptr(), _lib.addr(w),
+                                         2 if w is None else _lib.DT[w.dtype], _lib.addr(drows), _lib.addr(dw), n, ctx.k, H,
+                                         _lib.stream())
         _lib.check(rc, "atb_moe_ungather")
         return drows, None, None if dw is None else dw.view(probs.shape), None, None
 

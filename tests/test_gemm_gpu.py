@@ -430,6 +430,28 @@ def test_order_of_permute_may_be_changed_in_place():
     assert all(torch.equal(res[0], r) for r in res[1:])
 
 
+@pytest.mark.parametrize("probs", [None, torch.bfloat16])
+def test_unpermute_keeps_the_rows_only_for_the_gradient_of_the_probabilities(probs):
+    """Without such a gradient the rows are not kept: they may be changed in place after the call."""
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    T, k, E, H = 40, 2, 4, 64
+    order = torch.argsort(torch.rand(T, E, device="cuda").topk(k, dim=-1).indices.reshape(-1), stable=True)
+    p = None if probs is None else torch.rand(T, k, device="cuda").to(probs)
+    base, dout = _mk(T * k, H).requires_grad_(True), _mk(T, H)
+    res = []
+    for change in (False, True):
+        rows = base * 1.0
+        out = M.unpermute(rows, order, p, k, T)
+        if change:
+            rows.zero_()
+        kept = [t for t in out.grad_fn.saved_tensors if t is not None and t.shape == rows.shape]
+        assert not kept
+        res.append(torch.autograd.grad(out, base, dout)[0])
+    assert torch.equal(*res)
+
+
 def test_expert_ids_out_of_range_are_refused():
     from atorch_b200.modules.moe import Grouped_GEMM_MoE
 
