@@ -28,11 +28,13 @@ def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tenso
 
 def _watched(*ts: Optional[torch.Tensor]) -> bool:
     """Whether something other than reverse-mode autograd looks at these operations (a functorch transform, forward-mode
-    differentiation, a tracer, a tensor subclass): the row kernels would hide them from it, tensor operations do not."""
+    differentiation, a batch of gradients, a tracer or another dispatch mode, a tensor subclass): the row kernels would hide
+    them from it, tensor operations do not."""
     return (torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
-            or torch.compiler.is_compiling() or any(type(t) not in (torch.Tensor, torch.nn.Parameter)
-                                                    or torch.autograd.forward_ad.unpack_dual(t).tangent is not None
-                                                    for t in ts if t is not None))
+            or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0
+            or torch._ops._len_torch_dispatch_stack_pre_dispatch() > 0
+            or any(type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_legacy_batchedtensor(t)
+                   or torch.autograd.forward_ad.unpack_dual(t).tangent is not None for t in ts if t is not None))
 
 
 def _rows_ok(rows: torch.Tensor, order: torch.Tensor) -> bool:
@@ -82,7 +84,7 @@ class _Permute(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (slot,) = ctx.saved_tensors
-        if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
+        if torch.is_grad_enabled() or _watched(dy):     # operations that autograd and the others can follow
             return dy.index_select(0, slot).view(ctx.T, ctx.k, -1).sum(1), None, None, None
         return _gather_sum(_packed(dy), slot, None, ctx.T, ctx.k), None, None, None
 
@@ -100,7 +102,7 @@ class _Unpermute(torch.autograd.Function):
     def backward(ctx, dout):
         rows, order, probs = ctx.saved_tensors
         need_dw = ctx.needs_input_grad[2]
-        if torch.is_grad_enabled():             # differentiated again: operations that autograd can follow
+        if torch.is_grad_enabled() or _watched(dout):   # operations that autograd and the others can follow
             d, dw = dout.index_select(0, order // ctx.k), None
             if need_dw:
                 dots = (rows * d).sum(-1).to(probs.dtype)

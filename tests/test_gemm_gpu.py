@@ -452,6 +452,41 @@ def test_unpermute_keeps_the_rows_only_for_the_gradient_of_the_probabilities(pro
     assert torch.equal(*res)
 
 
+@pytest.mark.parametrize("probs_grad", [False, True])
+def test_routed_rows_under_batched_gradients_and_tracing(probs_grad):
+    """A batch of incoming gradients gives what one pass each gives (sums of k = 2 bf16 terms in another order: two
+    roundings), and a trace holds operations, not the results of the traced inputs."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from atorch_b200.ops import moe as M
+
+    torch.manual_seed(0)
+    T, k, E, H = 40, 2, 4, 64
+    idx = torch.rand(T, E, device="cuda").topk(k, dim=-1).indices
+    p = torch.rand(T, k, device="cuda").bfloat16().requires_grad_(probs_grad)
+
+    def f(x, p):
+        rows, order = M.permute(x, idx)
+        routed, order2, slots = M.route(x, idx, E)[1:]
+        return M.unpermute(rows, order, p, k, T), M.unpermute(routed, order2, p, k, T, slots)
+
+    x = _mk(T, H).requires_grad_(True)
+    wrt = [x, p] if probs_grad else [x]
+    dout = _mk(3 * T, H).view(3, T, H)
+    for out in f(x, p):
+        got = torch.autograd.grad(out, wrt, dout, is_grads_batched=True, retain_graph=True)
+        each = [torch.autograd.grad(out, wrt, d, retain_graph=True) for d in dout]
+        for i, g in enumerate(got):
+            ref = torch.stack([e[i] for e in each]).float()
+            assert (g.float() - ref).norm() <= 2 ** -7 * ref.norm()
+    with torch.no_grad():
+        x2 = _mk(T, H)
+        for pre in (False, True):
+            traced = make_fx(f, pre_dispatch=pre)(x.detach(), p.detach())
+            for a, b in zip(traced(x2, p.detach()), f(x2, p.detach())):
+                assert (a.float() - b.float()).norm() <= 2 ** -7 * b.float().norm()
+
+
 def test_expert_ids_out_of_range_are_refused():
     from atorch_b200.modules.moe import Grouped_GEMM_MoE
 
