@@ -452,29 +452,30 @@ ATB_DEVICE float block_max(float v, float* red) {
 // place in the sequence, and one CTA fills an SM: head after head, each from its heaviest block down, the last heads' heavy
 // blocks started when the other SMs were about to run dry. Here the heaviest blocks of all heads of all samples come first
 // and the lightest last (grid: head, place, run), in runs of as many heads as keep what their CTAs stream, two tensors of
-// `rows` rows, in half of the L2, a quarter for heads of 4 MB and more, whose many blocks leave a short tail in any run, but
-// of 4 heads at least (dK/dV, 16384 x 16 heads of 128: 1619 us in runs of 4, 1706 of 8, 1782 of 16, 1659 of 1; 4096 x 32: 253
-// in one run, 266 in runs of 16, 269 of 8, 295 of 1). Without a causal mask the blocks weigh the same, and neighbours that stream the same
+// `rows` rows, in three eighths of the L2, but of 4 heads at least, and all runs as long as each other or one head longer.
+// The share of the L2: a quarter and a half take 1 % more or less over 4096 to 16384 rows and 7 to 48 heads of 128 (forward
+// and backward, 7168 x 32: 1491, 1501, 1520 us with a quarter, three eighths, a half; 8192 x 32 1923, 1925, 1953; 10240 x 32
+// 2926, 2916, 2949; 10240 x 7 667, 645, 645; head after head 1575, 2001, 3011, 779). Equal runs: with a short last run the
+// order lost what it gains (7168 x 20 in 18 + 2 heads 1075, in 10 + 10 947, head after head 1034; 12288 x 16 2289, 2060,
+// 2182; 10240 x 20 1952, 1845, 1937). Without a causal mask the blocks weigh the same, and neighbours that stream the same
 // rows are worth more (4096 x 32 heads: 241 us forward, 254 in the other order): grid (place, head, sample) as it was.
-// Causal, before -> after: forward 16384 x 16 1049 -> 878 us, 8192 x 32 heads of 128 503 -> 448, 4096 x 32 157 -> 131,
-// 2 x 2048 x 16 60 -> 44; dQ 8192 x 32 672 -> 655, 4096 x 32 204 -> 193; dK/dV 257 -> 245, 2 x 2048 x 16 93 -> 84.
 struct BlockOrder {
   int heads, all;      // heads of a sample, of the batch; all == 0: the order without a causal mask
+  int run, longer;     // heads of a run; the first `longer` runs have one more
 };
 inline void make_block_order(BlockOrder* o, dim3* grid, int blocks, int heads, int batch, bool causal, long long rows,
                              int head_dim) {
-  const long long all = (long long)heads * batch, head = rows * head_dim * 4;
-  const long long fit = (head < (4LL << 20) ? 64LL << 20 : 32LL << 20) / head, least = fit < 4 ? 4 : fit;
-  const long long run = least < all ? least : all, runs = (all + run - 1) / run;
+  const long long all = (long long)heads * batch, fit = (48LL << 20) / (rows * head_dim * 4), least = fit < 4 ? 4 : fit;
+  const long long want = least < all ? least : all, runs = (all + want - 1) / want;
   if (causal && blocks <= 65535 && runs <= 65535 && all <= 0x7fffffffLL) {
-    *o = BlockOrder{heads, (int)all};
-    *grid = dim3((unsigned)run, blocks, (unsigned)runs);
+    *o = BlockOrder{heads, (int)all, (int)(all / runs), (int)(all % runs)};
+    *grid = dim3((unsigned)((all + runs - 1) / runs), blocks, (unsigned)runs);
   } else {
-    *o = BlockOrder{heads, 0};
+    *o = BlockOrder{heads, 0, 0, 0};
     *grid = dim3(blocks, heads, batch);
   }
 }
-// place: 0 = the heaviest block of its head. False: no block (the last run is shorter).
+// place: 0 = the heaviest block of its head. False: no block (a run that is one head shorter).
 ATB_DEVICE bool block_of(const BlockOrder& o, int& place, int& blocks, int& head, int& sample) {
   if (o.all == 0) {
     place = blockIdx.x;
@@ -483,11 +484,12 @@ ATB_DEVICE bool block_of(const BlockOrder& o, int& place, int& blocks, int& head
     sample = blockIdx.z;
     return true;
   }
+  const int run = blockIdx.z;
+  if ((int)blockIdx.x >= o.run + (run < o.longer ? 1 : 0)) return false;
   place = blockIdx.y;
   blocks = gridDim.y;
-  head = blockIdx.z * gridDim.x + blockIdx.x;
+  head = run * o.run + min(run, o.longer) + blockIdx.x;
   sample = 0;
-  if (head >= o.all) return false;
   if (o.all != o.heads) {
     sample = head / o.heads;
     head -= sample * o.heads;

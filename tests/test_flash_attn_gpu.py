@@ -476,10 +476,10 @@ def test_key_padding_with_the_forward_ahead_of_the_host_look(S, causal, D, monke
         assert torch.equal(fused, sep)
 
 
-@pytest.mark.parametrize("B,S,Hq,Hkv,D,fold_at", [(3, 300, 5, 5, 64, None), (1, 9000, 9, 9, 128, None), (2, 260, 8, 2, 128, 24),
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,fold_at", [(3, 300, 5, 5, 64, None), (1, 9000, 13, 13, 128, None), (2, 260, 8, 2, 128, 24),
                                                   (2, 260, 12, 2, 64, 24)])
 def test_causal_block_order_and_partly_folded_groups(B, S, Hq, Hkv, D, fold_at, monkeypatch):
-    """Heaviest blocks first over all heads and samples (9000 x 9 heads of 128: runs of 7 heads, the last one short), and
+    """Heaviest blocks first over all heads and samples (9000 x 13 heads of 128: runs of 7 and 6 heads), and
     groups of 4 and 6 query heads folded by 2 and 3 with the rest summed after: every block is computed once, by the same
     operations as in the order without a causal mask, which row intervals that spell the same mask select."""
     if fold_at is not None:
