@@ -452,20 +452,25 @@ ATB_DEVICE float block_max(float v, float* red) {
 // place in the sequence, and one CTA fills an SM: head after head, each from its heaviest block down, the last heads' heavy
 // blocks started when the other SMs were about to run dry. Here the heaviest blocks of all heads of all samples come first
 // and the lightest last (grid: head, place, run), in runs of as many heads as keep what their CTAs stream, two tensors of
-// `rows` rows, in three eighths of the L2, but of 4 heads at least, and all runs as long as each other or one head longer.
-// The share of the L2: a quarter and a half take 1 % more or less over 4096 to 16384 rows and 7 to 48 heads of 128 (forward
-// and backward, 7168 x 32: 1491, 1501, 1520 us with a quarter, three eighths, a half; 8192 x 32 1923, 1925, 1953; 10240 x 32
-// 2926, 2916, 2949; 10240 x 7 667, 645, 645; head after head 1575, 2001, 3011, 779). Equal runs: with a short last run the
-// order lost what it gains (7168 x 20 in 18 + 2 heads 1075, in 10 + 10 947, head after head 1034; 12288 x 16 2289, 2060,
-// 2182; 10240 x 20 1952, 1845, 1937). Without a causal mask the blocks weigh the same, and neighbours that stream the same
-// rows are worth more (4096 x 32 heads: 241 us forward, 254 in the other order): grid (place, head, sample) as it was.
+// `rows` rows, in half of the L2, three eighths for heads of 3 MB and more, but of 4 heads at least, and all runs as long as
+// each other or one head longer.
+// The share of the L2 (32 heads of 128, forward and backward, a quarter, three eighths, a half; head after head): 4096 rows
+// 568, 568, 566 us; 616. 5120 822, 828, 828; 880. 6144 1132, 1143, 1143; 1203. 7168 1491, 1501, 1520; 1575. 8192 1923, 1925,
+// 1953; 2001. 10240 2926, 2916, 2949; 3011. Over 7 to 48 heads three eighths are within 1 % of the best from 3 MB on. Below,
+// a half is as good under a plain causal mask and keeps 32 heads of 4096 in one run, which short packed documents like better
+// (mean of 8 draws of 9 documents, 32 heads on 8, forward 70.7 against 71.9 us).
+// Equal runs: with a short last run the order lost what it gains (7168 x 20 in 18 + 2 heads 1075, in 10 + 10 947, head after
+// head 1034; 12288 x 16 2289, 2060, 2182; 10240 x 20 1952, 1845, 1937). Without a causal mask the blocks weigh the same, and
+// neighbours that stream the same rows are worth more (4096 x 32 heads: 241 us forward, 254 in the other order): grid (place,
+// head, sample) as it was.
 struct BlockOrder {
   int heads, all;      // heads of a sample, of the batch; all == 0: the order without a causal mask
   int run, longer;     // heads of a run; the first `longer` runs have one more
 };
 inline void make_block_order(BlockOrder* o, dim3* grid, int blocks, int heads, int batch, bool causal, long long rows,
                              int head_dim) {
-  const long long all = (long long)heads * batch, fit = (48LL << 20) / (rows * head_dim * 4), least = fit < 4 ? 4 : fit;
+  const long long all = (long long)heads * batch, head = rows * head_dim * 4;
+  const long long fit = (head < (3LL << 20) ? 64LL << 20 : 48LL << 20) / head, least = fit < 4 ? 4 : fit;
   const long long want = least < all ? least : all, runs = (all + want - 1) / want;
   if (causal && blocks <= 65535 && runs <= 65535 && all <= 0x7fffffffLL) {
     *o = BlockOrder{heads, (int)all, (int)(all / runs), (int)(all % runs)};
