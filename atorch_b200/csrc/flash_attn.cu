@@ -11,6 +11,9 @@
 //
 // The MMA warp issues S_{j+1} before P_j V_j, so the tensor core works on the next scores while
 // the softmax warps exponentiate the current ones.
+// Waits are polled by whole warps and one lane of a converged warp issues (mbar_wait_warp in common.cuh). With waits that
+// every lane may leave on its own: 4096 x 8 heads on 1, dropout 133 us, 119 now; 16384 x 4 heads, all keys, dropout 1272,
+// 1096; 2048 x 32 heads on 8, batch 2, bias 482, 417; one query on 4096 keys, 4 x 32 heads on 8, 63, 54.
 //
 // Masks: every mask of the front end is a per-row key interval [lo, hi): causal (hi = i+1 + Sk-Sq),
 // GLM break-point (hi = max(i+1, g[b])), packed GLM (hi = max over spans), key padding (hi capped
@@ -93,7 +96,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [4]: t0, t1, full_lo, full_hi
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   // a wait already ran out somewhere in this stream of work: do not start, so that a failing
   // launch ends after one wait limit instead of one per wave of CTAs
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
@@ -158,76 +161,75 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  const int t0 = kv_range[0], t1 = kv_range[1];
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int t0 = warp_uniform(kv_range[0]), t1 = warp_uniform(kv_range[1]);
   const int full_lo = kv_range[2], full_hi = kv_range[3];
   const int ntiles = t1 - t0;
   const long long q_row0 = (long long)b * p.Sq + q0;
   const long long k_row0 = (long long)b * p.Sk;
 
   if (warp == 0) {
-    if (lane == 0 && ntiles > 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
+    if (ntiles > 0) {
+      const bool el = elect_one();
+      if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
       constexpr int TILE_B = (HDIM / 64) * PANEL;   // bytes of a [128 x HDIM] tile
-      mbar_expect_tx(q_full, TILE_B);
-      tma_load_2d(sQ, &tmQ, q_full, h * HDIM, (int)q_row0);
-      if (HDIM == 128) tma_load_2d(sQ + PANEL, &tmQ, q_full, h * HDIM + 64, (int)q_row0);
+      if (el) mbar_expect_tx(q_full, TILE_B);
+      if (el) tma_load_2d(sQ, &tmQ, q_full, h * HDIM, (int)q_row0);
+      if (HDIM == 128 && el) tma_load_2d(sQ + PANEL, &tmQ, q_full, h * HDIM + 64, (int)q_row0);
       for (int j = 0; j < ntiles; ++j) {
         const int s = j % KV_STAGES;
         const uint32_t ph = (j / KV_STAGES) & 1;
         const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
-        if (!mbar_wait(&k_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&k_full[s], TILE_B);
-        tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HDIM, krow);
-        if (HDIM == 128) tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HDIM + 64, krow);
-        if (!mbar_wait(&v_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        mbar_expect_tx(&v_full[s], TILE_B);
-        tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HDIM, krow);
-        if (HDIM == 128) tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HDIM + 64, krow);
+        if (!mbar_wait_warp(&k_empty[s], ph ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&k_full[s], TILE_B);
+        if (el) tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HDIM, krow);
+        if (HDIM == 128 && el) tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HDIM + 64, krow);
+        if (!mbar_wait_warp(&v_empty[s], ph ^ 1, abort_flag, p.status)) break;
+        if (el) mbar_expect_tx(&v_full[s], TILE_B);
+        if (el) tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HDIM, krow);
+        if (HDIM == 128 && el) tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HDIM + 64, krow);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && ntiles > 0) {
+    if (ntiles > 0) {
+      const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t idesc_s = umma_idesc(BQ, BKV, 1, 1, false, false);
       constexpr uint32_t idesc_o = umma_idesc(BQ, HDIM, 1, 1, false, true);
-      const uint32_t q_addr = smem_u32(sQ), p_addr = smem_u32(sP);
+      const uint32_t q_desc = umma_desc_lo(smem_u32(sQ), 16), p_desc = umma_desc_lo(smem_u32(sP), 16);
+      const uint32_t k_desc0 = umma_desc_lo(smem_u32(sK), 16), v_desc0 = umma_desc_lo(smem_u32(sV), PANEL);
       auto issue_s = [&](int j) -> bool {
         const int s = j % KV_STAGES, sb = j & 1;
-        if (!mbar_wait(&k_full[s], (j / KV_STAGES) & 1, abort_flag, p.status)) return false;
-        if (!mbar_wait(&s_free[sb], ((j >> 1) & 1) ^ 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&k_full[s], (j / KV_STAGES) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&s_free[sb], ((j >> 1) & 1) ^ 1, abort_flag, p.status)) return false;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + s * TILE);
+        const uint32_t kd = k_desc0 + ((s * TILE) >> 4);
 #pragma unroll
         for (int k = 0; k < HDIM / 16; ++k) {
-          const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tmem_base + sb * BKV, umma_desc_sw128(q_addr + off, 16, 1024),
-                      umma_desc_sw128(k_addr + off, 16, 1024), idesc_s, k != 0);
+          const uint32_t off = ((k >> 2) * PANEL + (k & 3) * 32) >> 4;
+          umma_ss_issue(tmem_base + sb * BKV, q_desc + off, kd + off, idesc_s, k != 0, el);
         }
-        umma_commit(&s_full[sb]);
-        umma_commit(&k_empty[s]);
+        umma_commit_issue(&s_full[sb], el);
+        umma_commit_issue(&k_empty[s], el);
         return true;
       };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status);
+      bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status);
       ok = ok && issue_s(0);
       for (int j = 0; ok && j < ntiles; ++j) {
         if (j + 1 < ntiles) ok = issue_s(j + 1);
         if (!ok) break;
         const int s = j % KV_STAGES;
-        if (!mbar_wait(p_full, j & 1, abort_flag, p.status)) break;
-        if (!mbar_wait(&v_full[s], (j / KV_STAGES) & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(p_full, j & 1, abort_flag, p.status)) break;
+        if (!mbar_wait_warp(&v_full[s], (j / KV_STAGES) & 1, abort_flag, p.status)) break;
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sV + s * TILE);
+        const uint32_t vd = v_desc0 + ((s * TILE) >> 4);
 #pragma unroll
         for (int k = 0; k < BKV / 16; ++k) {
-          const uint32_t a_off = (k >> 2) * PANEL + (k & 3) * 32;
-          umma_f16<1>(tmem_base + 2 * BKV, umma_desc_sw128(p_addr + a_off, 16, 1024),
-                      umma_desc_sw128(v_addr + k * 2048, PANEL, 1024), idesc_o, k != 0);
+          const uint32_t a_off = ((k >> 2) * PANEL + (k & 3) * 32) >> 4;
+          umma_ss_issue(tmem_base + 2 * BKV, p_desc + a_off, vd + k * 128, idesc_o, k != 0, el);
         }
-        umma_commit(o_full);
-        umma_commit(&v_empty[s]);
-        umma_commit(p_free);
+        umma_commit_issue(o_full, el);
+        umma_commit_issue(&v_empty[s], el);
+        umma_commit_issue(p_free, el);
       }
     }
   } else {
@@ -254,7 +256,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     bool ok = true;
 
     auto accumulate_o = [&](int j) -> bool {  // O := O * alpha_j + O_j
-      if (!__all_sync(0xffffffffu, mbar_wait(o_full, j & 1, abort_flag, p.status))) return false;
+      if (!mbar_wait_warp(o_full, j & 1, abort_flag, p.status)) return false;
       tc_fence_after();
 #pragma unroll
       for (int cc = 0; cc < HDIM / 64; ++cc) {
@@ -270,7 +272,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     for (int j = 0; j < ntiles; ++j) {
       const int sb = j & 1;
       const int kv0 = (t0 + j) * BKV;
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[sb], (j >> 1) & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(&s_full[sb], (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       float sv[64];
 #pragma unroll
@@ -326,7 +328,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       rm[half * 128 + r] = mx;
       __syncwarp();
       if (lane == 0) mbar_arrive(x_bar);
-      if (!__all_sync(0xffffffffu, mbar_wait(x_bar, j & 1, abort_flag, p.status))) { ok = false; break; }
+      if (!mbar_wait_warp(x_bar, j & 1, abort_flag, p.status)) { ok = false; break; }
       mx = fmaxf(mx, rm[(half ^ 1) * 128 + r]);
       // m_run / mx are raw (unscaled) score maxima; the softmax scale (> 0) is folded into the
       // exponent: p = 2^(s * c - m * c), one FFMA + one EX2 per element
@@ -362,7 +364,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // previous tile's P V product must be folded in (and must have finished reading sP)
       if (j > 0) {
         if (!accumulate_o(j - 1)) { ok = false; break; }
-        if (!__all_sync(0xffffffffu, mbar_wait(p_free, (j - 1) & 1, abort_flag, p.status))) { ok = false; break; }
+        if (!mbar_wait_warp(p_free, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
       }
       alpha_prev = alpha;
       // P tile, K-major 128B-swizzled: panel `half`, row r, 16-byte chunk c8 at slot (c8 ^ (r & 7))
@@ -382,7 +384,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     s_rowsum[half * 128 + r] = l_run;
     __syncwarp();
     if (lane == 0) mbar_arrive(x_bar);
-    ok = ok && mbar_wait(x_bar, ntiles & 1, abort_flag, p.status);
+    ok = ok && mbar_wait_warp(x_bar, ntiles & 1, abort_flag, p.status);
     const float l_tot = l_run + s_rowsum[(half ^ 1) * 128 + r];
     if (ok && row_valid) {
       const float inv = l_tot > 0.f ? (DROP ? p.drop.keep_scale : 1.f) / l_tot : 0.f;
