@@ -250,17 +250,6 @@ ATB_DEVICE void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, ui
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// fp8 (e4m3/e5m2) operands, fp32 accumulate
-ATB_DEVICE void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // Make the mbarrier track completion of all tcgen05 ops issued so far by this thread.
 ATB_DEVICE void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -364,6 +353,22 @@ ATB_DEVICE void umma_ss_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uin
   if constexpr (CTA_GROUP == 1) ATB_UMMA_SS("1");
   else ATB_UMMA_SS("2");
 #undef ATB_UMMA_SS
+}
+// kind::f8f6f4, shared-memory operands, one CTA
+ATB_DEVICE void umma_f8_issue(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
+                              uint32_t issue) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      ".reg .b64 a, b;\n"
+      "mov.b64 a, {%1, %3};\n"
+      "mov.b64 b, {%2, %3};\n"
+      "setp.ne.b32 p, %5, 0;\n"
+      "setp.ne.b32 q, %6, 0;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %4, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_lo), "r"(b_lo), "r"(UMMA_DESC_HI), "r"(idesc), "r"(accumulate), "r"(issue)
+      : "memory");
 }
 ATB_DEVICE void umma_ts_issue(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate,
                               uint32_t issue) {

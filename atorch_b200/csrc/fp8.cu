@@ -206,6 +206,8 @@ __global__ void dequant_kernel(const uint8_t* __restrict__ q, const float* __res
 // ---------------------------------------------------------------------------------------------
 // scaled GEMM
 // ---------------------------------------------------------------------------------------------
+// Waits are polled by whole warps and one lane of a converged warp issues (mbar_wait_warp in common.cuh); with waits that
+// every lane may leave on its own, 4096 x 11008 x 4096 took 419 us in place of 313, 8192 x 2048 x 2048 84 in place of 64.
 constexpr int GBM = 128, GBN = 128, GBK = 128, GST = 6;
 constexpr int G_TILE = 128 * 128;  // bytes per operand tile
 constexpr int G_BAR_OFF = GST * 2 * G_TILE;
@@ -232,7 +234,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) return;
   const int tiles_m = (M + GBM - 1) / GBM, tiles_n = (N + GBN - 1) / GBN;
   const int num_tiles = tiles_m * tiles_n;
@@ -248,16 +250,17 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * GBM, n0 = (tile / tiles_m) * GBN;
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % GST;
-          if (!mbar_wait(&empty[s], ((it / GST) & 1) ^ 1, abort_flag, status)) goto prod_done;
+    const bool el = elect_one();
+    uint32_t it = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const int m0 = (tile % tiles_m) * GBM, n0 = (tile / tiles_m) * GBN;
+      for (int kb = 0; kb < KB; ++kb, ++it) {
+        const int s = it % GST;
+        if (!mbar_wait_warp(&empty[s], ((it / GST) & 1) ^ 1, abort_flag, status)) goto prod_done;
+        if (el) {
           mbar_expect_tx(&full[s], 2 * G_TILE);
           tma_load_2d(sA + s * G_TILE, &tmA, &full[s], kb * GBK, m0);
           tma_load_2d(sB + s * G_TILE, &tmB, &full[s], kb * GBK, n0);
@@ -266,23 +269,22 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     }
   prod_done:;
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc(GBM, GBN, 0, 0, false, false);
-      uint32_t it = 0;
-      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % GST, buf = it & 1;
-          if (!mbar_wait(&tempty[buf], ((it >> 1) & 1) ^ 1, abort_flag, status)) goto mma_done;
-          if (!mbar_wait(&full[s], (it / GST) & 1, abort_flag, status)) goto mma_done;
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + s * G_TILE), b_addr = smem_u32(sB + s * G_TILE);
+    constexpr uint32_t idesc = umma_idesc(GBM, GBN, 0, 0, false, false);
+    const uint32_t el = elect_one();   // the lane that issues and commits
+    const uint32_t a_desc = umma_desc_lo(smem_u32(sA), 16), b_desc = umma_desc_lo(smem_u32(sB), 16);
+    uint32_t it = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      for (int kb = 0; kb < KB; ++kb, ++it) {
+        const int s = it % GST, buf = it & 1;
+        if (!mbar_wait_warp(&tempty[buf], ((it >> 1) & 1) ^ 1, abort_flag, status)) goto mma_done;
+        if (!mbar_wait_warp(&full[s], (it / GST) & 1, abort_flag, status)) goto mma_done;
+        tc_fence_after();
+        const uint32_t off = (s * G_TILE) >> 4;
 #pragma unroll
-          for (int k = 0; k < GBK / 32; ++k)
-            umma_f8(tmem_base + buf * GBN, umma_desc_sw128(a_addr + k * 32, 16, 1024),
-                    umma_desc_sw128(b_addr + k * 32, 16, 1024), idesc, k != 0);
-          umma_commit(&empty[s]);
-          umma_commit(&tfull[buf]);
-        }
+        for (int k = 0; k < GBK / 32; ++k)
+          umma_f8_issue(tmem_base + buf * GBN, a_desc + off + k * 2, b_desc + off + k * 2, idesc, k != 0, el);
+        umma_commit_issue(&empty[s], el);
+        umma_commit_issue(&tfull[buf], el);
       }
     }
   mma_done:;
@@ -299,7 +301,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       bool ok = true;
       for (int kb = 0; kb < KB; ++kb, ++it) {
         const int buf = it & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(&tfull[buf], (it >> 1) & 1, abort_flag, status))) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull[buf], (it >> 1) & 1, abort_flag, status)) { ok = false; break; }
         tc_fence_after();
         const float as = row_ok ? ep.a_s[(long long)row * KB + kb] : 0.f;
         const float bs_blk = ep.b_row_mode ? 0.f : ep.b_s[(long long)(n0 >> 7) * KB + kb];
