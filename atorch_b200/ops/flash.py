@@ -34,6 +34,10 @@ import weakref
 # 272 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 55 us against 82 us); ATB_FLASH_V2=0
 # keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
+# Head dim 64 keeps the single-tile kernel while its CTAs (128 rows) fit one wave: two tiles a CTA then leave half of the SMs
+# without work (16 heads, all keys, single / two tiles: 512 rows, 64 CTAs, 11.9 / 14.5 us; 1024, 128 CTAs, 16.5 / 20.6; two waves,
+# 64 heads of 512: 20.6 / 14.5; 32 heads of 1024: 30.8 / 22.7).
+ONE_WAVE = 148
 # backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch) where there is neither
 # dropout nor a bias. ATB_FLASH_BWD_SPLIT=0 selects the one key-block kernel with TMA reduce-adds of dQ everywhere.
 BWD_SPLIT = os.environ.get("ATB_FLASH_BWD_SPLIT", "1") == "1"
@@ -355,12 +359,14 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     out = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
     L = _lib.lib()
-    # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences; the single-tile kernel otherwise, and for
+    # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences (and enough blocks, see ONE_WAVE); the single-tile
+    # kernel otherwise, and for
     # dropout, a bias, and a scale that is not positive (hidden scores are -inf before they are scaled)
     p = _lib.addr
     args = (p(q), p(k), p(v), p(out), p(lse), p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q),
             _token_stride(k), _token_stride(v), int(causal), softmax_scale, _lib.stream(), _lib.status_addr(q))
-    if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0:
+    if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0 \
+            and (D == 128 or B * Hq * ((Sq + 127) // 128) > ONE_WAVE):
         rc = L.atb_flash_fwd_v2(*args, D, p(holes))
     elif D == 128 and bias is None and drop is None:
         rc = L.atb_flash_fwd(*args)

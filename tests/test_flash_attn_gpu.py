@@ -12,6 +12,12 @@ from atorch_b200.ops import flash
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def two_tiles_at_any_number_of_blocks(monkeypatch):
+    """The shapes here have few blocks; the two-tile kernel takes head dim 64 from more than a wave of them on."""
+    monkeypatch.setattr(flash, "ONE_WAVE", 0)
+
+
 def _qkv(B, Sq, Sk, Hq, Hkv, D=128, fused=False):
     if fused and Sq == Sk:
         qkv = torch.randn(B, Sq, Hq + 2 * Hkv, D, device="cuda", dtype=torch.bfloat16)
@@ -573,3 +579,27 @@ def test_head_dim_64_forward_is_as_exact_as_the_single_tile_kernel(B, S, H, caus
     torch.cuda.synchronize()
     _lib.check_status(torch.device("cuda", 0))
     assert err[True] <= 1.002 * err[False]
+
+
+@pytest.mark.parametrize("H,S,two", [(74, 256, False), (75, 256, True), (49, 300, False), (50, 300, True)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_head_dim_64_kernel_by_waves_of_blocks(H, S, two, causal, monkeypatch):
+    """One wave of 128-row blocks (148) stays on the single-tile kernel, one block more takes the two-tile kernel: both
+    against the fp32 reference (bf16 P and result: 2^-9 each)."""
+    monkeypatch.setattr(flash, "ONE_WAVE", 148)
+    torch.manual_seed(H)
+    q, k, v = (torch.randn(1, S, H, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+    names = []
+    real = _lib.lib()
+
+    class Spy:
+        def __getattr__(self, name):
+            names.append(name)
+            return getattr(real, name)
+
+    monkeypatch.setattr(_lib, "lib", lambda: Spy())
+    out, _ = flash.flash_fwd_raw(q, k, v, causal, 0.125, None, None)
+    assert names == ["atb_flash_fwd_v2" if two else "atb_flash_fwd_ex"]
+    ref = attention_reference(q, k, v, causal=causal).float()
+    torch.cuda.synchronize()
+    assert (out.float() - ref).norm() <= 2 ** -7 * ref.norm()
