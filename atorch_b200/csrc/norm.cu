@@ -216,17 +216,23 @@ __global__ void __launch_bounds__(NT, (VPT <= 2 && !LN) ? 4 : 1) norm_fwd_kernel
 // a time to hide it behind. So a step takes R rows, whose sums share one barrier (two sets of partial sums, used in turn),
 // and everything that the next R rows read - x, dy, dres and the row statistics - is requested before the reduction. R is
 // 2 for rows of up to 2048 16-bit elements and 1 above, where one row already keeps as many bytes in flight. The pieces
-// stay packed between the two passes (decoding them again is cheaper than 16 registers a piece, which cost the second CTA).
+// stay packed between the two passes (decoding them again is cheaper than 16 registers a piece, which cost the second CTA;
+// see KEEP). With and without a residual gradient are kernels of their own: the registers of the one slowed the other by up
+// to 9 % (4096 x 4096 bf16 RMSNorm without it, data in L2, 24.9 -> 22.8 us).
 // bf16 RMSNorm with a residual gradient, cold L2, before -> after: 4096 x 2048 26.6 -> 20.4 us, 4096 x 4096 45.9 -> 34.8,
 // 16384 x 2048 79.9 -> 57.4 (4.7 TB/s), 4096 x 8192 104 -> 61.5.
 // ------------------------------------------------------------------------------------------
-template <typename T, int VPT, int R, bool LN>
+template <typename T, int VPT, int R, bool LN, bool RES>
 __global__ void __launch_bounds__(NT, VPT == 1 || (VPT == 2 && (sizeof(T) == 2 || !LN)) ? 2 : 1)
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
                 T* __restrict__ dx, float* __restrict__ partial_dw, float* __restrict__ partial_db, int M, int N) {
   constexpr int NW = NT / 32, SUMS = LN ? 2 : 1;
-  constexpr bool AHEAD = VPT == 1 || (sizeof(T) == 2 && !LN);   // dres with the row; the others have no registers left
+  constexpr bool AHEAD = RES && (VPT == 1 || (sizeof(T) == 2 && !LN));   // dres with the row; the others have no registers left
+  // x^ and w dy stay decoded between the passes where there are registers for it and decoding twice shows: without a
+  // residual gradient, 16384 x 4096 bf16 RMSNorm 83.2 us decoded twice, 80.3 kept, 12000 x 8192 fp16 LayerNorm 141, 132,
+  // 16384 x 768 fp32 LayerNorm 57.4, 55.2
+  constexpr bool KEEP = !RES && (sizeof(T) == 4 ? LN && VPT == 1 : LN ? std::is_same_v<T, __half> && VPT == 4 : VPT == 2);
   __shared__ __align__(16) float red[2][SUMS * R][NW];
   const int nvec = N >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Raw8<T> wr[VPT];
@@ -255,7 +261,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
         if (c < nvec) {
           nx[r][i] = ldraw<T>(x + (size_t)(row + r) * N + c * 8);
           nd[r][i] = ldraw<T>(dy + (size_t)(row + r) * N + c * 8);
-          if (AHEAD && dres != nullptr) nr[r][i] = ldraw<T>(dres + (size_t)(row + r) * N + c * 8);
+          if (AHEAD) nr[r][i] = ldraw<T>(dres + (size_t)(row + r) * N + c * 8);
         }
       }
     }
@@ -264,6 +270,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
   int par = 0;
   for (int row = r0; row < r1; row += R, par ^= 1) {
     Raw8<T> cx[R][VPT], cd[R][VPT], cr[R][VPT];
+    float kx[KEEP ? R : 1][KEEP ? VPT : 1][8], kg[KEEP ? R : 1][KEEP ? VPT : 1][8];
     float rs[R], mn[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -284,6 +291,7 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float xh = (xv[j] - mn[r]) * rs[r], g = dyv[j] * wv[j];
+            if constexpr (KEEP) { kx[r][i][j] = xh; kg[r][i][j] = g; }
             c1 += xh * g;
             c2 += g;
             dwacc[i][j] += dyv[j] * xh;
@@ -314,13 +322,19 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
       for (int i = 0; i < VPT; ++i) {
         const int c = threadIdx.x + i * NT;
         if (c < nvec) {
-          float xv[8], dyv[8], wv[8], o[8];
-          decode8<T>(cx[r][i], xv);
-          decode8<T>(cd[r][i], dyv);
-          decode8<T>(wr[i], wv);
+          float o[8];
+          if constexpr (KEEP) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = (dyv[j] * wv[j] - (xv[j] - mn[r]) * rs[r] * c1 - c2) * rs[r];
-          if (dres != nullptr) {
+            for (int j = 0; j < 8; ++j) o[j] = (kg[r][i][j] - kx[r][i][j] * c1 - c2) * rs[r];
+          } else {
+            float xv[8], dyv[8], wv[8];
+            decode8<T>(cx[r][i], xv);
+            decode8<T>(cd[r][i], dyv);
+            decode8<T>(wr[i], wv);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = (dyv[j] * wv[j] - (xv[j] - mn[r]) * rs[r] * c1 - c2) * rs[r];
+          }
+          if constexpr (RES) {
             float rv[8];
             decode8<T>(AHEAD ? cr[r][i] : ldraw<T>(dres + (size_t)(row + r) * N + c * 8), rv);
 #pragma unroll
@@ -400,9 +414,15 @@ int launch_bwd(const void* dy, const void* x, const void* w, const float* mean, 
                void* dx, float* pdw, float* pdb, int parts, int M, int N, cudaStream_t st) {
   const int nvec = N >> 3;
   const int vpt = (nvec + NT - 1) / NT;
-#define L(V, R)                                                                                                 \
-  norm_bwd_kernel<T, V, R, LN><<<parts, NT, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd,       \
-                                                     (const T*)dres, (T*)dx, pdw, pdb, M, N)
+#define L(V, R)                                                                                                      \
+  do {                                                                                                               \
+    if (dres != nullptr)                                                                                             \
+      norm_bwd_kernel<T, V, R, LN, true><<<parts, NT, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd,   \
+                                                               (const T*)dres, (T*)dx, pdw, pdb, M, N);              \
+    else                                                                                                             \
+      norm_bwd_kernel<T, V, R, LN, false><<<parts, NT, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd,  \
+                                                                nullptr, (T*)dx, pdw, pdb, M, N);                    \
+  } while (0)
   if (vpt <= 1) L(1, (sizeof(T) == 2 ? 2 : 1));
   else if (vpt <= 2) L(2, 1);
   else if (vpt <= 4) L(4, 1);
