@@ -565,3 +565,25 @@ def test_gemm_k_groups(sizes, M, N, dtype, accumulate):
             tol = torch.finfo(dtype).eps + 2 * max(n, 1) ** 0.5 * 2 ** -23
             assert (out[g].float() - ref).norm() <= tol * max(ref.norm().item(), 1e-30)
         r += n
+
+
+@pytest.mark.parametrize("sizes", [(64, 0, 63, 65, 129), (7,) * 17])
+@pytest.mark.parametrize("M,N", [(8, 264), (264, 16), (512, 256)])
+def test_gemm_k_groups_accumulates_in_bf16(sizes, M, N):
+    """C += A_g^T B_g with a bf16 C, stored in 16-byte and in 32-byte pieces: one rounding of the fp32 sum (2^-9 of the result,
+    twice that at the outside); groups without rows are left alone."""
+    from atorch_b200.ops.gemm import gemm_k_groups, k_groups_ok
+
+    torch.manual_seed(M)
+    a, b = _mk(sum(sizes), M), _mk(sum(sizes), N)
+    out = torch.randn(len(sizes), M, N, device="cuda").bfloat16()
+    before = out.clone()
+    assert k_groups_ok(a, b, out)
+    gemm_k_groups(a, b, sizes, out, True)
+    torch.cuda.synchronize()
+    _lib.check_status(out.device)
+    r = 0
+    for g, n in enumerate(sizes):
+        ref = before[g].double() + a[r: r + n].double().t() @ b[r: r + n].double()
+        assert torch.equal(out[g], before[g]) if n == 0 else (out[g].double() - ref).norm() <= 2 ** -8 * ref.norm()
+        r += n

@@ -196,3 +196,38 @@ def test_grouped_gemm_with_other_numbers_of_groups_than_weights(sizes, swiglu, t
         assert torch.isfinite(w.grad[g]).all()
         assert bool(w.grad[g].any()) == (g in used)
     assert torch.isfinite(x.grad).all()
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("sizes", [(4, 0, 65), (0, 3) * 9 + (0, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_grouped_gemm_adds_into_main_grad(dtype, sizes, swiglu, trans_b, device):
+    """The weight gradient goes into ``main_grad`` in either layout and type (more groups than one launch takes, groups
+    without rows keep what is there): old + dW with dW as the same call returns it without one, which is rounded to bf16
+    (2^-9), and the sum to the type of main_grad."""
+    torch.manual_seed(len(sizes))
+    G = len(sizes)
+    x = torch.randn(sum(sizes), 64).bfloat16().to(device)
+    w0 = torch.randn(*((G, 32, 64) if trans_b else (G, 64, 32))).bfloat16().to(device)
+    old = torch.randn(w0.shape).to(dtype).to(device)
+    f = moe_ops.grouped_gemm_swiglu if swiglu else moe_ops.grouped_gemm
+    res = []
+    for main in (False, True):
+        w = w0.clone().requires_grad_(True)
+        if main:
+            w.main_grad = old.clone()
+        xs = x.clone().requires_grad_(True)
+        y = f(xs, w, list(sizes), trans_b)
+        y.backward(torch.ones_like(y))
+        res.append((w, xs.grad))
+    (wa, dxa), (wb, dxb) = res
+    assert wb.grad is None and wb.grad_added_to_main_grad and torch.equal(dxa, dxb)
+    dw, mg = wa.grad.float(), wb.main_grad.float()
+    for g, n in enumerate(sizes):
+        if n == 0:
+            assert torch.equal(wb.main_grad[g], old[g])
+        else:
+            tol = 2 ** -8 * dw[g].norm() + torch.finfo(dtype).eps * mg[g].norm()
+            assert (mg[g] - old[g].float() - dw[g]).norm() <= tol
