@@ -217,51 +217,6 @@ ATB_DEVICE void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
 ATB_DEVICE void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 ATB_DEVICE void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem]; `accumulate`==0 overwrites D.
-template <int CTA_GROUP = 1>
-ATB_DEVICE void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if constexpr (CTA_GROUP == 1)
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  else
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]  (A operand read from tensor memory)
-ATB_DEVICE void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Make the mbarrier track completion of all tcgen05 ops issued so far by this thread.
-ATB_DEVICE void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-// cta_group::2 commit onto ONE barrier given by its shared::cluster address (own or partner CTA).
-// A CTA pair that must be told on both sides issues two of these.
-ATB_DEVICE void umma_commit_cg2(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr)
-               : "memory");
-}
-
 // 32 lanes x 32 consecutive fp32 columns: thread t of the warp gets lane (base_lane + t).
 ATB_DEVICE void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -295,14 +250,6 @@ ATB_DEVICE void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
       "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
-ATB_DEVICE void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
 ATB_DEVICE void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 ATB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -310,26 +257,16 @@ ATB_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" :
 //   K-major  operand tile: rows of 64 x 16-bit (128 B); 8-row groups 1024 B apart (SBO).
 //   MN-major operand tile: k-rows of 64 x 16-bit along MN (128 B); 8 k-rows = 1024 B (SBO);
 //                          successive 64-element MN chunks `lbo_bytes` apart.
-ATB_DEVICE uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for sm_100
-  d |= (uint64_t)2 << 61;  // SWIZZLE_128B
-  return d;
-}
-
-// The same descriptor `bytes` further on in shared memory (the start-address field counts 16-byte units and
-// cannot carry out of its 14 bits for any address inside the 227 KB of a CTA): one 64-bit add per MMA in
-// place of rebuilding the descriptor, which matters when one thread issues an MMA every 64 clocks.
-ATB_DEVICE uint64_t umma_desc_advance(uint64_t desc, uint32_t bytes) { return desc + (uint64_t)(bytes >> 4); }
-
+// It is kept as its low word (start address in 16-byte units, which cannot carry out of its 14 bits inside the 227 KB of a
+// CTA, and LBO): adding to it moves on in shared memory, and the high word (SBO, descriptor version, swizzle) is the same for
+// every tile with 1024-byte row groups.
+//
 // The issue path of a whole warp: every lane runs the code, lanes with issue != 0 (one, from elect_one()) execute the
-// instruction. The predicate sits on the instruction itself, not on a branch around it, and a descriptor is its low word
-// (start address and LBO; the high word is the same for every tile with 1024-byte row groups). Measured for groups of 8
-// products of 32 clocks, each group behind a satisfied barrier: 268 clocks a group, 336 with `if (issue)` around 64-bit
-// descriptors.
+// instruction; the predicate sits on the instruction itself, not on a branch around it. D (+)= A B, accumulate == 0
+// overwrites D; `ss`: both operands from shared memory, `ts`: A from tensor memory. A commit makes the mbarrier (cg2: one
+// given by its shared::cluster address, own or partner CTA) track all tcgen05 operations that this lane has issued. Measured
+// for groups of 8 products of 32 clocks, each group behind a satisfied barrier: 268 clocks a group, 336 with `if (issue)`
+// around 64-bit descriptors.
 constexpr uint32_t UMMA_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 ATB_DEVICE uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFF) >> 4) | ((lbo_bytes >> 4) << 16);

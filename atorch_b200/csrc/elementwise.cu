@@ -127,7 +127,6 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
   }
 }
 
-// out[t, :] = inp[t, :] + bias[expert[t], :]   (MoE per-expert bias)
 // out[r] = sum over the g consecutive heads of row r, in fp32 and in order, for two tensors (blockIdx.y): the gradients of
 // a key/value head from those of its query heads. Bound by memory: one pass, each thread sums 8 columns of one row. As
 // tensor operations (to fp32, sum, back) 31 us for 2 x 4096 rows of 4 heads x 4 x 128, 5.7 us here.
@@ -154,6 +153,7 @@ __global__ void __launch_bounds__(256) head_sum_kernel(const uint4* __restrict__
                                          pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
 }
 
+// out[t, :] = inp[t, :] + bias[expert[t], :]   (MoE per-expert bias)
 __global__ void bias_gather_add_kernel(const __nv_bfloat16* __restrict__ inp, const __nv_bfloat16* __restrict__ bias,
                                        const int* __restrict__ expert, __nv_bfloat16* __restrict__ out, long long T,
                                        int H) {

@@ -917,9 +917,12 @@ extern "C" int atb_gemm_bf16_2cta_grouped(const void* A, const void* B, void* C,
     ep.rs_rows = g_fused_args.rs_rows;
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  // The 256-wide tile is the default. The 128-wide one fills the last wave better (256 tiles of 256x256
-  // occupy 74 CTA pairs for 4 waves at 86 %), but measured 1.5x slower per FLOP on B200: its 256-cycle
-  // stages leave the single MMA-issuing thread no slack. It stays selectable with tile_n = 128.
+  // The 256-wide tile is the default. The 128-wide one fills short waves better, but per product of a pair it reads one and a
+  // half times the operand bytes out of shared memory for the same work. Products of a 1.3B layer (hidden 2048, 5504),
+  // 256 / 128 wide, cold L2: 4096 rows 83 / 124 (q|k|v), 131 / 203 (gate|up), 37 / 54 us (o); 1500 rows 39 / 55, 64 / 89,
+  // 25 / 34; 777 rows 37 / 44, 50 / 66, 22.5 / 20.7. It wins only where the 256-wide tiles are fewer than the pairs, by 4 to
+  // 9 % (333 rows, o: 22.5 / 20.5; 777 rows, dgrad of gate|up: 65.5 / 59.6), and not in weight gradients. It stays
+  // selectable with tile_n = 128.
   const bool narrow = tile_n == 128;
 #define ATB_PAIR_DISPATCH(BN_)                                                                                     \
   do {                                                                                                             \
