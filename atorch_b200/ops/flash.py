@@ -160,15 +160,17 @@ class _HolesOnTheWay:
 AHEAD_MIN_CTAS = 296
 
 
-def _padded_intervals(q, k, causal, scale, key_padding_mask, others, drop):
+def _padded_intervals(q, heads, Sk, causal, scale, key_padding_mask, others, drop):
     """``(row_lo, row_hi, look)`` for a key padding mask of self-attention in front of the two-query-tile forward. The host
     has to know whether the mask has holes (those are unpadded), but the forward kernel need not wait for it: it is
     launched first and leaves at once if there are any, and ``look.check()`` comes after it, so that the GPU has work while
     the host waits and starts up again. ``None`` where another forward kernel would run, the mask comes with others or the
     forward is too short."""
-    B, S, H = q.shape[:3]
-    if key_padding_mask is None or drop or any(o is not None for o in others) or k.shape[1] != S or S < 256 \
-            or not FWD_TWO_TILES or not scale > 0 or B * H * ((S + 255) // 256) < AHEAD_MIN_CTAS:
+    if key_padding_mask is None:
+        return None
+    B, S = q.shape[:2]
+    if drop or any(o is not None for o in others) or Sk != S or S < 256 or not FWD_TWO_TILES or not scale > 0 \
+            or B * heads * ((S + 255) // 256) < AHEAD_MIN_CTAS:
         return None
     out = _launch_row_intervals(B, S, S, q.device, causal, None, None, key_padding_mask, None)
     return None if out is None else (out[0], out[1], _HolesOnTheWay(out[2]))
@@ -464,7 +466,7 @@ def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pa
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     if Sq == 1:
         causal = False   # single-query decode sees every key
-    padded = _padded_intervals(q, k, causal, scale, key_padding_mask,
+    padded = _padded_intervals(q, Hq, Sk, causal, scale, key_padding_mask,
                                (glm_mask, pack_glm_mask, cu_seqlens, additive_mask, additive_bias), dropout_p > 0.0)
     try:
         if padded is not None:
@@ -550,7 +552,7 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
     B, S, _, D = qkv.shape
     scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
     look = None
-    padded = _padded_intervals(qkv[:, :, :num_heads], qkv, causal, scale, mask_kwargs.get("key_padding_mask"),
+    padded = _padded_intervals(qkv, num_heads, S, causal, scale, mask_kwargs.get("key_padding_mask"),
                                [v for n, v in mask_kwargs.items() if n not in ("key_padding_mask", "dropout_p", "dropout_seed")],
                                mask_kwargs.get("dropout_p", 0.0) > 0.0)
     try:
