@@ -422,20 +422,21 @@ inline void make_block_order(BlockOrder* o, dim3* grid, int blocks, int heads, i
     *grid = dim3(blocks, heads, batch);
   }
 }
-// place: 0 = the heaviest block of its head. False: no block (a run that is one head shorter).
-ATB_DEVICE bool block_of(const BlockOrder& o, int& place, int& blocks, int& head, int& sample) {
+// place: 0 = the heaviest block of its head; idx: the block's index in the grid. False: no block (a run that is one head
+// shorter).
+ATB_DEVICE bool block_of(const BlockOrder& o, const uint3& idx, int& place, int& blocks, int& head, int& sample) {
   if (o.all == 0) {
-    place = blockIdx.x;
+    place = idx.x;
     blocks = gridDim.x;
-    head = blockIdx.y;
-    sample = blockIdx.z;
+    head = idx.y;
+    sample = idx.z;
     return true;
   }
-  const int run = blockIdx.z;
-  if ((int)blockIdx.x >= o.run + (run < o.longer ? 1 : 0)) return false;
-  place = blockIdx.y;
+  const int run = idx.z;
+  if ((int)idx.x >= o.run + (run < o.longer ? 1 : 0)) return false;
+  place = idx.y;
   blocks = gridDim.y;
-  head = run * o.run + min(run, o.longer) + blockIdx.x;
+  head = run * o.run + min(run, o.longer) + idx.x;
   sample = 0;
   if (o.all != o.heads) {
     sample = head / o.heads;
@@ -532,6 +533,21 @@ ATB_DEVICE uint32_t pack_bf16x2(float a, float b) {
 ATB_DEVICE float2 unpack_bf16x2(uint32_t u) {
   __nv_bfloat162 h = *reinterpret_cast<__nv_bfloat162*>(&u);
   return __bfloat1622float2(h);
+}
+
+// 32 fp32 bit patterns of a row as bf16: whole 32-byte sectors where the row allows it (`wide`), else 16-byte pieces
+ATB_DEVICE void store_bf16_32(__nv_bfloat16* p, const uint32_t (&x)[32], bool wide) {
+  uint32_t o[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) o[i] = pack_bf16x2(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
+  if (wide) {
+    stg_v8(p, o);
+    stg_v8(p + 16, o + 8);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<uint4*>(p + 8 * i) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+  }
 }
 
 template <typename T>

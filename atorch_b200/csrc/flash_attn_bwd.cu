@@ -558,18 +558,21 @@ extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, 
                                 const float* lse, float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
                                 long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
-                                void* stream, int* status);
+                                int* key_range, void* stream, int* status);
 
 extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k, const void* v, const float* lse,
                                  const float* delta, void* dk, void* dv, const int* row_lo, const int* row_hi, int B,
                                  int Sq, int Sk, int Hq, int Hkv, long long q_stride, long long k_stride,
                                  long long v_stride, long long do_stride, long long dkv_stride, int causal,
-                                 float softmax_scale, int fold, int head_dim, void* stream, int* status);
+                                 float softmax_scale, int fold, int head_dim, const int* key_range, void* stream,
+                                 int* status);
 
 // The two-kernel form, the default without dropout and bias: dK and dV per key block (flash_attn_bwd_dkv.cu; `fold`:
 // see there), dQ per query block (flash_attn_bwd_dq.cu, which runs first and writes delta). No atomics, results do not depend on scheduling. dq/dk/dv are
 // token-major rows of pitch dq_stride / dkv_stride elements (so they may be slices of one fused
-// [tokens, (Hq + 2 Hkv) * head_dim] gradient buffer); `delta` is scratch [B, Hq, Sq].
+// [tokens, (Hq + 2 Hkv) * head_dim] gradient buffer). `delta` is scratch, 8-byte aligned: [B, Hq, Sq] floats and, with
+// intervals, from the next multiple of 8 bytes on two ints per block of 128 query rows and sample (the keys its rows see:
+// the second kernel finds the query blocks of a key block there, where it went through the intervals of all rows before).
 extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* k, const void* v, const void* out,
                                    const float* lse, float* delta, void* dq, void* dk, void* dv, const int* row_lo,
                                    const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,
@@ -578,11 +581,15 @@ extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* 
                                    int fold, int head_dim) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if ((head_dim != 128 && head_dim != 64) || Hq % Hkv || (do_stride & 7)) return -1;
+  const long long rows = (long long)B * Hq * Sq;
+  int* key_range = row_lo != nullptr || row_hi != nullptr ? reinterpret_cast<int*>(delta + rows + (rows & 1)) : nullptr;
+  if (key_range != nullptr && (reinterpret_cast<uintptr_t>(key_range) & 7)) return -1;
   int rc = atb_flash_bwd_dq(dout, q, k, v, out, lse, delta, dq, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
-                            v_stride, do_stride, dq_stride, causal, softmax_scale, head_dim, stream, status);
+                            v_stride, do_stride, dq_stride, causal, softmax_scale, head_dim, key_range, stream, status);
   if (rc == 0)
     rc = atb_flash_bwd_dkv(dout, q, k, v, lse, delta, dk, dv, row_lo, row_hi, B, Sq, Sk, Hq, Hkv, q_stride, k_stride,
-                           v_stride, do_stride, dkv_stride, causal, softmax_scale, fold, head_dim, stream, status);
+                           v_stride, do_stride, dkv_stride, causal, softmax_scale, fold, head_dim, key_range, stream,
+                           status);
   return rc;
 }
 

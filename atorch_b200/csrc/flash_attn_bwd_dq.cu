@@ -11,11 +11,11 @@
 // second buffer); dQ of block j follows when dS(j) is in place.
 //
 // Warp 0 = TMA producer (Q, dO once; K in three stages because a K tile serves S and, later, dQ; V in two),
-// warp 1 = MMA issuer / TMEM owner, warps 2..9 = element-wise work: thread (row r, half h) owns columns
+// warp 1 = MMA issuer / TMEM owner, warp 2 = scheduler (block_queue.cuh), warps 4..11 = element-wise work: thread (row r, half h) owns columns
 // [64h, 64h+64) of row r. The two threads of a row sit in different warps and the bf16 dS of one overwrites
 // fp32 dP columns of the other, so the two warps of a lane quarter meet at a barrier between loading
 // and storing (an mbarrier with a bounded wait). Masks are per-row key intervals [lo, hi) as in the forward kernel.
-#include "common.cuh"
+#include "block_queue.cuh"
 
 namespace {
 using namespace atb;
@@ -24,7 +24,10 @@ constexpr int BQ = 128, BKV = 128;
 constexpr int PANEL = 128 * 64 * 2;
 constexpr int K_STAGES = 3, V_STAGES = 2;
 constexpr int N_EW = 256;
-constexpr int THREADS = 64 + N_EW;
+constexpr int THREADS = 128 + N_EW;
+// 168 registers a thread at launch (384 x 168 = 64512); the control warpgroup gives up what the element-wise warps need to
+// hold the loads of the next unit beside the results of the last one: 128 x 72 + 256 x 216 = 64512
+constexpr int REGS_CONTROL = 72, REGS_EW = 216;
 
 struct DqParams {
   const float* lse;            // [B, Hq, Sq]
@@ -36,6 +39,8 @@ struct DqParams {
   long long dq_stride;
   const int* row_lo;
   const int* row_hi;
+  int2* key_range;     // [B, query blocks], written for the dK/dV kernel unless null: first, last+1 key that a row sees
+  int wide;            // rows of dq start on 32-byte boundaries
   int B, Sq, Sk, Hq, Hkv, causal;
   float scale, scale_log2;
   int* status;
@@ -50,10 +55,12 @@ struct SmemQ {
   static constexpr int K_OFF = DO_OFF + TILE;
   static constexpr int V_OFF = K_OFF + K_STAGES * TILE;
   static constexpr int BAR_OFF = V_OFF + V_STAGES * TILE;  // 224 KB
-  static constexpr int NBARS = 1 + 2 * K_STAGES + 2 * V_STAGES + 4 + 4 + 1;
-  static constexpr int DOT_OFF = BAR_OFF + NBARS * 8 + 64;      // float [BQ]: dO . O of the rows
-  static constexpr int TOTAL = DOT_OFF + BQ * 4 + 1024;
+  static constexpr int NBARS = 2 + 2 * K_STAGES + 2 * V_STAGES + 4 + 4 + 2;
+  static constexpr int QUEUE_OFF = BAR_OFF + NBARS * 8 + 16;
+  static constexpr int DOT_OFF = QUEUE_OFF + (int)sizeof(WorkQueue);   // float [2][BQ]: dO . O of the rows of a unit
+  static constexpr int TOTAL = DOT_OFF + 2 * BQ * 4 + 1024;
 };
+static_assert(SmemQ<128>::QUEUE_OFF % 16 == 0 && SmemQ<64>::QUEUE_OFF % 16 == 0, "the queue is 16-byte aligned");
 static_assert(SmemQ<128>::TOTAL <= 232448, "shared memory of the dQ kernel exceeds 227 KB");
 
 template <int HD>
@@ -70,39 +77,39 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* sV = smem + L::V_OFF;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* qdo_full = bars;
-  uint64_t* k_full = bars + 1;                 // [K_STAGES]
+  uint64_t* qdo_free = bars + 1;               // the last S and dP of a unit have read Q and dO
+  uint64_t* k_full = bars + 2;                 // [K_STAGES]
   uint64_t* k_empty = k_full + K_STAGES;       // [K_STAGES]  dQ(j) has read K_j
   uint64_t* v_full = k_empty + K_STAGES;       // [V_STAGES]
   uint64_t* v_empty = v_full + V_STAGES;       // [V_STAGES]  dP(j) has read V_j
   uint64_t* sdp_full = v_empty + V_STAGES;     // S(j), dP(j) are in TMEM
   uint64_t* s_free = sdp_full + 1;             // every element-wise warp holds S(j), dP(j) in registers
   uint64_t* ds_full = s_free + 1;              // dS(j) is in TMEM
-  uint64_t* dq_full = ds_full + 1;             // the last dQ product has completed
-  uint64_t* pair_bar = dq_full + 1;            // [4] the two warps of a lane quarter both hold S(j), dP(j)
+  uint64_t* dq_full = ds_full + 1;             // the last dQ product of a unit has completed
+  uint64_t* acc_free = dq_full + 1;            // dQ of a unit has been read out of TMEM
+  uint64_t* pair_bar = acc_free + 1;           // [4] the two warps of a lane quarter both hold S(j), dP(j)
   uint64_t* dot_bar = pair_bar + 4;            // every element-wise warp has written its rows' dO . O
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // [4]: t0, t1, full_lo, full_hi
+  WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
-  int place, blocks, h, b;
-  if (!block_of(p.order, place, blocks, h, b)) return;
-  const int qb = blocks - 1 - place;   // heaviest (last) causal blocks first
-  const int hk = h / (p.Hq / p.Hkv);
-  const int q0 = qb * BQ;
   const int shift = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {
     mbar_init(qdo_full, 1);
+    mbar_init(qdo_free, 1);
     for (int i = 0; i < K_STAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < V_STAGES; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     mbar_init(sdp_full, 1);
     mbar_init(s_free, N_EW / 32);
     mbar_init(ds_full, N_EW / 32);
     mbar_init(dq_full, 1);
+    mbar_init(acc_free, N_EW / 32);
     for (int i = 0; i < 4; ++i) mbar_init(&pair_bar[i], 2);
     mbar_init(dot_bar, N_EW / 32);
+    queue_init(queue, 2 + N_EW / 32);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -110,81 +117,92 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_alloc<1>(tmem_slot, 512);
     tmem_relinquish<1>();
   }
-  if (warp == 2) {   // key range of this query block: union and intersection of the rows' intervals
-    int umin = INT_MAX, umax = 0, ilo = 0, ihi = INT_MAX;
-    int rlo[BQ / 32], rhi[BQ / 32];      // all loads first, then their use
-#pragma unroll
-    for (int e = 0; e < BQ / 32; ++e) {
-      const int i = min(q0 + lane + 32 * e, p.Sq - 1);
-      rlo[e] = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-      rhi[e] = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-    }
-#pragma unroll
-    for (int e = 0; e < BQ / 32; ++e) {
-      if (q0 + lane + 32 * e >= p.Sq) continue;
-      const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk);
-      if (hi <= lo) { ilo = INT_MAX; ihi = 0; continue; }
-      umin = min(umin, lo); umax = max(umax, hi);
-      ilo = max(ilo, lo); ihi = min(ihi, hi);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      umin = min(umin, __shfl_xor_sync(0xffffffffu, umin, o));
-      umax = max(umax, __shfl_xor_sync(0xffffffffu, umax, o));
-      ilo = max(ilo, __shfl_xor_sync(0xffffffffu, ilo, o));
-      ihi = min(ihi, __shfl_xor_sync(0xffffffffu, ihi, o));
-    }
-    if (lane == 0) {
-      kv_range[0] = umax > umin ? umin / BKV : 0;
-      kv_range[1] = umax > umin ? (umax + BKV - 1) / BKV : 0;
-      kv_range[2] = ilo;
-      kv_range[3] = ihi;
-    }
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int t0 = warp_uniform(kv_range[0]), n = warp_uniform(kv_range[1]) - t0;
-  const int full_lo = kv_range[2], full_hi = kv_range[3];
-  const long long q_row0 = (long long)b * p.Sq + q0;
-  const long long k_row0 = (long long)b * p.Sk;
-  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 384;   // dP buffer j&1 at tdP + 128*(j&1)
+  const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 384;   // dP buffer of block g at tdP + 128*(g&1)
 
-  if (warp == 0) {
-    if (n > 0) {
+  // Units of this CTA, one after another: query block w.place of head w.head and sample w.sample, key blocks
+  // [w.v0, w.v0 + w.v1), of which all rows see the keys [w.v2, w.v3). Barriers of the key blocks count on through all units
+  // (g), those of Q, dO and the accumulator count the units that have any block (u).
+  if (warp < 4) {
+    reg_dealloc<REGS_CONTROL>();
+    if (warp == 2) {
+      queue_run(queue, p.order, [&](Work& w, int blocks) {
+        w.place = blocks - 1 - w.place;   // heaviest (last) causal blocks first
+        const int q0 = w.place * BQ;
+        int umin = INT_MAX, umax = 0, ilo = 0, ihi = INT_MAX;   // union and intersection of the rows' intervals
+        int rlo[BQ / 32], rhi[BQ / 32];      // all loads first, then their use
+#pragma unroll
+        for (int e = 0; e < BQ / 32; ++e) {
+          const int i = min(q0 + lane + 32 * e, p.Sq - 1);
+          rlo[e] = p.row_lo ? p.row_lo[(long long)w.sample * p.Sq + i] : 0;
+          rhi[e] = p.row_hi ? p.row_hi[(long long)w.sample * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+        }
+#pragma unroll
+        for (int e = 0; e < BQ / 32; ++e) {
+          if (q0 + lane + 32 * e >= p.Sq) continue;
+          const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk);
+          if (hi <= lo) { ilo = INT_MAX; ihi = 0; continue; }
+          umin = min(umin, lo); umax = max(umax, hi);
+          ilo = max(ilo, lo); ihi = min(ihi, hi);
+        }
+        umin = __reduce_min_sync(0xffffffffu, umin);
+        umax = __reduce_max_sync(0xffffffffu, umax);
+        w.v0 = umax > umin ? umin / BKV : 0;
+        w.v1 = (umax > umin ? (umax + BKV - 1) / BKV : 0) - w.v0;
+        w.v2 = __reduce_max_sync(0xffffffffu, ilo);
+        w.v3 = __reduce_min_sync(0xffffffffu, ihi);
+        if (p.key_range != nullptr && w.head == 0 && lane == 0)
+          p.key_range[(long long)w.sample * blocks + w.place] = make_int2(umin, umax);
+      }, abort_flag, p.status);
+    } else if (warp == 0) {
       const bool el = elect_one();
       if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmdO); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
-      if (el) mbar_expect_tx(qdo_full, 2 * TILE);
-      if (el) tma_load_2d(sQ, &tmQ, qdo_full, h * HD, (int)q_row0);
-      if (HD == 128 && el) tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, (int)q_row0);
-      if (el) tma_load_2d(sdO, &tmdO, qdo_full, h * HD, (int)q_row0);
-      if (HD == 128 && el) tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, (int)q_row0);
-      for (int j = 0; j < n; ++j) {
-        const int ks = j % K_STAGES, vs = j % V_STAGES;
-        const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
-        if (!mbar_wait_warp(&k_empty[ks], ((j / K_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
-        if (el) mbar_expect_tx(&k_full[ks], TILE);
-        if (el) tma_load_2d(sK + ks * TILE, &tmK, &k_full[ks], hk * HD, krow);
-        if (HD == 128 && el) tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
-        if (!mbar_wait_warp(&v_empty[vs], ((j / V_STAGES) & 1) ^ 1, abort_flag, p.status)) break;
-        if (el) mbar_expect_tx(&v_full[vs], TILE);
-        if (el) tma_load_2d(sV + vs * TILE, &tmV, &v_full[vs], hk * HD, krow);
-        if (HD == 128 && el) tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
+      uint32_t g = 0;
+      int u = 0;
+      Work w;
+      for (int c = 0; queue_next(queue, c, w, abort_flag, p.status) && w.more; ++c) {
+        const int n = w.v1, h = w.head, hk = h / (p.Hq / p.Hkv);
+        if (n == 0) { queue_claim(queue); continue; }
+        const int qrow = (int)((long long)w.sample * p.Sq + w.place * BQ);
+        if (!mbar_wait_warp(qdo_free, (u & 1) ^ 1, abort_flag, p.status)) break;
+        ++u;
+        if (el) mbar_expect_tx(qdo_full, 2 * TILE);
+        if (el) tma_load_2d(sQ, &tmQ, qdo_full, h * HD, qrow);
+        if (HD == 128 && el) tma_load_2d(sQ + PANEL, &tmQ, qdo_full, h * HD + 64, qrow);
+        if (el) tma_load_2d(sdO, &tmdO, qdo_full, h * HD, qrow);
+        if (HD == 128 && el) tma_load_2d(sdO + PANEL, &tmdO, qdo_full, h * HD + 64, qrow);
+        bool ok = true;
+        for (int j = 0; j < n; ++j, ++g) {
+          if (j == max(n - 3, 0)) queue_claim(queue);
+          const int ks = g % K_STAGES, vs = g % V_STAGES;
+          const int krow = (int)((long long)w.sample * p.Sk + (long long)(w.v0 + j) * BKV);
+          ok = mbar_wait_warp(&k_empty[ks], ((g / K_STAGES) & 1) ^ 1, abort_flag, p.status);
+          if (!ok) break;
+          if (el) mbar_expect_tx(&k_full[ks], TILE);
+          if (el) tma_load_2d(sK + ks * TILE, &tmK, &k_full[ks], hk * HD, krow);
+          if (HD == 128 && el) tma_load_2d(sK + ks * TILE + PANEL, &tmK, &k_full[ks], hk * HD + 64, krow);
+          ok = mbar_wait_warp(&v_empty[vs], ((g / V_STAGES) & 1) ^ 1, abort_flag, p.status);
+          if (!ok) break;
+          if (el) mbar_expect_tx(&v_full[vs], TILE);
+          if (el) tma_load_2d(sV + vs * TILE, &tmV, &v_full[vs], hk * HD, krow);
+          if (HD == 128 && el) tma_load_2d(sV + vs * TILE + PANEL, &tmV, &v_full[vs], hk * HD + 64, krow);
+        }
+        if (!ok) break;
       }
-    }
-  } else if (warp == 1) {
-    if (n > 0) {
+    } else if (warp == 1) {
       const uint32_t el = elect_one();   // the lane that issues and commits
       constexpr uint32_t id_kk = umma_idesc(128, 128, 1, 1, false, false);
       constexpr uint32_t id_km = umma_idesc(128, HD, 1, 1, false, true);
       const uint32_t dQk = umma_desc_lo(smem_u32(sQ), 16), dOk = umma_desc_lo(smem_u32(sdO), 16);
       const uint32_t dKk0 = umma_desc_lo(smem_u32(sK), 16), dKm0 = umma_desc_lo(smem_u32(sK), PANEL);
       const uint32_t dVk0 = umma_desc_lo(smem_u32(sV), 16);
-      // S(j) = Q K_j^T and dP(j) = dO V_j^T
-      auto issue_sdp = [&](int j) -> bool {
-        const int ks = j % K_STAGES, vs = j % V_STAGES;
-        if (!mbar_wait_warp(&k_full[ks], (j / K_STAGES) & 1, abort_flag, p.status)) return false;
+      // S(g) = Q K_g^T and dP(g) = dO V_g^T
+      auto issue_sdp = [&](uint32_t g, bool last) -> bool {
+        const int ks = g % K_STAGES, vs = g % V_STAGES;
+        if (!mbar_wait_warp(&k_full[ks], (g / K_STAGES) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
         const uint32_t kd = dKk0 + ((ks * TILE) >> 4);
 #pragma unroll
@@ -192,10 +210,10 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
           umma_ss_issue(tS, dQk + (off >> 4), kd + (off >> 4), id_kk, k != 0, el);
         }
-        if (!mbar_wait_warp(&v_full[vs], (j / V_STAGES) & 1, abort_flag, p.status)) return false;
+        if (!mbar_wait_warp(&v_full[vs], (g / V_STAGES) & 1, abort_flag, p.status)) return false;
         tc_fence_after();
         const uint32_t vd = dVk0 + ((vs * TILE) >> 4);
-        const uint32_t dst = tdP + 128 * (j & 1);
+        const uint32_t dst = tdP + 128 * (g & 1);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
@@ -203,145 +221,176 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         umma_commit_issue(sdp_full, el);
         umma_commit_issue(&v_empty[vs], el);
+        if (last) umma_commit_issue(qdo_free, el);
         return true;
       };
-      bool ok = mbar_wait_warp(qdo_full, 0, abort_flag, p.status);
-      ok = ok && issue_sdp(0);
-      for (int j = 0; ok && j < n; ++j) {
-        if (j + 1 < n) {
-          if (!mbar_wait_warp(s_free, j & 1, abort_flag, p.status)) break;
-          tc_fence_after();
-          if (!issue_sdp(j + 1)) break;
-        }
-        if (!mbar_wait_warp(ds_full, j & 1, abort_flag, p.status)) break;
+      uint32_t g = 0;
+      int u = 0;
+      Work w;
+      for (int c = 0; queue_next(queue, c, w, abort_flag, p.status) && w.more; ++c) {
+        const int n = w.v1;
+        if (n == 0) continue;
+        // the first scores of a unit follow the last product of the one before and run under its results' way out
+        bool ok = mbar_wait_warp(qdo_full, u & 1, abort_flag, p.status) &&
+                  (g == 0 || mbar_wait_warp(s_free, (g - 1) & 1, abort_flag, p.status));
         tc_fence_after();
-        const uint32_t km = dKm0 + (((j % K_STAGES) * TILE) >> 4);
-        const uint32_t a = tdP + 128 * (j & 1);
+        ok = ok && issue_sdp(g, n == 1);
+        for (int j = 0; ok && j < n; ++j, ++g) {
+          if (j + 1 < n) {
+            ok = mbar_wait_warp(s_free, g & 1, abort_flag, p.status);
+            tc_fence_after();
+            ok = ok && issue_sdp(g + 1, j + 2 == n);
+          }
+          if (ok && j == 0 && u > 0) ok = mbar_wait_warp(acc_free, (u - 1) & 1, abort_flag, p.status);
+          ok = ok && mbar_wait_warp(ds_full, g & 1, abort_flag, p.status);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t km = dKm0 + (((g % K_STAGES) * TILE) >> 4);
+          const uint32_t a = tdP + 128 * (g & 1);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)   // dQ += dS K_j: 16 keys per step = 8 TMEM columns of packed bf16
-          umma_ts_issue(tdQ, a + k * 8, km + k * 128, id_km, (j | k) != 0, el);
-        umma_commit_issue(&k_empty[j % K_STAGES], el);
-        if (j == n - 1) umma_commit_issue(dq_full, el);
+          for (int k = 0; k < 8; ++k)   // dQ += dS K_j: 16 keys per step = 8 TMEM columns of packed bf16
+            umma_ts_issue(tdQ, a + k * 8, km + k * 128, id_km, (j | k) != 0, el);
+          umma_commit_issue(&k_empty[g % K_STAGES], el);
+          if (j == n - 1) umma_commit_issue(dq_full, el);
+        }
+        if (!ok) break;
+        ++u;
       }
     }
   } else {
+    reg_alloc<REGS_EW>();
     const int quarter = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int half = (warp - 4) >> 2;
     const int r = quarter * 32 + lane;
-    const int i = q0 + r;   // global query row
     const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16);
-    // delta = dO . O of the block's rows, 16 rows per warp and HD / 8 lanes per row, while the first tiles arrive and are
-    // multiplied: a separate pass over both tensors took 26 us at S=4096, 32 heads of 128
-    bool ok = true;
-    float delta;
-    {
-      constexpr int LANES = HD / 8, AT_ONCE = 32 / LANES, STEPS = 16 / AT_ONCE;
-      float* dots = reinterpret_cast<float*>(smem + L::DOT_OFF);
-      const int first = (warp - 2) * 16 + lane / LANES, sub = lane % LANES;
+    // delta = dO . O of the block's rows, 16 rows per warp and HD / 8 lanes per row: a separate pass over both tensors took
+    // 26 us at S=4096, 32 heads of 128. What a unit needs from memory is loaded before the results of the one before are stored.
+    constexpr int LANES = HD / 8, AT_ONCE = 32 / LANES, STEPS = 16 / AT_ONCE;
+    const int first = (warp - 4) * 16 + lane / LANES, sub = lane % LANES;
+    struct {
       uint4 x[STEPS], y[STEPS];
+      float lse;
+      int lo, hi;
+    } in;
+    auto load_unit = [&](const Work& w) {
+      if (!w.more) return;
+      const int b = w.sample, h = w.head, q0 = w.place * BQ;
 #pragma unroll
       for (int e = 0; e < STEPS; ++e) {
         const long long tok = (long long)b * p.Sq + min(q0 + first + e * AT_ONCE, p.Sq - 1);
-        x[e] = *reinterpret_cast<const uint4*>(p.dO + tok * p.do_stride + h * HD + sub * 8);
-        y[e] = *reinterpret_cast<const uint4*>(p.O + (tok * p.Hq + h) * HD + sub * 8);
+        in.x[e] = *reinterpret_cast<const uint4*>(p.dO + tok * p.do_stride + h * HD + sub * 8);
+        in.y[e] = *reinterpret_cast<const uint4*>(p.O + (tok * p.Hq + h) * HD + sub * 8);
       }
+      const int i = min(q0 + r, p.Sq - 1);
+      in.lse = p.lse[((long long)b * p.Hq + h) * p.Sq + i];
+      in.lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
+      in.hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+    };
+    uint32_t g = 0;
+    int u = 0;
+    Work w;
+    bool ok = queue_next(queue, 0, w, abort_flag, p.status);
+    if (ok) load_unit(w);
+    for (int c = 0; ok && w.more;) {
+      const int b = w.sample, h = w.head, n = w.v1, full_lo = w.v2, full_hi = w.v3;
+      const int i = w.place * BQ + r;   // global query row
+      float delta;
+      {
+        float* dots = reinterpret_cast<float*>(smem + L::DOT_OFF) + (c & 1) * BQ;
 #pragma unroll
-      for (int e = 0; e < STEPS; ++e) {
-        const uint32_t xs[4] = {x[e].x, x[e].y, x[e].z, x[e].w}, ys[4] = {y[e].x, y[e].y, y[e].z, y[e].w};
-        float acc = 0.f;
+        for (int e = 0; e < STEPS; ++e) {
+          const uint32_t xs[4] = {in.x[e].x, in.x[e].y, in.x[e].z, in.x[e].w};
+          const uint32_t ys[4] = {in.y[e].x, in.y[e].y, in.y[e].z, in.y[e].w};
+          float acc = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-          const float2 u = unpack_bf16x2(xs[w]), v = unpack_bf16x2(ys[w]);
-          acc += u.x * v.x + u.y * v.y;
+          for (int k = 0; k < 4; ++k) {
+            const float2 a = unpack_bf16x2(xs[k]), d = unpack_bf16x2(ys[k]);
+            acc += a.x * d.x + a.y * d.y;
+          }
+#pragma unroll
+          for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+          if (sub == 0) dots[first + e * AT_ONCE] = acc;
         }
-#pragma unroll
-        for (int o = LANES / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (sub == 0) dots[first + e * AT_ONCE] = acc;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dot_bar);
+        ok = mbar_wait_warp(dot_bar, c & 1, abort_flag, p.status);
+        if (!ok) break;
+        delta = dots[r];
+        if (half == 0 && i < p.Sq) p.delta[((long long)b * p.Hq + h) * p.Sq + i] = delta;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dot_bar);
-      ok = mbar_wait_warp(dot_bar, 0, abort_flag, p.status);
-      delta = dots[r];
-      if (ok && half == 0 && i < p.Sq) p.delta[((long long)b * p.Hq + h) * p.Sq + i] = delta;
-    }
-    bool valid = i < p.Sq;
-    int lo = 0, hi = 0;
-    float lse2 = 0.f;
-    if (valid) {
-      const float l = p.lse[((long long)b * p.Hq + h) * p.Sq + i];
-      if (l == -INFINITY) {
-        valid = false;
-        delta = 0.f;
-      } else {
-        lse2 = l * 1.4426950408889634f;
-        lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-        hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-        lo = max(lo, 0);
-        hi = min(hi, p.Sk);
-      }
-    }
-    const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
-    const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
-    for (int j = 0; ok && j < n; ++j) {
-      const int kv0 = (t0 + j) * BKV;
-      const uint32_t dp_addr = tdP + 128 * (j & 1) + lane_addr;
-      if (!mbar_wait_warp(sdp_full, j & 1, abort_flag, p.status)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t s0[32], s1[32], d0[32], d1[32];
-      tmem_ld_32x32(tS + lane_addr + half * 64, s0);
-      tmem_ld_32x32(tS + lane_addr + half * 64 + 32, s1);
-      tmem_ld_32x32(dp_addr + half * 64, d0);
-      tmem_ld_32x32(dp_addr + half * 64 + 32, d1);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(s_free);
-        mbar_arrive(&pair_bar[quarter]);
-      }
-      // both threads of every row of this lane quarter hold their S and dP before either stores dS (a bounded
-      // mbarrier wait, not a named barrier, so that a warp whose partner gave up cannot wait forever)
-      if (!mbar_wait_warp(&pair_bar[quarter], j & 1, abort_flag, p.status)) { ok = false; break; }
-      // tiles inside the intersection of the rows' intervals run without per-element tests
-      const bool tile_full = (kv0 >= full_lo) && (kv0 + BKV <= full_hi);
-      const int c0 = kv0 + half * 64;
-      float pa[32], pb[32];   // P for keys c0 .. c0+31 and c0+32 .. c0+63
-#pragma unroll
-      for (int c = 0; c < 32; c += 2) {
-        float a0, a1, b0, b1;
-        f2_unpack(f2_fma(f2_pack_bits(s0[c], s0[c + 1]), sc2, nl2), a0, a1);
-        f2_unpack(f2_fma(f2_pack_bits(s1[c], s1[c + 1]), sc2, nl2), b0, b1);
-        pa[c] = fast_exp2(a0); pa[c + 1] = fast_exp2(a1);
-        pb[c] = fast_exp2(b0); pb[c + 1] = fast_exp2(b1);
-      }
-      if (!tile_full) {   // a separate pass, so that fully visible tiles execute no interval tests at all
-        const uint32_t m0 = valid ? visible_keys(c0, lo, hi) : 0u, m1 = valid ? visible_keys(c0 + 32, lo, hi) : 0u;
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          if (!(m0 & (1u << c))) pa[c] = 0.f;
-          if (!(m1 & (1u << c))) pb[c] = 0.f;
+      const bool valid = i < p.Sq && in.lse != -INFINITY;
+      if (!valid) delta = 0.f;
+      const float lse2 = valid ? in.lse * 1.4426950408889634f : 0.f;
+      const int lo = valid ? max(in.lo, 0) : 0, hi = valid ? min(in.hi, p.Sk) : 0;
+      const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
+      const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
+      for (int j = 0; j < n; ++j, ++g) {
+        const int kv0 = (w.v0 + j) * BKV;
+        const uint32_t dp_addr = tdP + 128 * (g & 1) + lane_addr;
+        if (!mbar_wait_warp(sdp_full, g & 1, abort_flag, p.status)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t s0[32], s1[32], d0[32], d1[32];
+        tmem_ld_32x32(tS + lane_addr + half * 64, s0);
+        tmem_ld_32x32(tS + lane_addr + half * 64 + 32, s1);
+        tmem_ld_32x32(dp_addr + half * 64, d0);
+        tmem_ld_32x32(dp_addr + half * 64 + 32, d1);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(s_free);
+          mbar_arrive(&pair_bar[quarter]);
         }
-      }
-      uint32_t ds[32];
+        // both threads of every row of this lane quarter hold their S and dP before either stores dS (a bounded
+        // mbarrier wait, not a named barrier, so that a warp whose partner gave up cannot wait forever)
+        if (!mbar_wait_warp(&pair_bar[quarter], g & 1, abort_flag, p.status)) { ok = false; break; }
+        // tiles inside the intersection of the rows' intervals run without per-element tests
+        const bool tile_full = (kv0 >= full_lo) && (kv0 + BKV <= full_hi);
+        const int c0 = kv0 + half * 64;
+        float pa[32], pb[32];   // P for keys c0 .. c0+31 and c0+32 .. c0+63
 #pragma unroll
-      for (int c = 0; c < 32; c += 2) {
-        float x0, x1, y0, y1;   // dS = P (dP - delta) scale
-        f2_unpack(f2_mul(f2_mul(f2_pack(pa[c], pa[c + 1]), scl2), f2_add(f2_pack_bits(d0[c], d0[c + 1]), nd2)), x0, x1);
-        f2_unpack(f2_mul(f2_mul(f2_pack(pb[c], pb[c + 1]), scl2), f2_add(f2_pack_bits(d1[c], d1[c + 1]), nd2)), y0, y1);
-        ds[c >> 1] = pack_bf16x2(x0, x1);
-        ds[16 + (c >> 1)] = pack_bf16x2(y0, y1);
+        for (int c = 0; c < 32; c += 2) {
+          float a0, a1, b0, b1;
+          f2_unpack(f2_fma(f2_pack_bits(s0[c], s0[c + 1]), sc2, nl2), a0, a1);
+          f2_unpack(f2_fma(f2_pack_bits(s1[c], s1[c + 1]), sc2, nl2), b0, b1);
+          pa[c] = fast_exp2(a0); pa[c + 1] = fast_exp2(a1);
+          pb[c] = fast_exp2(b0); pb[c + 1] = fast_exp2(b1);
+        }
+        if (!tile_full) {   // a separate pass, so that fully visible tiles execute no interval tests at all
+          const uint32_t m0 = valid ? visible_keys(c0, lo, hi) : 0u, m1 = valid ? visible_keys(c0 + 32, lo, hi) : 0u;
+#pragma unroll
+          for (int c = 0; c < 32; ++c) {
+            if (!(m0 & (1u << c))) pa[c] = 0.f;
+            if (!(m1 & (1u << c))) pb[c] = 0.f;
+          }
+        }
+        uint32_t ds[32];
+#pragma unroll
+        for (int c = 0; c < 32; c += 2) {
+          float x0, x1, y0, y1;   // dS = P (dP - delta) scale
+          f2_unpack(f2_mul(f2_mul(f2_pack(pa[c], pa[c + 1]), scl2), f2_add(f2_pack_bits(d0[c], d0[c + 1]), nd2)), x0, x1);
+          f2_unpack(f2_mul(f2_mul(f2_pack(pb[c], pb[c + 1]), scl2), f2_add(f2_pack_bits(d1[c], d1[c + 1]), nd2)), y0, y1);
+          ds[c >> 1] = pack_bf16x2(x0, x1);
+          ds[16 + (c >> 1)] = pack_bf16x2(y0, y1);
+        }
+        // keys [64h, 64h+64) of the row as packed bf16: columns [32h, 32h+32) of the dP buffer
+        tmem_st_32x32(dp_addr + half * 32, ds);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_full);
       }
-      // keys [64h, 64h+64) of the row as packed bf16: columns [32h, 32h+32) of the dP buffer
-      tmem_st_32x32(dp_addr + half * 32, ds);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ds_full);
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (ok && n > 0) ok = mbar_wait_warp(dq_full, 0, abort_flag, p.status);
-    if (ok) {
-      if (n > 0) tc_fence_after();
+      if (!ok) break;
+      Work nw;
+      ok = queue_next(queue, ++c, nw, abort_flag, p.status);
+      if (!ok) break;
+      load_unit(nw);
+      if (n > 0) {
+        ok = mbar_wait_warp(dq_full, u & 1, abort_flag, p.status);
+        if (!ok) break;
+        ++u;
+        tc_fence_after();
+      }
       __nv_bfloat16* row = p.dq + ((long long)b * p.Sq + i) * p.dq_stride + h * HD + half * (HD / 2);
 #pragma unroll
       for (int cc = 0; cc < HD / 64; ++cc) {
@@ -349,22 +398,18 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (n > 0) {
           tmem_ld_32x32(tdQ + lane_addr + half * (HD / 2) + cc * 32, t);
           tmem_ld_wait();
+          if (cc == HD / 64 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_free);
+          }
         } else {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) t[c] = 0u;
+          for (int k = 0; k < 32; ++k) t[k] = 0u;
         }
-        if (i < p.Sq) {
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            uint4 v;
-            v.x = pack_bf16x2(__uint_as_float(t[c]), __uint_as_float(t[c + 1]));
-            v.y = pack_bf16x2(__uint_as_float(t[c + 2]), __uint_as_float(t[c + 3]));
-            v.z = pack_bf16x2(__uint_as_float(t[c + 4]), __uint_as_float(t[c + 5]));
-            v.w = pack_bf16x2(__uint_as_float(t[c + 6]), __uint_as_float(t[c + 7]));
-            *reinterpret_cast<uint4*>(row + cc * 32 + c) = v;
-          }
-        }
+        if (i < p.Sq) store_bf16_32(row + cc * 32, t, p.wide);
       }
+      w = nw;
     }
   }
 
@@ -412,7 +457,7 @@ extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, 
                                 const float* lse, float* delta, void* dq, const int* row_lo, const int* row_hi, int B, int Sq,
                                 int Sk, int Hq, int Hkv, long long q_stride, long long k_stride, long long v_stride,
                                 long long do_stride, long long dq_stride, int causal, float softmax_scale, int head_dim,
-                                void* stream, int* status) {
+                                int* key_range, void* stream, int* status) {
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
   if (Hq % Hkv || (head_dim != 128 && head_dim != 64)) return -1;
   if ((q_stride | k_stride | v_stride | do_stride | dq_stride) & 7) return -1;
@@ -420,7 +465,8 @@ extern "C" int atb_flash_bwd_dq(const void* dout, const void* q, const void* k, 
   DqParams p;
   p.dO = (const __nv_bfloat16*)dout; p.O = (const __nv_bfloat16*)out; p.do_stride = do_stride;
   p.lse = lse; p.delta = delta; p.dq = (__nv_bfloat16*)dq; p.dq_stride = dq_stride;
-  p.row_lo = row_lo; p.row_hi = row_hi;
+  p.row_lo = row_lo; p.row_hi = row_hi; p.key_range = reinterpret_cast<int2*>(key_range);
+  p.wide = (reinterpret_cast<uintptr_t>(dq) & 31) == 0 && (dq_stride & 15) == 0;
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv; p.causal = causal;
   p.scale = softmax_scale; p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;

@@ -1,7 +1,7 @@
 // Flash attention forward, two query tiles per CTA (head dim 128 or 64, bf16) for sm_100a.
 //
 // One CTA owns 256 query rows as two 128-row tiles A and B that share every K/V tile. Warp 0 = TMA
-// producer, warp 1 = MMA issuer / TMEM owner, warp 2 = key range, warps 4..7 = softmax of tile A, warps 8..11 =
+// producer, warp 1 = MMA issuer / TMEM owner, warp 2 = scheduler (block_queue.cuh), warps 4..7 = softmax of tile A, warps 8..11 =
 // softmax of tile B; a softmax thread owns one whole row (128 scores), so no row statistics are exchanged.
 //
 //   TMEM:  S_A | S_B | O_A | O_B   (4 x 128 fp32 columns); P_T (bf16) overwrites the first 64 columns of S_T
@@ -26,7 +26,7 @@
 //
 // Masks: per-row key interval [lo, hi) exactly as in flash_attn.cu; each query tile walks only the K/V
 // tiles up to the last one that any of its rows can see.
-#include "common.cuh"
+#include "block_queue.cuh"
 #include <type_traits>
 
 namespace {
@@ -54,6 +54,7 @@ struct Params {
   float scale_log2;
   int* status;
   const int* holes;    // [B] or null: if any is set, the launch does nothing
+  int wide;            // rows of O start on 32-byte boundaries
   BlockOrder order;
 };
 
@@ -64,8 +65,10 @@ struct L2 {
   static constexpr int K_OFF = Q_OFF + 2 * TILE;     // 2 stages
   static constexpr int V_OFF = K_OFF + 2 * TILE;     // 2 stages
   static constexpr int BAR_OFF = V_OFF + 2 * TILE;   // 192 KB
-  static constexpr int NBARS = 1 + 8 + 2 + 4 + 2;
-  static constexpr int TOTAL = BAR_OFF + NBARS * 8 + 64 + 1024;
+  static constexpr int NBARS = 2 + 8 + 2 + 4 + 2 + 2;
+  static constexpr int QUEUE_OFF = BAR_OFF + NBARS * 8 + 16;
+  static constexpr int TOTAL = QUEUE_OFF + (int)sizeof(WorkQueue) + 1024;
+  static_assert(QUEUE_OFF % 16 == 0, "the queue is 16-byte aligned");
 };
 
 // -inf in place of the scores of hidden keys: key kv0 + c is visible when it lies in [lo, hi)
@@ -115,16 +118,18 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint8_t* sV = smem + L::V_OFF;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
   uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;      // [2]
-  uint64_t* k_empty = bars + 3;     // [2]
-  uint64_t* v_full = bars + 5;      // [2]
-  uint64_t* v_empty = bars + 7;     // [2]
-  uint64_t* s_full = bars + 9;      // [2] per query tile: S_T(j) is in TMEM (and P_T(j-1) V has completed)
-  uint64_t* p_full = bars + 11;     // [2][2] per query tile and half of the keys: P_T(j) is in TMEM
-  uint64_t* o_full = bars + 15;     // [2] per query tile: the last P.V product has completed
+  uint64_t* q_free = bars + 1;      // the last scores of a unit have read Q
+  uint64_t* k_full = bars + 2;      // [2]
+  uint64_t* k_empty = bars + 4;     // [2]
+  uint64_t* v_full = bars + 6;      // [2]
+  uint64_t* v_empty = bars + 8;     // [2]
+  uint64_t* s_full = bars + 10;     // [2] per query tile: S_T(j) is in TMEM (and P_T(j-1) V has completed)
+  uint64_t* p_full = bars + 12;     // [2][2] per query tile and half of the keys: P_T(j) is in TMEM
+  uint64_t* o_full = bars + 16;     // [2] per query tile: the last P.V product of a unit has completed
+  uint64_t* o_free = bars + 18;     // [2] per query tile: O_T of a unit has been read out of TMEM
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + L::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  int* kv_range = const_cast<int*>(reinterpret_cast<volatile int*>(tmem_slot + 2));  // t0, t1 of tile A, t1 of tile B
+  WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
@@ -133,109 +138,118 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int i = threadIdx.x; i < p.B; i += THREADS) any |= p.holes[i];
     if (__syncthreads_or(any)) return;
   }
-  int place, blocks, h, b;
-  if (!block_of(p.order, place, blocks, h, b)) return;
-  const int qb = blocks - 1 - place;   // heaviest (last) causal blocks first
-  const int hk = h / (p.Hq / p.Hkv);
-  const int q0 = qb * 2 * BQ;
   const int shift = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
+    mbar_init(q_free, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
       mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&o_full[i], 1);
+      mbar_init(&s_full[i], 1); mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
     }
     for (int i = 0; i < 4; ++i) mbar_init(&p_full[i], 4);
+    queue_init(queue, 2 + 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == 1) { tmem_alloc<1>(tmem_slot, 512); tmem_relinquish<1>(); }
-  if (warp == 2) {   // union of the key intervals of the rows of each tile (all loads first, then their use)
-    int rlo[2 * BQ / 32], rhi[2 * BQ / 32];
-#pragma unroll
-    for (int e = 0; e < 2 * BQ / 32; ++e) {
-      const int i = min(q0 + lane + 32 * e, p.Sq - 1);
-      rlo[e] = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-      rhi[e] = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-    }
-    int umin = INT_MAX, umax[2] = {0, 0};
-#pragma unroll
-    for (int e = 0; e < 2 * BQ / 32; ++e) {
-      const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk), t = e / (BQ / 32);
-      if (q0 + lane + 32 * e < p.Sq && hi > lo) { umin = min(umin, lo); umax[t] = max(umax[t], hi); }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      umin = min(umin, __shfl_xor_sync(0xffffffffu, umin, o));
-      umax[0] = max(umax[0], __shfl_xor_sync(0xffffffffu, umax[0], o));
-      umax[1] = max(umax[1], __shfl_xor_sync(0xffffffffu, umax[1], o));
-    }
-    if (lane == 0) {
-      const int first = umin == INT_MAX ? 0 : umin / BKV;
-      kv_range[0] = first;
-      kv_range[1] = umax[0] > 0 ? (umax[0] + BKV - 1) / BKV : first;
-      kv_range[2] = umax[1] > 0 ? (umax[1] + BKV - 1) / BKV : first;
-    }
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
-  const int t0 = warp_uniform(kv_range[0]);
-  const int n_a = warp_uniform(kv_range[1]) - t0, n_b = warp_uniform(kv_range[2]) - t0;   // K/V tiles of query tile A / B
-  const int n = max(n_a, n_b);
-  const long long q_row0 = (long long)b * p.Sq + q0;
-  const long long k_row0 = (long long)b * p.Sk;
 
+  // Units of this CTA, one after another: 256 query rows w.place of head w.head and sample w.sample, w.v1 (w.v2) K/V tiles
+  // from w.v0 on for query tile A (B). Barriers of the K/V ring count its tiles through all units (g), those of a query tile
+  // the tiles that it multiplied, those of Q and O the units that have any.
   if (warp < 4) {
     reg_dealloc<REGS_CONTROL>();
-    if (warp == 0 && n > 0) {
+    if (warp == 2) {
+      queue_run(queue, p.order, [&](Work& w, int blocks) {
+        w.place = blocks - 1 - w.place;   // heaviest (last) causal blocks first
+        const int q0 = w.place * 2 * BQ;
+        // union of the key intervals of the rows of each tile (all loads first, then their use)
+        int rlo[2 * BQ / 32], rhi[2 * BQ / 32];
+#pragma unroll
+        for (int e = 0; e < 2 * BQ / 32; ++e) {
+          const int i = min(q0 + lane + 32 * e, p.Sq - 1);
+          rlo[e] = p.row_lo ? p.row_lo[(long long)w.sample * p.Sq + i] : 0;
+          rhi[e] = p.row_hi ? p.row_hi[(long long)w.sample * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
+        }
+        int umin = INT_MAX, umax[2] = {0, 0};
+#pragma unroll
+        for (int e = 0; e < 2 * BQ / 32; ++e) {
+          const int lo = max(rlo[e], 0), hi = min(rhi[e], p.Sk), t = e / (BQ / 32);
+          if (q0 + lane + 32 * e < p.Sq && hi > lo) { umin = min(umin, lo); umax[t] = max(umax[t], hi); }
+        }
+        umin = __reduce_min_sync(0xffffffffu, umin);
+        umax[0] = __reduce_max_sync(0xffffffffu, umax[0]);
+        umax[1] = __reduce_max_sync(0xffffffffu, umax[1]);
+        w.v0 = umin == INT_MAX ? 0 : umin / BKV;
+        w.v1 = umax[0] > 0 ? (umax[0] + BKV - 1) / BKV - w.v0 : 0;
+        w.v2 = umax[1] > 0 ? (umax[1] + BKV - 1) / BKV - w.v0 : 0;
+      }, abort_flag, p.status);
+    }
+    if (warp == 0) {
       const bool el = elect_one();
       if (el) { tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); }
-      if (el) mbar_expect_tx(q_full, 2 * TILE);
+      uint32_t g = 0;
+      int u = 0;
+      Work w;
+      for (int c = 0; queue_next(queue, c, w, abort_flag, p.status) && w.more; ++c) {
+        const int n = max(w.v1, w.v2), h = w.head, hk = h / (p.Hq / p.Hkv);
+        if (n == 0) { queue_claim(queue); continue; }
+        if (!mbar_wait_warp(q_free, (u & 1) ^ 1, abort_flag, p.status)) break;
+        ++u;
+        if (el) mbar_expect_tx(q_full, 2 * TILE);
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (el) tma_load_2d(sQ + t * TILE, &tmQ, q_full, h * HD, (int)(q_row0 + t * BQ));
-        if (HD == 128 && el) tma_load_2d(sQ + t * TILE + PANEL, &tmQ, q_full, h * HD + 64, (int)(q_row0 + t * BQ));
-      }
-      for (int j = 0; j < n; ++j) {
-        const int s = j & 1;
-        const uint32_t ph = (j >> 1) & 1;
-        const int krow = (int)(k_row0 + (long long)(t0 + j) * BKV);
-        if (!mbar_wait_warp(&k_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        if (el) mbar_expect_tx(&k_full[s], TILE);
-        if (el) tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HD, krow);
-        if (HD == 128 && el) tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HD + 64, krow);
-        if (!mbar_wait_warp(&v_empty[s], ph ^ 1, abort_flag, p.status)) break;
-        if (el) mbar_expect_tx(&v_full[s], TILE);
-        if (el) tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HD, krow);
-        if (HD == 128 && el) tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HD + 64, krow);
+        for (int t = 0; t < 2; ++t) {
+          const int qrow = (int)((long long)w.sample * p.Sq + w.place * 2 * BQ + t * BQ);
+          if (el) tma_load_2d(sQ + t * TILE, &tmQ, q_full, h * HD, qrow);
+          if (HD == 128 && el) tma_load_2d(sQ + t * TILE + PANEL, &tmQ, q_full, h * HD + 64, qrow);
+        }
+        bool ok = true;
+        for (int j = 0; j < n; ++j, ++g) {
+          if (j == max(n - 2, 0)) queue_claim(queue);
+          const int s = g & 1;
+          const uint32_t ph = (g >> 1) & 1;
+          const int krow = (int)((long long)w.sample * p.Sk + (long long)(w.v0 + j) * BKV);
+          ok = mbar_wait_warp(&k_empty[s], ph ^ 1, abort_flag, p.status);
+          if (!ok) break;
+          if (el) mbar_expect_tx(&k_full[s], TILE);
+          if (el) tma_load_2d(sK + s * TILE, &tmK, &k_full[s], hk * HD, krow);
+          if (HD == 128 && el) tma_load_2d(sK + s * TILE + PANEL, &tmK, &k_full[s], hk * HD + 64, krow);
+          ok = mbar_wait_warp(&v_empty[s], ph ^ 1, abort_flag, p.status);
+          if (!ok) break;
+          if (el) mbar_expect_tx(&v_full[s], TILE);
+          if (el) tma_load_2d(sV + s * TILE, &tmV, &v_full[s], hk * HD, krow);
+          if (HD == 128 && el) tma_load_2d(sV + s * TILE + PANEL, &tmV, &v_full[s], hk * HD + 64, krow);
+        }
+        if (!ok) break;
       }
     }
-    if (warp == 1 && n > 0) {
+    if (warp == 1) {
       const uint32_t el = elect_one();  // the lane that issues and commits
       constexpr uint32_t idesc_s = umma_idesc(BQ, BKV, 1, 1, false, false);
       constexpr uint32_t idesc_o = umma_idesc(BQ, HD, 1, 1, false, true);
-      int k_ready = -1, v_ready = -1;   // newest K / V tile whose arrival has been waited for
+      uint32_t k_ready = 0, v_ready = 0;   // K / V tiles whose arrival has been waited for
       // descriptors of the tiles' first MMA operands; the loops below only advance them
       // (kept in scalars and picked with selects: an array indexed at run time would live in local memory)
       const uint32_t q_desc0 = umma_desc_lo(smem_u32(sQ), 16), k_desc0 = umma_desc_lo(smem_u32(sK), 16),
                      v_desc0 = umma_desc_lo(smem_u32(sV), PANEL);
-      auto wait_k = [&](int j) -> bool {
-        if (k_ready >= j) return true;
-        k_ready = j;
-        return mbar_wait_warp(&k_full[j & 1], (j >> 1) & 1, abort_flag, p.status);
+      auto wait_k = [&](uint32_t g) -> bool {
+        if (k_ready > g) return true;
+        k_ready = g + 1;
+        return mbar_wait_warp(&k_full[g & 1], (g >> 1) & 1, abort_flag, p.status);
       };
-      auto wait_v = [&](int j) -> bool {
-        if (v_ready >= j) return true;
-        v_ready = j;
-        return mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, abort_flag, p.status);
+      auto wait_v = [&](uint32_t g) -> bool {
+        if (v_ready > g) return true;
+        v_ready = g + 1;
+        return mbar_wait_warp(&v_full[g & 1], (g >> 1) & 1, abort_flag, p.status);
       };
-      // S_T(j) = Q_T K_j^T into the tile's S columns (K_j has arrived)
-      auto issue_s = [&](int t, int j) {
-        const uint32_t qd = q_desc0 + ((t ? TILE : 0) >> 4), kd = k_desc0 + (((j & 1) ? TILE : 0) >> 4);
+      // S_T(g) = Q_T K_g^T into the tile's S columns (K_g has arrived)
+      auto issue_s = [&](int t, uint32_t g) {
+        const uint32_t qd = q_desc0 + ((t ? TILE : 0) >> 4), kd = k_desc0 + (((g & 1) ? TILE : 0) >> 4);
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) {
           const uint32_t off = (k >> 2) * PANEL + (k & 3) * 32;
@@ -243,122 +257,159 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         }
         umma_commit_issue(&s_full[t], el);
       };
-      bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status) && wait_k(0);
-      if (ok && n_a > 0) issue_s(0, 0);
-      if (ok && n_b > 0) issue_s(1, 0);
-      if (ok) umma_commit_issue(&k_empty[0], el);
-      // one half-step of the ping-pong for query tile T (compile-time, so that nothing is indexed at run time):
-      // P_T(j) V_j into O_T, then the next scores S_T(j+1). The waits for V_j and K_{j+1} come before the wait for P,
-      // so that nothing lies between P's arrival and the products that depend on it.
-      auto half_step = [&](auto tile, int j) -> bool {
-        constexpr int t = decltype(tile)::value;
-        const int n_t = t ? n_b : n_a;
-        const int s = j & 1;
-        if (j < n_t) {
-          if (!wait_v(j) || (j + 1 < n_t && !wait_k(j + 1))) return false;
-          const uint32_t vd = v_desc0 + ((s ? TILE : 0) >> 4);
+      uint32_t g = 0, done_a = 0, done_b = 0;      // K/V tiles so far: of the ring, multiplied by query tile A, B
+      int u = 0, units_a = 0, units_b = 0;
+      Work w;
+      for (int c = 0; queue_next(queue, c, w, abort_flag, p.status) && w.more; ++c) {
+        const int n_a = w.v1, n_b = w.v2, n = max(n_a, n_b);
+        if (n == 0) continue;
+        bool ok = mbar_wait_warp(q_full, u & 1, abort_flag, p.status) && wait_k(g);
+        if (!ok) break;
+        if (n_a > 0) issue_s(0, g);
+        if (n_b > 0) issue_s(1, g);
+        umma_commit_issue(&k_empty[g & 1], el);
+        if (n == 1) umma_commit_issue(q_free, el);
+        // one half-step of the ping-pong for query tile T (compile-time, so that nothing is indexed at run time):
+        // P_T(j) V_j into O_T, then the next scores S_T(j+1). The waits for V_j and K_{j+1} come before the wait for P,
+        // so that nothing lies between P's arrival and the products that depend on it.
+        auto half_step = [&](auto tile, int j) -> bool {
+          constexpr int t = decltype(tile)::value;
+          const int n_t = t ? n_b : n_a;
+          const uint32_t gj = g + j, ph = ((t ? done_b : done_a) + j) & 1;
+          const int s = gj & 1;
+          if (j < n_t) {
+            if (!wait_v(gj) || (j + 1 < n_t && !wait_k(gj + 1))) return false;
+            const int units = t ? units_b : units_a;
+            if (j == 0 && units > 0 && !mbar_wait_warp(&o_free[t], (units - 1) & 1, abort_flag, p.status)) return false;
+            const uint32_t vd = v_desc0 + ((s ? TILE : 0) >> 4);
 #pragma unroll
-          for (int k = 0; k < BKV / 16; ++k) {   // A = P_T: 16 bf16 keys per step = 8 TMEM columns
-            if (k % (BKV / 32) == 0) {
-              if (!mbar_wait_warp(&p_full[2 * t + k / (BKV / 32)], j & 1, abort_flag, p.status)) return false;
-              tc_fence_after();
+            for (int k = 0; k < BKV / 16; ++k) {   // A = P_T: 16 bf16 keys per step = 8 TMEM columns
+              if (k % (BKV / 32) == 0) {
+                if (!mbar_wait_warp(&p_full[2 * t + k / (BKV / 32)], ph, abort_flag, p.status)) return false;
+                tc_fence_after();
+              }
+              umma_ts_issue(tmem_base + 2 * BKV + t * HD, tmem_base + t * BKV + k * 8, vd + k * 128,
+                            idesc_o, (j | k) != 0, el);
             }
-            umma_ts_issue(tmem_base + 2 * BKV + t * HD, tmem_base + t * BKV + k * 8, vd + k * 128,
-                          idesc_o, (j | k) != 0, el);
+            if (j == n_t - 1) umma_commit_issue(&o_full[t], el);
           }
-          if (j == n_t - 1) umma_commit_issue(&o_full[t], el);
-        }
-        if (j + 1 < n_t) issue_s(t, j + 1);
-        if (t == 1) umma_commit_issue(&v_empty[s], el);
-        if (t == 1 && j + 1 < n) umma_commit_issue(&k_empty[(j + 1) & 1], el);
-        return true;
-      };
-      for (int j = 0; ok && j < n; ++j)
-        ok = half_step(std::integral_constant<int, 0>{}, j) && half_step(std::integral_constant<int, 1>{}, j);
+          if (j + 1 < n_t) issue_s(t, gj + 1);
+          if (t == 1) umma_commit_issue(&v_empty[s], el);
+          if (t == 1 && j + 1 < n) umma_commit_issue(&k_empty[(gj + 1) & 1], el);
+          if (t == 1 && j + 2 == n) umma_commit_issue(q_free, el);
+          return true;
+        };
+        for (int j = 0; ok && j < n; ++j)
+          ok = half_step(std::integral_constant<int, 0>{}, j) && half_step(std::integral_constant<int, 1>{}, j);
+        if (!ok) break;
+        g += n;
+        ++u;
+        done_a += n_a;
+        done_b += n_b;
+        units_a += n_a > 0;
+        units_b += n_b > 0;
+      }
     }
   } else {
     reg_alloc<REGS_SOFTMAX>();
     const int t = (warp - 4) >> 2;            // query tile of this warp
     const int quarter = warp & 3;             // TMEM lane quarter
     const int r = quarter * 32 + lane;        // row inside the tile
-    const int i = q0 + t * BQ + r;            // global query row
-    const bool row_valid = i < p.Sq;
-    const int n_t = t ? n_b : n_a;
-    int lo = 0, hi = 0;
-    if (row_valid) {
-      lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-      hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-      lo = max(lo, 0); hi = min(hi, p.Sk);
-    }
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t s_addr = lane_addr + t * BKV, o_addr = lane_addr + 2 * BKV + t * HD;
-    float m_ref = -INFINITY, l_run = 0.f;
-    bool ok = true;
-    for (int j = 0; j < n_t; ++j) {
-      const int kv0 = (t0 + j) * BKV;
-      if (!mbar_wait_warp(&s_full[t], j & 1, abort_flag, p.status)) { ok = false; break; }
-      tc_fence_after();
-      // the mask tests are compiled into a separate path taken only by warps with a partly visible row
-      const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
-      uint32_t x0[32], x1[32], x2[32], x3[32];
-      tmem_ld_32x32(s_addr, x0);
-      tmem_ld_32x32(s_addr + 32, x1);
-      tmem_ld_32x32(s_addr + 64, x2);
-      tmem_ld_32x32(s_addr + 96, x3);
-      tmem_ld_wait();
-      if (!full) {
-        mask_scores(x0, kv0, lo, hi);
-        mask_scores(x1, kv0 + 32, lo, hi);
-        mask_scores(x2, kv0 + 64, lo, hi);
-        mask_scores(x3, kv0 + 96, lo, hi);
+    int lo = 0, hi = 0;
+    auto load_unit = [&](const Work& w) {     // the row's interval, loaded before the results of the last unit are stored
+      const int i = w.place * 2 * BQ + t * BQ + r;
+      lo = hi = 0;
+      if (w.more && i < p.Sq) {
+        lo = p.row_lo ? p.row_lo[(long long)w.sample * p.Sq + i] : 0;
+        hi = p.row_hi ? p.row_hi[(long long)w.sample * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
       }
-      const float mx = fmaxf(fmaxf(max_of(x0), max_of(x1)), fmaxf(max_of(x2), max_of(x3)));
-      // raise the reference maximum only when it pays: 2^(gap) of a stale one fits bf16 and fp32
-      const bool raise = (mx > m_ref) && (m_ref == -INFINITY || (mx - m_ref) * p.scale_log2 > RESCALE_THRESHOLD<HD>);
-      if (__any_sync(0xffffffffu, raise)) {
-        float alpha = 1.f;
-        if (raise) {
-          alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * p.scale_log2);
-          m_ref = mx;
-          l_run *= alpha;
+    };
+    uint32_t g = 0;
+    int u = 0;
+    Work w;
+    bool ok = queue_next(queue, 0, w, abort_flag, p.status);
+    if (ok) load_unit(w);
+    for (int c = 0; ok && w.more;) {
+      const int b = w.sample, h = w.head, n_t = t ? w.v2 : w.v1;
+      const int i = w.place * 2 * BQ + t * BQ + r;     // global query row
+      const bool row_valid = i < p.Sq;
+      lo = max(lo, 0); hi = min(hi, p.Sk);
+      float m_ref = -INFINITY, l_run = 0.f;
+      for (int j = 0; j < n_t; ++j, ++g) {
+        const int kv0 = (w.v0 + j) * BKV;
+        if (!mbar_wait_warp(&s_full[t], g & 1, abort_flag, p.status)) { ok = false; break; }
+        tc_fence_after();
+        // the mask tests are compiled into a separate path taken only by warps with a partly visible row
+        const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
+        uint32_t x0[32], x1[32], x2[32], x3[32];
+        tmem_ld_32x32(s_addr, x0);
+        tmem_ld_32x32(s_addr + 32, x1);
+        tmem_ld_32x32(s_addr + 64, x2);
+        tmem_ld_32x32(s_addr + 96, x3);
+        tmem_ld_wait();
+        if (!full) {
+          mask_scores(x0, kv0, lo, hi);
+          mask_scores(x1, kv0 + 32, lo, hi);
+          mask_scores(x2, kv0 + 64, lo, hi);
+          mask_scores(x3, kv0 + 96, lo, hi);
         }
-        if (j > 0) {   // O_T holds the products up to tile j-1 (complete: S_T(j) was issued after them)
+        const float mx = fmaxf(fmaxf(max_of(x0), max_of(x1)), fmaxf(max_of(x2), max_of(x3)));
+        // raise the reference maximum only when it pays: 2^(gap) of a stale one fits bf16 and fp32
+        const bool raise = (mx > m_ref) && (m_ref == -INFINITY || (mx - m_ref) * p.scale_log2 > RESCALE_THRESHOLD<HD>);
+        if (__any_sync(0xffffffffu, raise)) {
+          float alpha = 1.f;
+          if (raise) {
+            alpha = (m_ref == -INFINITY) ? 0.f : fast_exp2((m_ref - mx) * p.scale_log2);
+            m_ref = mx;
+            l_run *= alpha;
+          }
+          if (j > 0) {   // O_T holds the products up to tile j-1 (complete: S_T(j) was issued after them)
 #pragma unroll 1
-          for (int cc = 0; cc < HD / 32; ++cc) {
-            uint32_t tr[32];
-            tmem_ld_32x32(o_addr + cc * 32, tr);
-            tmem_ld_wait();
+            for (int cc = 0; cc < HD / 32; ++cc) {
+              uint32_t tr[32];
+              tmem_ld_32x32(o_addr + cc * 32, tr);
+              tmem_ld_wait();
 #pragma unroll
-            for (int c = 0; c < 32; ++c) tr[c] = __float_as_uint(__uint_as_float(tr[c]) * alpha);
-            tmem_st_32x32(o_addr + cc * 32, tr);
+              for (int c = 0; c < 32; ++c) tr[c] = __float_as_uint(__uint_as_float(tr[c]) * alpha);
+              tmem_st_32x32(o_addr + cc * 32, tr);
+            }
           }
         }
+        // ---- P = 2^(S c - m c) as packed bf16 over the first 64 columns of S, in two halves
+        const float neg_ms = (m_ref == -INFINITY) ? 0.f : -m_ref * p.scale_log2;
+        const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nm2 = f2_pack(neg_ms, neg_ms);
+        uint64_t sum0 = 0ull, sum1 = 0ull;   // (0.f, 0.f)
+        uint32_t pk[32];
+        exp_half(x0, x1, sc2, nm2, sum0, sum1, pk);
+        tmem_st_32x32(s_addr, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[2 * t]);
+        exp_half(x2, x3, sc2, nm2, sum0, sum1, pk);
+        tmem_st_32x32(s_addr + 32, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[2 * t + 1]);
+        float a, b2, c2, d2;
+        f2_unpack(sum0, a, b2);
+        f2_unpack(sum1, c2, d2);
+        l_run += (a + b2) + (c2 + d2);
       }
-      // ---- P = 2^(S c - m c) as packed bf16 over the first 64 columns of S, in two halves
-      const float neg_ms = (m_ref == -INFINITY) ? 0.f : -m_ref * p.scale_log2;
-      const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nm2 = f2_pack(neg_ms, neg_ms);
-      uint64_t sum0 = 0ull, sum1 = 0ull;   // (0.f, 0.f)
-      uint32_t pk[32];
-      exp_half(x0, x1, sc2, nm2, sum0, sum1, pk);
-      tmem_st_32x32(s_addr, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[2 * t]);
-      exp_half(x2, x3, sc2, nm2, sum0, sum1, pk);
-      tmem_st_32x32(s_addr + 32, pk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[2 * t + 1]);
-      float a, b2, c2, d2;
-      f2_unpack(sum0, a, b2);
-      f2_unpack(sum1, c2, d2);
-      l_run += (a + b2) + (c2 + d2);
-    }
-    if (ok && n_t > 0) ok = mbar_wait_warp(&o_full[t], 0, abort_flag, p.status);
-    if (ok) {
-      if (n_t > 0) tc_fence_after();
+      if (!ok) break;
+      Work nw;
+      ok = queue_next(queue, ++c, nw, abort_flag, p.status);
+      if (!ok) break;
+      load_unit(nw);
+      if (n_t > 0) {
+        ok = mbar_wait_warp(&o_full[t], u & 1, abort_flag, p.status);
+        if (!ok) break;
+        ++u;
+        tc_fence_after();
+      }
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
       __nv_bfloat16* orow = p.O + (((long long)b * p.Sq + i) * p.Hq + h) * HD;
 #pragma unroll
@@ -367,25 +418,23 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         if (n_t > 0) {
           tmem_ld_32x32(o_addr + cc * 32, tr);
           tmem_ld_wait();
+          if (cc == HD / 32 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_free[t]);
+          }
+#pragma unroll
+          for (int k = 0; k < 32; ++k) tr[k] = __float_as_uint(__uint_as_float(tr[k]) * inv);
         } else {
 #pragma unroll
-          for (int c = 0; c < 32; ++c) tr[c] = 0u;
+          for (int k = 0; k < 32; ++k) tr[k] = 0u;
         }
-        if (row_valid) {
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            uint4 v;
-            v.x = pack_bf16x2(__uint_as_float(tr[c]) * inv, __uint_as_float(tr[c + 1]) * inv);
-            v.y = pack_bf16x2(__uint_as_float(tr[c + 2]) * inv, __uint_as_float(tr[c + 3]) * inv);
-            v.z = pack_bf16x2(__uint_as_float(tr[c + 4]) * inv, __uint_as_float(tr[c + 5]) * inv);
-            v.w = pack_bf16x2(__uint_as_float(tr[c + 6]) * inv, __uint_as_float(tr[c + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + cc * 32 + c) = v;
-          }
-        }
+        if (row_valid) store_bf16_32(orow + cc * 32, tr, p.wide);
       }
       if (row_valid)
         p.lse[((long long)b * p.Hq + h) * p.Sq + i] =
             l_run > 0.f ? (m_ref * p.scale_log2 + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
+      w = nw;
     }
   }
 
@@ -439,6 +488,7 @@ extern "C" int atb_flash_fwd_v2(const void* q, const void* k, const void* v, voi
   p.scale_log2 = softmax_scale * 1.4426950408889634f;
   p.status = status;
   p.holes = holes;
+  p.wide = (reinterpret_cast<uintptr_t>(o) & 31) == 0;     // rows of whole heads of 128 or 256 bytes
   return head_dim == 64 ? launch_fwd2<64>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream)
                         : launch_fwd2<128>(q, k, v, p, q_stride, k_stride, v_stride, (cudaStream_t)stream);
 }

@@ -398,7 +398,10 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
     split = BWD_SPLIT and drop is None and bias is None
     dq_acc = None if split else torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=q.device)
     fold = _fold(Hq // Hkv, B * Hkv * ((Sk + 127) // 128), (Sq + 127) // 128, bool(causal)) if split else 1
-    delta = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
+    # row sums; the two-kernel form with intervals keeps two words per query block behind them
+    rows = B * Hq * Sq
+    ranges = 2 * B * ((Sq + 127) // 128) if split and (row_lo is not None or row_hi is not None) else 0
+    delta = torch.empty(rows + (rows & 1) + ranges, dtype=torch.float32, device=q.device)
     if fused_out and Hkv == Hq and Sq == Sk:
         fused = torch.empty(B, Sq, 3 * Hq, D, dtype=q.dtype, device=q.device)
         dq, dk, dv = fused[:, :, :Hq], fused[:, :, Hq: 2 * Hq], fused[:, :, 2 * Hq:]

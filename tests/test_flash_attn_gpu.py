@@ -603,3 +603,32 @@ def test_head_dim_64_kernel_by_waves_of_blocks(H, S, two, causal, monkeypatch):
     ref = attention_reference(q, k, v, causal=causal).float()
     torch.cuda.synchronize()
     assert (out.float() - ref).norm() <= 2 ** -7 * ref.norm()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("mask", ["none", "padding"])
+def test_blocks_taken_over_by_running_ctas(mask, causal, D):
+    """More blocks than SMs in all three kernels (480 forward, 720 backward), so that every CTA does several of them, among
+    them blocks that see no key at all (samples without a valid key) next to full ones: the same as the fp32 reference,
+    and the same bits whichever CTA a block falls to."""
+    torch.manual_seed(D)
+    B, S, H = 6, 270, 40
+    q, k, v, dout = (torch.randn(B, S, H, D, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    kw = {"causal": causal}
+    if mask == "padding":
+        valid = torch.tensor([270, 0, 1, 129, 200, 0], device="cuda")[:, None]
+        kw["key_padding_mask"] = torch.arange(S, device="cuda")[None] < valid
+    lo, hi = flash.row_intervals(B, S, S, q.device, causal, key_padding_mask=kw.get("key_padding_mask"))
+    runs = []
+    for _ in range(3):
+        out, lse = flash.flash_fwd_raw(q, k, v, causal, D ** -0.5, lo, hi)
+        runs.append((out, lse, *flash.flash_bwd_raw(dout, q, k, v, out, lse, causal, D ** -0.5, lo, hi)))
+    torch.cuda.synchronize()
+    _lib.check_status(torch.device("cuda", 0))
+    for other in runs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(runs[0], other))
+    ins = [t.float().requires_grad_(True) for t in (q, k, v)]
+    ref = attention_reference(*ins, **kw)
+    for got, want in zip((runs[0][0], *runs[0][2:]), (ref, *torch.autograd.grad(ref, ins, dout.float()))):
+        assert (got.float() - want).norm() <= 1e-2 * want.norm()   # bf16 P, dS and results: 2^-9 each
