@@ -1,4 +1,4 @@
-"""ctypes loader for ``libatb.so`` (the sm_100a kernels of atorch_b200).
+"""Loader for ``libatb.so`` (the sm_100a kernels of atorch_b200).
 
 The library is built in-tree by :mod:`atorch_b200.build`. On a machine with a GPU a missing
 library is an error (ops must never fall back silently to eager PyTorch); on a CPU-only machine
@@ -8,6 +8,7 @@ the CPU test-suite exercises.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 from pathlib import Path
 from typing import Optional
@@ -24,9 +25,7 @@ class KernelError(RuntimeError):
 
 
 # Argument types of the launchers on the per-operator path (p: pointer, i: int, l: long long, f: float), checked against
-# csrc/ by a test. ctypes then converts plain Python numbers itself: building twenty ctypes objects per call and asking
-# for a Stream object cost more host time than the launch (an evaluation of a 1.3B model on one short document is bound
-# by the host: 67 launches took 3.1 ms, 2.75 ms this way).
+# csrc/ by a test. They are called through csrc/launcher.c with plain Python numbers; the others through ctypes.
 SIGNATURES = {
     "atb_gemm_bf16_2cta": "ppppiiillliiiifiiplpp",
     "atb_gemm_bf16_2cta_grouped": "ppppiiillliiiifiiplpiiiiipp",
@@ -54,35 +53,47 @@ SIGNATURES = {
 }
 _CTYPE = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
 
-launch_count = 0  # kernels of this library launched so far in this process
+_ctypes_launches = 0
 _NOT_LAUNCHES = {"atb_norm_bwd_parts", "atb_sumsq_parts", "atb_set_comm_wait_ns", "atb_noalloc_max_n"}
 
 
+def __getattr__(name):
+    if name == "launch_count":       # kernels of this library launched so far in this process
+        return _ctypes_launches + (0 if _lib is None else _lib.launcher.count())
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
 class _CountingLib:
-    """Proxy over the ctypes library that counts kernel launches (one per launcher call)."""
+    """The library's functions by name, each launcher counting its calls (one per kernel launch)."""
 
-    def __init__(self, cdll):
+    def __init__(self, cdll, launcher):
         self._cdll = cdll
-        self._cache = {}
+        self.launcher = launcher
 
-    def __getattr__(self, name):
-        fn = self._cache.get(name)
-        if fn is None:
-            raw = getattr(self._cdll, name)
-            if name in SIGNATURES:
-                raw.argtypes = [_CTYPE[c] for c in SIGNATURES[name]]
-            if name in _NOT_LAUNCHES:
-                fn = raw
-            else:
-                def fn(*a, _raw=raw):
-                    global launch_count
-                    launch_count += 1
-                    return _raw(*a)
-            self._cache[name] = fn
+    def __getattr__(self, name):     # once per name: the function becomes an attribute
+        raw = getattr(self._cdll, name)
+        if name in SIGNATURES:
+            fn = self.launcher.Launcher(ctypes.cast(raw, ctypes.c_void_p).value, SIGNATURES[name])
+        elif name in _NOT_LAUNCHES:
+            fn = raw
+        else:
+            def fn(*a, _raw=raw):
+                global _ctypes_launches
+                _ctypes_launches += 1
+                return _raw(*a)
+        self.__dict__[name] = fn
         return fn
 
     def has(self, name) -> bool:
-        return hasattr(self._cdll, name)
+        return name in self.__dict__ or hasattr(self._cdll, name)
+
+
+def _load_launcher():
+    """The extension module next to the library (csrc/launcher.c)."""
+    spec = importlib.util.spec_from_file_location("_launcher", _LIB_PATH.with_name("_launcher.so"))
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
 
 
 def lib_path() -> Path:
@@ -99,14 +110,14 @@ def lib():
     if _tried:
         raise KernelError(f"{_LIB_PATH} could not be loaded")
     _tried = True
-    if not _LIB_PATH.exists():
+    if not (_LIB_PATH.exists() and _LIB_PATH.with_name("_launcher.so").exists()):
         if os.environ.get("ATB_AUTO_BUILD", "1") == "1":
             from . import build as _build
 
             _build.build()
         else:
             raise KernelError(f"{_LIB_PATH} is missing: run `python -m atorch_b200.build`")
-    _lib = _CountingLib(ctypes.CDLL(str(_LIB_PATH)))
+    _lib = _CountingLib(ctypes.CDLL(str(_LIB_PATH)), _load_launcher())
     return _lib
 
 

@@ -2,8 +2,9 @@
 
 Every ``csrc/*.cu`` file is compiled with ``nvcc -gencode arch=compute_100a,code=sm_100a`` into an
 object file and the objects are linked into one shared library, ``atorch_b200/_C/libatb.so``, that
-exposes plain ``extern "C"`` launchers (loaded with ctypes by :mod:`atorch_b200._lib`). nvcc
-cross-compiles, so the build needs no GPU. Objects are rebuilt only when a source or header is newer.
+exposes plain ``extern "C"`` launchers (loaded by :mod:`atorch_b200._lib`). nvcc cross-compiles, so the build
+needs no GPU. Objects are rebuilt only when a source or header is newer. ``_C/_launcher.so`` beside it makes the launchers
+callable from Python at little cost (C, a second to compile).
 
 Plays the role of the JIT op builder of the reference (atorch/ops/op_builder/builder.py:120-681),
 but ahead of time and for one architecture only.
@@ -18,6 +19,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent
@@ -25,6 +27,7 @@ CSRC = ROOT / "csrc"
 OUT_DIR = ROOT / "_C"
 OBJ_DIR = OUT_DIR / "obj"
 LIB = OUT_DIR / "libatb.so"
+LAUNCHER = OUT_DIR / "_launcher.so"      # Python callables for the launchers (csrc/launcher.c)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -56,6 +59,19 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool) -> str:
     return res.stderr if verbose else ""
 
 
+def _build_launcher(force: bool) -> None:
+    src = CSRC / "launcher.c"
+    if not force and LAUNCHER.exists() and LAUNCHER.stat().st_mtime >= src.stat().st_mtime:
+        return
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
+    if cc is None:
+        raise RuntimeError("no C compiler found; set CC or add gcc to PATH")
+    cmd = [cc, "-O2", "-Wall", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(LAUNCHER)]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cc} failed for {src.name}:\n{res.stdout}\n{res.stderr}")
+
+
 def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
@@ -63,6 +79,7 @@ def sources() -> list[Path]:
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = find_nvcc()
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    _build_launcher(force)
     hdr_m = _newest_header_mtime()
     todo, objs = [], []
     for src in sources():

@@ -94,6 +94,10 @@ class LlamaConfig:
         return L * (proj * mult + attn * (mult if attention_recompute else 3)) + head * 3
 
 
+# attention arguments for which the kernels have to be asked (ops/flash.py: supported)
+_NOT_PLAIN = {"dropout_p", "additive_mask", "additive_bias"}
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float = 1e-5):
         super().__init__()
@@ -153,12 +157,15 @@ class LlamaDecoderLayer(nn.Module):
             S = qkv.shape[1]  # the projection may have gathered a sequence-sharded input (sequence parallelism)
             qkv = ops.rope(qkv, cos, sin, self.n_q + self.n_kv, d, positions, inplace=True)  # read by nothing else
         qkv = qkv.view(B, S, self.n_q + 2 * self.n_kv, d)
-        q = qkv[:, :, : self.n_q]
-        k = qkv[:, :, self.n_q: self.n_q + self.n_kv]
-        v = qkv[:, :, self.n_q + self.n_kv:]
         kw = attn_kwargs or {"causal": True}
-        if self.n_q == self.n_kv and flash.supported(q, k, v, kw.get("dropout_p", 0.0), kw.get("additive_mask"),
-                                                     kw.get("additive_bias")) and flash.backward_built():
+        fused = self.n_q == self.n_kv and not (kw.keys() & _NOT_PLAIN) and flash.supported_qkv(qkv, self.n_q)
+        if not fused:
+            q = qkv[:, :, : self.n_q]
+            k = qkv[:, :, self.n_q: self.n_q + self.n_kv]
+            v = qkv[:, :, self.n_q + self.n_kv:]
+            fused = self.n_q == self.n_kv and flash.supported(
+                q, k, v, kw.get("dropout_p", 0.0), kw.get("additive_mask"), kw.get("additive_bias")) and flash.backward_built()
+        if fused:
             cache = self._attn_cache if (self.training and self.config.reuse_attention_in_recompute) else None
             a = flash.flash_attention_qkv(qkv, self.n_q, recompute_cache=cache, **kw)   # fused gradient out
         else:

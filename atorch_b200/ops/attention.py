@@ -27,6 +27,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from .function import call
 
 
 def build_dense_mask(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask: Optional[torch.Tensor] = None,
@@ -101,7 +102,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
         if iv is not None:
             scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(q.shape[-1])
             drop = flash.dropout_config(dropout_p) if dropout_p > 0.0 else None
-            return flash._FlashAttn.apply(q, k, v, False, float(scale), iv[0], iv[1], drop)
+            return call(flash._FlashAttn, q, k, v, False, float(scale), iv[0], iv[1], drop)
     if flash.supported(q, k, v, dropout_p, additive_mask, additive_bias, key_padding_mask):
         return flash.flash_attention(q, k, v, causal=causal, softmax_scale=softmax_scale, glm_mask=glm_mask,
                                      pack_glm_mask=pack_glm_mask, key_padding_mask=key_padding_mask,

@@ -14,6 +14,7 @@ import torch
 import torch.distributed as dist
 
 from .. import _lib
+from .function import call
 
 
 def cross_entropy_reference(logits, labels, ignore_index=-100, label_smoothing=0.0, lse_square_scale=0.0):
@@ -106,7 +107,7 @@ def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int 
             return _vocab_parallel_reference(logits, labels, ignore_index, label_smoothing, lse_square_scale,
                                              process_group)
         return cross_entropy_reference(logits, labels, ignore_index, label_smoothing, lse_square_scale)
-    return _CrossEntropy.apply(logits, labels.contiguous(), ignore_index, float(label_smoothing),
+    return call(_CrossEntropy, logits, labels.contiguous(), ignore_index, float(label_smoothing),
                                float(lse_square_scale), inplace_backward, process_group)
 
 

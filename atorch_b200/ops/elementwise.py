@@ -11,6 +11,7 @@ from typing import Optional, Tuple
 import torch
 
 from .. import _lib
+from .function import call
 
 
 def rope_tables(seq_len: int, head_dim: int, base: float = 10000.0, device=None) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -97,7 +98,7 @@ def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, nheads: int, hea
         return _RopeRef.apply(x, cos, sin, positions, nheads, head_dim)
     if positions is not None and positions.dtype != torch.int32:
         positions = positions.to(torch.int32)
-    return _Rope.apply(x, cos, sin, positions, nheads, head_dim, bool(inplace) and not x.is_leaf)
+    return call(_Rope, x, cos, sin, positions, nheads, head_dim, bool(inplace) and not x.is_leaf)
 
 
 class _RopeRef(torch.autograd.Function):
@@ -157,7 +158,7 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for a fused ``[..., 2F]`` gate|up tensor."""
     if not (_lib.use_kernels(gate_up) and gate_up.dtype == torch.bfloat16 and gate_up.shape[-1] % 16 == 0):
         return swiglu_reference(gate_up)
-    return _SwiGLU.apply(gate_up)
+    return call(_SwiGLU, gate_up)
 
 
 def bias_gather_add_reference(inp, bias, expert_idx):

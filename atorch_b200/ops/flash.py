@@ -24,6 +24,7 @@ from typing import Optional, Tuple
 import torch
 
 from .. import _lib
+from .function import call
 
 
 import os
@@ -84,6 +85,13 @@ def supported(q, k, v, dropout_p=0.0, additive_mask=None, additive_bias=None, ke
         if s3 != 1 or s2 != D or s1 % 8 or s0 != s1 * t.shape[1]:
             return False
     return True
+
+
+def supported_qkv(qkv: torch.Tensor, num_heads: int) -> bool:
+    """:func:`supported` for the three thirds of a contiguous ``qkv [B, S, 3*H, D]`` without dropout, mask tensors or biases."""
+    return (_lib.use_kernels(qkv) and kernels_built() and backward_built() and qkv.dtype == torch.bfloat16
+            and qkv.is_contiguous() and qkv.shape[2] == 3 * num_heads
+            and (qkv.shape[3] == 128 or (qkv.shape[3] == 64 and _lib.lib().has("atb_flash_fwd_ex"))))
 
 
 def row_intervals(B: int, Sq: int, Sk: int, device, causal: bool = False, glm_mask=None, pack_glm_mask=None,
@@ -357,16 +365,32 @@ def flash_fwd_raw(q, k, v, causal, softmax_scale, row_lo, row_hi, drop=None, bia
     """Launch the forward kernel. Returns (out [B,Sq,Hq,D] bf16, lse [B,Hq,Sq] fp32). ``drop``: see
     ``dropout_config``; dropout runs in the single-tile kernel. ``holes``: see ``_padded_intervals`` (two-tile kernel)."""
     B, Sq, Hq, D = q.shape
-    Sk, Hkv = k.shape[1], k.shape[2]
-    out = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
-    lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
+    return _forward(q, (q.data_ptr(), k.data_ptr(), v.data_ptr()), (B, Sq, k.shape[1], Hq, k.shape[2]), D,
+                    (_token_stride(q), _token_stride(k), _token_stride(v)), causal, softmax_scale, row_lo, row_hi, drop,
+                    bias, holes)
+
+
+def _fused_heads(qkv, H):
+    """Addresses and token strides of the q, k and v heads of ``qkv [B, S, 3*H, D]`` (a slice takes longer to make than to
+    read)."""
+    step = H * qkv.shape[3] * qkv.element_size()
+    base = qkv.data_ptr()
+    return (base, base + step, base + 2 * step), (_token_stride(qkv),) * 3
+
+
+def _forward(like, qkv, sizes, D, strides, causal, softmax_scale, row_lo, row_hi, drop=None, bias=None, holes=None):
+    """:func:`flash_fwd_raw` on addresses ``qkv`` with token ``strides`` and ``sizes = (B, Sq, Sk, Hq, Hkv)``; ``like``: a
+    tensor of their device and dtype."""
+    B, Sq, _, Hq, _ = sizes
+    out = torch.empty(B, Sq, Hq, D, dtype=like.dtype, device=like.device)
+    lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=like.device)
     L = _lib.lib()
     # two-query-tile kernel (flash_attn_v2.cu) for long enough sequences (and enough blocks, see ONE_WAVE); the single-tile
     # kernel otherwise, and for
     # dropout, a bias, and a scale that is not positive (hidden scores are -inf before they are scaled)
     p = _lib.addr
-    args = (p(q), p(k), p(v), p(out), p(lse), p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q),
-            _token_stride(k), _token_stride(v), int(causal), softmax_scale, _lib.stream(), _lib.status_addr(q))
+    args = (*qkv, out.data_ptr(), lse.data_ptr(), p(row_lo), p(row_hi), *sizes, *strides, int(causal), softmax_scale,
+            _lib.stream(), _lib.status_addr(like))
     if FWD_TWO_TILES and Sq >= 256 and drop is None and bias is None and softmax_scale > 0 \
             and (D == 128 or B * Hq * ((Sq + 127) // 128) > ONE_WAVE):
         rc = L.atb_flash_fwd_v2(*args, D, p(holes))
@@ -394,31 +418,40 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
     equal query / key-value head counts) the three are slices of ONE ``[B, S, 3*H, D]`` buffer laid out
     like a fused q|k|v projection output, so the gradient of that projection needs no concatenation."""
     B, Sq, Hq, D = q.shape
-    Sk, Hkv = k.shape[1], k.shape[2]
+    return _backward(q, (q.data_ptr(), k.data_ptr(), v.data_ptr()), (B, Sq, k.shape[1], Hq, k.shape[2]), D,
+                     (_token_stride(q), _token_stride(k), _token_stride(v)), dout, out, lse, causal, softmax_scale, row_lo,
+                     row_hi, fused_out, drop, bias)
+
+
+def _backward(like, qkv, sizes, D, strides, dout, out, lse, causal, softmax_scale, row_lo, row_hi, fused_out=False, drop=None,
+              bias=None):
+    """:func:`flash_bwd_raw` on addresses, see :func:`_forward`."""
+    B, Sq, Sk, Hq, Hkv = sizes
+    dev, dt = like.device, like.dtype
     split = BWD_SPLIT and drop is None and bias is None
-    dq_acc = None if split else torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=q.device)
+    dq_acc = None if split else torch.zeros(B, Sq, Hq, D, dtype=torch.float32, device=dev)
     fold = _fold(Hq // Hkv, B * Hkv * ((Sk + 127) // 128), (Sq + 127) // 128, bool(causal)) if split else 1
     # row sums; the two-kernel form with intervals keeps two words per query block behind them
     rows = B * Hq * Sq
     ranges = 2 * B * ((Sq + 127) // 128) if split and (row_lo is not None or row_hi is not None) else 0
-    delta = torch.empty(rows + (rows & 1) + ranges, dtype=torch.float32, device=q.device)
+    delta = torch.empty(rows + (rows & 1) + ranges, dtype=torch.float32, device=dev)
     if fused_out and Hkv == Hq and Sq == Sk:
-        fused = torch.empty(B, Sq, 3 * Hq, D, dtype=q.dtype, device=q.device)
-        dq, dk, dv = fused[:, :, :Hq], fused[:, :, Hq: 2 * Hq], fused[:, :, 2 * Hq:]
+        fused = torch.empty(B, Sq, 3 * Hq, D, dtype=dt, device=dev)
+        grads, (dq_stride, dkv_stride, _) = _fused_heads(fused, Hq)
     else:
         fused = None
-        dq = torch.empty(B, Sq, Hq, D, dtype=q.dtype, device=q.device)
-        dk = torch.empty(B, Sk, Hq // fold, D, dtype=q.dtype, device=q.device)
-        dv = torch.empty(B, Sk, Hq // fold, D, dtype=q.dtype, device=q.device)
+        dq = torch.empty(B, Sq, Hq, D, dtype=dt, device=dev)
+        dk = torch.empty(B, Sk, Hq // fold, D, dtype=dt, device=dev)
+        dv = torch.empty(B, Sk, Hq // fold, D, dtype=dt, device=dev)
+        grads, dq_stride, dkv_stride = (dq.data_ptr(), dk.data_ptr(), dv.data_ptr()), Hq * D, Hq // fold * D
     dout = dout if (dout.stride(-1) == 1 and dout.stride(2) == D and dout.stride(0) == dout.stride(1) * Sq) \
         else dout.contiguous()
     L, p = _lib.lib(), _lib.addr
-    dims = (p(row_lo), p(row_hi), B, Sq, Sk, Hq, Hkv, _token_stride(q), _token_stride(k), _token_stride(v),
-            _token_stride(dout), _token_stride(dq), _token_stride(dk), int(causal), softmax_scale, _lib.stream(),
-            _lib.status_addr(q))
-    ins = (p(dout), p(q), p(k), p(v), p(out), p(lse), p(delta))
+    dims = (p(row_lo), p(row_hi), *sizes, *strides, _token_stride(dout), dq_stride, dkv_stride, int(causal), softmax_scale,
+            _lib.stream(), _lib.status_addr(like))
+    ins = (dout.data_ptr(), *qkv, out.data_ptr(), lse.data_ptr(), delta.data_ptr())
     if split:
-        rc = L.atb_flash_bwd_split(*ins, p(dq), p(dk), p(dv), *dims, fold, D)
+        rc = L.atb_flash_bwd_split(*ins, *grads, *dims, fold, D)
     else:
         if D != 128:
             bwd, extra = L.atb_flash_bwd_ex, _extra_args(drop, bias, D)
@@ -428,15 +461,15 @@ def flash_bwd_raw(dout, q, k, v, out, lse, causal, softmax_scale, row_lo, row_hi
             bwd, extra = L.atb_flash_bwd_dropout, _extra_args(drop, None)
         else:
             bwd, extra = L.atb_flash_bwd, ()
-        args = _as_ctypes("atb_flash_bwd_split", (*ins, p(dq), p(dk), p(dv), *dims))
+        args = _as_ctypes("atb_flash_bwd_split", (*ins, *grads, *dims))
         rc = bwd(*args[: len(ins)], _lib.ptr(dq_acc), *args[len(ins):], *extra)
     _lib.check(rc, "atb_flash_bwd")
-    if Hkv * fold != Hq:
-        parts, (dk, dv) = (dk, dv), (torch.empty(B, Sk, Hkv, D, dtype=q.dtype, device=q.device) for _ in range(2))
-        rc = L.atb_head_sum(*map(p, parts), p(dk), p(dv), B * Sk * Hkv, Hq // Hkv // fold, D, _lib.stream())
-        _lib.check(rc, "atb_head_sum")
     if fused is not None:
         return fused
+    if Hkv * fold != Hq:
+        parts, (dk, dv) = (dk, dv), (torch.empty(B, Sk, Hkv, D, dtype=dt, device=dev) for _ in range(2))
+        rc = L.atb_head_sum(*map(p, parts), p(dk), p(dv), B * Sk * Hkv, Hq // Hkv // fold, D, _lib.stream())
+        _lib.check(rc, "atb_head_sum")
     return dq, dk, dv
 
 
@@ -473,7 +506,7 @@ def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pa
                                (glm_mask, pack_glm_mask, cu_seqlens, additive_mask, additive_bias), dropout_p > 0.0)
     try:
         if padded is not None:
-            return _FlashAttn.apply(q, k, v, bool(causal), float(scale), padded[0], padded[1], None, None, padded[2])
+            return call(_FlashAttn, q, k, v, bool(causal), float(scale), padded[0], padded[1], None, None, padded[2])
         lo, hi = row_intervals(B, Sq, Sk, q.device, causal, glm_mask, pack_glm_mask, key_padding_mask, cu_seqlens)
     except NonContiguousKeyMask:
         if additive_mask is not None or additive_bias is not None:
@@ -487,7 +520,7 @@ def flash_attention(q, k, v, causal=False, softmax_scale=None, glm_mask=None, pa
     bias = None
     if additive_mask is not None or additive_bias is not None:
         bias = bias_config(B, Hq, Sq, Sk, additive_mask, additive_bias)
-    return _FlashAttn.apply(q, k, v, bool(causal), float(scale), lo, hi, drop, bias)
+    return call(_FlashAttn, q, k, v, bool(causal), float(scale), lo, hi, drop, bias)
 
 
 def _unpadded_attention(q, k, v, key_padding_mask, causal, scale, glm_mask, pack_glm_mask, cu_seqlens,
@@ -513,17 +546,23 @@ def _unpadded_attention(q, k, v, key_padding_mask, causal, scale, glm_mask, pack
     return out.view(B, S, H, D)
 
 
+def _fused_forward(qkv, H, causal, scale, row_lo, row_hi, look):
+    B, S, _, D = qkv.shape
+    heads, strides = _fused_heads(qkv, H)
+    return _forward(qkv, heads, (B, S, S, H, H), D, strides, causal, scale, row_lo, row_hi,
+                    holes=None if look is None else look.device)
+
+
 class _FlashAttnQKV(torch.autograd.Function):
     """Attention on a fused projection output ``qkv [B, S, 3*H, D]`` (q heads, then k, then v). The
     backward emits one fused gradient tensor in the same layout: no slice-backward zero fills or adds."""
 
     @staticmethod
     def forward(ctx, qkv, H, causal, scale, row_lo, row_hi, cached, look=None):
-        q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
         if cached is not None:
             out, lse = cached          # output and log-sum-exp kept from the first pass of a checkpointed block
         else:
-            out, lse = flash_fwd_raw(q, k, v, causal, scale, row_lo, row_hi, holes=None if look is None else look.device)
+            out, lse = _fused_forward(qkv, H, causal, scale, row_lo, row_hi, look)
         if look is not None:
             look.check()
         ctx.save_for_backward(qkv, out, lse, row_lo, row_hi)
@@ -534,8 +573,10 @@ class _FlashAttnQKV(torch.autograd.Function):
     def backward(ctx, dout):
         qkv, out, lse, row_lo, row_hi = ctx.saved_tensors
         H, causal, scale = ctx.cfg
-        q, k, v = qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:]
-        dqkv = flash_bwd_raw(dout, q, k, v, out, lse, causal, scale, row_lo, row_hi, fused_out=True)
+        B, S, _, D = qkv.shape
+        heads, strides = _fused_heads(qkv, H)
+        dqkv = _backward(qkv, heads, (B, S, S, H, H), D, strides, dout, out, lse, causal, scale, row_lo, row_hi,
+                         fused_out=True)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -570,9 +611,7 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
         if cur is not None:
             token, is_recompute = cur
             if not is_recompute and not torch.is_grad_enabled():
-                H = num_heads
-                out, lse = flash_fwd_raw(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], bool(causal),
-                                         float(scale), lo, hi, holes=None if look is None else look.device)
+                out, lse = _fused_forward(qkv, num_heads, bool(causal), float(scale), lo, hi, look)
                 if look is not None:
                     look.check()
                 recompute_cache[token] = (out, lse)
@@ -583,7 +622,7 @@ def flash_attention_qkv(qkv: torch.Tensor, num_heads: int, causal: bool = True, 
                 cached = recompute_cache.pop(token, None)
                 if cached is not None and cached[0].shape != (B, S, num_heads, D):
                     cached = None
-        return _FlashAttnQKV.apply(qkv, num_heads, bool(causal), float(scale), lo, hi, cached, look)
+        return call(_FlashAttnQKV, qkv, num_heads, bool(causal), float(scale), lo, hi, cached, look)
     except NonContiguousKeyMask:
         H = num_heads
         return flash_attention(qkv[:, :, :H], qkv[:, :, H: 2 * H], qkv[:, :, 2 * H:], causal=causal,

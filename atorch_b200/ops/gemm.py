@@ -21,6 +21,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from .function import call
 
 
 # CTA-pair kernel (tcgen05 cta_group::2, 256x256 tiles) for problems with M, N >= 256
@@ -272,7 +273,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
             and _lib.lib().has("atb_gemm_bf16_2cta_swiglu") and F % 8 == 0 and x.shape[-1] % 8 == 0
             and weight.stride(-1) == 1 and PAIR_KERNEL_DEFAULT):
         return swiglu(linear(x, weight))
-    return _LinearSwiGLU.apply(x, weight)
+    return call(_LinearSwiGLU, x, weight)
 
 
 class _LinearRope(torch.autograd.Function):
@@ -331,7 +332,7 @@ def linear_rope(x: torch.Tensor, weight: torch.Tensor, cos: torch.Tensor, sin: t
         return rope(linear(x, weight), cos, sin, nheads, head_dim, positions, inplace=inplace_grad)
     if positions is not None and positions.dtype != torch.int32:
         positions = positions.to(torch.int32)
-    return _LinearRope.apply(x, weight, cos, sin, positions, nheads, head_dim, inplace_grad)
+    return call(_LinearRope, x, weight, cos, sin, positions, nheads, head_dim, inplace_grad)
 
 
 class _Linear(torch.autograd.Function):
@@ -374,4 +375,4 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if x.dtype != torch.bfloat16 or not _lib.use_kernels(x, weight):
         y = torch.nn.functional.linear(x, weight.to(x.dtype), None if bias is None else bias.to(x.dtype))
         return y if residual is None else residual + y
-    return _Linear.apply(x, weight, bias, residual)
+    return call(_Linear, x, weight, bias, residual)

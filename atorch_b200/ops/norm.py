@@ -12,6 +12,7 @@ from typing import Optional
 import torch
 
 from .. import _lib
+from .function import call
 
 
 def rms_norm_reference(x, weight, eps=1e-6, residual=None):
@@ -92,6 +93,8 @@ class _Norm(torch.autograd.Function):
         ctx.w_ref, ctx.b_ref = weight, bias
         if residual is not None:
             return y.view(shp), s.view(shp)
+        if carry and not any(ctx.needs_input_grad):
+            return y.view(shp), x.detach()
         if carry:
             # second output: x itself (a second tensor over the same storage, no copy) for the residual path, so
             # that the gradient arriving through it is added inside the backward kernel
@@ -133,11 +136,11 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
         y = rms_norm_reference(x, weight, eps, residual)
         return (y, x) if (carry and residual is None) else y
     if carry and residual is None:
-        return _Norm.apply(x, None, weight, None, eps, False, True)
-    return _Norm.apply(x, residual, weight, None, eps, False)
+        return call(_Norm, x, None, weight, None, eps, False, True)
+    return call(_Norm, x, residual, weight, None, eps, False)
 
 
 def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, eps: float = 1e-5):
     if not _kernel_ok(x, weight) or (bias is not None and bias.dtype != x.dtype):
         return layer_norm_reference(x, weight, bias, eps)
-    return _Norm.apply(x, None, weight, bias, eps, True)
+    return call(_Norm, x, None, weight, bias, eps, True)

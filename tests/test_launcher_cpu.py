@@ -1,0 +1,90 @@
+"""The launcher extension's argument passing (csrc/launcher.c) and calls of autograd functions without gradients."""
+import ctypes
+import importlib.util
+import subprocess
+
+import pytest
+import torch
+from torch.autograd import forward_ad
+
+from atorch_b200 import build
+from atorch_b200.ops.function import call
+
+C_SOURCE = r"""
+#include <string.h>
+static double seen[64];
+const double* last(void) { return seen; }
+int mixed(void* a, const void* b, int c, long long d, float e, int g, void* h, long long i, int j, float k, int l, int m,
+          const int* n, int o, long long p, float q, int r, long long s, int t, int u) {
+  const double v[] = {(double)(long long)a, (double)(long long)b, c, (double)d, e, g, (double)(long long)h, (double)i, j, k,
+                      l, m, n[0], n[1], o, (double)p, q, r, (double)s, t, u};
+  memcpy(seen, v, sizeof(v));
+  return -7;
+}
+"""
+
+
+def _module(tmp_path):
+    build._build_launcher(False)
+    spec = importlib.util.spec_from_file_location("_launcher", build.LAUNCHER)
+    launcher = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(launcher)
+    (tmp_path / "callee.c").write_text(C_SOURCE)
+    subprocess.run(["gcc", "-O2", "-shared", "-fPIC", str(tmp_path / "callee.c"), "-o", str(tmp_path / "callee.so")], check=True)
+    lib = ctypes.CDLL(str(tmp_path / "callee.so"))
+    lib.last.restype = ctypes.POINTER(ctypes.c_double)
+    return launcher, lib, launcher.Launcher(ctypes.cast(lib.mixed, ctypes.c_void_p).value, "ppilfiplifiipilfilii")
+
+
+def test_arguments_in_registers_and_on_the_stack(tmp_path):
+    """Integers of both widths, pointers in every form and floats between them, more than the registers hold; numbers are cut
+    to the declared width like ctypes does; wrong counts and types are errors and call nothing."""
+    launcher, lib, fn = _module(tmp_path)
+    arr = (ctypes.c_int * 2)(21, -22)
+    args = (1 << 40, None, -3, -(1 << 40), 1.5, True, ctypes.c_void_p(0), 7, (1 << 33) | 5, 2, ctypes.c_int(9), -11, arr, -1,
+            (1 << 50) + 1, ctypes.c_float(0.25), 13, -14, -15, 16)
+    before = launcher.count()
+    assert fn(*args) == -7
+    assert lib.last()[:21] == [1 << 40, 0, -3, -(1 << 40), 1.5, 1, 0, 7, 5, 2, 9, -11, 21, -22, -1, (1 << 50) + 1, 0.25, 13,
+                               -14, -15, 16]
+    assert launcher.count() == before + 1
+    for bad in (args[:-1], args + (1,), ("x",) + args[1:], args[:2] + (1.5,) + args[3:], args[:4] + (None,) + args[5:]):
+        with pytest.raises((TypeError, AttributeError)):
+            fn(*bad)
+    assert launcher.count() == before + 1
+    with pytest.raises(ValueError):
+        launcher.Launcher(1, "px")
+
+
+class _Double(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        ctx.save_for_backward(x)
+        ctx.seen = ctx.needs_input_grad
+        _Double.last = tuple(ctx.needs_input_grad)
+        return x * 2
+
+    @staticmethod
+    def backward(ctx, g):
+        return g * 2
+
+
+def test_call_without_gradients():
+    """With gradients on, the node; off, the forward alone, which is told that nothing needs a gradient; what looks into
+    calls (forward-mode differentiation, transforms, the tracer) still meets ``apply``."""
+    x = torch.ones(3, requires_grad=True)
+    y = call(_Double, x)
+    assert y.requires_grad and _Double.last == (True,)
+    (g,) = torch.autograd.grad(y.sum(), x)
+    assert torch.equal(g, torch.full((3,), 2.0))
+    with torch.no_grad():
+        y = call(_Double, x)
+        assert not y.requires_grad and not any(_Double.last) and torch.equal(y, torch.full((3,), 2.0))
+        with forward_ad.dual_level(), pytest.raises(Exception):
+            call(_Double, forward_ad.make_dual(x.detach(), torch.ones(3)))
+        with pytest.raises(Exception):
+            torch.func.vmap(lambda t: call(_Double, t))(torch.ones(2, 3))
+        traced = torch.jit.trace(lambda t: call(_Double, t), (torch.ones(3),), check_trace=False)
+        assert "PythonOp" in str(traced.graph) or "_Double" in str(traced.graph)
+    with torch.inference_mode():
+        assert torch.equal(call(_Double, torch.ones(3)), torch.full((3,), 2.0))
