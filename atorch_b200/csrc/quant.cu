@@ -68,10 +68,14 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ x, 
   }
 }
 
-// The same quantisation with every group held in registers: one read of x. A warp (WARPS = 1) or a block of WARPS warps
-// owns a group of at most WARPS * 32 * V pieces of 8 elements; lane i of them takes pieces i, i + 32 WARPS, ...
-// Bound by memory: 16-byte loads, all V pieces of a thread in flight, 8- or 4-byte stores. 67 M bf16 values in groups
-// of 2048 to int8: 87.5 -> 45.2 us (201 MB, 4.5 TB/s); the kernel above reads x twice, 2 bytes a thread.
+// The same quantisation with every group held in registers: one read of x. LANES lanes of a warp, or a block of WARPS warps
+// (LANES = 32), own a group of at most WARPS * LANES * V pieces of 8 elements; the i-th of them takes pieces i,
+// i + LANES * WARPS, ...
+// Bound by memory: 16-byte loads, all V pieces of a thread in flight, 8- or 4-byte stores, and few enough instructions, which
+// bounded it before: extrema of 16-bit values two at a time, and codes by adding 1.5 * 2^23, whose low bits then are the
+// rounded integer, packed by byte permutes; rintf and the conversion to int each take a slot of the slow unit (16 a clock).
+// 67 M bf16 values in groups of 2048 to int8 (201 MB, cold): 47.1 us with those, 36.9 now (5.5 TB/s); fp32 57.4 either way.
+// The kernel above reads x twice, 2 bytes a thread: 87.5 us.
 template <typename T>
 struct Piece8 {
   uint4 r[sizeof(T) / 2];
@@ -82,34 +86,89 @@ struct Piece8 {
   ATB_DEVICE float at(int i) const { return to_f32<T>(reinterpret_cast<const T*>(r)[i]); }
 };
 
-template <typename T, int WARPS, int V>
+// Running extrema of pieces; NaN is passed over. abs_only: hi is that of the magnitudes, lo is not kept.
+template <typename T>
+struct Extrema {
+  float hi = -INFINITY, lo = INFINITY;
+  ATB_DEVICE void add(const Piece8<T>& v, bool abs_only) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      hi = fmaxf(hi, abs_only ? fabsf(v.at(j)) : v.at(j));
+      if (!abs_only) lo = fminf(lo, v.at(j));
+    }
+  }
+  ATB_DEVICE void done(float& h, float& l) const { h = hi; l = lo; }
+};
+template <typename T2>
+struct Extrema16 {
+  T2 hi, lo;
+  template <typename P>
+  ATB_DEVICE void add(const P& v, bool abs_only) {
+    const T2* x = reinterpret_cast<const T2*>(v.r);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      hi = __hmax2(hi, abs_only ? __habs2(x[j]) : x[j]);
+      if (!abs_only) lo = __hmin2(lo, x[j]);
+    }
+  }
+};
+template <>
+struct Extrema<__nv_bfloat16> : Extrema16<__nv_bfloat162> {
+  ATB_DEVICE Extrema() { hi = __float2bfloat162_rn(-INFINITY); lo = __float2bfloat162_rn(INFINITY); }
+  ATB_DEVICE void done(float& h, float& l) const {
+    h = fmaxf(__low2float(hi), __high2float(hi));
+    l = fminf(__low2float(lo), __high2float(lo));
+  }
+};
+template <>
+struct Extrema<__half> : Extrema16<__half2> {
+  ATB_DEVICE Extrema() { hi = __float2half2_rn(-INFINITY); lo = __float2half2_rn(INFINITY); }
+  ATB_DEVICE void done(float& h, float& l) const {
+    h = fmaxf(__low2float(hi), __high2float(hi));
+    l = fminf(__low2float(lo), __high2float(lo));
+  }
+};
+
+// Low bytes of four words in one.
+ATB_DEVICE uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
+// Low nibbles of the bytes of x as 16 bits.
+ATB_DEVICE uint32_t nibbles(uint32_t x) {
+  x &= 0x0F0F0F0Fu;
+  x = (x | (x >> 4)) & 0x00FF00FFu;
+  return (x | (x >> 8)) & 0xFFFFu;
+}
+
+template <typename T, int WARPS, int LANES, int V>
 __global__ void __launch_bounds__(128) quantize_regs_kernel(const T* __restrict__ x, int8_t* __restrict__ q,
                                                             float* __restrict__ params, int groups, int group_size,
                                                             int bits, int asym, const int* __restrict__ group_map) {
   __shared__ float red[2][4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = WARPS == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
-  if (g >= groups) return;                       // WARPS == 1 only: whole warps leave, nothing below syncs the block
-  const int t = WARPS == 1 ? lane : threadIdx.x;
+  constexpr int PER_WARP = 32 / LANES, TEAM = LANES * WARPS;      // groups of a warp; threads of a group
+  int g = WARPS == 1 ? (blockIdx.x * 4 + warp) * PER_WARP + lane / LANES : blockIdx.x;
+  if (WARPS == 1 && g - lane / LANES >= groups) return;      // whole warps leave, nothing below syncs the block
+  const bool mine = WARPS > 1 || g < groups;                 // the last warp may have lanes without a group
+  if (!mine) g = groups - 1;
+  const int t = WARPS == 1 ? lane % LANES : threadIdx.x;
   const int n = group_size / 8;
   const T* xg = x + (long long)g * group_size;
   Piece8<T> v[V];
 #pragma unroll
   for (int i = 0; i < V; ++i)
-    if (t + i * 32 * WARPS < n) v[i].load(xg + (t + i * 32 * WARPS) * 8);
-  float lo = INFINITY, hi = -INFINITY;
+    if (t + i * TEAM < n) v[i].load(xg + (t + i * TEAM) * 8);
+  Extrema<T> ext;
 #pragma unroll
-  for (int i = 0; i < V; ++i) {
-    if (t + i * 32 * WARPS < n) {
+  for (int i = 0; i < V; ++i)
+    if (t + i * TEAM < n) ext.add(v[i], !asym);
+  float lo, hi;
+  ext.done(hi, lo);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        lo = fminf(lo, v[i].at(j));
-        hi = fmaxf(hi, v[i].at(j));
-      }
-    }
+  for (int o = LANES / 2; o > 0; o >>= 1) {
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
   }
-  hi = warp_max(hi);
-  lo = -warp_max(-lo);
   if (WARPS > 1) {
     if (lane == 0) { red[0][warp] = hi; red[1][warp] = lo; }
     __syncthreads();
@@ -117,58 +176,60 @@ __global__ void __launch_bounds__(128) quantize_regs_kernel(const T* __restrict_
     for (int i = 0; i < WARPS; ++i) { hi = fmaxf(hi, red[0][i]); lo = fminf(lo, red[1][i]); }
   }
   const int qmax = (1 << (bits - 1)) - 1, half = 1 << (bits - 1);
-  float s = asym ? (hi - lo) / (float)((1 << bits) - 1) : fmaxf(fabsf(hi), fabsf(lo)) / (float)qmax;
+  float s = asym ? (hi - lo) / (float)((1 << bits) - 1) : fabsf(hi) / (float)qmax;
   const float off = asym ? lo : 0.f;
   if (s == 0.f) s = 1.f;
   const float inv = 1.f / s;
   const int og = group_map ? group_map[g] : g;
-  if (t == 0) {
+  if (t == 0 && mine) {
     params[(long long)og * (asym ? 2 : 1)] = s;
     if (asym) params[(long long)og * 2 + 1] = off;
   }
-  const float fh = (float)half, fm = (float)qmax, shift = asym ? fh : 0.f;
+  // rint(clamp(x)) is clamp(rint(x)) for whole bounds; asymmetric codes are rounded before the offset of half the range, which
+  // turns over their highest bit. NaN takes the lowest code, as fmaxf has it.
+  const float low = asym ? 0.f : -(float)half, high = asym ? (float)(2 * half - 1) : (float)qmax;
+  const uint32_t turn = !asym ? 0u : bits == 8 ? 0x80808080u : 0x08080808u;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
-    const int k = t + i * 32 * WARPS;
-    if (k >= n) continue;
+    const int k = t + i * TEAM;
+    if (k >= n || !mine) continue;
     uint32_t c[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      c[j] = (uint32_t)(int)fminf(fmaxf(rintf((v[i].at(j) - off) * inv) - shift, -fh), fm);
-    if (bits == 8) {
-      uint2 o = make_uint2(0u, 0u);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        o.x |= (c[j] & 0xFFu) << (8 * j);
-        o.y |= (c[4 + j] & 0xFFu) << (8 * j);
-      }
-      *reinterpret_cast<uint2*>(q + (long long)og * group_size + (long long)k * 8) = o;
-    } else {
-      uint32_t o = 0u;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) o |= (c[j] & 0xFu) << (4 * j);
-      *reinterpret_cast<uint32_t*>(q + (long long)og * (group_size / 2) + (long long)k * 4) = o;
+    for (int j = 0; j < 8; ++j) {
+      // off is 0 for symmetric codes; two roundings, product and sum, are wanted
+      const float x = __fmul_rn(asym ? v[i].at(j) - off : v[i].at(j), inv);
+      c[j] = __float_as_uint(__fadd_rn(fminf(fmaxf(x, low), high), 12582912.f));
     }
+    const uint32_t w0 = low_bytes(c[0], c[1], c[2], c[3]) ^ turn, w1 = low_bytes(c[4], c[5], c[6], c[7]) ^ turn;
+    if (bits == 8)
+      *reinterpret_cast<uint2*>(q + (long long)og * group_size + (long long)k * 8) = make_uint2(w0, w1);
+    else
+      *reinterpret_cast<uint32_t*>(q + (long long)og * (group_size / 2) + (long long)k * 4) = nibbles(w0) | (nibbles(w1) << 16);
   }
 }
 
-// A warp per group up to 2048 elements (8 pieces a lane: 32 registers of 16-bit, 64 of 32-bit values), a block of 4
-// warps up to 8192. Longer groups, groups that are no multiple of 8 and unaligned inputs take quantize_kernel.
+// Four pieces a lane as far as the group has them, and as many lanes as it takes: 8 up to 256 elements, 16 up to 512, a warp up
+// to 2048 (8 pieces a lane: 32 registers of 16-bit, 64 of 32-bit values), a block of 4 warps up to 8192. With a whole warp
+// for every group 67 M bf16 values in groups of 128 (512) took 121 (46) us, now
+// 45 (38); fp32 in groups of 128 119 -> 57. Longer groups, groups that are no
+// multiple of 8 and unaligned inputs take quantize_kernel.
 template <typename T>
 bool quantize_regs(const T* x, int8_t* q, float* params, int groups, int group_size, int bits, int asym,
                    const int* group_map, cudaStream_t st) {
   if (group_size % 8 || group_size > 8192 || (reinterpret_cast<uintptr_t>(x) & 15) ||
       (reinterpret_cast<uintptr_t>(q) & 7))
     return false;
-#define ATB_QUANT(W_, V_)                                                                                     \
-  quantize_regs_kernel<T, W_, V_><<<(W_) == 1 ? (groups + 3) / 4 : groups, 128, 0, st>>>(x, q, params, groups, \
-                                                                                         group_size, bits, asym, group_map)
-  if (group_size <= 256) ATB_QUANT(1, 1);
-  else if (group_size <= 512) ATB_QUANT(1, 2);
-  else if (group_size <= 1024) ATB_QUANT(1, 4);
-  else if (group_size <= 2048) ATB_QUANT(1, 8);
-  else if (group_size <= 4096) ATB_QUANT(4, 4);
-  else ATB_QUANT(4, 8);
+#define ATB_QUANT(W_, L_, V_)                                                                                           \
+  quantize_regs_kernel<T, W_, L_, V_><<<(W_) == 1 ? (groups + 4 * (32 / (L_)) - 1) / (4 * (32 / (L_))) : groups, 128, 0, st>>>( \
+      x, q, params, groups, group_size, bits, asym, group_map)
+  if (group_size <= 64) ATB_QUANT(1, 8, 1);
+  else if (group_size <= 128) ATB_QUANT(1, 8, 2);
+  else if (group_size <= 256) ATB_QUANT(1, 8, 4);
+  else if (group_size <= 512) ATB_QUANT(1, 16, 4);
+  else if (group_size <= 1024) ATB_QUANT(1, 32, 4);
+  else if (group_size <= 2048) ATB_QUANT(1, 32, 8);
+  else if (group_size <= 4096) ATB_QUANT(4, 32, 4);
+  else ATB_QUANT(4, 32, 8);
 #undef ATB_QUANT
   return true;
 }

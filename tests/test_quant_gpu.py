@@ -87,3 +87,25 @@ def test_quantize_group_lengths(group, dtype):
                 d = quantizer.dequantize(q, p, groups, bits, sym, out)
                 dr = quantizer.dequantize_reference(q, p, groups, bits, sym, out)     # one rounding to `out`
                 assert torch.equal(d, dr) or torch.allclose(d.float(), dr.float(), rtol=2 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("group", [8, 64, 72, 128, 256, 264, 512, 1024, 2048, 4104])
+def test_quantize_special_values_like_the_general_kernel(group, dtype):
+    """NaN, infinities, zeros and values whose scale has no finite reciprocal, for every split of a group over lanes: the same
+    codes and parameters as the general kernel, which inputs off a 16-byte boundary take. Odd numbers of groups leave lanes
+    without one."""
+    torch.manual_seed(group)
+    groups = 37
+    x = torch.randn(groups, group, device="cuda").to(dtype)
+    x[1, 3], x[2, 0], x[4, 7] = float("nan"), float("inf"), -float("inf")
+    x[5], x[6], x[7] = float("nan"), 0, float("inf")
+    x[8] = torch.where(torch.arange(group, device="cuda") % 2 == 0, 1e-45, -0.0).to(dtype)
+    x[36, group - 1] = 1e4
+    flat = x.reshape(-1)
+    shifted = torch.empty(flat.numel() + 1, device="cuda", dtype=dtype)[1:]
+    shifted.copy_(flat)
+    for bits in (8, 4):
+        for sym in (True, False):
+            (q, p), (qg, pg) = (quantizer.quantize(t, groups, bits, sym) for t in (flat, shifted))
+            assert torch.equal(q, qg) and torch.equal(p.nan_to_num(7.0), pg.nan_to_num(7.0))
