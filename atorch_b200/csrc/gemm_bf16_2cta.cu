@@ -25,6 +25,7 @@
 //   GEMM -> reduce-scatter  the epilogue adds every output row into the fp32 accumulation buffer of the
 //                        rank that owns the row (`red.add.f32` on peer pointers): no partial-sum tensor, no
 //                        separate collective, the reduction traffic overlaps the remaining tiles
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -40,14 +41,19 @@ constexpr int A_BYTES = BM * BK * 2;
 // BN = accumulator columns of the pair's tile (256 or 128); each CTA loads BN/2 rows of B.
 // The narrower tile exists for wave quantisation: 256 tiles of 256x256 fill 74 CTA pairs 3.46 times
 // (4 waves, 86 % busy), the same problem in 256x128 tiles takes 7 waves of half the length (99 %).
-template <int BN>
+//
+// SPLIT = 2: two pairs, a cluster of four CTAs, share a tile: pair p takes half p of the reduction and finishes half of the
+// columns, whose partial sums it gets from its counterpart (same rows) through distributed shared memory, 64 KB each way per
+// tile; half of the epilogue is left to each. For products with too few tiles, see split_pays.
+template <int BN, int SPLIT = 1>
 struct Cfg {
   static constexpr int BNH = BN / 2;
-  static constexpr int STAGES = BN == 256 ? 6 : 8;
+  static constexpr int STAGES = SPLIT == 2 ? 5 : BN == 256 ? 6 : 8;
   static constexpr int B_BYTES = BNH * BK * 2;
-  static constexpr int BAR_OFF = STAGES * (A_BYTES + B_BYTES);
+  static constexpr int X_OFF = STAGES * (A_BYTES + B_BYTES);         // partial sums from the other pair, fp32
+  static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 0);
   static constexpr int TQ = 4;                     // tile-id ring of the dynamic scheduler
-  static constexpr int SMEM_TOTAL = BAR_OFF + (2 * STAGES + 4 + 2 * TQ) * 8 + 16 + TQ * 4 + 1024;
+  static constexpr int SMEM_TOTAL = BAR_OFF + (2 * STAGES + 4 + 2 * TQ + 2) * 8 + 16 + TQ * 4 + 1024;
 };
 
 struct Epi {
@@ -76,6 +82,7 @@ struct Epi {
   const float* rope_sin;
   const int* rope_pos;
   int rope_s, rope_dim, rope_cols;
+  int split;  // (host) pairs per tile: 0 by split_pays, -1 one, 1 two wherever the kernel can
   int wide;   // every 16 columns of an output row start on a 32-byte boundary and N is a multiple of 16 (set by launch)
 };
 
@@ -217,6 +224,9 @@ struct Sched {
 ATB_DEVICE void st_remote_u32(uint32_t cluster_addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
+ATB_DEVICE void st_remote_v4(uint32_t cluster_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 // Wait (by a whole converged warp, one answer for all lanes) on a barrier whose phase is completed by an arrive of
 // another CTA of the cluster that published data with it.
 ATB_DEVICE bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status) {
@@ -259,14 +269,15 @@ ATB_DEVICE void mbar_arrive_remote(uint32_t bar_cluster_addr) {
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 
-template <int BN, bool A_MN, bool B_MN, bool KG>
+template <int BN, bool A_MN, bool B_MN, bool KG, int SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epi ep, int M,
                       int N, int K, Groups grp, Gate gate, Sched sched, const __grid_constant__ Ragged rag,
                       const __grid_constant__ KGroups<KG> kg, int* status) {
   static_assert(!KG || (A_MN && B_MN), "groups along the reduction are rows of MN-major operands");
-  constexpr int BNH = Cfg<BN>::BNH, STAGES = Cfg<BN>::STAGES, B_BYTES = Cfg<BN>::B_BYTES,
-                BAR_OFF = Cfg<BN>::BAR_OFF;
+  static_assert(SPLIT == 1 || (BN == 256 && !KG), "two pairs share a 256-wide tile");
+  using C = Cfg<BN, SPLIT>;
+  constexpr int BNH = C::BNH, STAGES = C::STAGES, B_BYTES = C::B_BYTES, BAR_OFF = C::BAR_OFF;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sA = smem;
@@ -275,15 +286,19 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint64_t* empty = full + STAGES;
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + 2;
-  constexpr int TQ = Cfg<BN>::TQ;
+  constexpr int TQ = C::TQ;
   uint64_t* tq_full = tempty + 2;
   uint64_t* tq_empty = tq_full + TQ;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tq_empty + TQ);
+  uint64_t* xfull = tq_empty + TQ;        // partial sums of the other pair are in the exchange buffer
+  uint64_t* xfree = xfull + 1;            // the other pair has read those sent to it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xfree + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* tq_tile = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [TQ] tile ids (-1: no more tiles)
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  const uint32_t rank = warp_uniform(cluster_ctarank());
+  const uint32_t cta = warp_uniform(cluster_ctarank());
+  const uint32_t rank = cta & 1, pair0 = cta & ~1u;     // place in the pair; the pair's first CTA in the cluster
+  const int part = SPLIT == 2 ? (int)(cta >> 1) : 0;    // which half of the reduction and of the columns
   const bool leader = rank == 0;
   // both CTAs of a pair read the same word, so they take the same decision
   const bool skip = warp_uniform((int)(status != nullptr && *reinterpret_cast<volatile int*>(status) != 0)) != 0;
@@ -294,11 +309,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   int groups = 1;
   if constexpr (KG) groups = kg.n;
   const int num_tiles = skip ? 0 : tiles_m * tiles_n * groups;
-  auto tile_kbs = [&](int b_idx) -> int {            // k-blocks of a tile
+  // k-blocks [first, end) of a tile for this pair
+  auto tile_kbs = [&](int b_idx, int& first) -> int {
+    first = 0;
     if constexpr (KG) return (kg.rows[b_idx] + BK - 1) / BK;
-    else return (K + BK - 1) / BK;
+    const int n = (K + BK - 1) / BK, mid = (n + 1) / 2;
+    if constexpr (SPLIT == 2) {
+      first = part ? mid : 0;
+      return part ? n : mid;
+    }
+    return n;
   };
-  const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
+  const int cluster_id = blockIdx.x / (2 * SPLIT), num_clusters = gridDim.x / (2 * SPLIT);
   constexpr int BAND = 8;
 
   if (threadIdx.x == 0) {
@@ -314,6 +336,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(&tq_full[i], 1);
       mbar_init(&tq_empty[i], 2 + 2 * EPI_WARPS);   // leader: MMA + epilogue warps; partner: producer + epilogue warps
     }
+    mbar_init(xfull, EPI_WARPS);
+    mbar_init(xfree, EPI_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -401,9 +425,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     if (!mbar_wait_warp(&tq_empty[slot], ((idx / TQ) & 1) ^ 1, abort_flag, status)) return false;
     if (lane == 0) {
       tq_tile[slot] = t;
-      st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), 1), (uint32_t)t);
+      st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), pair0 + 1), (uint32_t)t);
       mbar_arrive(&tq_full[slot]);
-      mbar_arrive_remote(map_to_cta(&tq_full[slot], 1));     // release.cluster: orders the store above
+      mbar_arrive_remote(map_to_cta(&tq_full[slot], pair0 + 1));     // release.cluster: orders the store above
     }
     return true;
   };
@@ -415,7 +439,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   };
   auto free_tile_slot = [&](int idx) {                        // once per consumer warp, after read_tile by all its lanes
     __syncwarp();
-    if (dyn && lane == 0) mbar_arrive_remote(map_to_cta(&tq_empty[idx % TQ], 0));
+    if (dyn && lane == 0) mbar_arrive_remote(map_to_cta(&tq_empty[idx % TQ], pair0));
   };
 
   if (warp == 0) {
@@ -449,7 +473,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         int m0, n0, m_end, b_idx;
         tile_coords(tile, m0, n0, m_end, b_idx);
         if (!tile_active(m0, b_idx)) continue;
-        const int num_kb = tile_kbs(b_idx);
+        int kb_first;
+        const int kb_end = tile_kbs(b_idx, kb_first);
         const CUtensorMap *mapA = &tmA, *mapB = &tmB;
         if constexpr (KG) {
           mapA = &kg.a[b_idx];
@@ -467,14 +492,14 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                              : gate_wait(gate, am0, min(am0 + BM, M), abort_flag, status);
           if (!__all_sync(0xffffffffu, here)) goto producer_done;
         }
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_first; kb < kb_end; ++kb) {
           if (!kb_active(kb)) continue;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait_warp(&empty[s], ph ^ 1, abort_flag, status)) goto producer_done;
           if (lane == 0) {
             if (leader) mbar_expect_tx(&full[s], 2 * (A_BYTES + B_BYTES));
-            const uint32_t bar = map_to_cta(&full[s], 0);
+            const uint32_t bar = map_to_cta(&full[s], pair0);
             uint8_t* a_dst = sA + s * A_BYTES;
             uint8_t* b_dst = sB + s * B_BYTES;
             if constexpr (!A_MN) {
@@ -500,7 +525,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     if (leader) {
       const uint32_t el = elect_one();      // the lane that issues and commits
       const uint32_t a_desc = umma_desc_lo(smem_u32(sA), A_MN ? 8192 : 16), b_desc = umma_desc_lo(smem_u32(sB), B_MN ? 8192 : 16);
-      const uint32_t empty0 = smem_u32(empty), empty1 = map_to_cta(empty, 1), tfull0 = smem_u32(tfull), tfull1 = map_to_cta(tfull, 1);
+      const uint32_t empty0 = map_to_cta(empty, pair0), empty1 = map_to_cta(empty, pair0 + 1);
+      const uint32_t tfull0 = map_to_cta(tfull, pair0), tfull1 = map_to_cta(tfull, pair0 + 1);
       constexpr uint32_t idesc = umma_idesc(2 * BM, BN, 1, 1, A_MN, B_MN);
       uint32_t it = 0;
       int local = 0;
@@ -508,12 +534,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         const int tile = read_tile(idx);
         free_tile_slot(idx);
         if (tile < 0) break;
-        int num_kb;
+        int kb_first, kb_end;
         {
           int m0, n0, m_end, b_idx;
           tile_coords(tile, m0, n0, m_end, b_idx);
           if (!tile_active(m0, b_idx)) continue;
-          num_kb = tile_kbs(b_idx);
+          kb_end = tile_kbs(b_idx, kb_first);
         }
         const int acc = local & 1;
         const uint32_t acc_ph = (local >> 1) & 1;
@@ -521,7 +547,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         bool first_kb = true;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_first; kb < kb_end; ++kb) {
           if (!kb_active(kb)) continue;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -548,7 +574,110 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int half = (warp - 2) >> 2;       // column half
     const bool wide = ep.wide != 0;
     int local = 0;
-    const uint32_t tempty_leader[2] = {map_to_cta(&tempty[0], 0), map_to_cta(&tempty[1], 0)};
+    const uint32_t tempty_leader[2] = {map_to_cta(&tempty[0], pair0), map_to_cta(&tempty[1], pair0)};
+    // What becomes of 32 accumulators of a row (the operands' sum over the whole reduction) at column col0 of the output.
+    // gate and up of the same 32 features
+    auto finish_gated = [&](const uint32_t (&g)[32], const uint32_t (&u)[32], int row, int col0) {
+      __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
+      __nv_bfloat16* grow = ep.gu_out == nullptr ? nullptr
+          : reinterpret_cast<__nv_bfloat16*>(ep.gu_out) + (long long)row * ep.ldgu + col0;
+      uint32_t gp[16], up[16], op[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        // round to bf16 first: the same values and the same formula as the separate SwiGLU kernel
+        gp[j] = pack_bf16x2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
+        up[j] = pack_bf16x2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
+        const float2 a = unpack_bf16x2(gp[j]), b = unpack_bf16x2(up[j]);
+        op[j] = pack_bf16x2(a.x / (1.f + __expf(-a.x)) * b.x, a.y / (1.f + __expf(-a.y)) * b.y);
+      }
+      store_row_bf16(crow, op, N - col0, wide);
+      if (grow != nullptr) {
+        store_row_bf16(grow, gp, N - col0, wide);
+        store_row_bf16(grow + N, up, N - col0, wide);
+      }
+    };
+    // the two sides of a rotation, x1 at col0 and x2 half a head further
+    auto finish_rope = [&](const uint32_t (&x1)[32], const uint32_t (&x2)[32], int row, int col0) {
+      const int hd2 = ep.rope_dim / 2, pos = ep.rope_pos != nullptr ? ep.rope_pos[row] : row % ep.rope_s;
+      const long long at = (long long)pos * hd2 + (col0 % ep.rope_dim);
+      uint32_t o1[16], o2[16];
+#pragma unroll
+      for (int i = 0; i < 32; i += 4) {
+        const float4 cs = *reinterpret_cast<const float4*>(ep.rope_cos + at + i);
+        const float4 sn = *reinterpret_cast<const float4*>(ep.rope_sin + at + i);
+        const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+        float a[4], b[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float u = __uint_as_float(x1[i + e]) * ep.alpha, v = __uint_as_float(x2[i + e]) * ep.alpha;
+          a[e] = u * cv[e] - v * sv[e];
+          b[e] = v * cv[e] + u * sv[e];
+        }
+        o1[i / 2] = pack_bf16x2(a[0], a[1]);
+        o1[i / 2 + 1] = pack_bf16x2(a[2], a[3]);
+        o2[i / 2] = pack_bf16x2(b[0], b[1]);
+        o2[i / 2 + 1] = pack_bf16x2(b[2], b[3]);
+      }
+      __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
+      store_row_bf16(crow, o1, N - col0, wide);
+      store_row_bf16(crow + hd2, o2, N - col0 - hd2, wide);
+    };
+    auto finish_plain = [&](const uint32_t (&r)[32], int row, int col0, long long c_row0) {
+      float v[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ep.alpha;
+      if (ep.bias != nullptr) {
+        const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(ep.bias);
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (col0 + i < N) v[i] += __bfloat162float(bias[col0 + i]);
+      }
+      if (ep.rs_rows > 0) {
+        const int owner = row / ep.rs_rows;
+        float* crow = ep.rs_base[owner] + (long long)(row - owner * ep.rs_rows) * ep.ldc + col0;
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          if (col0 + i < N)
+            asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(crow + i), "f"(v[i]),
+                         "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3])
+                         : "memory");
+        }
+      } else if (ep.out_fp32) {
+        float* crow = reinterpret_cast<float*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          if (col0 + i < N) {
+            if (ep.accumulate) {
+              const float4 old = *reinterpret_cast<const float4*>(crow + i);
+              v[i] += old.x; v[i + 1] += old.y; v[i + 2] += old.z; v[i + 3] += old.w;
+            }
+            if (!wide) *reinterpret_cast<float4*>(crow + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+          }
+        }
+        if (wide) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            if (col0 + i < N) stg_v8(crow + i, reinterpret_cast<const uint32_t*>(v + i));
+        }
+      } else {
+        __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
+        if (ep.accumulate || ep.residual != nullptr) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            if (col0 + i < N) {
+              if (ep.accumulate) add_row_bf16(crow + i, v + i);
+              if (ep.residual != nullptr)
+                add_row_bf16(reinterpret_cast<const __nv_bfloat16*>(ep.residual) + (long long)row * ep.ldr + col0 + i,
+                             v + i);
+            }
+          }
+        }
+        uint32_t o[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+        store_row_bf16(crow, o, N - col0, wide);
+      }
+    };
     for (int idx = 0;; ++idx) {
       const int tile = read_tile(idx);
       free_tile_slot(idx);
@@ -580,6 +709,61 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       tc_fence_after();
       const int row = m0 + (int)rank * BM + q * 32 + lane;
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      const bool in = row < m_end;
+      if constexpr (SPLIT == 2) {
+        // 32-column pieces: this CTA finishes four of the eight, 4 part .. 4 part + 3, of gate|up columns two of each. This warp
+        // sends two of the counterpart's and finishes two of its own, the two sides of what belongs together.
+        const bool cross = ep.gated || (ep.rope_cos != nullptr && ep.rope_dim == 128 && n0 + part * 128 < ep.rope_cols);
+        auto piece = [&](int owner, int i) -> int { return ep.gated ? (i >> 1) * 4 + 2 * owner + (i & 1) : 4 * owner + i; };
+        const int first = cross ? half : 2 * half, second = cross ? half + 2 : 2 * half + 1;      // of the four
+        const uint32_t other = cta ^ 2;
+        if (!mbar_wait_cluster(xfree, (local & 1) ^ 1, abort_flag, status)) break;
+        const uint32_t xout = map_to_cta(smem + C::X_OFF, other) + (q * 32 + lane) * 16;
+        uint32_t ra[32], rb[32];
+        tmem_ld_32x32(t_addr + piece(1 - part, first) * 32, ra);
+        tmem_ld_32x32(t_addr + piece(1 - part, second) * 32, rb);
+        tmem_ld_wait();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {      // four columns of 128 rows are 2 KB: lanes write and read 16 bytes side by side
+          st_remote_v4(xout + (first * 8 + k) * BM * 16, ra[4 * k], ra[4 * k + 1], ra[4 * k + 2], ra[4 * k + 3]);
+          st_remote_v4(xout + (second * 8 + k) * BM * 16, rb[4 * k], rb[4 * k + 1], rb[4 * k + 2], rb[4 * k + 3]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(map_to_cta(xfull, other));
+        tmem_ld_32x32(t_addr + piece(part, first) * 32, ra);
+        tmem_ld_32x32(t_addr + piece(part, second) * 32, rb);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(tempty_leader[acc]);
+        if (!mbar_wait_cluster(xfull, local & 1, abort_flag, status)) break;
+        const uint8_t* xin = smem + C::X_OFF + (q * 32 + lane) * 16;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float4 a = *reinterpret_cast<const float4*>(xin + (first * 8 + k) * BM * 16);
+          const float4 b = *reinterpret_cast<const float4*>(xin + (second * 8 + k) * BM * 16);
+          const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            ra[4 * k + e] = __float_as_uint(__uint_as_float(ra[4 * k + e]) + av[e]);
+            rb[4 * k + e] = __float_as_uint(__uint_as_float(rb[4 * k + e]) + bv[e]);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(map_to_cta(xfree, other));
+        ++local;
+        const int col_a = n0 + piece(part, first) * 32, col_b = n0 + piece(part, second) * 32;
+        if (!in) continue;
+        if (ep.gated) {
+          if (col_a < N) finish_gated(ra, rb, row, col_a);
+        } else if (ep.rope_cos != nullptr && col_a < ep.rope_cols) {
+          if (col_a < N) finish_rope(ra, rb, row, col_a);
+        } else {
+          if (col_a < N) finish_plain(ra, row, col_a, c_row0);
+          if (col_b < N) finish_plain(rb, row, col_b, c_row0);
+        }
+        continue;
+      }
       if (ep.gated) {
 #pragma unroll 1
         for (int c = half * (BN / 128); c < (half + 1) * (BN / 128); ++c) {
@@ -587,40 +771,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           tmem_ld_32x32(t_addr + c * 32, g);
           tmem_ld_32x32(t_addr + BN / 2 + c * 32, u);
           tmem_ld_wait();
-          const int col0 = n0 + c * 32;
-          if (row < m_end && col0 < N) {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
-            __nv_bfloat16* grow = ep.gu_out == nullptr ? nullptr
-                : reinterpret_cast<__nv_bfloat16*>(ep.gu_out) + (long long)row * ep.ldgu + col0;
-            uint32_t gp[16], up[16], op[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              // round to bf16 first: the same values and the same formula as the separate SwiGLU kernel
-              gp[j] = pack_bf16x2(__uint_as_float(g[2 * j]), __uint_as_float(g[2 * j + 1]));
-              up[j] = pack_bf16x2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1]));
-              const float2 a = unpack_bf16x2(gp[j]), b = unpack_bf16x2(up[j]);
-              op[j] = pack_bf16x2(a.x / (1.f + __expf(-a.x)) * b.x, a.y / (1.f + __expf(-a.y)) * b.y);
-            }
-            store_row_bf16(crow, op, N - col0, wide);
-            if (grow != nullptr) {
-              store_row_bf16(grow, gp, N - col0, wide);
-              store_row_bf16(grow + N, up, N - col0, wide);
-            }
-          }
+          if (in && n0 + c * 32 < N) finish_gated(g, u, row, n0 + c * 32);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(tempty_leader[acc]);
-        ++local;
-        continue;
-      }
-      if (ep.rope_cos != nullptr && n0 + half * (BN / 2) < ep.rope_cols) {
+      } else if (ep.rope_cos != nullptr && n0 + half * (BN / 2) < ep.rope_cols) {
         // this warp's half of the columns is one head of 128 or two of 64 (launch checks BN == 256): the pieces that
         // hold the two sides of a rotation are loaded together
         const int gap = ep.rope_dim / 64;      // pieces between them: 2 or 1
-        const bool in = row < m_end;
-        const int pos = !in ? 0 : ep.rope_pos != nullptr ? ep.rope_pos[row] : row % ep.rope_s;
-        const int hd2 = ep.rope_dim / 2;
 #pragma unroll 1
         for (int pr = 0; pr < 2; ++pr) {
           const int c = half * (BN / 64) + pr * (gap == 1 ? 2 : 1);     // first piece of the pair
@@ -628,104 +784,20 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           tmem_ld_32x32(t_addr + c * 32, x1);
           tmem_ld_32x32(t_addr + (c + gap) * 32, x2);
           tmem_ld_wait();
-          const int col0 = n0 + c * 32;
-          if (in && col0 < N) {
-            const long long at = (long long)pos * hd2 + (col0 % ep.rope_dim);
-            uint32_t o1[16], o2[16];
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 cs = *reinterpret_cast<const float4*>(ep.rope_cos + at + i);
-              const float4 sn = *reinterpret_cast<const float4*>(ep.rope_sin + at + i);
-              const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
-              float a[4], b[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float u = __uint_as_float(x1[i + e]) * ep.alpha, v = __uint_as_float(x2[i + e]) * ep.alpha;
-                a[e] = u * cv[e] - v * sv[e];
-                b[e] = v * cv[e] + u * sv[e];
-              }
-              o1[i / 2] = pack_bf16x2(a[0], a[1]);
-              o1[i / 2 + 1] = pack_bf16x2(a[2], a[3]);
-              o2[i / 2] = pack_bf16x2(b[0], b[1]);
-              o2[i / 2 + 1] = pack_bf16x2(b[2], b[3]);
-            }
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (long long)row * ep.ldc + col0;
-            store_row_bf16(crow, o1, N - col0, wide);
-            store_row_bf16(crow + hd2, o2, N - col0 - hd2, wide);
-          }
+          if (in && n0 + c * 32 < N) finish_rope(x1, x2, row, n0 + c * 32);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_remote(tempty_leader[acc]);
-        ++local;
-        continue;
-      }
-      constexpr int CH = BN / 64;              // 32-column pieces of this warp's half
-      uint32_t ra[32], rb[32];
-      tmem_ld_32x32(t_addr + half * (BN / 2), ra);
+      } else {
+        constexpr int CH = BN / 64;              // 32-column pieces of this warp's half
+        uint32_t ra[32], rb[32];
+        tmem_ld_32x32(t_addr + half * (BN / 2), ra);
 #pragma unroll
-      for (int cc = 0; cc < CH; ++cc) {
-        const int c = half * CH + cc;
-        uint32_t (&r)[32] = (cc & 1) ? rb : ra;
-        uint32_t (&rn)[32] = (cc & 1) ? ra : rb;
-        tmem_ld_wait();
-        if (cc + 1 < CH) tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
-        const int col0 = n0 + c * 32;
-        if (row < m_end && col0 < N) {
-          float v[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ep.alpha;
-          if (ep.bias != nullptr) {
-            const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(ep.bias);
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col0 + i < N) v[i] += __bfloat162float(bias[col0 + i]);
-          }
-          if (ep.rs_rows > 0) {
-            const int owner = row / ep.rs_rows;
-            float* crow = ep.rs_base[owner] + (long long)(row - owner * ep.rs_rows) * ep.ldc + col0;
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              if (col0 + i < N)
-                asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(crow + i), "f"(v[i]),
-                             "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3])
-                             : "memory");
-            }
-          } else if (ep.out_fp32) {
-            float* crow = reinterpret_cast<float*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              if (col0 + i < N) {
-                if (ep.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(crow + i);
-                  v[i] += old.x; v[i + 1] += old.y; v[i + 2] += old.z; v[i + 3] += old.w;
-                }
-                if (!wide) *reinterpret_cast<float4*>(crow + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-              }
-            }
-            if (wide) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 8)
-                if (col0 + i < N) stg_v8(crow + i, reinterpret_cast<const uint32_t*>(v + i));
-            }
-          } else {
-            __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
-            if (ep.accumulate || ep.residual != nullptr) {
-#pragma unroll
-              for (int i = 0; i < 32; i += 8) {
-                if (col0 + i < N) {
-                  if (ep.accumulate) add_row_bf16(crow + i, v + i);
-                  if (ep.residual != nullptr)
-                    add_row_bf16(reinterpret_cast<const __nv_bfloat16*>(ep.residual) + (long long)row * ep.ldr + col0 + i,
-                                 v + i);
-                }
-              }
-            }
-            uint32_t o[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
-            store_row_bf16(crow, o, N - col0, wide);
-          }
+        for (int cc = 0; cc < CH; ++cc) {
+          const int c = half * CH + cc;
+          uint32_t (&r)[32] = (cc & 1) ? rb : ra;
+          uint32_t (&rn)[32] = (cc & 1) ? ra : rb;
+          tmem_ld_wait();
+          if (cc + 1 < CH) tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
+          if (in && n0 + c * 32 < N) finish_plain(r, row, n0 + c * 32, c_row0);
         }
       }
       tc_fence_before();
@@ -800,10 +872,63 @@ int* sched_counters(cudaStream_t stream) {
   return reinterpret_cast<int*>(p);
 }
 
-template <int BN, bool A_MN, bool B_MN, bool KG = false>
+// Clusters of four CTAs of the split kernel that run at a time (fewer than a quarter of the SMs where a GPC's number of
+// them is no multiple of four); 0 if none. The same for all operand layouts: asked once.
+int split_clusters() {
+  static std::atomic<int> known{-1};
+  int n = known.load(std::memory_order_relaxed);
+  if (n >= 0) return n;
+  auto kern = gemm_bf16_2cta_kernel<256, false, false, false, 2>;
+  constexpr int smem = Cfg<256, 2>::SMEM_TOTAL;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(4 * sm_count(), 1, 1);
+  cfg.blockDim = dim3(THREADS, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 4;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  n = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  known.store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Whether two pairs per tile finish earlier than one, in waves of k-blocks: a wave of half tiles takes a tenth longer per
+// k-block when all SMs load, and the exchange at its end costs as much as 14 k-blocks (4 us). Cold L2, one / two pairs (us), tiles and
+// k-blocks: 8 x 172 61.4 / 41.0; 16 x 86 37.7 / 28.8; 32 x 86 39.6 / 31.5; 96 x 86 71.7 / 63.5; 96 x 172 122.9 / 106.5; about
+// even: 32 x 32 22.5 / 21.3, 96 x 32 36.9 / 36.9; not: 48 x 86 41.0 / 45.1, 172 x 32 49.9 / 56.0, 16 x 8 14.4 / 16.4.
+bool split_pays(int tiles, int kbs, int wish) {
+  if (kbs < 2 || wish < 0) return false;
+  const int pairs = sm_count() / 2;
+  const long long whole = (long long)((tiles + pairs - 1) / pairs) * kbs;
+  auto pays = [&](int clusters) {
+    return clusters > 0 &&
+           (wish > 0 || (long long)((tiles + clusters - 1) / clusters) * ((kbs + 1) / 2) * 110 + 1400 < whole * 95);
+  };
+  return pays(pairs / 2) && pays(split_clusters());      // the second number takes a driver call: only where it can matter
+}
+
+template <int BN, bool A_MN, bool B_MN, bool KG = false, int SPLIT = 1>
 int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, long long lda, long long ldb,
            int max_ctas, const Groups& grp, int b_extent_rows, const Gate& gate, const Ragged& rag, cudaStream_t stream,
            int* status, const KGroups<KG>& kg = KGroups<KG>()) {
+  const int tile_cols = ep.gated ? BN / 2 : BN;
+  int tiles = (rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
+  if constexpr (KG) tiles *= kg.n;
+  if constexpr (SPLIT == 1 && BN == 256 && !KG) {
+    if (rag.n == 0 && grp.counts == nullptr && grp.b_rows == 0 && gate.flags == nullptr && ep.rs_rows <= 0 && max_ctas <= 0 &&
+        split_pays(tiles, (K + BK - 1) / BK, ep.split))
+      return launch<BN, A_MN, B_MN, KG, 2>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent_rows, gate, rag, stream, status,
+                                           kg);
+  }
   CUtensorMap tmA = {}, tmB = {};
   bool ok = true;
   if (KG) {              // a map per group, made by the caller
@@ -827,17 +952,14 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   epw.wide = ep.C != nullptr && ep.rs_rows <= 0 && N % 16 == 0 && (reinterpret_cast<uintptr_t>(ep.C) & 31) == 0 &&
              (ep.ldc * out_bytes) % 32 == 0 &&
              (ep.gu_out == nullptr || ((reinterpret_cast<uintptr_t>(ep.gu_out) & 31) == 0 && (ep.ldgu * 2) % 32 == 0));
-  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, KG>;
-  constexpr int SMEM_TOTAL = Cfg<BN>::SMEM_TOTAL;
+  auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, KG, SPLIT>;
+  constexpr int SMEM_TOTAL = Cfg<BN, SPLIT>::SMEM_TOTAL;
   static bool attr_set = false;
   if (!attr_set) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_TOTAL) != cudaSuccess) return -4;
     attr_set = true;
   }
-  const int tile_cols = ep.gated ? BN / 2 : BN;
-  int tiles = (rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM)) * ((N + tile_cols - 1) / tile_cols);
-  if constexpr (KG) tiles *= kg.n;
-  int clusters = sm_count() / 2;
+  int clusters = SPLIT == 2 ? split_clusters() : sm_count() / 2;
   if (tiles < clusters) clusters = tiles;
   if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   // dynamic tile scheduling for plain launches with more tiles than CTA pairs (see Sched)
@@ -846,17 +968,17 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     const char* e = getenv("ATB_GEMM_DYNAMIC");
     g_dynamic = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
-  if (g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
+  if (SPLIT == 1 && g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
       gate.flags == nullptr)
     sched.counters = sched_counters(stream);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * clusters, 1, 1);
+  cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
   cfg.blockDim = dim3(THREADS, 1, 1);
   cfg.dynamicSmemBytes = SMEM_TOTAL;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = 2 * SPLIT;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -924,6 +1046,7 @@ extern "C" int atb_gemm_bf16_2cta_grouped(const void* A, const void* B, void* C,
   // 9 % (333 rows, o: 22.5 / 20.5; 777 rows, dgrad of gate|up: 65.5 / 59.6), and not in weight gradients. It stays
   // selectable with tile_n = 128.
   const bool narrow = tile_n == 128;
+  ep.split = tile_n == 256 ? -1 : tile_n == 512 ? 1 : 0;
 #define ATB_PAIR_DISPATCH(BN_)                                                                                     \
   do {                                                                                                             \
     if (!a_mn_major && !b_mn_major)                                                                                \

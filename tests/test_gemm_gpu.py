@@ -587,3 +587,48 @@ def test_gemm_k_groups_accumulates_in_bf16(sizes, M, N):
         ref = before[g].double() + a[r: r + n].double().t() @ b[r: r + n].double()
         assert torch.equal(out[g], before[g]) if n == 0 else (out[g].double() - ref).norm() <= 2 ** -8 * ref.norm()
         r += n
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 128), (264, 264, 136), (8, 520, 1000), (1000, 2056, 192), (2560, 2560, 200)])
+def test_gemm_two_pairs_per_tile(M, N, K, a_mn, b_mn):
+    """A cluster of four CTAs per tile (tile_n = 512): the two halves of the reduction (unequal ones, of a single k-block, with a
+    ragged end), more tiles than clusters, edges of rows and columns, every kind of output."""
+    torch.manual_seed(M + N + K)
+    a = _mk(K, M) if a_mn else _mk(M, K)
+    b = _mk(K, N) if b_mn else _mk(N, K)
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double()
+    bias, res, c0 = _mk(1, N)[0], _mk(M, N), torch.randn(M, N, device="cuda")
+    got = gemm(a, b, a_mn, b_mn, tile_n=512, kernel="2cta")
+    both = gemm(a, b, a_mn, b_mn, tile_n=512, kernel="2cta", bias=bias, residual=res, alpha=0.5)
+    acc = gemm(a, b, a_mn, b_mn, tile_n=512, kernel="2cta", out=c0.clone(), accumulate=True)
+    torch.cuda.synchronize()
+    _lib.check_status(a.device)
+    for out, want, tol in ((got, ref, 2 ** -9), (both, 0.5 * ref + bias.double() + res.double(), 2 ** -9),   # one rounding to bf16
+                           (acc, c0.double() + ref, 1e-5)):
+        assert (out.double() - want).norm() <= tol * want.norm()
+
+
+@pytest.mark.parametrize("T", [300, 512])
+def test_fused_epilogues_with_two_pairs_per_tile(T):
+    """SwiGLU and rotary epilogues on products of few tiles and a long reduction, which the rule gives two pairs per tile: gate
+    and up, and the two sides of a rotation, meet in one thread again (heads of 128 and 64, columns that are not rotated, an
+    edge inside a tile)."""
+    from atorch_b200.ops import linear_rope, linear_swiglu
+    from atorch_b200.ops.elementwise import rope_reference, rope_tables
+
+    torch.manual_seed(T)
+    K = 6144
+    x, w = _mk(T, K), _mk(2 * 200, K) * 0.02
+    g, u = (x.double() @ w.double().t()).to(torch.bfloat16).double().chunk(2, -1)
+    act = linear_swiglu(x, w)
+    want = torch.nn.functional.silu(g) * u
+    assert (act.double() - want).norm() <= 2 ** -7 * want.norm()          # gate, up and the result are rounded to bf16
+    for heads, kv, D in ((3, 2, 128), (4, 4, 64)):
+        cos, sin = rope_tables(T, D, device="cuda")
+        wq = _mk((heads + kv) * D, K) * 0.02
+        got = linear_rope(x, wq, cos, sin, heads, D)
+        want = rope_reference((x.double() @ wq.double().t()).float(), cos, sin, heads, D)
+        torch.cuda.synchronize()
+        _lib.check_status(x.device)
+        assert (got.float() - want).norm() <= 2 ** -8 * want.norm()
