@@ -51,9 +51,12 @@ struct Cfg {
   static constexpr int STAGES = SPLIT == 2 ? 5 : BN == 256 ? 6 : 8;
   static constexpr int B_BYTES = BNH * BK * 2;
   static constexpr int X_OFF = STAGES * (A_BYTES + B_BYTES);         // partial sums from the other pair, fp32
-  static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 0);
+  // output boxes on their way out (see the epilogue): 4 KB per epilogue warp, [32 rows][128 bytes] with 128-byte swizzle
+  static constexpr int OUT_OFF = X_OFF;
+  static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 8 * 4096);
   static constexpr int TQ = 4;                     // tile-id ring of the dynamic scheduler
-  static constexpr int SMEM_TOTAL = BAR_OFF + (2 * STAGES + 4 + 2 * TQ + 2) * 8 + 16 + TQ * 4 + 1024;
+  static constexpr int SMEM_TOTAL = BAR_OFF + (2 * STAGES + 4 + 2 * TQ + 3) * 8 + 16 + TQ * 4 + 1024;
+  static_assert(SMEM_TOTAL <= 232448, "shared memory of the pair kernel exceeds 227 KB");
 };
 
 struct Epi {
@@ -83,6 +86,7 @@ struct Epi {
   const int* rope_pos;
   int rope_s, rope_dim, rope_cols;
   int split;  // (host) pairs per tile: 0 by split_pays, -1 one, 1 two wherever the kernel can
+  int boxed;  // nothing but a rounding to bf16 on the way out, and a tensor map for it (set by launch)
   int wide;   // every 16 columns of an output row start on a 32-byte boundary and N is a multiple of 16 (set by launch)
 };
 
@@ -188,14 +192,22 @@ struct KGroups<true> {
   int n;
 };
 
+template <bool KG>
+uint64_t kg_count(const KGroups<KG>& kg) {
+  if constexpr (KG) return kg.n;
+  return 1;
+}
+
 ATB_DEVICE uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+ATB_DEVICE void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+ATB_DEVICE void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 ATB_DEVICE void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive_all();
+  cluster_wait_all();
 }
 // shared::cluster address of `ptr` (a shared::cta pointer of this CTA) in CTA `rank` of the cluster
 ATB_DEVICE uint32_t map_to_cta(const void* ptr, uint32_t rank) {
@@ -271,7 +283,8 @@ constexpr int THREADS = 64 + 32 * EPI_WARPS;
 
 template <int BN, bool A_MN, bool B_MN, bool KG, int SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Epi ep, int M,
+gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, Epi ep, int M,
                       int N, int K, Groups grp, Gate gate, Sched sched, const __grid_constant__ Ragged rag,
                       const __grid_constant__ KGroups<KG> kg, int* status) {
   static_assert(!KG || (A_MN && B_MN), "groups along the reduction are rows of MN-major operands");
@@ -291,7 +304,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   uint64_t* tq_empty = tq_full + TQ;
   uint64_t* xfull = tq_empty + TQ;        // partial sums of the other pair are in the exchange buffer
   uint64_t* xfree = xfull + 1;            // the other pair has read those sent to it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xfree + 1);
+  uint64_t* tmem_ready = xfree + 1;       // tensor memory has been allocated
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_ready + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* tq_tile = reinterpret_cast<volatile int*>(tmem_slot + 4);   // [TQ] tile ids (-1: no more tiles)
 
@@ -300,15 +314,13 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t rank = cta & 1, pair0 = cta & ~1u;     // place in the pair; the pair's first CTA in the cluster
   const int part = SPLIT == 2 ? (int)(cta >> 1) : 0;    // which half of the reduction and of the columns
   const bool leader = rank == 0;
-  // both CTAs of a pair read the same word, so they take the same decision
-  const bool skip = warp_uniform((int)(status != nullptr && *reinterpret_cast<volatile int*>(status) != 0)) != 0;
-
+  // all CTAs of a cluster read the same word, so they take the same decision (on its way while the barriers are set up)
+  const int stopped = status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
   const int tiles_m = rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM);
   const int tile_cols = ep.gated ? BN / 2 : BN;      // output columns per tile
   const int tiles_n = (N + tile_cols - 1) / tile_cols;
   int groups = 1;
   if constexpr (KG) groups = kg.n;
-  const int num_tiles = skip ? 0 : tiles_m * tiles_n * groups;
   // k-blocks [first, end) of a tile for this pair
   auto tile_kbs = [&](int b_idx, int& first) -> int {
     first = 0;
@@ -323,24 +335,32 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int cluster_id = blockIdx.x / (2 * SPLIT), num_clusters = gridDim.x / (2 * SPLIT);
   constexpr int BAND = 8;
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 1);
+  // What every role waits for is the barriers of all CTAs of the cluster, so they come first, and the wait for them last: the
+  // allocation of tensor memory and the coordinates of the first tile lie between arriving and waiting. One after the other
+  // the first load went out 4060 clocks after the start of a CTA, now 3140.
+  if (warp == 2) {
+    if (lane == 0) {
+      for (int i = 0; i < STAGES; ++i) {
+        mbar_init(&full[i], 1);
+        mbar_init(&empty[i], 1);
+      }
+      mbar_init(&tfull[0], 1);
+      mbar_init(&tfull[1], 1);
+      mbar_init(&tempty[0], 2 * EPI_WARPS);
+      mbar_init(&tempty[1], 2 * EPI_WARPS);
+      for (int i = 0; i < TQ; ++i) {
+        mbar_init(&tq_full[i], 1);
+        mbar_init(&tq_empty[i], 2 + 2 * EPI_WARPS);   // leader: MMA + epilogue warps; partner: producer + epilogue warps
+      }
+      mbar_init(xfull, EPI_WARPS);
+      mbar_init(xfree, EPI_WARPS);
+      mbar_init(tmem_ready, 1);
+      *abort_flag = 0;
+      mbar_fence_init();
     }
-    mbar_init(&tfull[0], 1);
-    mbar_init(&tfull[1], 1);
-    mbar_init(&tempty[0], 2 * EPI_WARPS);
-    mbar_init(&tempty[1], 2 * EPI_WARPS);
-    for (int i = 0; i < TQ; ++i) {
-      mbar_init(&tq_full[i], 1);
-      mbar_init(&tq_empty[i], 2 + 2 * EPI_WARPS);   // leader: MMA + epilogue warps; partner: producer + epilogue warps
-    }
-    mbar_init(xfull, EPI_WARPS);
-    mbar_init(xfree, EPI_WARPS);
-    *abort_flag = 0;
-    mbar_fence_init();
+    __syncwarp();
   }
+  cluster_arrive_all();
   if (!KG && warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -348,11 +368,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   if (warp == 1) {
     tmem_alloc<2>(tmem_slot, 2 * BN);
     tmem_relinquish<2>();
+    tc_fence_before();
   }
-  tc_fence_before();
-  cluster_sync_all();  // barriers of both CTAs initialised and visible before any remote arrive
-  tc_fence_after();
-  const uint32_t tmem_base = warp_uniform(*tmem_slot);
+  const int num_tiles = warp_uniform(stopped) != 0 ? 0 : tiles_m * tiles_n * groups;
 
   // identical decisions in every role: which tiles and which k-blocks carry data
   auto tile_active = [&](int m0, int b_idx) -> bool {
@@ -452,10 +470,22 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         return warp_uniform(d);
       };
       int drawn = (dyn && leader) ? draw() : 0;
+      // the first tile, as far as it is known without the cluster
+      int tile = dyn ? (leader && drawn < num_tiles ? drawn : -1) : static_tile(0);
+      int m0 = 0, n0 = 0, m_end = 0, b_idx = 0;
+      if (tile >= 0) tile_coords(tile, m0, n0, m_end, b_idx);
+      cluster_wait_all();
       for (int idx = 0;; ++idx) {
-        int tile;
+        if (idx > 0 || (dyn && !leader)) {
+          if (dyn && leader) {
+            tile = drawn < num_tiles ? drawn : -1;
+          } else {
+            tile = read_tile(idx);
+            free_tile_slot(idx);
+          }
+          if (tile >= 0) tile_coords(tile, m0, n0, m_end, b_idx);
+        }
         if (dyn && leader) {
-          tile = drawn < num_tiles ? drawn : -1;
           if (tile >= 0) drawn = draw();                       // the next one, fetched under this tile's loads
           if (!publish_tile(idx, tile)) goto producer_done;
           if (tile < 0 && lane == 0) {   // every pair draws exactly one number past the end; the last to do so resets
@@ -465,13 +495,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
               __threadfence();
             }
           }
-        } else {
-          tile = read_tile(idx);
-          free_tile_slot(idx);
         }
         if (tile < 0) break;
-        int m0, n0, m_end, b_idx;
-        tile_coords(tile, m0, n0, m_end, b_idx);
         if (!tile_active(m0, b_idx)) continue;
         int kb_first;
         const int kb_end = tile_kbs(b_idx, kb_first);
@@ -522,6 +547,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   producer_done:;
   } else if (warp == 1) {
+    cluster_wait_all();
+    tc_fence_after();
+    const uint32_t tmem_base = warp_uniform(*tmem_slot);
+    if (lane == 0) mbar_arrive(tmem_ready);
     if (leader) {
       const uint32_t el = elect_one();      // the lane that issues and commits
       const uint32_t a_desc = umma_desc_lo(smem_u32(sA), A_MN ? 8192 : 16), b_desc = umma_desc_lo(smem_u32(sB), B_MN ? 8192 : 16);
@@ -570,8 +599,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   mma_done:;
   } else {
+    cluster_wait_all();
     const int q = warp & 3;                 // lane quarter
     const int half = (warp - 2) >> 2;       // column half
+    const bool have_tmem = mbar_wait_warp(tmem_ready, 0, abort_flag, status);
+    tc_fence_after();
+    const uint32_t tmem_base = warp_uniform(*tmem_slot);
     const bool wide = ep.wide != 0;
     int local = 0;
     const uint32_t tempty_leader[2] = {map_to_cta(&tempty[0], pair0), map_to_cta(&tempty[1], pair0)};
@@ -622,7 +655,19 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       store_row_bf16(crow, o1, N - col0, wide);
       store_row_bf16(crow + hd2, o2, N - col0 - hd2, wide);
     };
-    auto finish_plain = [&](const uint32_t (&r)[32], int row, int col0, long long c_row0) {
+    // 32 bf16 values that are added to a row's accumulators, the residual or, when accumulating, the output so far, in four loads
+    // at once; with a test of the column around each, they came one after the other, 16 times the latency of the L2 per tile
+    // (not in the grouped weight gradients, which the registers for it made 1.5 % slower)
+    const __nv_bfloat16* added = KG ? nullptr : ep.residual != nullptr ? reinterpret_cast<const __nv_bfloat16*>(ep.residual)
+                                 : ep.accumulate && !ep.out_fp32 ? reinterpret_cast<const __nv_bfloat16*>(ep.C) : nullptr;
+    const long long added_ld = ep.residual != nullptr ? ep.ldr : ep.ldc;
+    auto fetch = [&](uint4 (&x)[4], long long row, int col0) {
+      const uint4* p = reinterpret_cast<const uint4*>(added + row * added_ld + col0);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = p[i];
+    };
+    // x: as fetched, if `fetched` (whole pieces)
+    auto finish_plain = [&](const uint32_t (&r)[32], int row, int col0, long long c_row0, const uint4 (&x)[4], bool fetched) {
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ep.alpha;
@@ -661,12 +706,25 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       } else {
         __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
-        if (ep.accumulate || ep.residual != nullptr) {
+        if (fetched) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float2 f = unpack_bf16x2(w[k]);
+              v[8 * i + 2 * k] += f.x;
+              v[8 * i + 2 * k + 1] += f.y;
+            }
+          }
+        }
+        const bool more = ep.accumulate && ep.residual != nullptr;      // both: the second one here
+        if (more || ((ep.accumulate || ep.residual != nullptr) && !fetched)) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             if (col0 + i < N) {
               if (ep.accumulate) add_row_bf16(crow + i, v + i);
-              if (ep.residual != nullptr)
+              if (ep.residual != nullptr && !fetched)
                 add_row_bf16(reinterpret_cast<const __nv_bfloat16*>(ep.residual) + (long long)row * ep.ldr + col0 + i,
                              v + i);
             }
@@ -678,10 +736,15 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         store_row_bf16(crow, o, N - col0, wide);
       }
     };
-    for (int idx = 0;; ++idx) {
-      const int tile = read_tile(idx);
-      free_tile_slot(idx);
-      if (tile < 0) break;
+    int next = -1;
+    if (have_tmem) {
+      next = read_tile(0);
+      free_tile_slot(0);
+    }
+    for (int idx = 0; next >= 0; ++idx) {
+      const int tile = next;
+      next = read_tile(idx + 1);      // known by the time this tile's accumulators are: the producer is past its loads
+      free_tile_slot(idx + 1);
       int m0, n0, m_end, b_idx;
       tile_coords(tile, m0, n0, m_end, b_idx);
       const long long c_row0 = KG ? (long long)b_idx * M : 0;      // this group's rows of C
@@ -705,11 +768,53 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
       const int acc = local & 1;
       const uint32_t acc_ph = (local >> 1) & 1;
+      const int row = m0 + (int)rank * BM + q * 32 + lane;
+      const bool fetching = added != nullptr && row < m_end;
+      uint4 xa[4], xb[4];
+      if (SPLIT == 1 && fetching && n0 + half * (BN / 2) + 32 <= N) fetch(xa, c_row0 + row, n0 + half * (BN / 2));
       if (!mbar_wait_warp(&tfull[acc], acc_ph, abort_flag, status)) break;
       tc_fence_after();
-      const int row = m0 + (int)rank * BM + q * 32 + lane;
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       const bool in = row < m_end;
+      const int row0 = m0 + (int)rank * BM + q * 32;      // first of this warp's rows
+      // The last tile's epilogue is exposed in full: boxes of 32 rows x 64 columns go through shared memory (swizzled, no bank
+      // conflicts) and the TMA unit. 512 x 512 x 512: 11.6 -> 10.3 us, 2048 x 2048 x 4096 weight gradient 30.8 -> 28.8. Earlier tiles keep to direct stores: the operands of the
+      // products that run beside them take the whole bandwidth of shared memory.
+      if (SPLIT == 1 && ep.boxed != 0 && next < 0 && row0 + 32 <= m_end && n0 + (half + 1) * (BN / 2) <= N) {
+        uint8_t* box = smem + C::OUT_OFF + (warp - 2) * 4096;
+#pragma unroll 1
+        for (int e = 0; e < BN / 128; ++e) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(t_addr + half * (BN / 2) + e * 64, r0);
+          tmem_ld_32x32(t_addr + half * (BN / 2) + e * 64 + 32, r1);
+          tmem_ld_wait();
+          if (e > 0) {                   // the box before has been read
+            if (lane == 0) tma_store_wait_read<0>();
+            __syncwarp();
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint32_t (&r)[32] = i < 4 ? r0 : r1;
+            const int k = (i & 3) * 8;
+            uint4 o;
+            o.x = pack_bf16x2(__uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+            o.y = pack_bf16x2(__uint_as_float(r[k + 2]), __uint_as_float(r[k + 3]));
+            o.z = pack_bf16x2(__uint_as_float(r[k + 4]), __uint_as_float(r[k + 5]));
+            o.w = pack_bf16x2(__uint_as_float(r[k + 6]), __uint_as_float(r[k + 7]));
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((i ^ (lane & 7)) << 4)) = o;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tmC, box, n0 + half * (BN / 2) + e * 64, (int)(c_row0 + row0));
+            tma_store_commit();
+          }
+        }
+        if (lane == 0) tma_store_wait_read<0>();      // shared memory has to outlive its readers
+        tc_fence_before();
+        __syncwarp();
+        break;
+      }
       if constexpr (SPLIT == 2) {
         // 32-column pieces: this CTA finishes four of the eight, 4 part .. 4 part + 3, of gate|up columns two of each. This warp
         // sends two of the counterpart's and finishes two of its own, the two sides of what belongs together.
@@ -736,6 +841,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(tempty_leader[acc]);
+        const int col_a = n0 + piece(part, first) * 32, col_b = n0 + piece(part, second) * 32;
+        if (fetching && col_a + 32 <= N) fetch(xa, c_row0 + row, col_a);
+        if (fetching && col_b + 32 <= N) fetch(xb, c_row0 + row, col_b);
         if (!mbar_wait_cluster(xfull, local & 1, abort_flag, status)) break;
         const uint8_t* xin = smem + C::X_OFF + (q * 32 + lane) * 16;
 #pragma unroll
@@ -752,15 +860,14 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(map_to_cta(xfree, other));
         ++local;
-        const int col_a = n0 + piece(part, first) * 32, col_b = n0 + piece(part, second) * 32;
         if (!in) continue;
         if (ep.gated) {
           if (col_a < N) finish_gated(ra, rb, row, col_a);
         } else if (ep.rope_cos != nullptr && col_a < ep.rope_cols) {
           if (col_a < N) finish_rope(ra, rb, row, col_a);
         } else {
-          if (col_a < N) finish_plain(ra, row, col_a, c_row0);
-          if (col_b < N) finish_plain(rb, row, col_b, c_row0);
+          if (col_a < N) finish_plain(ra, row, col_a, c_row0, xa, fetching && col_a + 32 <= N);
+          if (col_b < N) finish_plain(rb, row, col_b, c_row0, xb, fetching && col_b + 32 <= N);
         }
         continue;
       }
@@ -796,8 +903,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           uint32_t (&r)[32] = (cc & 1) ? rb : ra;
           uint32_t (&rn)[32] = (cc & 1) ? ra : rb;
           tmem_ld_wait();
-          if (cc + 1 < CH) tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
-          if (in && n0 + c * 32 < N) finish_plain(r, row, n0 + c * 32, c_row0);
+          if (cc + 1 < CH) {
+            tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
+            if (fetching && n0 + (c + 2) * 32 <= N) fetch((cc & 1) ? xa : xb, c_row0 + row, n0 + (c + 1) * 32);
+          }
+          if (in && n0 + c * 32 < N)
+            finish_plain(r, row, n0 + c * 32, c_row0, (cc & 1) ? xb : xa, fetching && n0 + (c + 1) * 32 <= N);
         }
       }
       tc_fence_before();
@@ -818,7 +929,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc<2>(tmem_base, 2 * BN);
+    tmem_dealloc<2>(warp_uniform(*tmem_slot), 2 * BN);
   }
 }
 
@@ -929,7 +1040,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
       return launch<BN, A_MN, B_MN, KG, 2>(A, B, ep, M, N, K, lda, ldb, max_ctas, grp, b_extent_rows, gate, rag, stream, status,
                                            kg);
   }
-  CUtensorMap tmA = {}, tmB = {};
+  CUtensorMap tmA = {}, tmB = {}, tmC = {};
   bool ok = true;
   if (KG) {              // a map per group, made by the caller
   } else if (!A_MN)
@@ -952,6 +1063,10 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   epw.wide = ep.C != nullptr && ep.rs_rows <= 0 && N % 16 == 0 && (reinterpret_cast<uintptr_t>(ep.C) & 31) == 0 &&
              (ep.ldc * out_bytes) % 32 == 0 &&
              (ep.gu_out == nullptr || ((reinterpret_cast<uintptr_t>(ep.gu_out) & 31) == 0 && (ep.ldgu * 2) % 32 == 0));
+  epw.boxed = SPLIT == 1 && ep.C != nullptr && ep.rs_rows <= 0 && ep.bias == nullptr && ep.residual == nullptr && !ep.accumulate &&
+              !ep.out_fp32 && ep.alpha == 1.f && !ep.gated && ep.rope_cos == nullptr &&
+              make_tmap_2d(&tmC, ep.C, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M * kg_count(kg), N, ep.ldc, 32, 64,
+                           CU_TENSOR_MAP_SWIZZLE_128B);
   auto kern = gemm_bf16_2cta_kernel<BN, A_MN, B_MN, KG, SPLIT>;
   constexpr int SMEM_TOTAL = Cfg<BN, SPLIT>::SMEM_TOTAL;
   static bool attr_set = false;
@@ -983,7 +1098,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, epw, M, N, K, grp, gate, sched, rag, kg, status);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, epw, M, N, K, grp, gate, sched, rag, kg, status);
   return e == cudaSuccess ? 0 : -5;
 }
 
