@@ -356,6 +356,19 @@ template <int N>
 ATB_DEVICE void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ----------------------------------------------------------------------------------
+// Launches that overlap the end of the kernel before them (programmatic dependent launch)
+// ----------------------------------------------------------------------------------
+// grid_go(): the next launch of the stream, if it is made by launch_after(), may take the SMs that become free from here on.
+// grid_wait(): the kernels before have completed and their writes are visible. A kernel launched by launch_after() waits in
+// every thread that touches device memory, before it does, on every path: barriers, tensor memory and tensor maps are set up
+// before it, under the last blocks of the kernel in front. Its inputs must not be read through the read-only path (const
+// __restrict__ pointers, which promise that nobody writes while the kernel runs), so the kernels that use it only say
+// grid_go(). The gap between two kernels was 1.9 us. Loss of 8 layers of a 1.3B model on 777 tokens (68 launches) 1479 -> 1444 us,
+// forward and backward of one layer on 3000 tokens (23) 1073 -> 1049, a training step of 8 layers of it (286) 18687 -> 18431.
+ATB_DEVICE void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+ATB_DEVICE void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------------
 // small helpers
 // ----------------------------------------------------------------------------------
 ATB_DEVICE float warp_sum(float v) {
@@ -572,7 +585,29 @@ ATB_DEVICE __half from_f32<__half>(float v) { return __float2half_rn(v); }
 // Host-side: encode a 2-D tiled tensor map through the driver entry point (no libcuda link).
 #include <mutex>
 #include <cstdio>
+#include <utility>
 namespace atb {
+// Launch that may start before the kernel in front has ended (see grid_wait), in clusters of `cluster` CTAs.
+template <typename... P, typename... A>
+inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, int cluster,
+                                A&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(CE_NT) ce_fwd_kernel(const T* __restrict__ log
                                                        float* __restrict__ sum_logits_out, int V, long long stride,
                                                        int vocab_start, long long v_total, long long ignore_index,
                                                        float smoothing, float z_scale) {
+  grid_go();
   __shared__ float red[33];
   const long long row = blockIdx.x;
   const T* x = logits + row * stride;
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(CE_NT) ce_bwd_kernel(const T* __restrict__ log
                                                        float grad_scalar, T* __restrict__ dlogits, int V,
                                                        long long stride, int vocab_start, long long v_total,
                                                        long long ignore_index, float smoothing, float z_scale) {
+  grid_go();
   const long long row = blockIdx.x;
   const T* x = logits + row * stride;
   T* dx = dlogits + row * stride;

@@ -21,6 +21,7 @@ __global__ void rope_kernel(__nv_bfloat16* x, const __nv_bfloat16* src,
                             const float* __restrict__ cosT, const float* __restrict__ sinT,
                             const int* __restrict__ pos, long long T, int S, int nheads, int D, long long row_stride,
                             long long src_stride, int tail8, float sign) {
+  grid_go();
   const int half = D >> 1;
   const int vec_per_head = half >> 3;  // 8 bf16 per 16-byte vector
   const long long total = T * (long long)nheads * vec_per_head;
@@ -70,6 +71,7 @@ __global__ void rope_kernel(__nv_bfloat16* x, const __nv_bfloat16* src,
 // out[t, f] = silu(gu[t, f]) * gu[t, F + f]
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T,
                                   int F, long long gu_stride, long long out_stride) {
+  grid_go();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -97,6 +99,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int F, long long gu_stride,
                                   long long dout_stride) {
+  grid_go();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;

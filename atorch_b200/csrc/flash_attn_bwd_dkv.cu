@@ -107,7 +107,10 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) {
+    grid_wait();
+    return;
+  }
   const int shift = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {
@@ -128,6 +131,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     queue_init(queue, 2 + N_EW / 32);
     *abort_flag = 0;
     mbar_fence_init();
+    grid_go();
   }
   if (warp == 1) {
     tmem_alloc<1>(tmem_slot, 512);
@@ -136,6 +140,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_wait();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   // Units of this CTA, one after another: key block w.place (the first is the heaviest) of head w.head of the results and
   // sample w.sample, query blocks [w.v0, w.v0 + w.v1). Block i of a unit: query block v0 + i % v1 of query head
@@ -470,8 +475,7 @@ int launch_dkv(const void* dout, const void* q, const void* k, const void* v, Dk
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sk + BKV - 1) / BKV, p.Hq / p.fold, p.B, p.causal != 0, p.Sq, HD);
-  flash_bwd_dkv_kernel<HD><<<grid, THREADS, SmemK<HD>::TOTAL, stream>>>(tmQ, tmdO, tmK, tmV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return launch_after(flash_bwd_dkv_kernel<HD>, grid, THREADS, SmemK<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p) == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

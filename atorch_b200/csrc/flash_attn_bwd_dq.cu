@@ -94,7 +94,10 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) {
+    grid_wait();
+    return;
+  }
   const int shift = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {
@@ -112,6 +115,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     queue_init(queue, 2 + N_EW / 32);
     *abort_flag = 0;
     mbar_fence_init();
+    grid_go();
   }
   if (warp == 1) {
     tmem_alloc<1>(tmem_slot, 512);
@@ -120,6 +124,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_wait();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
   const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdQ = tmem_base + 384;   // dP buffer of block g at tdP + 128*(g&1)
 
@@ -445,8 +450,7 @@ int launch_dq(const void* dout, const void* q, const void* k, const void* v, DqP
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sq + BQ - 1) / BQ, p.Hq, p.B, p.causal != 0, p.Sk, HD);
-  flash_bwd_dq_kernel<HD><<<grid, THREADS, SmemQ<HD>::TOTAL, stream>>>(tmQ, tmdO, tmK, tmV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return launch_after(flash_bwd_dq_kernel<HD>, grid, THREADS, SmemQ<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p) == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

@@ -132,8 +132,12 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) {
+    grid_wait();
+    return;
+  }
   if (p.holes != nullptr) {
+    grid_wait();
     int any = 0;
     for (int i = threadIdx.x; i < p.B; i += THREADS) any |= p.holes[i];
     if (__syncthreads_or(any)) return;
@@ -152,11 +156,13 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     queue_init(queue, 2 + 8);
     *abort_flag = 0;
     mbar_fence_init();
+    grid_go();
   }
   if (warp == 1) { tmem_alloc<1>(tmem_slot, 512); tmem_relinquish<1>(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_wait();
   const uint32_t tmem_base = warp_uniform(*tmem_slot);
 
   // Units of this CTA, one after another: 256 query rows w.place of head w.head and sample w.sample, w.v1 (w.v2) K/V tiles
@@ -466,8 +472,7 @@ int launch_fwd2(const void* q, const void* k, const void* v, Params p, long long
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B, p.causal != 0, p.Sk, HD);
-  flash_fwd2_kernel<HD><<<grid, THREADS, L2<HD>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -5;
+  return launch_after(flash_fwd2_kernel<HD>, grid, THREADS, L2<HD>::TOTAL, stream, 1, tmQ, tmK, tmV, p) == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

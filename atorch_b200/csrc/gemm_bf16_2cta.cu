@@ -361,6 +361,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     __syncwarp();
   }
   cluster_arrive_all();
+  // A launch that waits for other ranks keeps the SMs that it was told to leave free for the transfer.
+  if (threadIdx.x == 0 && gate.flags == nullptr) grid_go();
   if (!KG && warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -469,6 +471,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         if (lane == 0) d = atomicAdd(&sched.counters[0], 1);
         return warp_uniform(d);
       };
+      grid_wait();
       int drawn = (dyn && leader) ? draw() : 0;
       // the first tile, as far as it is known without the cluster
       int tile = dyn ? (leader && drawn < num_tiles ? drawn : -1) : static_tile(0);
@@ -552,6 +555,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const uint32_t tmem_base = warp_uniform(*tmem_slot);
     if (lane == 0) mbar_arrive(tmem_ready);
     if (leader) {
+      grid_wait();                          // counts of rows lie in device memory; a wait with a limit starts when work can
       const uint32_t el = elect_one();      // the lane that issues and commits
       const uint32_t a_desc = umma_desc_lo(smem_u32(sA), A_MN ? 8192 : 16), b_desc = umma_desc_lo(smem_u32(sB), B_MN ? 8192 : 16);
       const uint32_t empty0 = map_to_cta(empty, pair0), empty1 = map_to_cta(empty, pair0 + 1);
@@ -602,6 +606,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     cluster_wait_all();
     const int q = warp & 3;                 // lane quarter
     const int half = (warp - 2) >> 2;       // column half
+    grid_wait();
     const bool have_tmem = mbar_wait_warp(tmem_ready, 0, abort_flag, status);
     tc_fence_after();
     const uint32_t tmem_base = warp_uniform(*tmem_slot);
@@ -1086,19 +1091,8 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   if (SPLIT == 1 && g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
       gate.flags == nullptr)
     sched.counters = sched_counters(stream);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * SPLIT * clusters, 1, 1);
-  cfg.blockDim = dim3(THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SMEM_TOTAL;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2 * SPLIT;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmC, epw, M, N, K, grp, gate, sched, rag, kg, status);
+  const cudaError_t e = launch_after(kern, dim3(2 * SPLIT * clusters), THREADS, SMEM_TOTAL, stream, 2 * SPLIT, tmA, tmB, tmC, epw, M,
+                                     N, K, grp, gate, sched, rag, kg, status);
   return e == cudaSuccess ? 0 : -5;
 }
 

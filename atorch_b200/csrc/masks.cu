@@ -21,6 +21,7 @@ ATB_DEVICE long long ld_index(const void* p, int is64, long long i) {
 __global__ void __launch_bounds__(256) row_intervals_kernel(int* __restrict__ row_lo, int* __restrict__ row_hi,
                                                             int* __restrict__ holes, int Sq, int Sk, int causal_like,
                                                             MaskArgs m) {
+  grid_go();
   __shared__ int s_cnt, s_first, s_last;
   const int b = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x;
   if (m.keys != nullptr) {

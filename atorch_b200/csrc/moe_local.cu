@@ -27,6 +27,7 @@ __global__ void invert_perm_kernel(const long long* __restrict__ order, int* __r
 __global__ void __launch_bounds__(256) gather_sum_kernel(const __nv_bfloat16* __restrict__ src,
                                                          const int* __restrict__ slot_of, const void* __restrict__ w,
                                                          int w_dtype, __nv_bfloat16* __restrict__ out, int k, int H) {
+  grid_go();
   const long long t = blockIdx.x;
   for (int c = threadIdx.x; c < H / 8; c += 256) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256) ungather_kernel(const __nv_bfloat16* __re
                                                        const long long* __restrict__ order, const void* __restrict__ w,
                                                        int w_dtype, __nv_bfloat16* __restrict__ dsrc,
                                                        void* __restrict__ dw, int k, int H) {
+  grid_go();
   __shared__ float red[33];
   const long long s = order[blockIdx.x];
   if (s < 0 || s >= (long long)gridDim.x) return;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(1024) route_kernel(const long long* __restrict
 
 __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ src, const long long* __restrict__ order,
                                                           uint4* __restrict__ out, int k, int pieces) {
+  grid_go();
   const long long s = order[blockIdx.x] / k;
   for (int c = threadIdx.x; c < pieces; c += 256) out[(long long)blockIdx.x * pieces + c] = src[s * pieces + c];
 }

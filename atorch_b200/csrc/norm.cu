@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(NT, (VPT <= 2 && !LN) ? 4 : 1) norm_fwd_kernel
                                                       T* __restrict__ y, T* __restrict__ sum_out,
                                                       float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                       int M, int N, float eps) {
+  grid_go();
   __shared__ float red[33];
   const int nvec = N >> 3;
   float wv[VPT][8], bv[VPT][8];
@@ -227,6 +228,7 @@ __global__ void __launch_bounds__(NT, VPT == 1 || (VPT == 2 && (sizeof(T) == 2 |
 norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                 const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
                 T* __restrict__ dx, float* __restrict__ partial_dw, float* __restrict__ partial_db, int M, int N) {
+  grid_go();
   constexpr int NW = NT / 32, SUMS = LN ? 2 : 1;
   constexpr bool AHEAD = RES && (VPT == 1 || (sizeof(T) == 2 && !LN));   // dres with the row; the others have no registers left
   // x^ and w dy stay decoded between the passes where there are registers for it and decoding twice shows: without a
@@ -363,6 +365,7 @@ constexpr int CS_COLS = 32, CS_GROUPS = 8;
 template <typename TO>
 __global__ void __launch_bounds__(CS_COLS * CS_GROUPS)
 colsum_kernel(const float* __restrict__ partial, TO* __restrict__ out, int P, int N, int accumulate) {
+  grid_go();
   __shared__ float part[CS_GROUPS][CS_COLS];
   const int cl = threadIdx.x % CS_COLS, g = threadIdx.x / CS_COLS;
   const int c = blockIdx.x * CS_COLS + cl;

@@ -632,3 +632,47 @@ def test_fused_epilogues_with_two_pairs_per_tile(T):
         torch.cuda.synchronize()
         _lib.check_status(x.device)
         assert (got.float() - want).norm() <= 2 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("rows", [256, 777])
+def test_kernels_that_start_early_wait_for_their_inputs(rows):
+    """Every kernel of a chain reads what the one before wrote, and buffers are written again while they could still be read:
+    the same bits with a synchronisation after each launch, without, and replayed from a graph."""
+    from atorch_b200 import ops
+    from atorch_b200.ops.flash import flash_attention
+
+    torch.manual_seed(0)
+    H = 512
+    w = [(torch.randn(n, k, device="cuda") / k ** 0.5).bfloat16() for n, k in ((3 * H, H), (H, H), (4 * H, H), (H, 2 * H))]
+    g = torch.ones(H, device="cuda").bfloat16()
+    x0 = torch.randn(rows, H, device="cuda").bfloat16()
+    x, act, out = torch.empty_like(x0), torch.empty(rows, 2 * H, device="cuda").bfloat16(), torch.empty_like(x0)
+    bufs = [torch.empty(rows, n, device="cuda").bfloat16() for n in (3 * H, 4 * H)]
+
+    def run(sync):
+        x.copy_(x0)
+        for _ in range(6):
+            for step in (
+                lambda: ops.gemm(ops.rms_norm(x, g, 1e-5), w[0], out=bufs[0]),
+                lambda: out.copy_(flash_attention(*bufs[0].view(1, rows, 12, 128).split(4, 2), causal=True).view(rows, H)),
+                lambda: ops.gemm(out, w[1], out=x, accumulate=True),
+                lambda: ops.gemm(ops.rms_norm(x, g, 1e-5), w[2], out=bufs[1]),
+                lambda: act.copy_(ops.swiglu(bufs[1])),
+                lambda: ops.gemm(act, w[3], out=x, accumulate=True),
+            ):
+                step()
+                if sync:
+                    torch.cuda.synchronize()
+        return x.clone()
+
+    with torch.no_grad():
+        want = run(True)
+        assert all(torch.equal(run(False), want) for _ in range(20))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = run(False)
+        for _ in range(5):
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(got, want)
+    assert bool(torch.isfinite(want).all())
