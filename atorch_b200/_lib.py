@@ -36,6 +36,7 @@ SIGNATURES = {
     "atb_moe_gather_rows": "pppiiip",
     "atb_gemm_bf16_2cta_kgroups": "pppiiillpiiipp",
     "atb_head_sum": "ppppliip",
+    "atb_embedding_bwd": "ppppiiiiip",
     "atb_gemm_bf16_2cta_ragged": "pppiiilllipiippp",
     "atb_norm_fwd": "ppppppppiifiip",
     "atb_norm_bwd": "pppppppppiiiiip",

@@ -214,7 +214,7 @@ class LlamaModel(nn.Module):
                 return_logits: bool = True):
         B, S = input_ids.shape
         cos, sin = self.rope(S, input_ids.device)
-        h = self.embed_tokens(input_ids)
+        h = ops.embedding(self.embed_tokens, input_ids)
         for layer in self.layers:
             if self.config.gradient_checkpointing and self.training and torch.is_grad_enabled():
                 h = checkpoint_module(layer, h, cos, sin, positions, attn_kwargs)

@@ -123,7 +123,7 @@ class MixtralModel(nn.Module):
         if key not in self._rope:
             self._rope = {key: ops.rope_tables(S, self.config.head_dim, self.config.rope_theta, input_ids.device)}
         cos, sin = self._rope[key]
-        h = self.embed_tokens(input_ids)
+        h = ops.embedding(self.embed_tokens, input_ids)
         for layer in self.layers:
             if self.config.gradient_checkpointing and self.training and torch.is_grad_enabled():
                 h = checkpoint_module(layer, h, cos, sin)

@@ -7,6 +7,7 @@ from .gemm import gemm, gemm_reference, linear, linear_rope, linear_swiglu
 from .norm import rms_norm, rms_norm_reference, layer_norm, layer_norm_reference
 from .elementwise import (rope, rope_reference, rope_tables, swiglu, swiglu_reference, bias_gather_add,
                           bias_gather_add_reference)
+from .embedding import embedding
 from .cross_entropy import cross_entropy, cross_entropy_reference
 from .optim import (adamw_step, adamw_reference, agd_step, agd_reference, sum_squares, outer_sgd_step,
                     outer_sgd_reference)

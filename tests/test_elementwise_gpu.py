@@ -265,3 +265,57 @@ def test_norm_backward_row_pairs(M, N, dtype, layernorm):
     assert (pw.double().sum(0) - dw).norm() <= 16 * eps32 * max(1.0, M ** 0.5) * dw.norm()
     if layernorm:
         assert (pb.double().sum(0) - dyd.sum(0)).norm() <= 16 * eps32 * max(1.0, M ** 0.5) * dyd.sum(0).norm()
+
+
+@pytest.mark.parametrize("T,V,H,out_dtype,accumulate,ids_of", [
+    (1, 1, 8, torch.bfloat16, False, "uniform"),
+    (777, 1000, 520, torch.bfloat16, True, "uniform"),
+    (8193, 32000, 256, torch.float32, True, "uniform"),
+    (4100, 151937, 64, torch.bfloat16, False, "uniform"),       # ranges of 1024 rows, the last one ragged
+    (5000, 149, 1032, torch.float32, False, "padding"),         # most tokens on one row: a block sums it
+    (300, 31, 512, torch.bfloat16, True, "edge"),               # 63 to 66 tokens a row
+])
+def test_embedding_gradient(T, V, H, out_dtype, accumulate, ids_of):
+    from atorch_b200.ops.embedding import embedding_grad
+
+    g = torch.Generator().manual_seed(T)
+    ids = torch.randint(0, V, (T,), generator=g)
+    if ids_of == "padding":
+        ids[torch.rand(T, generator=g) < 0.8] = V - 1
+    elif ids_of == "edge":
+        ids = torch.cat([torch.full((n,), i * 7) for i, n in enumerate((63, 64, 65, 66, 42))])[torch.randperm(T, generator=g)]
+    dy = torch.randn(T, H, generator=g).bfloat16()
+    old = torch.randn(V, H, generator=g).to(out_dtype)
+    out = old.cuda() if accumulate else torch.full((V, H), float("nan"), dtype=out_dtype, device="cuda")
+    embedding_grad(dy.cuda(), ids.cuda(), out, accumulate)
+    want = (old.double() if accumulate else torch.zeros(V, H, dtype=torch.float64)).index_add(0, ids, dy.double())
+    size = (old.double().abs() if accumulate else torch.zeros(V, H, dtype=torch.float64)).index_add(0, ids, dy.double().abs())
+    n = torch.bincount(ids, minlength=V).max().item() + 1
+    # n fp32 additions and one rounding to the output type
+    bound = size * n * 2.0 ** -23 + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0)
+    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+    again = old.cuda() if accumulate else torch.empty_like(out)
+    assert torch.equal(embedding_grad(dy.cuda(), ids.cuda(), again, accumulate), out)     # same bits whatever the timing
+
+
+def test_embedding_module_gradient_and_fallbacks():
+    m = torch.nn.Embedding(300, 64).cuda().bfloat16()
+    ids = torch.randint(0, 300, (3, 50), device="cuda")
+    w = torch.randn(3, 50, 64, device="cuda")
+    out = ops.embedding(m, ids)
+    (out.float() * w).sum().backward()
+    got, m.weight.grad = m.weight.grad, None
+    assert torch.equal(out, torch.nn.functional.embedding(ids, m.weight))
+    dy = w.bfloat16().double().view(-1, 64)
+    want = torch.zeros(300, 64, dtype=torch.float64, device="cuda").index_add(0, ids.view(-1), dy)
+    # one rounding of an fp32 sum (the library adds up in bf16 where there are few tokens)
+    torch.testing.assert_close(got.double(), want, rtol=2.0 ** -8, atol=1e-6)
+    m.weight.grad = None
+    m.weight.main_grad = torch.ones(300, 64, device="cuda")
+    (ops.embedding(m, ids).float() * w).sum().backward()
+    assert m.weight.grad is None and m.weight.grad_added_to_main_grad
+    torch.testing.assert_close(m.weight.main_grad.double() - 1, want, rtol=0.0, atol=2.0 ** -20)     # fp32 sums below 8
+    seen = []
+    m.register_forward_hook(lambda *a: seen.append(1))
+    ops.embedding(m, ids)
+    assert seen == [1]
