@@ -18,10 +18,11 @@ using namespace atb;
 // When `src` differs from `x` the result is written to `x` from `src` (out of place) and the columns after the
 // rotated heads (`tail8` 16-byte vectors per row, e.g. the v heads) are copied through unchanged.
 __global__ void rope_kernel(__nv_bfloat16* x, const __nv_bfloat16* src,
-                            const float* __restrict__ cosT, const float* __restrict__ sinT,
-                            const int* __restrict__ pos, long long T, int S, int nheads, int D, long long row_stride,
+                            const float* cosT, const float* sinT,
+                            const int* pos, long long T, int S, int nheads, int D, long long row_stride,
                             long long src_stride, int tail8, float sign) {
   grid_go();
+  grid_wait();
   const int half = D >> 1;
   const int vec_per_head = half >> 3;  // 8 bf16 per 16-byte vector
   const long long total = T * (long long)nheads * vec_per_head;
@@ -69,9 +70,10 @@ __global__ void rope_kernel(__nv_bfloat16* x, const __nv_bfloat16* src,
 }
 
 // out[t, f] = silu(gu[t, f]) * gu[t, F + f]
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, long long T,
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* __restrict__ out, long long T,
                                   int F, long long gu_stride, long long out_stride) {
   grid_go();
+  grid_wait();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -96,10 +98,11 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 }
 
 // dgu[t, f] = dout * up * (sig + gate*sig*(1-sig)) ; dgu[t, F+f] = dout * silu(gate)
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
+__global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* dout,
                                   __nv_bfloat16* __restrict__ dgu, long long T, int F, long long gu_stride,
                                   long long dout_stride) {
   grid_go();
+  grid_wait();
   const int vpr = F >> 3;
   const long long total = T * vpr;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -213,16 +216,15 @@ extern "C" int atb_rope(void* x, const void* src, const float* cosT, const float
   if ((D & 15) || (row_stride & 7) || (src_stride & 7) || (tail_cols & 7)) return -1;
   const long long total = T * (long long)nheads * (D >> 4);
   const __nv_bfloat16* s = src ? (const __nv_bfloat16*)src : (const __nv_bfloat16*)x;
-  rope_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, s, cosT, sinT, pos, T, S, nheads,
-                                                                      D, row_stride, src ? src_stride : row_stride,
-                                                                      tail_cols >> 3, backward ? -1.f : 1.f);
+  launch_after(rope_kernel, grid_for(total, 256), 256, 0, (cudaStream_t)stream, 1, (__nv_bfloat16*)x, s, cosT, sinT, pos, T, S,
+               nheads, D, row_stride, src ? src_stride : row_stride, tail_cols >> 3, backward ? -1.f : 1.f);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 extern "C" int atb_swiglu_fwd(const void* gu, void* out, long long T, int F, long long gu_stride, long long out_stride,
                               void* stream) {
   if (T <= 0) return 0;
   if ((F & 7) || (gu_stride & 7) || (out_stride & 7)) return -1;
-  swiglu_fwd_kernel<<<grid_for(T * (F >> 3), 256), 256, 0, (cudaStream_t)stream>>>(
+  launch_after(swiglu_fwd_kernel, grid_for(T * (F >> 3), 256), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, T, F, gu_stride, out_stride);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
@@ -230,7 +232,7 @@ extern "C" int atb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long 
                               long long dout_stride, void* stream) {
   if (T <= 0) return 0;
   if ((F & 7) || (gu_stride & 7) || (dout_stride & 7)) return -1;
-  swiglu_bwd_kernel<<<grid_for(T * (F >> 3), 256), 256, 0, (cudaStream_t)stream>>>(
+  launch_after(swiglu_bwd_kernel, grid_for(T * (F >> 3), 256), 256, 0, (cudaStream_t)stream, 1,
       (const __nv_bfloat16*)gu, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dgu, T, F, gu_stride, dout_stride);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -113,12 +113,13 @@ ATB_DEVICE float round_through(float x) {
 // If `residual` is given, the sum x + residual is also written to `sum_out` (pre-norm stream).
 // ------------------------------------------------------------------------------------------
 template <typename T, int VPT, bool LN, bool RES>
-__global__ void __launch_bounds__(NT, (VPT <= 2 && !LN) ? 4 : 1) norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ residual,
-                                                      const T* __restrict__ w, const T* __restrict__ b,
+__global__ void __launch_bounds__(NT, (VPT <= 2 && !LN) ? 4 : 1) norm_fwd_kernel(const T* x, const T* residual,
+                                                      const T* w, const T* b,
                                                       T* __restrict__ y, T* __restrict__ sum_out,
                                                       float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                       int M, int N, float eps) {
   grid_go();
+  grid_wait();
   __shared__ float red[33];
   const int nvec = N >> 3;
   float wv[VPT][8], bv[VPT][8];
@@ -225,10 +226,10 @@ __global__ void __launch_bounds__(NT, (VPT <= 2 && !LN) ? 4 : 1) norm_fwd_kernel
 // ------------------------------------------------------------------------------------------
 template <typename T, int VPT, int R, bool LN, bool RES>
 __global__ void __launch_bounds__(NT, VPT == 1 || (VPT == 2 && (sizeof(T) == 2 || !LN)) ? 2 : 1)
-norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
-                const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const T* __restrict__ dres,
+norm_bwd_kernel(const T* dy, const T* x, const T* w, const float* mean_in, const float* rstd_in, const T* dres,
                 T* __restrict__ dx, float* __restrict__ partial_dw, float* __restrict__ partial_db, int M, int N) {
   grid_go();
+  grid_wait();
   constexpr int NW = NT / 32, SUMS = LN ? 2 : 1;
   constexpr bool AHEAD = RES && (VPT == 1 || (sizeof(T) == 2 && !LN));   // dres with the row; the others have no registers left
   // x^ and w dy stay decoded between the passes where there are registers for it and decoding twice shows: without a
@@ -364,8 +365,9 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
 constexpr int CS_COLS = 32, CS_GROUPS = 8;
 template <typename TO>
 __global__ void __launch_bounds__(CS_COLS * CS_GROUPS)
-colsum_kernel(const float* __restrict__ partial, TO* __restrict__ out, int P, int N, int accumulate) {
+colsum_kernel(const float* partial, TO* __restrict__ out, int P, int N, int accumulate) {
   grid_go();
+  grid_wait();
   __shared__ float part[CS_GROUPS][CS_COLS];
   const int cl = threadIdx.x % CS_COLS, g = threadIdx.x / CS_COLS;
   const int c = blockIdx.x * CS_COLS + cl;
@@ -397,11 +399,11 @@ int launch_fwd(const void* x, const void* res, const void* w, const void* b, voi
 #define L(V)                                                                                                       \
   do {                                                                                                             \
     if (res != nullptr)                                                                                            \
-      norm_fwd_kernel<T, V, LN, true><<<grid, NT, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (const T*)b,   \
-                                                           (T*)y, (T*)sum_out, mean, rstd, M, N, eps);            \
+      launch_after(norm_fwd_kernel<T, V, LN, true>, grid, NT, 0, st, 1, (const T*)x, (const T*)res, (const T*)w,   \
+                   (const T*)b, (T*)y, (T*)sum_out, mean, rstd, M, N, eps);                                        \
     else                                                                                                           \
-      norm_fwd_kernel<T, V, LN, false><<<grid, NT, 0, st>>>((const T*)x, (const T*)res, (const T*)w, (const T*)b,  \
-                                                            (T*)y, (T*)sum_out, mean, rstd, M, N, eps);           \
+      launch_after(norm_fwd_kernel<T, V, LN, false>, grid, NT, 0, st, 1, (const T*)x, (const T*)res, (const T*)w,  \
+                   (const T*)b, (T*)y, (T*)sum_out, mean, rstd, M, N, eps);                                        \
   } while (0)
   if (vpt <= 1) L(1);
   else if (vpt <= 2) L(2);
@@ -420,11 +422,11 @@ int launch_bwd(const void* dy, const void* x, const void* w, const float* mean, 
 #define L(V, R)                                                                                                      \
   do {                                                                                                               \
     if (dres != nullptr)                                                                                             \
-      norm_bwd_kernel<T, V, R, LN, true><<<parts, NT, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd,   \
-                                                               (const T*)dres, (T*)dx, pdw, pdb, M, N);              \
+      launch_after(norm_bwd_kernel<T, V, R, LN, true>, parts, NT, 0, st, 1, (const T*)dy, (const T*)x, (const T*)w,  \
+                   mean, rstd, (const T*)dres, (T*)dx, pdw, pdb, M, N);                                              \
     else                                                                                                             \
-      norm_bwd_kernel<T, V, R, LN, false><<<parts, NT, 0, st>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd,  \
-                                                                nullptr, (T*)dx, pdw, pdb, M, N);                    \
+      launch_after(norm_bwd_kernel<T, V, R, LN, false>, parts, NT, 0, st, 1, (const T*)dy, (const T*)x, (const T*)w, \
+                   mean, rstd, (const T*)nullptr, (T*)dx, pdw, pdb, M, N);                                           \
   } while (0)
   if (vpt <= 1) L(1, (sizeof(T) == 2 ? 2 : 1));
   else if (vpt <= 2) L(2, 1);
@@ -479,9 +481,9 @@ extern "C" int atb_norm_bwd(const void* dy, const void* x, const void* w, const 
 extern "C" int atb_colsum(const float* partial, void* out, int P, int N, int out_dtype, int accumulate, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const int grid = (N + CS_COLS - 1) / CS_COLS, threads = CS_COLS * CS_GROUPS;
-  if (out_dtype == 0) colsum_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(partial, (__nv_bfloat16*)out, P, N, accumulate);
-  else if (out_dtype == 1) colsum_kernel<__half><<<grid, threads, 0, st>>>(partial, (__half*)out, P, N, accumulate);
-  else colsum_kernel<float><<<grid, threads, 0, st>>>(partial, (float*)out, P, N, accumulate);
+  if (out_dtype == 0) launch_after(colsum_kernel<__nv_bfloat16>, grid, threads, 0, st, 1, partial, (__nv_bfloat16*)out, P, N, accumulate);
+  else if (out_dtype == 1) launch_after(colsum_kernel<__half>, grid, threads, 0, st, 1, partial, (__half*)out, P, N, accumulate);
+  else launch_after(colsum_kernel<float>, grid, threads, 0, st, 1, partial, (float*)out, P, N, accumulate);
   return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
