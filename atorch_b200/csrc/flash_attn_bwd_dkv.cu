@@ -13,7 +13,7 @@
 //   S(i+1) is issued as soon as the warps hold S(i) in registers and runs under the exponentials of block i,
 //   dV(i) starts when P(i) is stored and runs under dS(i),
 //   dK(i), dP(i+1) run under the exponentials of block i+1.
-// S=8192, 32 heads of 128, causal: 1188 -> 865 us (2800 clocks a block, 1024 of them exponentials); before, S(i+1) was issued after P and dS were
+// S=8192, 32 heads of 128, causal: 1188 -> 822 us (861 with a CTA per block; 2800 clocks a block, 1024 of them exponentials); before, S(i+1) was issued after P and dS were
 // both stored, or (for long causal inputs) P^T and dS^T went through tensor memory instead, whose element-wise warps need
 // the row statistics per column.
 // For grouped queries the gradients of the group are summed in the accumulator in fp32; with one CTA per query head the

@@ -31,23 +31,25 @@ import os
 import weakref
 
 # forward kernel with two 128-row query tiles per CTA that share every K/V tile (csrc/flash_attn_v2.cu): the
-# default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 135 us against
-# 231 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 55 us against 74 us); ATB_FLASH_V2=0
+# default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 125 us against
+# 232 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 42 us against 68 us); ATB_FLASH_V2=0
 # keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
 # Head dim 64 keeps the single-tile kernel while its CTAs (128 rows) fit one wave: two tiles a CTA then leave half of the SMs
-# without work (16 heads, all keys, single / two tiles: 512 rows, 64 CTAs, 11.9 / 14.5 us; 1024, 128 CTAs, 16.5 / 20.6; two waves,
-# 64 heads of 512: 20.6 / 14.5; 32 heads of 1024: 30.8 / 22.7).
+# without work (16 heads, all keys, single / two tiles: 512 rows, 64 CTAs, 12.4 / 12.8 us; 1024, 128 CTAs, 17.5 / 21.2; two waves,
+# 64 heads of 512: 20.7 / 13.9; 32 heads of 1024: 32.5 / 22.3).
 ONE_WAVE = 148
 # backward as two kernels (dK/dV per key block + dQ per query block; no atomics, no fp32 scratch) where there is neither
 # dropout nor a bias. ATB_FLASH_BWD_SPLIT=0 selects the one key-block kernel with TMA reduce-adds of dQ everywhere.
 BWD_SPLIT = os.environ.get("ATB_FLASH_BWD_SPLIT", "1") == "1"
 # dK/dV kernel: a CTA sums the query heads of its group in tensor memory, as many of them (a divisor of the group) as still
 # leave this many CTAs; what is left of a group is summed by a pass over the bf16 results. A CTA per SM will do while a
-# head is short (10 x 512, 16 heads on 4, backward in all: 95 us with 160 CTAs, 114 with 320, 132 with 640), from 16 query
-# blocks on half as many again (2560, 32 on 8: 232 us with 160, 210 with 320, 226 with 640; 3584: 345 with 224, 349 with 448,
-# 374 with 896). Long heads that all see every key fold whole groups or none (4000, 32 on 4: 785 us unfolded, 802 by 4).
+# head is short (10 x 512, 16 heads on 4, causal, backward in all: 75 us with 160 CTAs, 83 with 320, 89 with 640). From 12 query
+# blocks on the last CTAs weigh more, and it takes FOLD_LONG_CTAS (2 x 1536, 32 on 4: 167 us with 192, 156 with 384; 2560, 32 on 8:
+# 222 with 160, 188 with 320, 192 with 640; 3584: 338 with 224, 327 with 448, 333 with 896; 4096: 400 with 256, 403 with 512).
+# Long heads that all see every key fold whole groups or none (4000, 32 on 4: 758 us unfolded, 807 by 4, 996 by 2).
 FOLD_MIN_CTAS = 148
+FOLD_LONG_CTAS = 240
 
 
 def kernels_built() -> bool:
@@ -407,7 +409,7 @@ def _forward(like, qkv, sizes, D, strides, causal, softmax_scale, row_lo, row_hi
 
 def _fold(group: int, ctas: int, q_blocks: int, causal: bool) -> int:
     """Query heads per CTA of the dK/dV kernel (see FOLD_MIN_CTAS); ``ctas``: its CTAs with whole groups."""
-    need = FOLD_MIN_CTAS if q_blocks < 16 else FOLD_MIN_CTAS * 3 // 2
+    need = FOLD_MIN_CTAS if q_blocks < 12 else FOLD_LONG_CTAS
     return next((f for f in range(group, 1, -1) if group % f == 0 and ctas * (group // f) >= need
                  and (f == group or causal or q_blocks < 16)), 1)
 

@@ -90,6 +90,9 @@ def gemm(
     ``a`` is stored ``[M,K]`` (or ``[K,M]`` when ``a_mn``), ``b`` is stored ``[N,K]`` (or ``[K,N]``
     when ``b_mn``). Inputs are bf16, accumulation is fp32, the output is bf16 or fp32.
 
+    ``tile_n`` (CTA-pair kernel): 0 = by a rule on the sizes, 128 or 256 = tiles of that width, 512 = tiles of 256 columns
+    with two pairs of CTAs each, half of the reduction a pair.
+
     ``groups`` (mixture-of-experts buffers, CTA-pair kernel only): ``{"counts": int32 device tensor,
     "m_rows": r}`` - rows of A come in groups of ``r`` slots (a multiple of 256) of which only the first
     ``counts[g]`` hold data and the rest is zero: tiles beyond the count are not computed, their output is
