@@ -19,8 +19,8 @@
 // While tile A's warps exponentiate, the tensor core works for tile B and vice versa:
 // issue order  PV_A(j), S_A(j+1), PV_B(j), S_B(j+1).
 //
-// 8192 keys, 32 heads of 128: full 818 us (1344 TFLOP/s), causal 436 us (450 with a CTA per block; before: 945 and 578-625 us; 497
-// before BlockOrder); 16 x 512, 16 heads of 64, all keys 50 -> 42 us by the running CTAs. A step of both tiles takes 3100 clocks, 1900 of them softmax and 1200 tensor work of the same tile. Tried: K/V tiles of 64 keys with
+// 8192 keys, 32 heads of 128: full 775 us (1420 TFLOP/s), causal 419 us (450 with a CTA per block; before: 945 and 578-625 us; 497
+// before BlockOrder); 16 x 512, 16 heads of 64, all keys 50 -> 40 us by the running CTAs. A step of both tiles takes 3100 clocks, 1900 of them softmax and 1200 tensor work of the same tile. Tried: K/V tiles of 64 keys with
 // two score buffers per tile, which takes the tensor work out of that chain - 887 us, because a 128 x 64 x 16 score
 // product takes 48 clocks for its shared-memory operands where it should take 32; P in one piece - 859 us.
 //
@@ -334,21 +334,20 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     };
     uint32_t g = 0;
     int u = 0;
-    Work w;
-    bool ok = queue_next(queue, 0, w, abort_flag, p.status);
-    if (ok) load_unit(w);
-    for (int c = 0; ok && w.more;) {
-      const int b = w.sample, h = w.head, n_t = t ? w.v2 : w.v1;
-      const int i = w.place * 2 * BQ + t * BQ + r;     // global query row
-      const bool row_valid = i < p.Sq;
-      lo = max(lo, 0); hi = min(hi, p.Sk);
+    bool ok = queue_wait(queue, 0, abort_flag, p.status);
+    if (ok) load_unit(queue_read(queue, 0));
+    for (int c = 0; ok; ++c) {
+      const Work unit = queue_read(queue, c);
+      if (!unit.more) break;
+      const int n_t = t ? unit.v2 : unit.v1;
+      lo = max(lo, 0); hi = min(hi, p.Sk);             // (0, 0) in a row that there is not
       float m_ref = -INFINITY, l_run = 0.f;
       for (int j = 0; j < n_t; ++j, ++g) {
-        const int kv0 = (w.v0 + j) * BKV;
+        const int kv0 = (unit.v0 + j) * BKV;
         if (!mbar_wait_warp(&s_full[t], g & 1, abort_flag, p.status)) { ok = false; break; }
         tc_fence_after();
         // the mask tests are compiled into a separate path taken only by warps with a partly visible row
-        const bool full = __all_sync(0xffffffffu, row_valid && lo <= kv0 && hi >= kv0 + BKV);
+        const bool full = __all_sync(0xffffffffu, lo <= kv0 && hi >= kv0 + BKV);
         uint32_t x0[32], x1[32], x2[32], x3[32];
         tmem_ld_32x32(s_addr, x0);
         tmem_ld_32x32(s_addr + 32, x1);
@@ -406,10 +405,12 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         l_run += (a + b2) + (c2 + d2);
       }
       if (!ok) break;
-      Work nw;
-      ok = queue_next(queue, ++c, nw, abort_flag, p.status);
+      ok = queue_wait(queue, c + 1, abort_flag, p.status);
       if (!ok) break;
-      load_unit(nw);
+      load_unit(queue_read(queue, c + 1));
+      const Work w = queue_read(queue, c);
+      const int b = w.sample, h = w.head, i = w.place * 2 * BQ + t * BQ + r;     // global query row
+      const bool row_valid = i < p.Sq;
       if (n_t > 0) {
         ok = mbar_wait_warp(&o_full[t], u & 1, abort_flag, p.status);
         if (!ok) break;
@@ -440,7 +441,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       if (row_valid)
         p.lse[((long long)b * p.Hq + h) * p.Sq + i] =
             l_run > 0.f ? (m_ref * p.scale_log2 + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-      w = nw;
+      queue_free(queue, c);
     }
   }
 

@@ -31,8 +31,8 @@ import os
 import weakref
 
 # forward kernel with two 128-row query tiles per CTA that share every K/V tile (csrc/flash_attn_v2.cu): the
-# default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 125 us against
-# 232 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 42 us against 68 us); ATB_FLASH_V2=0
+# default from 256 query rows on for head dims 128 and 64 (measured at S=4096, H=32, D=128, causal: 118 us against
+# 232 us for the single-tile kernel; at B=16, S=512, H=16, D=64, all keys: 40 us against 68 us); ATB_FLASH_V2=0
 # keeps the single-tile kernel everywhere
 FWD_TWO_TILES = os.environ.get("ATB_FLASH_V2", "1") == "1"
 # Head dim 64 keeps the single-tile kernel while its CTAs (128 rows) fit one wave: two tiles a CTA then leave half of the SMs
