@@ -312,10 +312,11 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       return row_info(w.sample, w.head * p.fold, w.v0 * BQ + r, w.more && w.v1 > 0);
     };
     uint32_t g = 0;
-    Work w;
-    bool ok = queue_next(queue, 0, w, abort_flag, p.status);
-    RowInfo raw = ok ? first_row(w) : RowInfo{};
-    for (int c = 0; ok && w.more;) {
+    bool ok = queue_wait(queue, 0, abort_flag, p.status);
+    RowInfo raw = ok ? first_row(queue_read(queue, 0)) : RowInfo{};
+    for (int c = 0; ok; ++c) {
+      const Work w = queue_read(queue, c);
+      if (!w.more) break;
       const int b = w.sample, ho = w.head, kv0 = w.place * BKV, n = w.v1 * p.fold;
       const int c0 = kv0 + half * 64;              // first key of this thread
       int h = ho * p.fold, qb = 0;
@@ -405,18 +406,18 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       if (!ok) break;
       // the next unit is known and its first values are on their way before this one's results leave
-      Work nw;
-      ok = queue_next(queue, ++c, nw, abort_flag, p.status);
+      ok = queue_wait(queue, c + 1, abort_flag, p.status);
       if (!ok) break;
-      raw = first_row(nw);
+      raw = first_row(queue_read(queue, c + 1));
       if (n > 0)
         ok = mbar_wait_warp(p_free, (g - 1) & 1, abort_flag, p.status) &&
              mbar_wait_warp(ds_free, (g - 1) & 1, abort_flag, p.status);
       if (!ok) break;
       // dV / dK of this key block: TMEM lane = key row. tcgen05.ld is a warp-wide (.sync.aligned)
       // instruction: every lane executes it, only the global stores are predicated per row.
-      const int j = kv0 + r;
-      const long long at = ((long long)b * p.Sk + j) * p.dkv_stride + ho * HD + half * (HD / 2);
+      const Work again = queue_read(queue, c);
+      const int j = again.place * BKV + r;
+      const long long at = ((long long)again.sample * p.Sk + j) * p.dkv_stride + again.head * HD + half * (HD / 2);
       if (n > 0) tc_fence_after();
 #pragma unroll
       for (int cc = 0; cc < HD / 64; ++cc) {
@@ -439,7 +440,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           store_bf16_32(p.dk + at + cc * 32, tk, p.wide);
         }
       }
-      w = nw;
+      queue_free(queue, c);
     }
   }
 
