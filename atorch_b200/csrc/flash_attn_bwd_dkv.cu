@@ -476,7 +476,8 @@ int launch_dkv(const void* dout, const void* q, const void* k, const void* v, Dk
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sk + BKV - 1) / BKV, p.Hq / p.fold, p.B, p.causal != 0, p.Sq, HD);
-  return launch_after(flash_bwd_dkv_kernel<HD>, grid, THREADS, SmemK<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p) == cudaSuccess ? 0 : -5;
+  launch_after(flash_bwd_dkv_kernel<HD>, grid, THREADS, SmemK<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

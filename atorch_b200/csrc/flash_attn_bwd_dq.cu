@@ -450,7 +450,8 @@ int launch_dq(const void* dout, const void* q, const void* k, const void* v, DqP
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sq + BQ - 1) / BQ, p.Hq, p.B, p.causal != 0, p.Sk, HD);
-  return launch_after(flash_bwd_dq_kernel<HD>, grid, THREADS, SmemQ<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p) == cudaSuccess ? 0 : -5;
+  launch_after(flash_bwd_dq_kernel<HD>, grid, THREADS, SmemQ<HD>::TOTAL, stream, 1, tmQ, tmdO, tmK, tmV, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace

@@ -473,7 +473,8 @@ int launch_fwd2(const void* q, const void* k, const void* v, Params p, long long
   }
   dim3 grid;
   make_block_order(&p.order, &grid, (p.Sq + 2 * BQ - 1) / (2 * BQ), p.Hq, p.B, p.causal != 0, p.Sk, HD);
-  return launch_after(flash_fwd2_kernel<HD>, grid, THREADS, L2<HD>::TOTAL, stream, 1, tmQ, tmK, tmV, p) == cudaSuccess ? 0 : -5;
+  launch_after(flash_fwd2_kernel<HD>, grid, THREADS, L2<HD>::TOTAL, stream, 1, tmQ, tmK, tmV, p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 
 }  // namespace
