@@ -97,11 +97,13 @@ ATB_DEVICE bool clc_answer(const WorkQueue* q, uint3& idx) {
   return warp_uniform(ok) != 0;
 }
 
-// The scheduler warp's whole life, by all its lanes. describe(Work&, blocks) fills in v0..v3 of a block (`blocks`: blocks of
-// a head); its lanes may load and shuffle.
+// The scheduler warp's whole life, by all its lanes, after grid_wait. describe(Work&, blocks) fills in v0..v3 of a block
+// (`blocks`: blocks of a head); its lanes may load and shuffle. After an error of a kernel before this one the first unit
+// is published as none: one warp looks, the roles all take the same from the queue, and the load runs beside those of the unit.
 template <class F>
 ATB_DEVICE void queue_run(WorkQueue* q, const BlockOrder& order, F describe, volatile int* abort_flag, int* status) {
   const bool first_lane = (threadIdx.x & 31) == 0;
+  const int failed = status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
   uint3 idx = blockIdx;
   bool have = true;
   uint32_t asked = 0;
@@ -124,8 +126,9 @@ ATB_DEVICE void queue_run(WorkQueue* q, const BlockOrder& order, F describe, vol
     int blocks = 0;
     while (have && !block_of(order, idx, w.place, blocks, w.head, w.sample))   // an index without a block
       if (!ask()) return;
-    w.more = have;
     if (have) describe(w, blocks);
+    if (c == 0 && warp_uniform(failed) != 0) have = false;
+    w.more = have;
     const int e = c & 1;
     if (!mbar_wait_warp(&q->empty[e], ((c >> 1) & 1) ^ 1, abort_flag, status)) return;
     if (first_lane) {

@@ -107,10 +107,6 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) {
-    grid_wait();
-    return;
-  }
   const int shift = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {

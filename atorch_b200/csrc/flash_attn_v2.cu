@@ -132,10 +132,6 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   WorkQueue* queue = reinterpret_cast<WorkQueue*>(smem + L::QUEUE_OFF);
 
   const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) {
-    grid_wait();
-    return;
-  }
   if (p.holes != nullptr) {
     grid_wait();
     int any = 0;

@@ -126,6 +126,12 @@ struct Gate {
 
 __device__ unsigned long long g_gate_wait_ns = ATB_WAIT_LIMIT_NS;
 
+// An error that a kernel has recorded in the status word.
+ATB_DEVICE bool error_recorded(const int* status) {
+  return status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
+}
+
+// True as well, at once, when an error has been recorded: what would arrive is not needed any more (see `stopped`).
 ATB_DEVICE bool gate_wait(const Gate& gate, int row_lo, int row_hi, volatile int* abort_flag, int* status) {
   for (int g = row_lo / gate.rows; g <= (row_hi - 1) / gate.rows; ++g) {
     const unsigned int* f = gate.flags + g;
@@ -138,6 +144,7 @@ ATB_DEVICE bool gate_wait(const Gate& gate, int row_lo, int row_hi, volatile int
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
       if ((int)(v - gate.epoch) >= 0) break;
       if (*abort_flag) return false;
+      if (error_recorded(status)) return true;
       if (globaltimer_ns() - t0 > limit) {
         *abort_flag = 1;
         if (status) atomicCAS(status, 0, (int)ATB_ERR_PEER_TIMEOUT);
@@ -314,8 +321,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const uint32_t rank = cta & 1, pair0 = cta & ~1u;     // place in the pair; the pair's first CTA in the cluster
   const int part = SPLIT == 2 ? (int)(cta >> 1) : 0;    // which half of the reduction and of the columns
   const bool leader = rank == 0;
-  // all CTAs of a cluster read the same word, so they take the same decision (on its way while the barriers are set up)
-  const int stopped = status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
   const int tiles_m = rag.n > 0 ? rag.mt0[rag.n] : (M + 2 * BM - 1) / (2 * BM);
   const int tile_cols = ep.gated ? BN / 2 : BN;      // output columns per tile
   const int tiles_n = (N + tile_cols - 1) / tile_cols;
@@ -372,7 +377,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     tmem_relinquish<2>();
     tc_fence_before();
   }
-  const int num_tiles = warp_uniform(stopped) != 0 ? 0 : tiles_m * tiles_n * groups;
+  const int num_tiles = tiles_m * tiles_n * groups;
 
   // identical decisions in every role: which tiles and which k-blocks carry data
   auto tile_active = [&](int m0, int b_idx) -> bool {
@@ -607,6 +612,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     const int q = warp & 3;                 // lane quarter
     const int half = (warp - 2) >> 2;       // column half
     grid_wait();
+    // After an error of a kernel before this one nothing is stored. Only the epilogue asks, and here, where that kernel has
+    // completed: every role of every CTA of the cluster goes through all tiles either way, so no answer has to be the same in
+    // two of them. The load runs under the first tile's products.
+    bool stopped = warp_uniform((int)error_recorded(status)) != 0;
     const bool have_tmem = mbar_wait_warp(tmem_ready, 0, abort_flag, status);
     tc_fence_after();
     const uint32_t tmem_base = warp_uniform(*tmem_slot);
@@ -756,7 +765,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (!tile_active(m0, b_idx)) {
         // an empty tile: its output is all zeros (left alone when accumulating)
         const int zrow = m0 + (int)rank * BM + q * 32 + lane;
-        if (!ep.accumulate && ep.rs_rows <= 0 && zrow < M) {
+        if (!stopped && !ep.accumulate && ep.rs_rows <= 0 && zrow < M) {
           for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 8) {
             if (n0 + c >= N) break;
             if (ep.out_fp32) {
@@ -779,6 +788,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       if (SPLIT == 1 && fetching && n0 + half * (BN / 2) + 32 <= N) fetch(xa, c_row0 + row, n0 + half * (BN / 2));
       if (!mbar_wait_warp(&tfull[acc], acc_ph, abort_flag, status)) break;
       tc_fence_after();
+      // a producer that found an error in place of its rows went on without them: look again behind it
+      if (gate.flags != nullptr) stopped = stopped || warp_uniform((int)error_recorded(status)) != 0;
+      if (stopped) m_end = m0;
       const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       const bool in = row < m_end;
       const int row0 = m0 + (int)rank * BM + q * 32;      // first of this warp's rows

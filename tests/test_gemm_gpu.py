@@ -676,3 +676,77 @@ def test_kernels_that_start_early_wait_for_their_inputs(rows):
             torch.cuda.synchronize()
             assert torch.equal(got, want)
     assert bool(torch.isfinite(want).all())
+
+
+@pytest.mark.parametrize("kind", ["one wave", "many tiles", "two pairs per tile", "accumulate", "attention", "attention backward"])
+def test_kernel_behind_an_error_stores_nothing(kind):
+    """The kernel in front records an error (the status word is the last element that it writes) after the kernel behind has
+    started early: the kernel behind stores nothing, and no wait of it runs out. With a clear word it stores everything."""
+    torch.manual_seed(0)
+    L, st = _lib.lib(), _lib.stream()
+    a = torch.ones(4096, 8192, device="cuda", dtype=torch.bfloat16)
+    front = torch.zeros(4096, 4096, device="cuda", dtype=torch.bfloat16)
+    rnd = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    if kind.startswith("attention"):
+        B, S, H, D = 2, 640, 16, 128
+        q, k, v, do, o = (rnd(B, S, H, D) for _ in range(5))
+        lse, delta = torch.zeros(B, H, S, device="cuda"), torch.zeros(B * H * S, device="cuda")
+        outs = [torch.zeros_like(q) for _ in range(3)]
+        dims = (0, 0, B, S, S, H, H, H * D, H * D, H * D)
+
+        def launch(status):
+            p = [t.data_ptr() for t in outs]
+            if kind == "attention":
+                return L.atb_flash_fwd_v2(q.data_ptr(), k.data_ptr(), v.data_ptr(), p[0], lse.data_ptr(), *dims, 1, D ** -0.5,
+                                          st, status, D, 0)
+            return L.atb_flash_bwd_split(do.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
+                                         lse.data_ptr(), delta.data_ptr(), *p, *dims, H * D, H * D, H * D, 1, D ** -0.5, st,
+                                         status, 1, D)
+        outs_written = outs[:1] if kind == "attention" else outs
+    else:
+        M, N, K = {"one wave": (512, 512, 512), "accumulate": (777, 520, 256)}.get(kind, (4096, 4096, 1024))
+        x, w, c = rnd(M, K), rnd(N, K), torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+        outs_written = [c]
+
+        def launch(status):
+            return L.atb_gemm_bf16_2cta(x.data_ptr(), w.data_ptr(), c.data_ptr(), 0, M, N, K, K, K, N, 0, 0, 0,
+                                        int(kind == "accumulate"), 1.0, 512 if kind == "two pairs per tile" else 0, 0, 0, 0, st,
+                                        status)
+    word = front.view(torch.int32)[-1, -1:]
+    for _ in range(3):
+        front.zero_()
+        gemm(a, a[:4096], out=front)
+        assert launch(word.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert front.view(torch.int32)[-1, -1].item() == 0x46004600      # 8192 twice: what the product wrote, no error code
+        assert not any(bool(t.any()) for t in outs_written)
+    clear = torch.zeros(1, device="cuda", dtype=torch.int32)
+    assert launch(clear.data_ptr()) == 0
+    torch.cuda.synchronize()
+    assert clear.item() == 0 and all(bool(t.any()) for t in outs_written)
+
+
+def test_gate_behind_an_error_does_not_wait():
+    """Rows that have not arrived are not waited for once an error has been recorded, and nothing is stored."""
+    import ctypes
+    import time
+
+    M, N, K = 512, 1024, 512
+    x, w = _mk(M, K), _mk(N, K)
+    c = torch.zeros(M, N, device="cuda", dtype=torch.bfloat16)
+    flags = torch.zeros(8, device="cuda", dtype=torch.int32)
+    status = torch.full((1,), 4, device="cuda", dtype=torch.int32)
+    ll, p = ctypes.c_longlong, lambda t: ctypes.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    t0 = time.time()
+    for _ in range(4):
+        assert _lib.lib().atb_gemm_bf16_2cta_wgather(p(x), p(w), p(c), M, N, K, ll(K), ll(K), ll(N), p(flags),
+                                                     ctypes.c_uint(1), 128, 256, _lib.stream_ptr(), p(status)) == 0
+    torch.cuda.synchronize()
+    assert time.time() - t0 < 1.0                # the limit of one wait is 2 s
+    assert not bool(c.any()) and status.item() == 4
+    status.zero_()
+    flags.fill_(1)
+    assert _lib.lib().atb_gemm_bf16_2cta_wgather(p(x), p(w), p(c), M, N, K, ll(K), ll(K), ll(N), p(flags), ctypes.c_uint(1),
+                                                 128, 256, _lib.stream_ptr(), p(status)) == 0
+    _check(c, x.float() @ w.float().t(), K)
