@@ -238,6 +238,7 @@ ATB_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tm, uint32_t
 // between launches (the pair that finishes last clears them).
 struct Sched {
   int* counters;   // nullptr: static schedule (tile = pair + i * pairs)
+  int early;       // the launch after this one may take the SMs that this one leaves
 };
 
 ATB_DEVICE void st_remote_u32(uint32_t cluster_addr, uint32_t v) {
@@ -366,8 +367,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     __syncwarp();
   }
   cluster_arrive_all();
-  // A launch that waits for other ranks keeps the SMs that it was told to leave free for the transfer.
-  if (threadIdx.x == 0 && gate.flags == nullptr) grid_go();
+  if (threadIdx.x == 0 && sched.early) grid_go();
   if (!KG && warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -1094,8 +1094,10 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   int clusters = SPLIT == 2 ? split_clusters() : sm_count() / 2;
   if (tiles < clusters) clusters = tiles;
   if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
-  // dynamic tile scheduling for plain launches with more tiles than CTA pairs (see Sched)
-  Sched sched{nullptr};
+  // Dynamic tile scheduling for plain launches with more tiles than CTA pairs (see Sched). A launch that waits for other ranks, and
+  // one with a limit on its CTAs, keep the SMs that they leave free for what runs beside them, a transfer: the launch after
+  // them would sit there and wait.
+  Sched sched{nullptr, gate.flags == nullptr && max_ctas <= 0};
   if (g_dynamic < 0) {
     const char* e = getenv("ATB_GEMM_DYNAMIC");
     g_dynamic = (e != nullptr && e[0] == '0') ? 0 : 1;

@@ -750,3 +750,25 @@ def test_gate_behind_an_error_does_not_wait():
     assert _lib.lib().atb_gemm_bf16_2cta_wgather(p(x), p(w), p(c), M, N, K, ll(K), ll(K), ll(N), p(flags), ctypes.c_uint(1),
                                                  128, 256, _lib.stream_ptr(), p(status)) == 0
     _check(c, x.float() @ w.float().t(), K)
+
+
+def test_launch_with_a_limit_leaves_the_other_sms_free():
+    """20 CTAs for some milliseconds and a product of the same stream behind them: one of another stream, which needs SMs to
+    itself, ends long before they do."""
+    a, small = _mk(8192, 8192), _mk(2048, 2048)
+    side = torch.cuda.Stream()
+    first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    gemm(a, a, max_ctas=20)
+    gemm(small, small)
+    with torch.cuda.stream(side):
+        gemm(small, small)
+    torch.cuda.synchronize()
+    gemm(a, a, max_ctas=20)
+    gemm(small, small)
+    with torch.cuda.stream(side):
+        gemm(small, small)
+        first.record()
+    last.record()
+    torch.cuda.synchronize()
+    _lib.check_status(a.device)
+    assert first.elapsed_time(last) > 1.0
