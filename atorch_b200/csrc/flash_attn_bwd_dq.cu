@@ -111,11 +111,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     queue_init(queue, 2 + N_EW / 32);
     *abort_flag = 0;
     mbar_fence_init();
-    grid_go();
   }
   if (warp == 1) {
     tmem_alloc<1>(tmem_slot, 512);
     tmem_relinquish<1>();
+    if (lane == 0) grid_go();
   }
   tc_fence_before();
   __syncthreads();

@@ -152,9 +152,12 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     queue_init(queue, 2 + 8);
     *abort_flag = 0;
     mbar_fence_init();
-    grid_go();
   }
-  if (warp == 1) { tmem_alloc<1>(tmem_slot, 512); tmem_relinquish<1>(); }
+  if (warp == 1) {
+    tmem_alloc<1>(tmem_slot, 512);
+    tmem_relinquish<1>();
+    if (lane == 0) grid_go();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -367,7 +367,6 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     __syncwarp();
   }
   cluster_arrive_all();
-  if (threadIdx.x == 0 && sched.early) grid_go();
   if (!KG && warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
@@ -376,6 +375,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     tmem_alloc<2>(tmem_slot, 2 * BN);
     tmem_relinquish<2>();
     tc_fence_before();
+    if (lane == 0 && sched.early) grid_go();
   }
   const int num_tiles = tiles_m * tiles_n * groups;
 

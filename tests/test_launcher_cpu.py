@@ -88,3 +88,21 @@ def test_call_without_gradients():
         assert "PythonOp" in str(traced.graph) or "_Double" in str(traced.graph)
     with torch.inference_mode():
         assert torch.equal(call(_Double, torch.ones(3)), torch.full((3,), 2.0))
+
+
+def test_kernels_let_their_successor_in_after_their_tensor_memory():
+    """A successor that starts early must not take tensor memory that the kernel in front has yet to allocate, since it waits
+    for that kernel: grid_go() follows the allocation in the warp that allocates."""
+    import re
+
+    found = 0
+    for src in build.sources():
+        code = re.sub(r"//[^\n]*", "", src.read_text())
+        for kernel in code.split("__global__")[1:]:
+            if "tmem_alloc<" not in kernel or "grid_go(" not in kernel:
+                continue
+            found += 1
+            alloc, go = kernel.index("tmem_alloc<"), kernel.index("grid_go(")
+            # one block of one warp: nothing between the two closes it
+            assert alloc < go and "}" not in kernel[alloc:go], src.name
+    assert found == 4
