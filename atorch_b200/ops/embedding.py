@@ -3,10 +3,12 @@ from __future__ import annotations
 
 import torch
 import torch.nn as nn
-from torch.autograd import forward_ad
 from torch.nn.modules import module as nn_module
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from .. import _lib
+from .function import watched
 
 
 def embedding_grad(dy: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, accumulate: bool) -> torch.Tensor:
@@ -33,9 +35,10 @@ class _EmbeddingFn(torch.autograd.Function):
         return torch.embedding(weight, ids)
 
     @staticmethod
-    @torch.autograd.function.once_differentiable
     def backward(ctx, dy):
         ids, = ctx.saved_tensors
+        if torch.is_grad_enabled() or watched(dy, ids):   # a second derivative, a batch of gradients, a dispatch mode
+            return None, torch.ops.aten.embedding_dense_backward(dy, ids, ctx.weight_shape[0], -1, False)
         mg = getattr(ctx.weight_ref, "main_grad", None)
         if mg is None:
             return None, embedding_grad(dy, ids, torch.empty(ctx.weight_shape, dtype=dy.dtype, device=dy.device), False)
@@ -53,9 +56,10 @@ class _EmbeddingFn(torch.autograd.Function):
 def _plain(m: nn.Module) -> bool:
     """Nothing but ``F.embedding`` on the weight: no option of it, and nobody who watches or replaces the call."""
     return (type(m) is nn.Embedding and m.padding_idx is None and m.max_norm is None and not m.sparse
-            and not m.scale_grad_by_freq and "forward" not in m.__dict__
+            and not m.scale_grad_by_freq and "forward" not in m.__dict__ and m._compiled_call_impl is None
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks)
-            and not nn_module._has_any_global_hook())
+            and not nn_module._has_any_global_hook()
+            and all(type(mode) is DeviceContext for mode in _get_current_function_mode_stack()))
 
 
 def embedding(module: nn.Module, ids: torch.Tensor) -> torch.Tensor:
@@ -64,7 +68,6 @@ def embedding(module: nn.Module, ids: torch.Tensor) -> torch.Tensor:
         w = module.weight
         if (w.requires_grad and type(w) is nn.Parameter and w.is_cuda and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0
                 and ids.numel() < 2 ** 30 and w.numel() > 0 and not w._backward_hooks and not w._post_accumulate_grad_hooks
-                and _lib.use_kernels(w) and not torch._C._are_functorch_transforms_active()
-                and forward_ad._current_level < 0 and torch._C._get_tracing_state() is None):
+                and _lib.use_kernels(w) and not watched(ids, w)):
             return _EmbeddingFn.apply(ids, w)
     return module(ids)

@@ -1,8 +1,21 @@
-"""Calls of the operators' autograd functions where nothing can ask for a gradient."""
+"""Who looks at the operators' calls, and calls of their autograd functions where nothing can ask for a gradient."""
 from __future__ import annotations
+
+from typing import Optional
 
 import torch
 from torch.autograd import forward_ad
+
+
+def watched(*ts: Optional[torch.Tensor]) -> bool:
+    """Whether something other than reverse-mode autograd looks at operations on these tensors (a functorch transform,
+    forward-mode differentiation, a batch of gradients, a tracer or another dispatch mode, a tensor subclass): kernels called by
+    address would hide them from it, tensor operations do not."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
+            or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0
+            or torch._ops._len_torch_dispatch_stack_pre_dispatch() > 0
+            or any(type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_legacy_batchedtensor(t)
+                   or forward_ad.unpack_dual(t).tangent is not None for t in ts if t is not None))
 
 
 class _NoGradContext:

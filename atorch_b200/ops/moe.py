@@ -18,6 +18,7 @@ import torch
 
 from .. import _lib
 from .elementwise import swiglu, swiglu_backward
+from .function import watched
 from .gemm import gemm, gemm_k_groups, gemm_ragged, k_groups_ok, linear, ragged_ok
 
 
@@ -26,22 +27,11 @@ def tokens_per_expert(expert_idx: torch.Tensor, num_experts: int) -> torch.Tenso
     return torch.bincount(expert_idx.reshape(-1), minlength=num_experts)
 
 
-def _watched(*ts: Optional[torch.Tensor]) -> bool:
-    """Whether something other than reverse-mode autograd looks at these operations (a functorch transform, forward-mode
-    differentiation, a batch of gradients, a tracer or another dispatch mode, a tensor subclass): the row kernels would hide
-    them from it, tensor operations do not."""
-    return (torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
-            or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0
-            or torch._ops._len_torch_dispatch_stack_pre_dispatch() > 0
-            or any(type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_legacy_batchedtensor(t)
-                   or torch.autograd.forward_ad.unpack_dual(t).tangent is not None for t in ts if t is not None))
-
-
 def _rows_ok(rows: torch.Tensor, order: torch.Tensor) -> bool:
     """Whether the row kernels (csrc/moe_local.cu) take these rows: bf16 on the GPU in 16-byte pieces, int64 order."""
     return (_lib.use_kernels(rows, order) and rows.dtype == torch.bfloat16 and rows.dim() == 2 and rows.shape[1] % 8 == 0
             and rows.shape[1] > 0 and order.dtype == torch.int64 and order.dim() == 1 and order.is_contiguous()
-            and 0 < order.numel() < 1 << 31 and not _watched(rows, order))
+            and 0 < order.numel() < 1 << 31 and not watched(rows, order))
 
 
 def _slots(order: torch.Tensor) -> torch.Tensor:
@@ -84,7 +74,7 @@ class _Permute(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (slot,) = ctx.saved_tensors
-        if torch.is_grad_enabled() or _watched(dy):     # operations that autograd and the others can follow
+        if torch.is_grad_enabled() or watched(dy):     # operations that autograd and the others can follow
             return dy.index_select(0, slot).view(ctx.T, ctx.k, -1).sum(1), None, None, None
         return _gather_sum(_packed(dy), slot, None, ctx.T, ctx.k), None, None, None
 
@@ -102,7 +92,7 @@ class _Unpermute(torch.autograd.Function):
     def backward(ctx, dout):
         rows, order, probs = ctx.saved_tensors
         need_dw = ctx.needs_input_grad[2]
-        if torch.is_grad_enabled() or _watched(dout):   # operations that autograd and the others can follow
+        if torch.is_grad_enabled() or watched(dout):   # operations that autograd and the others can follow
             d, dw = dout.index_select(0, order // ctx.k), None
             if need_dw:
                 dots = (rows * d).sum(-1).to(probs.dtype)
@@ -170,7 +160,7 @@ def unpermute(permuted: torch.Tensor, sorted_idx: torch.Tensor, probs: Optional[
     if topk >= 1 and _rows_ok(permuted, sorted_idx) and n_slots == sorted_idx.numel() == permuted.shape[0] \
             and n_slots % topk == 0 and (probs is None or (probs.numel() == n_slots and probs.is_cuda
                                                            and probs.dtype in (torch.bfloat16, torch.float32)
-                                                           and not _watched(probs))):
+                                                           and not watched(probs))):
         return _Unpermute.apply(permuted, sorted_idx, probs, topk, slots)
     return unpermute_reference(permuted, sorted_idx, probs, topk, n_slots)
 

@@ -319,3 +319,44 @@ def test_embedding_module_gradient_and_fallbacks():
     m.register_forward_hook(lambda *a: seen.append(1))
     ops.embedding(m, ids)
     assert seen == [1]
+
+
+@pytest.mark.parametrize("dtype,off", [(torch.bfloat16, 0), (torch.float32, 1), (torch.float64, 0)])
+def test_embedding_into_an_untouched_buffer(dtype, off):
+    """A gradient buffer that nothing has been written to is overwritten, also one that the kernels do not take."""
+    m = torch.nn.Embedding(300, 64).cuda().bfloat16()
+    ids = torch.randint(0, 300, (150,), device="cuda")
+    m.weight.main_grad = torch.full((300 * 64 + off,), float("nan"), dtype=dtype, device="cuda")[off:].view(300, 64)
+    m.weight._atb_first = True
+    w = torch.randn(150, 64, device="cuda").bfloat16()
+    ops.embedding(m, ids).backward(w)
+    want = torch.zeros(300, 64, dtype=torch.float64, device="cuda").index_add(0, ids, w.double())
+    torch.testing.assert_close(m.weight.main_grad.double(), want, rtol=2.0 ** -8, atol=1e-6)     # one rounding to bf16
+    assert m.weight._atb_first is False and m.weight.grad_added_to_main_grad
+
+
+def test_embedding_leaves_watched_calls_to_the_module():
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    m = torch.nn.Embedding(300, 64).cuda().bfloat16()
+    ids = torch.randint(0, 300, (150,), device="cuda")
+    node = lambda: ops.embedding(m, ids).grad_fn.name()
+    own = node()
+    assert "_EmbeddingFn" in own
+    with torch.device("cuda"):          # says where tensors are made, looks at nothing
+        assert node() == own
+    for mode in (Dispatch(), Function()):
+        with mode:
+            assert node() != own
+    seen = []
+    m._compiled_call_impl = lambda *a: seen.append(a) or m.forward(*a)      # what module.compile() sets
+    assert node() != own and len(seen) == 1
