@@ -4,6 +4,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+from torch._functorch.utils import unwrap_dead_wrappers
 from torch.autograd import forward_ad
 
 
@@ -32,8 +33,9 @@ def call(function, *args):
     and re-wraps every argument and reports ``needs_input_grad`` by the flags of the inputs even then (5 of the 21 us that a
     linear layer takes on the host, and the gate|up tensor of the first pass of a checkpointed block was written for nobody:
     90 MB per layer at 4096 x 5504). Anything that looks into calls, a transform, forward-mode differentiation or a tracer,
-    still gets ``apply``, which either serves it or refuses."""
+    still gets ``apply``, which either serves it or refuses. (Under a dispatch mode and for a tensor subclass ``apply`` runs the
+    same ``forward`` on the same arguments.) A tensor that has outlived its transform is unwrapped, as ``apply`` does."""
     if torch.is_grad_enabled() or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0 \
             or torch._C._get_tracing_state() is not None:
         return function.apply(*args)
-    return function.forward(_NoGradContext(), *args)
+    return function.forward(_NoGradContext(), *unwrap_dead_wrappers(args))

@@ -90,6 +90,23 @@ def test_call_without_gradients():
         assert torch.equal(call(_Double, torch.ones(3)), torch.full((3,), 2.0))
 
 
+class _Address(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return torch.tensor(x.data_ptr())
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_call_on_a_tensor_that_outlived_its_transform():
+    kept = []
+    torch.func.grad(lambda t: (kept.append(t), (t * t).sum())[1])(torch.ones(3))
+    with torch.no_grad():
+        assert call(_Address, kept[0]).item() == _Address.apply(kept[0]).item() != 0
+
+
 def test_kernels_let_their_successor_in_after_their_tensor_memory():
     """A successor that starts early must not take tensor memory that the kernel in front has yet to allocate, since it waits
     for that kernel: grid_go() follows the allocation in the warp that allocates."""
