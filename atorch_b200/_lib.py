@@ -25,7 +25,8 @@ class KernelError(RuntimeError):
 
 
 # Argument types of the launchers on the per-operator path (p: pointer, i: int, l: long long, f: float), checked against
-# csrc/ by a test. They are called through csrc/launcher.c with plain Python numbers; the others through ctypes.
+# csrc/ by a test. They are called through csrc/launcher.c with plain Python numbers; the others, and all of them where that
+# module has not been built for this Python, through ctypes.
 SIGNATURES = {
     "atb_gemm_bf16_2cta": "ppppiiillliiiifiiplpp",
     "atb_gemm_bf16_2cta_grouped": "ppppiiillliiiifiiplpiiiiipp",
@@ -60,7 +61,7 @@ _NOT_LAUNCHES = {"atb_norm_bwd_parts", "atb_sumsq_parts", "atb_set_comm_wait_ns"
 
 def __getattr__(name):
     if name == "launch_count":       # kernels of this library launched so far in this process
-        return _ctypes_launches + (0 if _lib is None else _lib.launcher.count())
+        return _ctypes_launches + (0 if _lib is None or _lib.launcher is None else _lib.launcher.count())
     raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
@@ -73,11 +74,14 @@ class _CountingLib:
 
     def __getattr__(self, name):     # once per name: the function becomes an attribute
         raw = getattr(self._cdll, name)
-        if name in SIGNATURES:
+        if name in SIGNATURES and self.launcher is not None:
             fn = self.launcher.Launcher(ctypes.cast(raw, ctypes.c_void_p).value, SIGNATURES[name])
         elif name in _NOT_LAUNCHES:
             fn = raw
         else:
+            if name in SIGNATURES:
+                raw.argtypes = [_CTYPE[c] for c in SIGNATURES[name]]
+
             def fn(*a, _raw=raw):
                 global _ctypes_launches
                 _ctypes_launches += 1
@@ -90,8 +94,12 @@ class _CountingLib:
 
 
 def _load_launcher():
-    """The extension module next to the library (csrc/launcher.c)."""
-    spec = importlib.util.spec_from_file_location("_launcher", _LIB_PATH.with_name("_launcher.so"))
+    """The extension module next to the library (csrc/launcher.c), or None where this Python has none and cannot build it."""
+    from . import build as _build
+
+    if not _build.LAUNCHER.exists() and not (os.environ.get("ATB_AUTO_BUILD", "1") == "1" and _build.build_launcher()):
+        return None
+    spec = importlib.util.spec_from_file_location("_launcher", _build.LAUNCHER)
     module = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(module)
     return module
@@ -111,7 +119,7 @@ def lib():
     if _tried:
         raise KernelError(f"{_LIB_PATH} could not be loaded")
     _tried = True
-    if not (_LIB_PATH.exists() and _LIB_PATH.with_name("_launcher.so").exists()):
+    if not _LIB_PATH.exists():
         if os.environ.get("ATB_AUTO_BUILD", "1") == "1":
             from . import build as _build
 

@@ -3,8 +3,9 @@
 Every ``csrc/*.cu`` file is compiled with ``nvcc -gencode arch=compute_100a,code=sm_100a`` into an
 object file and the objects are linked into one shared library, ``atorch_b200/_C/libatb.so``, that
 exposes plain ``extern "C"`` launchers (loaded by :mod:`atorch_b200._lib`). nvcc cross-compiles, so the build
-needs no GPU. Objects are rebuilt only when a source or header is newer. ``_C/_launcher.so`` beside it makes the launchers
-callable from Python at little cost (C, a second to compile).
+needs no GPU. Objects are rebuilt only when a source or header is newer. ``_C/_launcher.<ABI>.so`` beside it makes the launchers
+callable from Python at little cost (C, a second to compile); it belongs to one Python, so its name says to which. Without a
+C compiler or Python's headers it is left out, and the launchers are called through ctypes.
 
 Plays the role of the JIT op builder of the reference (atorch/ops/op_builder/builder.py:120-681),
 but ahead of time and for one architecture only.
@@ -20,6 +21,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent
@@ -27,7 +29,8 @@ CSRC = ROOT / "csrc"
 OUT_DIR = ROOT / "_C"
 OBJ_DIR = OUT_DIR / "obj"
 LIB = OUT_DIR / "libatb.so"
-LAUNCHER = OUT_DIR / "_launcher.so"      # Python callables for the launchers (csrc/launcher.c)
+# Python callables for the launchers (csrc/launcher.c), for this Python
+LAUNCHER = OUT_DIR / ("_launcher" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -66,10 +69,24 @@ def _build_launcher(force: bool) -> None:
     cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
     if cc is None:
         raise RuntimeError("no C compiler found; set CC or add gcc to PATH")
-    cmd = [cc, "-O2", "-Wall", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(LAUNCHER)]
+    OUT_DIR.mkdir(parents=True, exist_ok=True)
+    tmp = LAUNCHER.with_name(f"{LAUNCHER.name}.{os.getpid()}.tmp")     # other processes see the whole file or none
+    cmd = [cc, "-O2", "-Wall", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(tmp)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
+        tmp.unlink(missing_ok=True)
         raise RuntimeError(f"{cc} failed for {src.name}:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, LAUNCHER)
+
+
+def build_launcher(force: bool = False) -> bool:
+    """Whether there is a launcher module for this Python, after building it where that can be done."""
+    try:
+        _build_launcher(force)
+    except (RuntimeError, OSError) as e:
+        warnings.warn(f"kernels will be launched through ctypes, 2 us a call more: {e}")
+        return False
+    return True
 
 
 def sources() -> list[Path]:
@@ -79,7 +96,6 @@ def sources() -> list[Path]:
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = find_nvcc()
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
-    _build_launcher(force)
     hdr_m = _newest_header_mtime()
     todo, objs = [], []
     for src in sources():
@@ -99,6 +115,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_launcher(force)
     return LIB
 
 

@@ -56,6 +56,36 @@ def test_arguments_in_registers_and_on_the_stack(tmp_path):
         launcher.Launcher(1, "px")
 
 
+def test_launcher_belongs_to_one_python(tmp_path, monkeypatch):
+    """Its name says to which; it appears whole; what is left where it cannot be built is ctypes, with the same calls."""
+    import sysconfig
+
+    from atorch_b200 import _lib
+
+    assert build.LAUNCHER.name == "_launcher" + sysconfig.get_config_var("EXT_SUFFIX")
+    launcher, lib, _ = _module(tmp_path)
+    monkeypatch.setattr(build, "OUT_DIR", tmp_path)
+    monkeypatch.setattr(build, "LAUNCHER", tmp_path / build.LAUNCHER.name)
+    monkeypatch.setenv("CC", "false")
+    with pytest.warns(UserWarning, match="ctypes"):
+        assert not build.build_launcher()
+    with pytest.warns(UserWarning, match="ctypes"):
+        assert _lib._load_launcher() is None
+    assert not list(tmp_path.glob("_launcher*"))
+    monkeypatch.setitem(_lib.SIGNATURES, "mixed", "ppilfiplifiipilfilii")
+    monkeypatch.setattr(_lib, "_ctypes_launches", 0)
+    arr = (ctypes.c_int * 2)(21, -22)
+    args = (1 << 40, None, -3, -(1 << 40), 1.5, True, None, 7, 5, 2.0, 9, -11, ctypes.addressof(arr), -1, 1 << 50, 0.25, 13, -14,
+            -15, 16)
+    seen = []
+    for module in (launcher, None):
+        assert _lib._CountingLib(lib, module).mixed(*args) == -7
+        seen.append(lib.last()[:21])
+    assert seen[0] == seen[1] and _lib._ctypes_launches == 1
+    monkeypatch.delenv("CC")
+    assert build.build_launcher() and [f.name for f in tmp_path.glob("_launcher*")] == [build.LAUNCHER.name]
+
+
 class _Double(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x):
