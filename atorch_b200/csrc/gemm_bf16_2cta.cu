@@ -234,8 +234,8 @@ ATB_DEVICE void tma_load_2d_pair(void* smem_dst, const CUtensorMap* tm, uint32_t
 // Dynamic tile scheduling: tiles are handed out by an atomic counter instead of a fixed stride, so that a CTA pair
 // that shares its SMs with another kernel (a reduce-scatter or copy kernel of the communication streams takes part
 // of the SM's path to L2, on which this kernel's operand loads depend) simply takes fewer tiles, instead of making
-// the whole launch wait for it. counters[0] = next tile, counters[1] = pairs that have finished; both are zero
-// between launches (the pair that finishes last clears them).
+// the whole launch wait for it. Where two pairs share a tile, their cluster of four draws as one. counters[0] = next tile,
+// counters[1] = clusters that have finished; both are zero between launches (the cluster that finishes last clears them).
 struct Sched {
   int* counters;   // nullptr: static schedule (tile = pair + i * pairs)
   int early;       // the launch after this one may take the SMs that this one leaves
@@ -356,7 +356,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(&tempty[1], 2 * EPI_WARPS);
       for (int i = 0; i < TQ; ++i) {
         mbar_init(&tq_full[i], 1);
-        mbar_init(&tq_empty[i], 2 + 2 * EPI_WARPS);   // leader: MMA + epilogue warps; partner: producer + epilogue warps
+        mbar_init(&tq_empty[i], SPLIT * (2 + 2 * EPI_WARPS) + SPLIT - 1);   // every CTA's epilogue warps, every pair's MMA
+                                                                             // warp, every producer but the one that draws
       }
       mbar_init(xfull, EPI_WARPS);
       mbar_init(xfree, EPI_WARPS);
@@ -437,34 +438,40 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     }
   };
 
-  // The idx-th tile of this pair, the same number in every role of both CTAs. Static: a fixed stride. Dynamic: the
-  // leader's producer thread draws it from the global counter and publishes it through a ring of tile ids in the
-  // shared memory of both CTAs; every other role reads it there and frees the slot.
-  const bool dyn = sched.counters != nullptr;
+  // The idx-th tile of this cluster, the same number in every role of all its CTAs. Static: a fixed stride. Dynamic: the
+  // first CTA's producer thread draws it from the global counter and publishes it through a ring of tile ids in the
+  // shared memory of all CTAs; every other role reads it there and frees the slot.
+  const bool dyn = sched.counters != nullptr, draws = cta == 0;
+  // A cluster of four begins with the tile of its own number and draws and publishes the next one AHEAD k-blocks before
+  // the end of its loads: four CTAs take longer to hear of it.
+  constexpr int GIVEN = SPLIT == 2 ? 1 : 0, AHEAD = 8;
   auto static_tile = [&](int idx) -> int {
     const int t = cluster_id + idx * num_clusters;
     return t < num_tiles ? t : -1;
   };
-  auto publish_tile = [&](int idx, int t) -> bool {          // leader's producer warp
-    const int slot = idx % TQ;
-    if (!mbar_wait_warp(&tq_empty[slot], ((idx / TQ) & 1) ^ 1, abort_flag, status)) return false;
+  auto publish_tile = [&](int idx, int t) -> bool {          // the producer warp that draws
+    const int slot = (idx - GIVEN) % TQ;
+    if (!mbar_wait_warp(&tq_empty[slot], (((idx - GIVEN) / TQ) & 1) ^ 1, abort_flag, status)) return false;
     if (lane == 0) {
       tq_tile[slot] = t;
-      st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), pair0 + 1), (uint32_t)t);
       mbar_arrive(&tq_full[slot]);
-      mbar_arrive_remote(map_to_cta(&tq_full[slot], pair0 + 1));     // release.cluster: orders the store above
+#pragma unroll
+      for (uint32_t to = 1; to < 2 * SPLIT; ++to) {
+        st_remote_u32(map_to_cta(const_cast<int*>(&tq_tile[slot]), to), (uint32_t)t);
+        mbar_arrive_remote(map_to_cta(&tq_full[slot], to));     // release.cluster: orders the store above
+      }
     }
     return true;
   };
   auto read_tile = [&](int idx) -> int {                      // any other role, a whole warp
-    if (!dyn) return static_tile(idx);
-    const int slot = idx % TQ;
-    if (!mbar_wait_cluster(&tq_full[slot], (idx / TQ) & 1, abort_flag, status)) return -1;
+    if (!dyn || idx < GIVEN) return static_tile(idx);
+    const int slot = (idx - GIVEN) % TQ;
+    if (!mbar_wait_cluster(&tq_full[slot], ((idx - GIVEN) / TQ) & 1, abort_flag, status)) return -1;
     return warp_uniform((int)tq_tile[slot]);
   };
   auto free_tile_slot = [&](int idx) {                        // once per consumer warp, after read_tile by all its lanes
     __syncwarp();
-    if (dyn && lane == 0) mbar_arrive_remote(map_to_cta(&tq_empty[idx % TQ], pair0));
+    if (dyn && idx >= GIVEN && lane == 0) mbar_arrive_remote(map_to_cta(&tq_empty[(idx - GIVEN) % TQ], 0));
   };
 
   if (warp == 0) {
@@ -474,18 +481,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       auto draw = [&]() -> int {
         int d = 0;
         if (lane == 0) d = atomicAdd(&sched.counters[0], 1);
-        return warp_uniform(d);
+        return warp_uniform(d) + GIVEN * num_clusters;
       };
       grid_wait();
-      int drawn = (dyn && leader) ? draw() : 0;
+      int drawn = (dyn && draws && GIVEN == 0) ? draw() : 0;
       // the first tile, as far as it is known without the cluster
-      int tile = dyn ? (leader && drawn < num_tiles ? drawn : -1) : static_tile(0);
+      int tile = dyn && GIVEN == 0 ? (draws && drawn < num_tiles ? drawn : -1) : static_tile(0);
       int m0 = 0, n0 = 0, m_end = 0, b_idx = 0;
       if (tile >= 0) tile_coords(tile, m0, n0, m_end, b_idx);
       cluster_wait_all();
       for (int idx = 0;; ++idx) {
-        if (idx > 0 || (dyn && !leader)) {
-          if (dyn && leader) {
+        if (idx > 0 || (dyn && !draws && GIVEN == 0)) {
+          if (dyn && draws) {
             tile = drawn < num_tiles ? drawn : -1;
           } else {
             tile = read_tile(idx);
@@ -493,10 +500,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           }
           if (tile >= 0) tile_coords(tile, m0, n0, m_end, b_idx);
         }
-        if (dyn && leader) {
-          if (tile >= 0) drawn = draw();                       // the next one, fetched under this tile's loads
-          if (!publish_tile(idx, tile)) goto producer_done;
-          if (tile < 0 && lane == 0) {   // every pair draws exactly one number past the end; the last to do so resets
+        if (dyn && draws) {
+          if (GIVEN == 0) {
+            if (tile >= 0) drawn = draw();                     // the next one, fetched under this tile's loads
+            if (!publish_tile(idx, tile)) goto producer_done;
+          }
+          if (tile < 0 && lane == 0) {   // every cluster draws exactly one number past the end; the last to do so resets
             if (atomicAdd(&sched.counters[1], 1) == num_clusters - 1) {
               sched.counters[0] = 0;
               sched.counters[1] = 0;
@@ -526,6 +535,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           if (!__all_sync(0xffffffffu, here)) goto producer_done;
         }
         for (int kb = kb_first; kb < kb_end; ++kb) {
+          if (GIVEN > 0 && dyn && draws && kb == max(kb_end - AHEAD, kb_first)) {
+            drawn = draw();
+            if (!publish_tile(idx + 1, drawn < num_tiles ? drawn : -1)) goto producer_done;
+          }
           if (!kb_active(kb)) continue;
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -1030,16 +1043,20 @@ int split_clusters() {
 }
 
 // Whether two pairs per tile finish earlier than one, in waves of k-blocks: a wave of half tiles takes a tenth longer per
-// k-block when all SMs load, and the exchange at its end costs as much as 14 k-blocks (4 us). Cold L2, one / two pairs (us), tiles and
-// k-blocks: 8 x 172 61.4 / 41.0; 16 x 86 37.7 / 28.8; 32 x 86 39.6 / 31.5; 96 x 86 71.7 / 63.5; 96 x 172 122.9 / 106.5; about
-// even: 32 x 32 22.5 / 21.3, 96 x 32 36.9 / 36.9; not: 48 x 86 41.0 / 45.1, 172 x 32 49.9 / 56.0, 16 x 8 14.4 / 16.4.
+// k-block when all SMs load, the exchange at its end costs as much as 14 k-blocks (4 us), and a further tile, drawn by four CTAs,
+// 1.5 more. Cold L2, one / two pairs (us), tiles and k-blocks: 8 x 172 59.4 / 43.0; 16 x 86 36.9 / 28.7; 32 x 86 36.9 / 30.7;
+// 96 x 86 71.7 / 67.6; 96 x 172 124.9 / 110.6; about even: 80 x 64 55.3 / 55.3, 96 x 64 57.3 / 55.3; not: 80 x 58 51.2 / 53.2,
+// 48 x 86 38.9 / 49.2, 104 x 86 73.7 / 81.9, 222 x 86 104.4 / 133.1.
+// Beside a kernel that takes 24 SMs for itself fewer clusters of four find room than pairs: 16 x 86 36.9 / 32.8, 24 x 86 36.9 / 34.8, but
+// 32 x 86 38.9 / 57.3, 96 x 86 73.7 / 92.2 (115.6 with a fixed share of tiles); one that takes 8, 96 x 86 73.7 / 67.6.
 bool split_pays(int tiles, int kbs, int wish) {
   if (kbs < 2 || wish < 0) return false;
   const int pairs = sm_count() / 2;
   const long long whole = (long long)((tiles + pairs - 1) / pairs) * kbs;
   auto pays = [&](int clusters) {
-    return clusters > 0 &&
-           (wish > 0 || (long long)((tiles + clusters - 1) / clusters) * ((kbs + 1) / 2) * 110 + 1400 < whole * 95);
+    if (clusters <= 0) return false;
+    const long long waves = (tiles + clusters - 1) / clusters;
+    return wish > 0 || waves * ((kbs + 1) / 2) * 110 + 1400 + 150 * (waves - 1) < whole * 95;
   };
   return pays(pairs / 2) && pays(split_clusters());      // the second number takes a driver call: only where it can matter
 }
@@ -1094,7 +1111,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
   int clusters = SPLIT == 2 ? split_clusters() : sm_count() / 2;
   if (tiles < clusters) clusters = tiles;
   if (max_ctas > 0 && clusters > max_ctas / 2) clusters = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
-  // Dynamic tile scheduling for plain launches with more tiles than CTA pairs (see Sched). A launch that waits for other ranks, and
+  // Dynamic tile scheduling for plain launches with more tiles than clusters (see Sched). A launch that waits for other ranks, and
   // one with a limit on its CTAs, keep the SMs that they leave free for what runs beside them, a transfer: the launch after
   // them would sit there and wait.
   Sched sched{nullptr, gate.flags == nullptr && max_ctas <= 0};
@@ -1102,7 +1119,7 @@ int launch(const void* A, const void* B, const Epi& ep, int M, int N, int K, lon
     const char* e = getenv("ATB_GEMM_DYNAMIC");
     g_dynamic = (e != nullptr && e[0] == '0') ? 0 : 1;
   }
-  if (SPLIT == 1 && g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
+  if (g_dynamic > 0 && tiles > clusters && grp.counts == nullptr && (grp.b_rows == 0 || rag.n > 0) &&
       gate.flags == nullptr)
     sched.counters = sched_counters(stream);
   const cudaError_t e = launch_after(kern, dim3(2 * SPLIT * clusters), THREADS, SMEM_TOTAL, stream, 2 * SPLIT, tmA, tmB, tmC, epw, M,

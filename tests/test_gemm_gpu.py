@@ -772,3 +772,27 @@ def test_launch_with_a_limit_leaves_the_other_sms_free():
     torch.cuda.synchronize()
     _lib.check_status(a.device)
     assert first.elapsed_time(last) > 1.0
+
+
+def test_shared_tiles_beside_another_kernel():
+    """Two pairs per tile, six tiles per cluster, while a launch of another stream holds 24 SMs: the clusters that fit share the
+    tiles. With a fixed share of six, those that start when the first ones end double the time."""
+    held, side = _mk(8192, 8192), torch.cuda.Stream()
+    x, w = _mk(37 * 256, 2048), _mk(6 * 256, 2048)
+    out, ms = torch.empty(37 * 256, 6 * 256, device="cuda", dtype=torch.bfloat16), {}
+    for hold in (False, True, False, True):
+        torch.cuda.synchronize()
+        if hold:
+            with torch.cuda.stream(side):
+                gemm(held, held, max_ctas=24)
+        first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        out.fill_(float("nan"))
+        torch.cuda._sleep(400000)            # the launch of the other stream has its SMs
+        first.record()
+        gemm(x, w, out=out, tile_n=512)
+        last.record()
+        torch.cuda.synchronize()
+        ms[hold] = first.elapsed_time(last)
+        _check(out, x.float() @ w.float().t(), 2048)
+    _lib.check_status(x.device)
+    assert ms[True] < 1.5 * ms[False], ms
