@@ -56,7 +56,8 @@ SIGNATURES = {
 _CTYPE = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float}
 
 _ctypes_launches = 0
-_NOT_LAUNCHES = {"atb_norm_bwd_parts", "atb_sumsq_parts", "atb_set_comm_wait_ns", "atb_noalloc_max_n"}
+_NOT_LAUNCHES = {"atb_norm_bwd_parts", "atb_sumsq_parts", "atb_set_comm_wait_ns", "atb_noalloc_max_n",
+                 "atb_embedding_bwd_scratch"}
 
 
 def __getattr__(name):

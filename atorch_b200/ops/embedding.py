@@ -1,6 +1,9 @@
 """Token embedding whose gradient goes straight into ``weight.main_grad`` (``csrc/embedding.cu``)."""
 from __future__ import annotations
 
+import ctypes
+import functools
+
 import torch
 import torch.nn as nn
 from torch.nn.modules import module as nn_module
@@ -11,15 +14,22 @@ from .. import _lib
 from .function import watched
 
 
+@functools.cache
+def _words():
+    fn = _lib.lib().atb_embedding_bwd_scratch
+    fn.restype = ctypes.c_longlong
+    return fn
+
+
 def embedding_grad(dy: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, accumulate: bool) -> torch.Tensor:
-    """``out[v] (+)= sum of dy over the tokens whose id is v`` (bf16 ``dy``; fp32 sums in the order of the tokens)."""
+    """``out[v] (+)= sum of dy over the tokens whose id is v`` (bf16 ``dy``; fp32 sums in an order that the ids alone decide)."""
     V, H = out.shape
     T = ids.numel()
     dy = dy.reshape(T, H).contiguous()
     if dy.data_ptr() % 16:
         dy = dy.clone()
     ids = ids.contiguous()
-    scratch = torch.empty(V + 1 + T, dtype=torch.int32, device=out.device)
+    scratch = torch.empty(_words()(T, V, H), dtype=torch.int32, device=out.device)
     rc = _lib.lib().atb_embedding_bwd(dy.data_ptr(), ids.data_ptr(), out.data_ptr(), scratch.data_ptr(), T, V, H,
                                       int(out.dtype == torch.float32), int(accumulate), _lib.stream())
     _lib.check(rc, f"atb_embedding_bwd T={T} V={V} H={H}")

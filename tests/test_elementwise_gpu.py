@@ -360,3 +360,51 @@ def test_embedding_leaves_watched_calls_to_the_module():
     seen = []
     m._compiled_call_impl = lambda *a: seen.append(a) or m.forward(*a)      # what module.compile() sets
     assert node() != own and len(seen) == 1
+
+
+@pytest.mark.parametrize("out_dtype,accumulate", [(torch.bfloat16, False), (torch.float32, True)])
+@pytest.mark.parametrize("counts,V,H", [
+    ((512,), 1, 8),                                        # the most that one block sums, and one more
+    ((513,), 2, 520),
+    ((1, 511, 512, 513, 1023, 1024, 1025, 0, 200, 600, 1400, 1), 40, 264),    # rows that begin and end everywhere in a part
+    ((600, 0, 600, 600, 5, 6000), 3000, 1032),
+])
+def test_embedding_gradient_of_long_rows(counts, V, H, out_dtype, accumulate):
+    from atorch_b200.ops.embedding import embedding_grad
+
+    g = torch.Generator().manual_seed(sum(counts))
+    rows = torch.randperm(V, generator=g)[: len(counts)].sort().values
+    ids = torch.repeat_interleave(rows, torch.tensor(counts[: len(rows)]))
+    ids = ids[torch.randperm(ids.numel(), generator=g)]
+    dy = torch.randn(ids.numel(), H, generator=g).bfloat16()
+    old = torch.randn(V, H, generator=g).to(out_dtype)
+    out = old.cuda() if accumulate else torch.full((V, H), float("nan"), dtype=out_dtype, device="cuda")
+    embedding_grad(dy.cuda(), ids.cuda(), out, accumulate)
+    want = (old.double() if accumulate else torch.zeros(V, H, dtype=torch.float64)).index_add(0, ids, dy.double())
+    size = (old.double().abs() if accumulate else torch.zeros(V, H, dtype=torch.float64)).index_add(0, ids, dy.double().abs())
+    # as many fp32 additions as a row has tokens, and one rounding to the output type
+    bound = size * (max(counts) + 1) * 2.0 ** -23 + (want.abs() * 2.0 ** -8 if out_dtype == torch.bfloat16 else 0.0)
+    assert bool(((out.double().cpu() - want).abs() <= bound).all())
+    again = old.cuda() if accumulate else torch.empty_like(out)
+    assert torch.equal(embedding_grad(dy.cuda(), ids.cuda(), again, accumulate), out)
+
+
+def test_embedding_gradient_time_does_not_depend_on_the_ids():
+    """A row with most of the tokens (padding), and a table of few rows, take about as long as tokens spread over a large one."""
+    from atorch_b200.ops.embedding import embedding_grad
+
+    T, H, us = 65536, 1024, {}
+    dy = torch.randn(T, H, device="cuda").bfloat16()
+    for name, V, ids in (("spread", 32000, torch.randint(0, 32000, (T,), device="cuda")),
+                         ("one", 32000, torch.zeros(T, dtype=torch.int64, device="cuda")),
+                         ("few", 256, torch.randint(0, 256, (T,), device="cuda"))):
+        out = torch.zeros(V, H, device="cuda", dtype=torch.bfloat16)
+        for _ in range(5):
+            first, last = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda._sleep(200000)
+            first.record()
+            embedding_grad(dy, ids, out, True)
+            last.record()
+            torch.cuda.synchronize()
+            us[name] = min(us.get(name, 1e9), 1e3 * first.elapsed_time(last))
+    assert us["one"] < 3 * us["spread"] and us["few"] < 3 * us["spread"], us
