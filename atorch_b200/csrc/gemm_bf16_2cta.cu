@@ -51,9 +51,11 @@ struct Cfg {
   static constexpr int STAGES = SPLIT == 2 ? 5 : BN == 256 ? 6 : 8;
   static constexpr int B_BYTES = BNH * BK * 2;
   static constexpr int X_OFF = STAGES * (A_BYTES + B_BYTES);         // partial sums from the other pair, fp32
-  // output boxes on their way out (see the epilogue): 4 KB per epilogue warp, [32 rows][128 bytes] with 128-byte swizzle
-  static constexpr int OUT_OFF = X_OFF;
-  static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 8 * 4096);
+  // output boxes on their way out (see the epilogue): 4 KB per epilogue warp, [32 rows][128 bytes] with 128-byte swizzle, in the place
+  // of the operands, all of which have been multiplied by then. Space of their own took half of the L1 cache, in which an
+  // epilogue that adds to fp32 values keeps their lines: 4096 x 4096 x 256 67.6 -> 84.2 us.
+  static constexpr int OUT_OFF = 0;
+  static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 0);
   static constexpr int TQ = 4;                     // tile-id ring of the dynamic scheduler
   static constexpr int SMEM_TOTAL = BAR_OFF + (2 * STAGES + 4 + 2 * TQ + 3) * 8 + 16 + TQ * 4 + 1024;
   static_assert(SMEM_TOTAL <= 232448, "shared memory of the pair kernel exceeds 227 KB");
