@@ -28,6 +28,7 @@
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -684,10 +685,18 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       store_row_bf16(crow, o1, N - col0, wide);
       store_row_bf16(crow + hd2, o2, N - col0 - hd2, wide);
     };
+    // A body for each kind of output, chosen outside of the loop over the columns: with one for all, the registers for what is
+    // added and the choices cost those that need neither 6 % (32000 x 2048 x 512 75.8 us, with one body 81.9; with a bias 101 and 120).
+    constexpr int PLAIN = 0, FP32 = 1, ADD = 2, ANY = 3;   // bf16; fp32, alone or added to; bf16 and one thing added; the rest
+    constexpr std::integral_constant<int, ANY> any{};
+    const int output = ep.bias != nullptr || ep.rs_rows > 0 || (ep.residual != nullptr && (ep.accumulate || ep.out_fp32)) ? ANY
+                       : ep.out_fp32 ? FP32 : ep.residual == nullptr && !ep.accumulate ? PLAIN : ADD;
     // 32 bf16 values that are added to a row's accumulators, the residual or, when accumulating, the output so far, in four loads
-    // at once; with a test of the column around each, they came one after the other, 16 times the latency of the L2 per tile
-    // (not in the grouped weight gradients, which the registers for it made 1.5 % slower)
-    const __nv_bfloat16* added = KG ? nullptr : ep.residual != nullptr ? reinterpret_cast<const __nv_bfloat16*>(ep.residual)
+    // at once; with a test of the column around each, they came one after the other, 16 times the latency of the L2 per tile.
+    // They are asked for one piece ahead; in the grouped weight gradients, where that slowed down the plain body (8 groups of
+    // 1024 rows, 4096 x 14336, 766 -> 836 us), with the piece: added to 861 us, one after the other 972.
+    const bool bias16 = (reinterpret_cast<uintptr_t>(ep.bias) & 15) == 0;
+    const __nv_bfloat16* added = ep.residual != nullptr ? reinterpret_cast<const __nv_bfloat16*>(ep.residual)
                                  : ep.accumulate && !ep.out_fp32 ? reinterpret_cast<const __nv_bfloat16*>(ep.C) : nullptr;
     const long long added_ld = ep.residual != nullptr ? ep.ldr : ep.ldc;
     auto fetch = [&](uint4 (&x)[4], long long row, int col0) {
@@ -695,18 +704,36 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #pragma unroll
       for (int i = 0; i < 4; ++i) x[i] = p[i];
     };
+    auto add8 = [&](float* v, const uint4& x) {
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack_bf16x2(w[k]);
+        v[2 * k] += f.x;
+        v[2 * k + 1] += f.y;
+      }
+    };
     // x: as fetched, if `fetched` (whole pieces)
-    auto finish_plain = [&](const uint32_t (&r)[32], int row, int col0, long long c_row0, const uint4 (&x)[4], bool fetched) {
+    auto finish_plain = [&](auto kind, const uint32_t (&r)[32], int row, int col0, long long c_row0, uint4 (&x)[4], bool fetched) {
+      constexpr int KIND = decltype(kind)::value;
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]) * ep.alpha;
-      if (ep.bias != nullptr) {
+      if (KIND == ANY && ep.bias != nullptr) {
         const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(ep.bias);
+        if (bias16 && col0 + 32 <= N) {
+          uint4 b[4];
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (col0 + i < N) v[i] += __bfloat162float(bias[col0 + i]);
+          for (int i = 0; i < 4; ++i) b[i] = *reinterpret_cast<const uint4*>(bias + col0 + 8 * i);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) add8(v + 8 * i, b[i]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (col0 + i < N) v[i] += __bfloat162float(bias[col0 + i]);
+        }
       }
-      if (ep.rs_rows > 0) {
+      if (KIND == ANY && ep.rs_rows > 0) {
         const int owner = row / ep.rs_rows;
         float* crow = ep.rs_base[owner] + (long long)(row - owner * ep.rs_rows) * ep.ldc + col0;
 #pragma unroll
@@ -716,7 +743,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                          "f"(v[i + 1]), "f"(v[i + 2]), "f"(v[i + 3])
                          : "memory");
         }
-      } else if (ep.out_fp32) {
+      } else if (KIND == FP32 || (KIND == ANY && ep.out_fp32)) {
         float* crow = reinterpret_cast<float*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
@@ -735,20 +762,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       } else {
         __nv_bfloat16* crow = reinterpret_cast<__nv_bfloat16*>(ep.C) + (c_row0 + row) * ep.ldc + col0;
-        if (fetched) {
+        if ((KIND == ANY || KIND == ADD) && fetched) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t w[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 f = unpack_bf16x2(w[k]);
-              v[8 * i + 2 * k] += f.x;
-              v[8 * i + 2 * k + 1] += f.y;
-            }
-          }
+          for (int i = 0; i < 4; ++i) add8(v + 8 * i, x[i]);
         }
         const bool more = ep.accumulate && ep.residual != nullptr;      // both: the second one here
-        if (more || ((ep.accumulate || ep.residual != nullptr) && !fetched)) {
+        if ((KIND == ANY && more) || ((KIND == ANY || KIND == ADD) && (ep.accumulate || ep.residual != nullptr) && !fetched)) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             if (col0 + i < N) {
@@ -800,7 +819,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const int row = m0 + (int)rank * BM + q * 32 + lane;
       const bool fetching = added != nullptr && row < m_end;
       uint4 xa[4], xb[4];
-      if (SPLIT == 1 && fetching && n0 + half * (BN / 2) + 32 <= N) fetch(xa, c_row0 + row, n0 + half * (BN / 2));
+      if (SPLIT == 1 && !KG && fetching && n0 + half * (BN / 2) + 32 <= N) fetch(xa, c_row0 + row, n0 + half * (BN / 2));
       if (!mbar_wait_warp(&tfull[acc], acc_ph, abort_flag, status)) break;
       tc_fence_after();
       // a producer that found an error in place of its rows went on without them: look again behind it
@@ -898,8 +917,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         } else if (ep.rope_cos != nullptr && col_a < ep.rope_cols) {
           if (col_a < N) finish_rope(ra, rb, row, col_a);
         } else {
-          if (col_a < N) finish_plain(ra, row, col_a, c_row0, xa, fetching && col_a + 32 <= N);
-          if (col_b < N) finish_plain(rb, row, col_b, c_row0, xb, fetching && col_b + 32 <= N);
+          if (col_a < N) finish_plain(any, ra, row, col_a, c_row0, xa, fetching && col_a + 32 <= N);
+          if (col_b < N) finish_plain(any, rb, row, col_b, c_row0, xb, fetching && col_b + 32 <= N);
         }
         continue;
       }
@@ -927,21 +946,30 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
       } else {
         constexpr int CH = BN / 64;              // 32-column pieces of this warp's half
-        uint32_t ra[32], rb[32];
-        tmem_ld_32x32(t_addr + half * (BN / 2), ra);
+        auto pieces = [&](auto kind) {
+          uint32_t ra[32], rb[32];
+          tmem_ld_32x32(t_addr + half * (BN / 2), ra);
 #pragma unroll
-        for (int cc = 0; cc < CH; ++cc) {
-          const int c = half * CH + cc;
-          uint32_t (&r)[32] = (cc & 1) ? rb : ra;
-          uint32_t (&rn)[32] = (cc & 1) ? ra : rb;
-          tmem_ld_wait();
-          if (cc + 1 < CH) {
-            tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
-            if (fetching && n0 + (c + 2) * 32 <= N) fetch((cc & 1) ? xa : xb, c_row0 + row, n0 + (c + 1) * 32);
+          for (int cc = 0; cc < CH; ++cc) {
+            const int c = half * CH + cc;
+            uint32_t (&r)[32] = (cc & 1) ? rb : ra;
+            uint32_t (&rn)[32] = (cc & 1) ? ra : rb;
+            tmem_ld_wait();
+            if (cc + 1 < CH) {
+              tmem_ld_32x32(t_addr + (c + 1) * 32, rn);
+              if (kind == ADD && !KG && fetching && n0 + (c + 2) * 32 <= N)
+                fetch((cc & 1) ? xa : xb, c_row0 + row, n0 + (c + 1) * 32);
+            }
+            if (kind == ADD && KG && fetching && n0 + (c + 1) * 32 <= N) fetch(xa, c_row0 + row, n0 + c * 32);
+            if (in && n0 + c * 32 < N)
+              finish_plain(kind, r, row, n0 + c * 32, c_row0, (kind == ADD && !KG && (cc & 1)) ? xb : xa,
+                           (kind == ADD || (cc == 0 && !KG)) && fetching && n0 + (c + 1) * 32 <= N);
           }
-          if (in && n0 + c * 32 < N)
-            finish_plain(r, row, n0 + c * 32, c_row0, (cc & 1) ? xb : xa, fetching && n0 + (c + 1) * 32 <= N);
-        }
+        };
+        if (output == PLAIN) pieces(std::integral_constant<int, PLAIN>{});
+        else if (output == FP32) pieces(std::integral_constant<int, FP32>{});
+        else if (output == ADD) pieces(std::integral_constant<int, ADD>{});
+        else pieces(any);
       }
       tc_fence_before();
       __syncwarp();
