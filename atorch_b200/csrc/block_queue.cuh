@@ -40,10 +40,9 @@ ATB_DEVICE void queue_init(WorkQueue* q, int reader_warps) {
 }
 
 // The c-th unit of this CTA, by every lane of a reader warp: wait for it (false: the wait ran out), read it, give its place back.
-// The element-wise warps of the forward and the dK/dV kernel hold it until its results are stored, and read it again where they need it: eight values kept
-// in registers through the loop over the tiles slowed that loop by 6 to 8 % (one wave of 8192 keys: head dim 64 139 -> 128 us, 128
-// 128 -> 121; backward of 16 heads of 64 on 8192 keys, all visible 1274 -> 1225, 32 heads of 128, causal 1508 -> 1505, on 8 4096 404 -> 399,
-// but 4096, all visible 762 -> 770). The dQ kernel has registers to spare (1460 -> 1463 us of backward).
+// The element-wise warps of the forward and the dK/dV kernel hold it until its results are stored, and read it again where
+// they need it: eight values kept in registers through the loop over the tiles slowed that loop by 6 to 8 % (one wave of
+// 8192 keys: head dim 64 139 -> 128 us, 128 128 -> 121). In the dQ kernel it makes no difference.
 ATB_DEVICE bool queue_wait(WorkQueue* q, int c, volatile int* abort_flag, int* status) {
   return mbar_wait_warp(&q->full[c & 1], (c >> 1) & 1, abort_flag, status);
 }

@@ -25,9 +25,6 @@ constexpr int PANEL = 128 * 64 * 2;
 constexpr int K_STAGES = 3, V_STAGES = 2;
 constexpr int N_EW = 256;
 constexpr int THREADS = 128 + N_EW;
-// 168 registers a thread at launch (384 x 168 = 64512); the control warpgroup gives up what the element-wise warps need to
-// hold the loads of the next unit beside the results of the last one: 128 x 72 + 256 x 216 = 64512
-constexpr int REGS_CONTROL = 72, REGS_EW = 216;
 
 struct DqParams {
   const float* lse;            // [B, Hq, Sq]
@@ -128,7 +125,6 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // [w.v0, w.v0 + w.v1), of which all rows see the keys [w.v2, w.v3). Barriers of the key blocks count on through all units
   // (g), those of Q, dO and the accumulator count the units that have any block (u).
   if (warp < 4) {
-    reg_dealloc<REGS_CONTROL>();
     if (warp == 2) {
       queue_run(queue, p.order, [&](Work& w, int blocks) {
         w.place = blocks - 1 - w.place;   // heaviest (last) causal blocks first
@@ -259,49 +255,41 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   } else {
-    reg_alloc<REGS_EW>();
     const int quarter = warp & 3;
     const int half = (warp - 4) >> 2;
     const int r = quarter * 32 + lane;
     const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16);
     // delta = dO . O of the block's rows, 16 rows per warp and HD / 8 lanes per row: a separate pass over both tensors took
-    // 26 us at S=4096, 32 heads of 128. What a unit needs from memory is loaded before the results of the one before are stored.
+    // 26 us at S=4096, 32 heads of 128. A unit's values are loaded when it begins, under its first products: holding them from the
+    // end of the unit before took registers that the loop over the tiles needs (16 heads on 8192 keys, all visible, head dim 64
+    // 565 us, now 512; 128 604, now 562; 16 x 512, 16 heads of 64, 59 either way).
     constexpr int LANES = HD / 8, AT_ONCE = 32 / LANES, STEPS = 16 / AT_ONCE;
     const int first = (warp - 4) * 16 + lane / LANES, sub = lane % LANES;
-    struct {
-      uint4 x[STEPS], y[STEPS];
-      float lse;
-      int lo, hi;
-    } in;
-    auto load_unit = [&](const Work& w) {
-      if (!w.more) return;
-      const int b = w.sample, h = w.head, q0 = w.place * BQ;
-#pragma unroll
-      for (int e = 0; e < STEPS; ++e) {
-        const long long tok = (long long)b * p.Sq + min(q0 + first + e * AT_ONCE, p.Sq - 1);
-        in.x[e] = *reinterpret_cast<const uint4*>(p.dO + tok * p.do_stride + h * HD + sub * 8);
-        in.y[e] = *reinterpret_cast<const uint4*>(p.O + (tok * p.Hq + h) * HD + sub * 8);
-      }
-      const int i = min(q0 + r, p.Sq - 1);
-      in.lse = p.lse[((long long)b * p.Hq + h) * p.Sq + i];
-      in.lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + i] : 0;
-      in.hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + i] : (p.causal ? i + 1 + shift : p.Sk);
-    };
     uint32_t g = 0;
     int u = 0;
     Work w;
     bool ok = queue_next(queue, 0, w, abort_flag, p.status);
-    if (ok) load_unit(w);
     for (int c = 0; ok && w.more;) {
       const int b = w.sample, h = w.head, n = w.v1, full_lo = w.v2, full_hi = w.v3;
       const int i = w.place * BQ + r;   // global query row
-      float delta;
+      float delta, lse;
+      int lo, hi;
       {
+        uint4 x[STEPS], y[STEPS];
+#pragma unroll
+        for (int e = 0; e < STEPS; ++e) {
+          const long long tok = (long long)b * p.Sq + min(w.place * BQ + first + e * AT_ONCE, p.Sq - 1);
+          x[e] = *reinterpret_cast<const uint4*>(p.dO + tok * p.do_stride + h * HD + sub * 8);
+          y[e] = *reinterpret_cast<const uint4*>(p.O + (tok * p.Hq + h) * HD + sub * 8);
+        }
+        const int at = min(i, p.Sq - 1);
+        lse = p.lse[((long long)b * p.Hq + h) * p.Sq + at];
+        lo = p.row_lo ? p.row_lo[(long long)b * p.Sq + at] : 0;
+        hi = p.row_hi ? p.row_hi[(long long)b * p.Sq + at] : (p.causal ? at + 1 + shift : p.Sk);
         float* dots = reinterpret_cast<float*>(smem + L::DOT_OFF) + (c & 1) * BQ;
 #pragma unroll
         for (int e = 0; e < STEPS; ++e) {
-          const uint32_t xs[4] = {in.x[e].x, in.x[e].y, in.x[e].z, in.x[e].w};
-          const uint32_t ys[4] = {in.y[e].x, in.y[e].y, in.y[e].z, in.y[e].w};
+          const uint32_t xs[4] = {x[e].x, x[e].y, x[e].z, x[e].w}, ys[4] = {y[e].x, y[e].y, y[e].z, y[e].w};
           float acc = 0.f;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -319,10 +307,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         delta = dots[r];
         if (half == 0 && i < p.Sq) p.delta[((long long)b * p.Hq + h) * p.Sq + i] = delta;
       }
-      const bool valid = i < p.Sq && in.lse != -INFINITY;
+      const bool valid = i < p.Sq && lse != -INFINITY;
       if (!valid) delta = 0.f;
-      const float lse2 = valid ? in.lse * 1.4426950408889634f : 0.f;
-      const int lo = valid ? max(in.lo, 0) : 0, hi = valid ? min(in.hi, p.Sk) : 0;
+      const float lse2 = valid ? lse * 1.4426950408889634f : 0.f;
+      lo = valid ? max(lo, 0) : 0;
+      hi = valid ? min(hi, p.Sk) : 0;
       const uint64_t sc2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
       const uint64_t nd2 = f2_pack(-delta, -delta), scl2 = f2_pack(p.scale, p.scale);
       for (int j = 0; j < n; ++j, ++g) {
@@ -385,7 +374,6 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       Work nw;
       ok = queue_next(queue, ++c, nw, abort_flag, p.status);
       if (!ok) break;
-      load_unit(nw);
       if (n > 0) {
         ok = mbar_wait_warp(dq_full, u & 1, abort_flag, p.status);
         if (!ok) break;
