@@ -811,3 +811,47 @@ def test_adding_to_fp32_costs_reading_it():
         torch.cuda.synchronize()
         us[add] = min(us.get(add, 1e9), 1e3 * first.elapsed_time(last))
     assert us[True] < 2.6 * us[False], us
+
+
+@pytest.mark.parametrize("rows", [300, 2048])
+def test_early_starts_forward_backward_and_across_streams(rows):
+    """A layer and its gradients, with its products that two pairs share, and a product of another stream behind an event: the
+    same bits with a synchronisation after every operator of both passes and without."""
+    from atorch_b200 import ops
+    from atorch_b200.ops.flash import flash_attention_qkv
+
+    torch.manual_seed(1)
+    H, F, side = 1024, 6144, torch.cuda.Stream()
+    w = [(torch.randn(n, k, device="cuda") / k ** 0.5).bfloat16().requires_grad_() for n, k in ((3 * H, H), (H, H), (2 * F, H), (H, F))]
+    g = torch.ones(H, device="cuda").bfloat16().requires_grad_()
+    x0, dy = torch.randn(1, rows, H, device="cuda").bfloat16().requires_grad_(), torch.randn(1, rows, H, device="cuda").bfloat16()
+    cos, sin = ops.rope_tables(rows, 128, 10000.0, "cuda")
+
+    def run(sync):
+        def mark(t):
+            if sync:
+                torch.cuda.synchronize()
+                t.register_hook(lambda d: torch.cuda.synchronize())
+            return t
+
+        qkv = mark(ops.rope(mark(ops.linear(mark(ops.rms_norm(x0, g, 1e-5)), w[0])), cos, sin, 16, 128))
+        a = mark(flash_attention_qkv(qkv.view(1, rows, 24, 128), 8))
+        x = mark(ops.linear(a.view(1, rows, H), w[1], residual=x0))
+        act = mark(ops.swiglu(mark(ops.linear(mark(ops.rms_norm(x, g, 1e-5)), w[2]))))
+        y = mark(ops.linear(act, w[3], residual=x))
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            z = ops.gemm(y.detach().view(rows, H), y.detach().view(rows, H))
+        grads = torch.autograd.grad(y, (x0, g, *w), dy)
+        torch.cuda.current_stream().wait_stream(side)
+        with torch.no_grad():
+            z = ops.gemm(z[:256], z[:256])
+        torch.cuda.synchronize()
+        return (y.detach(), z, *grads)
+
+    want = run(True)
+    assert all(bool(torch.isfinite(t).all()) for t in want)
+    for _ in range(8):
+        for a, b in zip(run(False), want):
+            assert torch.equal(a, b)
+    _lib.check_status(x0.device)
