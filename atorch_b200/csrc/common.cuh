@@ -361,14 +361,14 @@ ATB_DEVICE void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0
 // grid_go(): the next launch of the stream, if it is made by launch_after(), may take the SMs that become free from here on.
 // grid_wait(): the kernels before have completed and their writes are visible. A kernel launched by launch_after() waits in
 // every thread that touches device memory, before it does, on every path: barriers, tensor memory and tensor maps are set up
-// before it, under the last blocks of the kernel in front. A kernel that allocates tensor memory says grid_go() in the warp that
-// allocates, after it: then no CTA of a successor runs before every CTA of this grid has its tensor memory, and none can
-// hold, while it waits for this kernel, what this kernel still needs. Such a kernel takes its inputs by plain pointers: const __restrict__
-// selects the read-only path, which promises that nobody writes while the kernel runs. Kernels that are not worth it
-// only say grid_go(). The gap between two kernels was 1.9 us. Matrix products and attention first: loss of 8 layers of a 1.3B model
-// on 777 tokens (68 launches) 1479 -> 1444 us, forward and backward of one layer on 3000 tokens (23) 1073 -> 1049, a training step
-// of 8 layers of it (286) 18687 -> 18431; then norms, SwiGLU and rotary: the loss 1485 -> 1466, a step of a small model (83 launches, where
-// the launch itself is also cheaper on the host) 2901 -> 2816, the large ones even.
+// before it, under the last blocks of the kernel in front. A kernel that allocates tensor memory says grid_go() in the warp
+// that allocates, after it: then no CTA of a successor runs before every CTA of this grid has its tensor memory, and none can
+// hold, while it waits for this kernel, what this kernel still needs. Such a kernel takes its inputs by plain pointers: const
+// __restrict__ selects the read-only path, which promises that nobody writes while the kernel runs. Kernels that are not worth
+// it only say grid_go(). The gap between two kernels was 1.9 us. Before / after matrix products and attention had it: loss of 8
+// layers of a 1.3B model on 777 tokens (68 launches) 1479 / 1444 us, forward and backward of one layer on 3000 tokens (23) 1073
+// / 1049, a training step of 8 layers (286) 18687 / 18431. Norms, SwiGLU and rotary then: the loss 1485 / 1466, a step of a
+// small model (83 launches) 2901 / 2816, the large ones even.
 ATB_DEVICE void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 ATB_DEVICE void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -1,13 +1,14 @@
-// Gradient of an embedding table: row v (+)= the sum of the gradients of the tokens whose id is v, in fp32, rounded once. A row of up
-// to MANY tokens is summed in their order, a longer one as eight interleaved sums, from PART tokens on eight per PART tokens, which
-// are then added in a fixed order. Two kernels, no atomics on values and no order that depends on timing:
+// Gradient of an embedding table: row v (+)= the sum of the gradients of the tokens whose id is v, in fp32, rounded once. A row
+// of up to MANY tokens is summed in their order, a longer one as eight interleaved sums, from PART tokens on eight per PART
+// tokens, which are then added in a fixed order. Two kernels, no atomics on values and no order that depends on timing:
 //   embed_sort    a stable counting sort of the ids. A CTA owns a range of rows and reads all ids twice: the first time it counts
 //                 its own per row and warp and the ids below its range (which is where its part of the result begins), the
 //                 second time it writes the tokens. The ids are small (64 KB for 8192) and come out of L2; in exchange no CTA
 //                 waits for another.
 //   embed_rows    a warp per row and 512 columns; a row with many tokens by the eight warps of its block, a long one by several
 //                 blocks. With one block for every row and 32 rows a block, 65536 tokens took, nine in ten of them on one row
-//                 (padding; 32000 x 2048), 2670 us, now 163; on a table of 256 x 1024 482, now 67; spread over 32000 x 2048 155, now 152.
+//                 (padding; 32000 x 2048), 2670 us, now 163; on a table of 256 x 1024 482, now 67; spread over 32000 x
+//                 2048 155, now 152.
 // Bound by memory: the gradients of the tokens are read once, the rows that have any are read and written. The library wrote a
 // gradient of the whole table (zeros, then rows) that was then added to the gradient buffer, three more passes over the
 // table, after a sort in several launches. 4096 tokens on 32000 rows of 2048, random ids, cold: 357 us in 30 launches, now 48.
@@ -21,8 +22,8 @@ constexpr int SORT_WARPS = 16, BATCH = 8;
 constexpr int MAX_RANGE = 1024;          // rows of a CTA: 16 warps x 1024 counters are 64 KB of shared memory
 constexpr int COLS = 512;                // columns of a block; its rows are 32, 8 or 2
 constexpr int FEW_BLOCKS = 2 * 148;      // blocks that there should be (4096 tokens on 1000 x 256: 32 rows a block 34 us, 2 17)
-constexpr int MANY = 64;                 // tokens above which the whole block sums a row (16 to 128 all even; 256 takes half as long again on
-                                         // 256 x 1024 with 65536 tokens)
+// Tokens above which the whole block sums a row: 16 to 128 are all even, 256 takes half as long again on 256 x 1024 with 65536 tokens.
+constexpr int MANY = 64;
 constexpr int PART = 512;                // tokens above which several blocks sum a row, as many of them each
 
 __global__ void __launch_bounds__(SORT_WARPS * 32)
@@ -282,8 +283,8 @@ void launch_rows(const void* dy, const long long* ids, const int* start, const i
 
 }  // namespace
 
-// Words of the scratch, 16-byte aligned: int32 [V + 1 + T], with more than 512 tokens also counters and, from the next multiple of 16
-// bytes on, fp32 sums of the parts of long rows.
+// Words of the scratch, 16-byte aligned: int32 [V + 1 + T], with more than 512 tokens also counters and, from the next multiple
+// of 16 bytes on, fp32 sums of the parts of long rows.
 extern "C" long long atb_embedding_bwd_scratch(int T, int V, int H) {
   const long long parts = T > PART ? (T + PART - 1) / PART : 0, words = (long long)V + 1 + T + 2 * parts * ((H + COLS - 1) / COLS);
   return parts > 0 ? ((words + 3) & ~3ll) + 2 * parts * H : words;

@@ -567,12 +567,12 @@ extern "C" int atb_flash_bwd_dkv(const void* dout, const void* q, const void* k,
                                  float softmax_scale, int fold, int head_dim, const int* key_range, void* stream,
                                  int* status);
 
-// The two-kernel form, the default without dropout and bias: dK and dV per key block (flash_attn_bwd_dkv.cu; `fold`:
-// see there), dQ per query block (flash_attn_bwd_dq.cu, which runs first and writes delta). No atomics, results do not depend on scheduling. dq/dk/dv are
-// token-major rows of pitch dq_stride / dkv_stride elements (so they may be slices of one fused
+// The two-kernel form, the default without dropout and bias: dK and dV per key block (flash_attn_bwd_dkv.cu; `fold`: see
+// there), dQ per query block (flash_attn_bwd_dq.cu, which runs first and writes delta). No atomics, results do not depend on
+// scheduling. dq/dk/dv are token-major rows of pitch dq_stride / dkv_stride elements (so they may be slices of one fused
 // [tokens, (Hq + 2 Hkv) * head_dim] gradient buffer). `delta` is scratch, 8-byte aligned: [B, Hq, Sq] floats and, with
-// intervals, from the next multiple of 8 bytes on two ints per block of 128 query rows and sample (the keys its rows see:
-// the second kernel finds the query blocks of a key block there, where it went through the intervals of all rows before).
+// intervals, from the next multiple of 8 bytes on two ints per block of 128 query rows and sample (the keys its rows see: the
+// second kernel finds the query blocks of a key block there).
 extern "C" int atb_flash_bwd_split(const void* dout, const void* q, const void* k, const void* v, const void* out,
                                    const float* lse, float* delta, void* dq, void* dk, void* dv, const int* row_lo,
                                    const int* row_hi, int B, int Sq, int Sk, int Hq, int Hkv, long long q_stride,

@@ -13,14 +13,15 @@
 //   S(i+1) is issued as soon as the warps hold S(i) in registers and runs under the exponentials of block i,
 //   dV(i) starts when P(i) is stored and runs under dS(i),
 //   dK(i), dP(i+1) run under the exponentials of block i+1.
-// S=8192, 32 heads of 128, causal: 1188 -> 822 us (861 with a CTA per block; 2800 clocks a block, 1024 of them exponentials); before, S(i+1) was issued after P and dS were
-// both stored, or (for long causal inputs) P^T and dS^T went through tensor memory instead, whose element-wise warps need
-// the row statistics per column.
+// S=8192, 32 heads of 128, causal: 822 us (861 with a CTA per block; 1188 when S(i+1) was issued after P and dS were both
+// stored); 2800 clocks a block, 1024 of them exponentials. For long causal inputs P^T and dS^T once went through tensor memory
+// instead, whose element-wise warps need the row statistics per column.
 // For grouped queries the gradients of the group are summed in the accumulator in fp32; with one CTA per query head the
 // bf16 results have to be added by a separate pass over them.
 //
-// Warp 0 = TMA producer, warp 1 = MMA issuer / TMEM owner, warp 10 = scheduler (block_queue.cuh), warps 2..9 =
-// element-wise work: thread (row r, half h) owns columns [64h, 64h+64) of row r. Masks are per-row key intervals [lo, hi) as in the forward kernel.
+// Warp 0 = TMA producer, warp 1 = MMA issuer / TMEM owner, warp 10 = scheduler (block_queue.cuh), warps 2..9 = element-wise
+// work: thread (row r, half h) owns columns [64h, 64h+64) of row r. Masks are per-row key intervals [lo, hi) as in the forward
+// kernel.
 #include "block_queue.cuh"
 
 namespace {

@@ -10,11 +10,11 @@
 // core already forms S and dP of block j+1 (S is free as soon as the warps hold it in registers, dP has a
 // second buffer); dQ of block j follows when dS(j) is in place.
 //
-// Warp 0 = TMA producer (Q, dO once; K in three stages because a K tile serves S and, later, dQ; V in two),
-// warp 1 = MMA issuer / TMEM owner, warp 2 = scheduler (block_queue.cuh), warps 4..11 = element-wise work: thread (row r, half h) owns columns
-// [64h, 64h+64) of row r. The two threads of a row sit in different warps and the bf16 dS of one overwrites
-// fp32 dP columns of the other, so the two warps of a lane quarter meet at a barrier between loading
-// and storing (an mbarrier with a bounded wait). Masks are per-row key intervals [lo, hi) as in the forward kernel.
+// Warp 0 = TMA producer (Q, dO once; K in three stages because a K tile serves S and, later, dQ; V in two), warp 1 = MMA issuer
+// / TMEM owner, warp 2 = scheduler (block_queue.cuh), warps 4..11 = element-wise work: thread (row r, half h) owns columns
+// [64h, 64h+64) of row r. The two threads of a row sit in different warps and the bf16 dS of one overwrites fp32 dP columns of
+// the other, so the two warps of a lane quarter meet at a barrier between loading and storing (an mbarrier with a bounded
+// wait). Masks are per-row key intervals [lo, hi) as in the forward kernel.
 #include "block_queue.cuh"
 
 namespace {

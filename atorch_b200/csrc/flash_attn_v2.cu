@@ -19,10 +19,11 @@
 // While tile A's warps exponentiate, the tensor core works for tile B and vice versa:
 // issue order  PV_A(j), S_A(j+1), PV_B(j), S_B(j+1).
 //
-// 8192 keys, 32 heads of 128: full 775 us (1420 TFLOP/s), causal 419 us (450 with a CTA per block; before: 945 and 578-625 us; 497
-// before BlockOrder); 16 x 512, 16 heads of 64, all keys 50 -> 40 us by the running CTAs. A step of both tiles takes 3100 clocks, 1900 of them softmax and 1200 tensor work of the same tile. Tried: K/V tiles of 64 keys with
-// two score buffers per tile, which takes the tensor work out of that chain - 887 us, because a 128 x 64 x 16 score
-// product takes 48 clocks for its shared-memory operands where it should take 32; P in one piece - 859 us.
+// 8192 keys, 32 heads of 128: full 775 us (1420 TFLOP/s), causal 419 us (450 with a CTA per block); 16 x 512, 16 heads of 64,
+// all keys 45 us (55 with a CTA per block). A step of both tiles takes 3100 clocks, 1900 of them softmax and 1200 tensor work
+// of the same tile. Tried: K/V tiles of 64 keys with two score buffers per tile, which takes the tensor work out of that chain
+// - 887 us, because a 128 x 64 x 16 score product takes 48 clocks for its shared-memory operands where it should take 32; P in
+// one piece - 859 us.
 //
 // Masks: per-row key interval [lo, hi) exactly as in flash_attn.cu; each query tile walks only the K/V
 // tiles up to the last one that any of its rows can see.

@@ -52,9 +52,9 @@ struct Cfg {
   static constexpr int STAGES = SPLIT == 2 ? 5 : BN == 256 ? 6 : 8;
   static constexpr int B_BYTES = BNH * BK * 2;
   static constexpr int X_OFF = STAGES * (A_BYTES + B_BYTES);         // partial sums from the other pair, fp32
-  // output boxes on their way out (see the epilogue): 4 KB per epilogue warp, [32 rows][128 bytes] with 128-byte swizzle, in the place
-  // of the operands, all of which have been multiplied by then. Space of their own took half of the L1 cache, in which an
-  // epilogue that adds to fp32 values keeps their lines: 4096 x 4096 x 256 67.6 -> 84.2 us.
+  // output boxes on their way out (see the epilogue): 4 KB per epilogue warp, [32 rows][128 bytes] with 128-byte swizzle, in
+  // the place of the operands, all of which have been multiplied by then. Space of their own took half of the L1 cache, in
+  // which an epilogue that adds to fp32 values keeps their lines: 4096 x 4096 x 256 68.0 us, 84.2 with it.
   static constexpr int OUT_OFF = 0;
   static constexpr int BAR_OFF = X_OFF + (SPLIT == 2 ? BM * (BN / 2) * 4 : 0);
   static constexpr int TQ = 4;                     // tile-id ring of the dynamic scheduler
@@ -359,8 +359,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       mbar_init(&tempty[1], 2 * EPI_WARPS);
       for (int i = 0; i < TQ; ++i) {
         mbar_init(&tq_full[i], 1);
-        mbar_init(&tq_empty[i], SPLIT * (2 + 2 * EPI_WARPS) + SPLIT - 1);   // every CTA's epilogue warps, every pair's MMA
-                                                                             // warp, every producer but the one that draws
+        // read by every CTA's epilogue warps, every pair's MMA warp and every producer but the one that draws
+        mbar_init(&tq_empty[i], SPLIT * (2 + 2 * EPI_WARPS) + SPLIT - 1);
       }
       mbar_init(xfull, EPI_WARPS);
       mbar_init(xfree, EPI_WARPS);
@@ -686,7 +686,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       store_row_bf16(crow + hd2, o2, N - col0 - hd2, wide);
     };
     // A body for each kind of output, chosen outside of the loop over the columns: with one for all, the registers for what is
-    // added and the choices cost those that need neither 6 % (32000 x 2048 x 512 75.8 us, with one body 81.9; with a bias 101 and 120).
+    // added and the choices cost those that need neither 6 % (32000 x 2048 x 512 75.8 us, with one body 81.9; with a bias 101
+    // and 120).
     constexpr int PLAIN = 0, FP32 = 1, ADD = 2, ANY = 3;   // bf16; fp32, alone or added to; bf16 and one thing added; the rest
     constexpr std::integral_constant<int, ANY> any{};
     const int output = ep.bias != nullptr || ep.rs_rows > 0 || (ep.residual != nullptr && (ep.accumulate || ep.out_fp32)) ? ANY
@@ -829,8 +830,9 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       const bool in = row < m_end;
       const int row0 = m0 + (int)rank * BM + q * 32;      // first of this warp's rows
       // The last tile's epilogue is exposed in full: boxes of 32 rows x 64 columns go through shared memory (swizzled, no bank
-      // conflicts) and the TMA unit. 512 x 512 x 512: 11.6 -> 10.3 us, 2048 x 2048 x 4096 weight gradient 30.8 -> 28.8. Earlier tiles keep to direct stores: the operands of the
-      // products that run beside them take the whole bandwidth of shared memory.
+      // conflicts) and the TMA unit. 512 x 512 x 512: 11.6 -> 10.3 us, 2048 x 2048 x 4096 weight gradient 30.8 -> 28.8. Earlier
+      // tiles keep to direct stores: the operands of the products that run beside them take the whole bandwidth of shared
+      // memory.
       if (SPLIT == 1 && ep.boxed != 0 && next < 0 && row0 + 32 <= m_end && n0 + (half + 1) * (BN / 2) <= N) {
         uint8_t* box = smem + C::OUT_OFF + (warp - 2) * 4096;
 #pragma unroll 1
@@ -1077,8 +1079,9 @@ int split_clusters() {
 // 1.5 more. Cold L2, one / two pairs (us), tiles and k-blocks: 8 x 172 59.4 / 43.0; 16 x 86 36.9 / 28.7; 32 x 86 36.9 / 30.7;
 // 96 x 86 71.7 / 67.6; 96 x 172 124.9 / 110.6; about even: 80 x 64 55.3 / 55.3, 96 x 64 57.3 / 55.3; not: 80 x 58 51.2 / 53.2,
 // 48 x 86 38.9 / 49.2, 104 x 86 73.7 / 81.9, 222 x 86 104.4 / 133.1.
-// Beside a kernel that takes 24 SMs for itself fewer clusters of four find room than pairs: 16 x 86 36.9 / 32.8, 24 x 86 36.9 / 34.8, but
-// 32 x 86 38.9 / 57.3, 96 x 86 73.7 / 92.2 (115.6 with a fixed share of tiles); one that takes 8, 96 x 86 73.7 / 67.6.
+// Beside a kernel that takes 24 SMs for itself fewer clusters of four find room than pairs: 16 x 86 36.9 / 32.8, 24 x 86 36.9 /
+// 34.8, but 32 x 86 38.9 / 57.3, 96 x 86 73.7 / 92.2 (115.6 with a fixed share of tiles); one that takes 8, 96 x 86 73.7 /
+// 67.6.
 bool split_pays(int tiles, int kbs, int wish) {
   if (kbs < 2 || wish < 0) return false;
   const int pairs = sm_count() / 2;

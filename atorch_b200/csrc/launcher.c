@@ -1,5 +1,5 @@
 /* Launchers of libatb.so as Python callables with declared argument types ("ppii f...": p pointer, i int, l long long,
- * f float). A ctypes call with twenty arguments costs 2.3 us before the launch itself (3 us), this one 0.3.
+ * f float). A ctypes call with twenty arguments costs 2.3 us before the launch itself (3 us), this one 0.25.
  *
  * All arguments of integer class go to the callee in their order, in registers and then in 8-byte stack slots, the floats
  * in vector registers in theirs, wherever they stand between the integers (System V x86-64 and Linux AArch64): so one

@@ -46,7 +46,9 @@ BWD_SPLIT = os.environ.get("ATB_FLASH_BWD_SPLIT", "1") == "1"
 # leave this many CTAs; what is left of a group is summed by a pass over the bf16 results. A CTA per SM will do while a
 # head is short (10 x 512, 16 heads on 4, causal, backward in all: 75 us with 160 CTAs, 83 with 320, 89 with 640). From 12 query
 # blocks on the last CTAs weigh more, and it takes FOLD_LONG_CTAS (2 x 1536, 32 on 4: 167 us with 192, 156 with 384; 2560, 32 on 8:
-# 222 with 160, 188 with 320, 192 with 640; 3584: 338 with 224, 327 with 448, 333 with 896; 4096: 400 with 256, 403 with 512).
+# 222 with 160, 188 with 320, 192 with 640; 3584: 338 with 224, 327 with 448, 333 with 896; 4096: 400 with 256, 403 with 512), with
+# every key visible too (2 x 1536, 32 on 8: 306 with 192, 281 with 384; 1664, 64 on 16: 335 with 208, 304 with 416; 3 x 1792, 32 on
+# 4: 632 with 168, 550 with 336; 4 x 1920, 12 on 3: 343 with 180, 310 with 360; head dim 64, 2 x 1536, 32 on 8: 263 and 237).
 # Long heads that all see every key fold whole groups or none (4000, 32 on 4: 758 us unfolded, 807 by 4, 996 by 2).
 FOLD_MIN_CTAS = 148
 FOLD_LONG_CTAS = 240
