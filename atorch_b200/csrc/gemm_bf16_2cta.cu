@@ -1020,17 +1020,18 @@ int g_dynamic = -1;      // -1: read ATB_GEMM_DYNAMIC on first use (default on)
 std::mutex g_sched_mu;
 
 int* sched_counters(cudaStream_t stream) {
+  // A graph may be replayed on any stream, beside launches of the one that it was captured on.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
   std::lock_guard<std::mutex> lock(g_sched_mu);
   int dev = 0;
   cudaGetDevice(&dev);
   for (int i = 0; i < g_sched_n; ++i)
     if (g_sched_ws[i].dev == dev && g_sched_ws[i].stream == stream) return g_sched_ws[i].counters;
   if (g_sched_n >= SCHED_MAX_STREAMS) return nullptr;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return nullptr;
-  }
   void* p = nullptr;
   if (cudaMalloc(&p, 256) != cudaSuccess) {
     cudaGetLastError();

@@ -855,3 +855,39 @@ def test_early_starts_forward_backward_and_across_streams(rows):
         for a, b in zip(run(False), want):
             assert torch.equal(a, b)
     _lib.check_status(x0.device)
+
+
+@pytest.mark.parametrize("tile_n", [256, 512])
+def test_graphs_of_one_stream_replayed_beside_each_other(tile_n):
+    """Two graphs captured on a stream that has run the same products before, replayed on two other streams while that one
+    runs them too: each result is whole."""
+    side, streams = torch.cuda.Stream(), [torch.cuda.Stream() for _ in range(2)]
+    x, w = [_mk(4096, 512) for _ in range(3)], _mk(4096, 512)
+    outs = [torch.empty(4096, 4096, device="cuda", dtype=torch.bfloat16) for _ in x]
+
+    def run(i):
+        for _ in range(8):
+            gemm(x[i], w, out=outs[i], tile_n=tile_n)
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        run(2)
+    torch.cuda.synchronize()
+    graphs = [torch.cuda.CUDAGraph() for _ in streams]
+    for i, g in enumerate(graphs):
+        with torch.cuda.graph(g, stream=side):
+            run(i)
+    want = [gemm(t, w, tile_n=tile_n) for t in x]
+    for _ in range(20):
+        for o in outs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(side):
+            run(2)
+        torch.cuda.synchronize()
+        for o, t in zip(outs, want):
+            assert torch.equal(o, t)
+    _lib.check_status(w.device)
