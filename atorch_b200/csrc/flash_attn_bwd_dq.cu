@@ -262,7 +262,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // delta = dO . O of the block's rows, 16 rows per warp and HD / 8 lanes per row: a separate pass over both tensors took
     // 26 us at S=4096, 32 heads of 128. A unit's values are loaded when it begins, under its first products: holding them from the
     // end of the unit before took registers that the loop over the tiles needs (16 heads on 8192 keys, all visible, head dim 64
-    // 565 us, now 512; 128 604, now 562; 16 x 512, 16 heads of 64, 59 either way).
+    // 565 us, now 512; 128 604, now 562). They are asked into L2 there (backward of 4096 in 30 documents, 32 heads of 128 on 8,
+    // 148 us without, 144 with).
     constexpr int LANES = HD / 8, AT_ONCE = 32 / LANES, STEPS = 16 / AT_ONCE;
     const int first = (warp - 4) * 16 + lane / LANES, sub = lane % LANES;
     uint32_t g = 0;
@@ -374,6 +375,16 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       Work nw;
       ok = queue_next(queue, ++c, nw, abort_flag, p.status);
       if (!ok) break;
+      if (nw.more) {      // on their way into L2 while this unit's results leave
+#pragma unroll
+        for (int e = 0; e < STEPS; ++e) {
+          const long long tok = (long long)nw.sample * p.Sq + min(nw.place * BQ + first + e * AT_ONCE, p.Sq - 1);
+          if ((sub & 3) == 0) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.dO + tok * p.do_stride + nw.head * HD + sub * 8));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.O + (tok * p.Hq + nw.head) * HD + sub * 8));
+          }
+        }
+      }
       if (n > 0) {
         ok = mbar_wait_warp(dq_full, u & 1, abort_flag, p.status);
         if (!ok) break;
